@@ -15,12 +15,13 @@ CHECKING = os.environ.get("FSB_BOUNDS_CHECK", "") not in ("", "0")
 LIB_PATH = os.path.join(_HERE, "csrc", "libfsb_check.so" if CHECKING else "libfsb.so")
 
 FSB_F32, FSB_F64 = 0, 1
-FSB_F16, FSB_BF16, FSB_C64, FSB_C128 = 2, 3, 4, 5     # fsb_spmv_csr_wide only
+FSB_F16, FSB_BF16, FSB_C64, FSB_C128 = 2, 3, 4, 5     # the *_wide and *_stored entry points
 FSB_I32, FSB_I64 = 0, 1
 FSB_SPMV_AUTO, FSB_SPMV_VECTOR, FSB_SPMV_STREAM = 0, 1, 2
 FSB_SPMV_PANEL = 3  # host-side tag only: the panel kernel has its own entry point
 FSB_SPMM_AUTO, FSB_SPMM_PLAIN, FSB_SPMM_BULK = 0, 1, 2
 FSB_SPMM_ACCUMULATE = 16  # or-ed into the selector: C += A B
+FSB_SPMM_LONG_ROWS = 32   # or-ed into the selector: long rows are shared by a block
 FSB_CUDA_ERROR_BASE = 1000
 
 _ERRORS = {
@@ -72,6 +73,10 @@ SIGNATURES = {
     "fsb_spmm_csr": (
         _i32,
         [_i32, _i32, _i32, _vp, _vp, _vp, _vp, _i64, _vp, _i64, _i64, _i64, _i64, _i64, _i32, _vp, _vp, _sz, _vp, _vp],
+    ),
+    "fsb_spmm_stored_scratch_bytes": (_sz, [_i32, _i64, _i64]),
+    "fsb_spmm_csr_stored": (
+        _i32, [_i32, _i32, _vp, _vp, _vp, _vp, _i64, _vp, _i64, _i64, _i64, _i64, _i64, _i32, _vp, _sz, _vp],
     ),
     "fsb_spmv_csr_wide": (_i32, [_i32, _i32, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _vp]),
     "fsb_spmm_csr_wide": (_i32, [_i32, _i32, _vp, _vp, _vp, _vp, _i64, _vp, _i64, _i64, _i64, _i64, _i64, _vp]),

@@ -11,12 +11,16 @@
 // Rows ending in the tile are written to C with streaming stores; a row continuing into the next tile
 // leaves its partial row in carry[t, :], a row that began in an earlier tile leaves it in head[t, :],
 // and a second kernel adds them up in a fixed order (deterministic, no atomics).
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
+
 #include "fsb_common.cuh"
 
 namespace fsb {
 
 constexpr int kMmThreads = 256;
 constexpr int kMmTile = 1024;  // nnz per tile
+constexpr int kMmMinPiece = 32; // shortest piece of a long segment
 constexpr int kWaitSpins = 1 << 22;
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -56,22 +60,123 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t phase)
   return false;
 }
 
-// ACCUM: add to what C holds instead of overwriting it (rows without entries are then left alone) -- the later
-// passes of a product that the host code splits into column panels of A.
-template <typename V, typename I, typename P, int VW, bool BULK, bool ACCUM>
-__global__ void __launch_bounds__(kMmThreads)
-spmm_tile_kernel(const V* __restrict__ data, const I* __restrict__ idx, const P* __restrict__ ptr,
-                 const V* __restrict__ B, int64_t ldb, V* __restrict__ C, int64_t ldc,
-                 const int32_t* __restrict__ tile_row, V* __restrict__ carry, V* __restrict__ head,
-                 int64_t nnz, int n_dense, int LR, int32_t* __restrict__ status) {
+// ---- stored value types: what is accumulated, and how a value enters a sum ---------------------------------------
+// half precisions are accumulated in float32 and rounded once when a row of C is stored
+template <typename S>
+struct MmOps {
+  typedef S Acc;
+  static __device__ __forceinline__ void fma(Acc& acc, S a, S b) { acc += a * b; }
+  static __device__ __forceinline__ Acc add(Acc a, Acc b) { return a + b; }
+  static __device__ __forceinline__ Acc widen(S v) { return v; }
+  static __device__ __forceinline__ S narrow(Acc v) { return v; }
+  static __device__ __forceinline__ Acc zero() { return (Acc)0; }
+};
+template <>
+struct MmOps<__half> {
+  typedef float Acc;
+  static __device__ __forceinline__ void fma(Acc& acc, __half a, __half b) {
+    acc = fmaf(__half2float(a), __half2float(b), acc);
+  }
+  static __device__ __forceinline__ Acc add(Acc a, Acc b) { return a + b; }
+  static __device__ __forceinline__ Acc widen(__half v) { return __half2float(v); }
+  static __device__ __forceinline__ __half narrow(Acc v) { return __float2half_rn(v); }
+  static __device__ __forceinline__ Acc zero() { return 0.f; }
+};
+template <>
+struct MmOps<__nv_bfloat16> {
+  typedef float Acc;
+  static __device__ __forceinline__ void fma(Acc& acc, __nv_bfloat16 a, __nv_bfloat16 b) {
+    acc = fmaf(__bfloat162float(a), __bfloat162float(b), acc);
+  }
+  static __device__ __forceinline__ Acc add(Acc a, Acc b) { return a + b; }
+  static __device__ __forceinline__ Acc widen(__nv_bfloat16 v) { return __bfloat162float(v); }
+  static __device__ __forceinline__ __nv_bfloat16 narrow(Acc v) { return __float2bfloat16_rn(v); }
+  static __device__ __forceinline__ Acc zero() { return 0.f; }
+};
+template <typename C2>
+struct MmComplex {
+  typedef C2 Acc;
+  static __device__ __forceinline__ void fma(Acc& acc, C2 a, C2 b) {
+    // written out: which products the compiler would fuse differs between the kernels
+    acc.x = ::fma(-a.y, b.y, ::fma(a.x, b.x, acc.x));
+    acc.y = ::fma(a.y, b.x, ::fma(a.x, b.y, acc.y));
+  }
+  static __device__ __forceinline__ Acc add(Acc a, Acc b) {
+    a.x += b.x;
+    a.y += b.y;
+    return a;
+  }
+  static __device__ __forceinline__ Acc widen(C2 v) { return v; }
+  static __device__ __forceinline__ C2 narrow(Acc v) { return v; }
+  static __device__ __forceinline__ Acc zero() {
+    Acc z;
+    z.x = 0;
+    z.y = 0;
+    return z;
+  }
+};
+template <> struct MmOps<float2> : MmComplex<float2> {};
+template <> struct MmOps<double2> : MmComplex<double2> {};
+
+template <int BYTES> struct RawVec;
+template <> struct RawVec<2> { typedef unsigned short type; };
+template <> struct RawVec<4> { typedef unsigned int type; };
+template <> struct RawVec<8> { typedef uint2 type; };
+template <> struct RawVec<16> { typedef uint4 type; };
+
+// VW stored values moved as one access of VW * sizeof(S) bytes
+template <typename S, int VW>
+struct Pack {
+  typedef typename RawVec<VW * (int)sizeof(S)>::type Raw;
+  Raw raw;
+  __device__ __forceinline__ void gather(const S* p) { raw = __ldg(reinterpret_cast<const Raw*>(p)); }
+  __device__ __forceinline__ void load_stream(const S* p) { raw = __ldcs(reinterpret_cast<const Raw*>(p)); }
+  __device__ __forceinline__ void store_stream(S* p) const { __stcs(reinterpret_cast<Raw*>(p), raw); }
+  __device__ __forceinline__ S get(int i) const { return reinterpret_cast<const S*>(&raw)[i]; }
+  __device__ __forceinline__ void set(int i, S v) { reinterpret_cast<S*>(&raw)[i] = v; }
+};
+
+// Resident CTAs the register budget is set for: 40 registers hold the four gathers of one access per lane; left to itself
+// the compiler fits 32 and issues them one after the other (54 columns, 28386 rows of 45 entries, float32: 60 us, 44 us).
+__host__ __device__ constexpr int mm_ctas(int nc, size_t size, bool with_long) {
+  return nc == 1 ? (size == 16 ? 4 : with_long ? 5 : 6) : with_long ? 2 : nc == 2 ? 4 : 3;
+}
+
+// A group of LR lanes takes one segment (the part of a row that lies in the tile) at a time, four gathers of B on their
+// way.  LONG: segments of more than 2 * piece entries are left to a second pass: cut into pieces, dealt to all groups of
+// the CTA, their partial rows added in shared memory.  Without it the group that meets a long row of a skewed matrix
+// walks it alone while the others wait (float32, 300000 rows of Zipf lengths, 3.6 M entries, 128 columns: 413 us, with it
+// 300 us; bfloat16, 200003 such rows, 4 M entries, 128 columns, through a kernel of whole rows on widened copies of B and
+// C: 6490 us, here 291 us).  Handing out equal slices of the tile instead, whatever rows they cross,
+// balances as well but pays a row-end test per entry, and an even matrix then loses what a skewed one gains (2^20 rows
+// of 16 entries, 64 columns, float32: 615 us against 531 us).  `piece` depends on the number of columns and the value
+// type only (not on the alignment, which picks VW and LR), so the order of additions does too.
+// n_dense is covered by LR * NC accesses of VW elements per entry; wider products take column tiles (gridDim.y).
+// ACCUM: add to what C holds instead of overwriting it (rows without entries are then left alone) -- the later passes
+// of a product that the host code splits into column panels of A.
+template <typename S, typename I, int VW, int NC, bool LONG, bool ACCUM>
+__global__ void __launch_bounds__(kMmThreads, mm_ctas(NC, sizeof(S), LONG))
+spmm_tile_kernel(const S* __restrict__ data, const I* __restrict__ idx, const void* __restrict__ ptr, int ptr64,
+                 const S* __restrict__ B, int64_t ldb, S* __restrict__ C, int64_t ldc,
+                 const int32_t* __restrict__ tile_row, typename MmOps<S>::Acc* __restrict__ carry,
+                 typename MmOps<S>::Acc* __restrict__ head, int64_t nnz, int n_dense, int LR, int piece,
+                 int use_bulk, int32_t* __restrict__ status) {
+  typedef MmOps<S> Ops;
+  typedef typename Ops::Acc A;
   constexpr int T = kMmTile;
   constexpr int RC = T;
-  __shared__ __align__(128) V s_val[T];
+  constexpr int U = 4;                                    // entries whose gathers are in flight together
+  constexpr int PIECES = T / kMmMinPiece + T / (2 * kMmMinPiece);   // most pieces the long segments of a tile have
+  __shared__ __align__(128) S s_val[T];
   __shared__ __align__(128) I s_idx[T];
   __shared__ int32_t s_off[RC + 1];
+  __shared__ int32_t s_piece_at[LONG ? PIECES : 1];       // a piece: first entry | end << 16
+  __shared__ int32_t s_long[LONG ? T / (2 * kMmMinPiece) : 1];   // a long segment: number | first piece << 16
   __shared__ __align__(8) uint64_t s_bar;
   __shared__ int s_head_partial;
   __shared__ int s_failed;
+  __shared__ int s_n_long, s_n_pieces;
+  extern __shared__ __align__(16) unsigned char s_parts[];
 
   const int tid = threadIdx.x;
   const int64_t t = blockIdx.x;
@@ -81,7 +186,7 @@ spmm_tile_kernel(const V* __restrict__ data, const I* __restrict__ idx, const P*
   const int32_t rb = tile_row[t + 1];
 
   // ---- stage the tile -------------------------------------------------------------------------
-  bool bulk = BULK && cnt == T;
+  const bool bulk = use_bulk && cnt == T;
   if (bulk) {
     if (tid == 0) {
       s_failed = 0;
@@ -90,8 +195,8 @@ spmm_tile_kernel(const V* __restrict__ data, const I* __restrict__ idx, const P*
     }
     __syncthreads();
     if (tid == 0) {
-      mbar_expect_tx(&s_bar, (uint32_t)(T * (sizeof(V) + sizeof(I))));
-      bulk_g2s(s_val, data + lo, (uint32_t)(T * sizeof(V)), &s_bar);
+      mbar_expect_tx(&s_bar, (uint32_t)(T * (sizeof(S) + sizeof(I))));
+      bulk_g2s(s_val, data + lo, (uint32_t)(T * sizeof(S)), &s_bar);
       bulk_g2s(s_idx, idx + lo, (uint32_t)(T * sizeof(I)), &s_bar);
     }
   } else {
@@ -101,13 +206,82 @@ spmm_tile_kernel(const V* __restrict__ data, const I* __restrict__ idx, const P*
     }
   }
 
+  // segments: rows ra .. rb-1 end in this tile, segment nrf is the row that continues
   const int nrf = rb - ra;
   const int nseg = nrf + 1;
   const int lane = tid & (LR - 1);
   const int grp = tid / LR;
   const int ngrp = kMmThreads / LR;
-  const int col0 = (blockIdx.y * LR + lane) * VW;
-  const bool col_ok = col0 < n_dense;
+  const int width = LR * NC * VW;                          // columns of this column tile
+  const int col0 = (int)blockIdx.y * width + lane * VW;    // first column of access 0; access i is LR * VW further on
+
+  auto clear = [](A (&acc)[NC][VW]) {
+#pragma unroll
+    for (int i = 0; i < NC; ++i)
+#pragma unroll
+      for (int j = 0; j < VW; ++j) acc[i][j] = Ops::zero();
+  };
+  // acc += sum over the entries p .. e-1 of value * row of B
+  auto walk = [&](int p, int e, A (&acc)[NC][VW]) {
+    for (; p + U <= e; p += U) {
+      Pack<S, VW> b[U][NC];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const S* row = B + (int64_t)s_idx[p + u] * ldb + col0;
+#pragma unroll
+        for (int i = 0; i < NC; ++i)
+          if (i == 0 || col0 + i * LR * VW < n_dense) b[u][i].gather(row + i * LR * VW);
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const S v = s_val[p + u];
+#pragma unroll
+        for (int i = 0; i < NC; ++i)
+#pragma unroll
+          for (int j = 0; j < VW; ++j) Ops::fma(acc[i][j], v, b[u][i].get(j));
+      }
+    }
+    for (; p < e; ++p) {
+      const S* row = B + (int64_t)s_idx[p] * ldb + col0;
+      const S v = s_val[p];
+#pragma unroll
+      for (int i = 0; i < NC; ++i) {
+        if (i == 0 || col0 + i * LR * VW < n_dense) {
+          Pack<S, VW> b;
+          b.gather(row + i * LR * VW);
+#pragma unroll
+          for (int j = 0; j < VW; ++j) Ops::fma(acc[i][j], v, b.get(j));
+        }
+      }
+    }
+  };
+  // the sum of segment g: to C, or to the arrays that the fix-up adds up
+  auto finish = [&](int g, bool has_entries, const A (&acc)[NC][VW]) {
+    const bool to_carry = g == nrf, to_head = g == 0 && s_head_partial;
+#pragma unroll
+    for (int i = 0; i < NC; ++i) {
+      const int col = col0 + i * LR * VW;
+      if (i > 0 && col >= n_dense) break;
+      if (to_carry || to_head) {
+        A* dst = (to_carry ? carry : head) + t * n_dense + col;
+#pragma unroll
+        for (int j = 0; j < VW; ++j) dst[j] = acc[i][j];
+      } else {
+        S* dst = C + ((int64_t)ra + g) * ldc + col;
+        Pack<S, VW> out;
+        if (!ACCUM) {
+#pragma unroll
+          for (int j = 0; j < VW; ++j) out.set(j, Ops::narrow(acc[i][j]));
+          out.store_stream(dst);
+        } else if (has_entries) {     // a row without entries leaves its row of C alone
+          out.load_stream(dst);
+#pragma unroll
+          for (int j = 0; j < VW; ++j) out.set(j, Ops::narrow(Ops::add(acc[i][j], Ops::widen(out.get(j)))));
+          out.store_stream(dst);
+        }
+      }
+    }
+  };
 
   for (int base = 0; base < nseg; base += RC) {
     const int m = (nseg - base) < RC ? (nseg - base) : RC;
@@ -116,11 +290,17 @@ spmm_tile_kernel(const V* __restrict__ data, const I* __restrict__ idx, const P*
       const int g = base + k;
       int32_t o = cnt;
       if (g <= nrf) {
-        const int64_t d = (int64_t)ptr[(int64_t)ra + g] - lo;
+        const int64_t row = (int64_t)ra + g;
+        const int64_t d = (ptr64 ? static_cast<const int64_t*>(ptr)[row]
+                                 : (int64_t) static_cast<const int32_t*>(ptr)[row]) - lo;
         o = d < 0 ? 0 : (d > cnt ? cnt : (int32_t)d);
         if (g == 0) s_head_partial = (d < 0 && nrf > 0) ? 1 : 0;
       }
       s_off[k] = o;
+    }
+    if (LONG && tid == 0) {
+      s_n_long = 0;
+      s_n_pieces = 0;
     }
     if (bulk && base == 0) {
       // every thread polls the barrier itself: completion makes the copied bytes visible to it
@@ -136,62 +316,67 @@ spmm_tile_kernel(const V* __restrict__ data, const I* __restrict__ idx, const P*
 
     for (int k = grp; k < m; k += ngrp) {
       const int s = s_off[k], e = s_off[k + 1];
-      V acc[VW];
-#pragma unroll
-      for (int i = 0; i < VW; ++i) acc[i] = 0;
-      if (col_ok) {
-        int p = s;
-        for (; p + 4 <= e; p += 4) {
-          V a[4];
-          int64_t c[4];
-          V b[4][VW];
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            a[u] = s_val[p + u];
-            c[u] = (int64_t)s_idx[p + u];
+      if (LONG && e - s > 2 * piece) {
+        if (lane == 0) {
+          const int n = (e - s + piece - 1) / piece;
+          const int first = atomicAdd(&s_n_pieces, n);
+          s_long[atomicAdd(&s_n_long, 1)] = k | first << 16;
+          for (int q = 0; q < n; ++q) {
+            const int p = s + q * piece;
+            s_piece_at[first + q] = p | (p + piece < e ? p + piece : e) << 16;
           }
-#pragma unroll
-          for (int u = 0; u < 4; ++u) ld_dense<V, VW>(B + c[u] * ldb + col0, b[u]);
-#pragma unroll
-          for (int u = 0; u < 4; ++u)
-#pragma unroll
-            for (int i = 0; i < VW; ++i) acc[i] += a[u] * b[u][i];
         }
-        for (; p < e; ++p) {
-          const V a = s_val[p];
-          V b[VW];
-          ld_dense<V, VW>(B + (int64_t)s_idx[p] * ldb + col0, b);
+      } else if (col0 < n_dense) {
+        A acc[NC][VW];
+        clear(acc);
+        walk(s, e, acc);
+        finish(base + k, e > s, acc);
+      }
+    }
+    if (!LONG) continue;
+    __syncthreads();
+    const int n_long = s_n_long;
+    if (n_long > 0) {
+      A* parts = reinterpret_cast<A*>(s_parts);
+      const int n_pieces = s_n_pieces;
+      for (int q = grp; q < n_pieces; q += ngrp) {
+        if (col0 < n_dense) {
+          A acc[NC][VW];
+          clear(acc);
+          walk(s_piece_at[q] & 0xFFFF, s_piece_at[q] >> 16, acc);
 #pragma unroll
-          for (int i = 0; i < VW; ++i) acc[i] += a * b[i];
+          for (int i = 0; i < NC; ++i)
+#pragma unroll
+            for (int j = 0; j < VW; ++j) parts[q * width + (i * LR + lane) * VW + j] = acc[i][j];
         }
-        const int g = base + k;
-        if (g == nrf) {
+      }
+      __syncthreads();
+      for (int q = grp; q < n_long; q += ngrp) {
+        const int k = s_long[q] & 0xFFFF, first = s_long[q] >> 16;
+        const int n = (s_off[k + 1] - s_off[k] + piece - 1) / piece;
+        if (col0 < n_dense) {
+          A acc[NC][VW];
+          clear(acc);
+          for (int p = first; p < first + n; ++p)
 #pragma unroll
-          for (int i = 0; i < VW; ++i) carry[t * n_dense + col0 + i] = acc[i];
-        } else if (g == 0 && s_head_partial) {
+            for (int i = 0; i < NC; ++i)
 #pragma unroll
-          for (int i = 0; i < VW; ++i) head[t * n_dense + col0 + i] = acc[i];
-        } else if (!ACCUM) {
-          st_dense_stream<V, VW>(C + ((int64_t)ra + g) * ldc + col0, acc);
-        } else if (e > s) {
-          V* dst = C + ((int64_t)ra + g) * ldc + col0;
-          V old[VW];
-          ld_dense_stream<V, VW>(dst, old);
-#pragma unroll
-          for (int i = 0; i < VW; ++i) acc[i] += old[i];
-          st_dense_stream<V, VW>(dst, acc);
+              for (int j = 0; j < VW; ++j)
+                acc[i][j] = Ops::add(acc[i][j], parts[p * width + (i * LR + lane) * VW + j]);
+          finish(base + k, true, acc);
         }
       }
     }
   }
 }
 
-// one thread per (tile t >= 1, column): finish the row that started before tile t and ends in it
-template <typename V, typename P, bool ACCUM>
+// one thread per (tile t >= 1, column): finish the row that started before tile t and ends in it.  R: real type of the
+// partial sums, D: real type of C (complex columns are taken as pairs of real ones)
+template <typename R, typename D, typename P>
 __global__ void __launch_bounds__(kMmThreads)
 spmm_fixup_kernel(const P* __restrict__ ptr, const int32_t* __restrict__ tile_row,
-                  const V* __restrict__ carry, const V* __restrict__ head, V* __restrict__ C, int64_t ldc,
-                  int64_t n_tiles, int n_dense, int log2_tile) {
+                  const R* __restrict__ carry, const R* __restrict__ head, D* __restrict__ C, int64_t ldc,
+                  int64_t n_tiles, int n_dense, int log2_tile, int accumulate) {
   const int64_t gid = (int64_t)blockIdx.x * kMmThreads + threadIdx.x;
   const int64_t t = gid / n_dense + 1;
   const int j = (int)(gid % n_dense);
@@ -209,16 +394,18 @@ spmm_fixup_kernel(const P* __restrict__ ptr, const int32_t* __restrict__ tile_ro
     comp += (fabs(sum) >= fabs(v)) ? ((sum - s2) + v) : ((v - s2) + sum);
     sum = s2;
   }
-  V* dst = C + (int64_t)ra * ldc + j;
-  *dst = ACCUM ? (V)(((double)*dst + sum) + comp) : (V)(sum + comp);
+  D* dst = C + (int64_t)ra * ldc + j;
+  // rounded to the accumulator type first, like every other row
+  const R r = accumulate ? (R)(((double)MmOps<D>::widen(*dst) + sum) + comp) : (R)(sum + comp);
+  *dst = MmOps<D>::narrow(r);
 }
 
 template <typename V>
 __global__ void __launch_bounds__(kMmThreads) zero_rows_kernel(V* __restrict__ C, int64_t ldc, int64_t n_rows,
-                                                              int n_dense) {
+                                                              int64_t n_dense) {
   const int64_t gid = (int64_t)blockIdx.x * kMmThreads + threadIdx.x;
   const int64_t r = gid / n_dense;
-  const int j = (int)(gid % n_dense);
+  const int64_t j = gid % n_dense;
   if (r < n_rows) C[r * ldc + j] = (V)0;
 }
 
@@ -227,69 +414,192 @@ struct SpmmArgs {
   int64_t ldb;
   void* C;
   int64_t ldc, n_rows, n_dense, nnz;
-  int algo;
-  bool accumulate;
+  int algo, ptype;
+  bool accumulate, long_rows;
   const int32_t* tile_row;
   void* scratch;
   int32_t* status;
   cudaStream_t st;
 };
 
-template <typename V, typename I, typename P, int VW>
-static int launch_spmm(const SpmmArgs& a) {
+template <typename S> struct RealOf { typedef S Out; typedef typename MmOps<S>::Acc Acc; static constexpr int parts = 1; };
+template <> struct RealOf<float2> { typedef float Out; typedef float Acc; static constexpr int parts = 2; };
+template <> struct RealOf<double2> { typedef double Out; typedef double Acc; static constexpr int parts = 2; };
+
+static int pow2_at_least(int v) {
+  int p = 1;
+  while (p < v) p <<= 1;
+  return p;
+}
+
+template <typename S, typename I, int VW, int NC>
+static int launch_spmm(const SpmmArgs& a, int LR, int piece) {
+  typedef typename MmOps<S>::Acc A;
   constexpr int T = kMmTile;
+  constexpr bool REAL = sizeof(S) >= 4 && RealOf<S>::parts == 1;   // the types that are ever accumulated into C
   const int64_t n_tiles = (a.nnz + T - 1) / T;
   const int n_dense = (int)a.n_dense;
-  int need = (n_dense + VW - 1) / VW;  // lanes needed to cover a row of B
-  int LR = 1;
-  while (LR < 32 && LR < need) LR <<= 1;
-  const int col_tiles = (need + LR - 1) / LR;
-  V* carry = (V*)a.scratch;
-  V* head = carry + n_tiles * n_dense;
-  bool bulk = a.algo != FSB_SPMM_PLAIN && aligned_to(a.data, 16) && aligned_to(a.idx, 16);
-  dim3 grid((unsigned)n_tiles, (unsigned)col_tiles);
-#define FSB_SPMM_LAUNCH(BULK_, ACC_)                                                                          \
-  spmm_tile_kernel<V, I, P, VW, BULK_, ACC_><<<grid, kMmThreads, 0, a.st>>>(                                  \
-      (const V*)a.data, (const I*)a.idx, (const P*)a.ptr, (const V*)a.B, a.ldb, (V*)a.C, a.ldc, a.tile_row,   \
-      carry, head, a.nnz, n_dense, LR, a.status)
-  if (bulk) {
-    if (a.accumulate) FSB_SPMM_LAUNCH(true, true); else FSB_SPMM_LAUNCH(true, false);
+  const int width = LR * NC * VW;
+  const int64_t col_tiles = (n_dense + width - 1) / width;
+  if (col_tiles > 65535) return FSB_ERANGE;
+  A* carry = (A*)a.scratch;
+  A* head = carry + n_tiles * n_dense;
+  const int bulk = a.algo != FSB_SPMM_PLAIN && aligned_to(a.data, 16) && aligned_to(a.idx, 16);
+  const dim3 grid((unsigned)n_tiles, (unsigned)col_tiles);
+#define FSB_SPMM_LAUNCH(LONG_, ACC_, SMEM_)                                                                          \
+  spmm_tile_kernel<S, I, VW, NC, LONG_, ACC_><<<grid, kMmThreads, SMEM_, a.st>>>(                                    \
+      (const S*)a.data, (const I*)a.idx, a.ptr, a.ptype == FSB_I64, (const S*)a.B, a.ldb, (S*)a.C, a.ldc, a.tile_row, \
+      carry, head, a.nnz, n_dense, LR, piece, bulk, a.status)
+  // the long segments of a tile (more than 2 * piece entries each) have at most T / piece + T / (2 * piece) pieces
+  const size_t parts = a.long_rows ? (size_t)(T / piece + T / (2 * piece)) * width * sizeof(A) : 0;
+  if (a.accumulate) {
+    if constexpr (REAL) {
+      if (a.long_rows) FSB_SPMM_LAUNCH(true, true, parts); else FSB_SPMM_LAUNCH(false, true, 0);
+    } else {
+      return FSB_EINVAL;
+    }
   } else {
-    if (a.accumulate) FSB_SPMM_LAUNCH(false, true); else FSB_SPMM_LAUNCH(false, false);
+    if (a.long_rows) FSB_SPMM_LAUNCH(true, false, parts); else FSB_SPMM_LAUNCH(false, false, 0);
   }
 #undef FSB_SPMM_LAUNCH
   FSB_RETURN_IF_LAUNCH_FAILED();
   if (n_tiles > 1) {
+    typedef RealOf<S> R;
     int log2_tile = 0;
     while ((1 << log2_tile) < T) ++log2_tile;
-    const int64_t n = (n_tiles - 1) * n_dense;
-    const int64_t g = (n + kMmThreads - 1) / kMmThreads;
+    const int cols = n_dense * R::parts;
+    const int64_t g = ((n_tiles - 1) * cols + kMmThreads - 1) / kMmThreads;
     if (g >= INT32_MAX) return FSB_ERANGE;
-    if (a.accumulate)
-      spmm_fixup_kernel<V, P, true><<<(unsigned)g, kMmThreads, 0, a.st>>>((const P*)a.ptr, a.tile_row, carry, head,
-                                                                         (V*)a.C, a.ldc, n_tiles, n_dense, log2_tile);
-    else
-      spmm_fixup_kernel<V, P, false><<<(unsigned)g, kMmThreads, 0, a.st>>>((const P*)a.ptr, a.tile_row, carry, head,
-                                                                          (V*)a.C, a.ldc, n_tiles, n_dense, log2_tile);
+#define FSB_SPMM_FIXUP(P_)                                                                                          \
+  spmm_fixup_kernel<typename R::Acc, typename R::Out, P_><<<(unsigned)g, kMmThreads, 0, a.st>>>(                   \
+      (const P_*)a.ptr, a.tile_row, (const typename R::Acc*)carry, (const typename R::Acc*)head,                   \
+      (typename R::Out*)a.C, a.ldc * R::parts, n_tiles, cols, log2_tile, a.accumulate)
+    if (a.ptype == FSB_I64) FSB_SPMM_FIXUP(int64_t); else FSB_SPMM_FIXUP(int32_t);
+#undef FSB_SPMM_FIXUP
     FSB_RETURN_IF_LAUNCH_FAILED();
   }
   return FSB_OK;
 }
 
-template <typename V, typename I, typename P>
+// Lanes per entry (LR, a power of two) and accesses per lane (NC).  Up to 32 accesses there is one per lane (5 columns as
+// 2 lanes x 3: 66 us, as 8 lanes: 48 us, 200000 rows of 20 entries).  Beyond, the pair with the fewest idle lanes: 33
+// single columns take 16 lanes x 3 instead of two passes over the matrix with 32 lanes.  NC is bounded by what a lane
+// accumulates in registers (32 bytes).
+template <typename S, typename I, int VW>
+static int spmm_shape(const SpmmArgs& a) {
+  typedef typename MmOps<S>::Acc A;
+  constexpr int VMAX = 16 / (int)sizeof(S);
+  constexpr int HELD = VW * (int)sizeof(A);      // accumulator bytes of one access
+  // (16-byte values: one, or the pieces of long segments would not fit beside the staged tile)
+  constexpr int NC_MAX = sizeof(S) == 16 || HELD >= 32 ? 1 : (32 / HELD < 4 ? 32 / HELD : 4);
+  const int64_t need = (a.n_dense + VW - 1) / VW;
+  const int64_t need_widest = (a.n_dense + VMAX - 1) / VMAX;
+  const int LR_min = pow2_at_least((int)(need_widest < 32 ? need_widest : 32));   // what a 16-byte access would use
+  // half a group's even share of a tile, at least kMmMinPiece: a segment is long from twice that on
+  const int share = kMmTile / kMmThreads * LR_min;
+  const int piece = share / 2 > kMmMinPiece ? share / 2 : kMmMinPiece;
+  int LR = 32, NC = 1;
+  if (need <= 32) {
+    LR = pow2_at_least((int)need);
+  } else {
+    int64_t best = -1;
+    for (int nc = 1; nc <= NC_MAX; ++nc)
+      for (int lr = LR_min; lr <= 32; lr <<= 1) {
+        const int64_t passes = (need + lr * nc - 1) / (lr * nc);
+        const int64_t cost = passes * lr * nc * 64 + passes;   // idle lanes first, then passes over the matrix
+        if (best < 0 || cost < best) {
+          best = cost;
+          LR = lr;
+          NC = nc;
+        }
+      }
+  }
+  if constexpr (NC_MAX >= 2) {
+    if (NC == 2) return launch_spmm<S, I, VW, 2>(a, LR, piece);
+  }
+  if constexpr (NC_MAX >= 4) {
+    if (NC == 3) return launch_spmm<S, I, VW, 3>(a, LR, piece);
+    if (NC == 4) return launch_spmm<S, I, VW, 4>(a, LR, piece);
+  }
+  return launch_spmm<S, I, VW, 1>(a, LR, piece);
+}
+
+template <typename S, typename I>
 static int spmm_typed(const SpmmArgs& a) {
   // widest access that divides the row length and keeps every row of B and C aligned
-  constexpr int VMAX = 16 / sizeof(V);
+  constexpr int VMAX = 16 / (int)sizeof(S);
   int vw = VMAX;
   while (vw > 1 && !(a.n_dense % vw == 0 && a.ldb % vw == 0 && a.ldc % vw == 0 &&
-                     aligned_to(a.B, vw * sizeof(V)) && aligned_to(a.C, vw * sizeof(V)) &&
-                     aligned_to(a.scratch, vw * sizeof(V))))
+                     aligned_to(a.B, vw * sizeof(S)) && aligned_to(a.C, vw * sizeof(S))))
     vw >>= 1;
-  if constexpr (VMAX == 4) {
-    if (vw == 4) return launch_spmm<V, I, P, 4>(a);
+  if constexpr (VMAX >= 8) {
+    if (vw == 8) return spmm_shape<S, I, 8>(a);
   }
-  if (vw == 2) return launch_spmm<V, I, P, 2>(a);
-  return launch_spmm<V, I, P, 1>(a);
+  if constexpr (VMAX >= 4) {
+    if (vw == 4) return spmm_shape<S, I, 4>(a);
+  }
+  if constexpr (VMAX >= 2) {
+    if (vw == 2) return spmm_shape<S, I, 2>(a);
+  }
+  return spmm_shape<S, I, 1>(a);
+}
+
+static size_t stored_size(int vtype) {
+  return vtype == FSB_F16 || vtype == FSB_BF16 ? 2 : vtype == FSB_F32 ? 4 : vtype == FSB_C128 ? 16 : 8;
+}
+static size_t acc_size(int vtype) { return stored_size(vtype) < 4 ? 4 : stored_size(vtype); }
+
+static size_t spmm_scratch_bytes(int vtype, int64_t nnz, int64_t n_dense) {
+  const int64_t n_tiles = fsb_csr_num_tiles(nnz, kMmTile);
+  const size_t b = (size_t)n_tiles * 2 * (size_t)(n_dense > 0 ? n_dense : 0) * acc_size(vtype);
+  return (b + 255) & ~(size_t)255;
+}
+
+static int spmm_run(int vtype, int itype, int ptype, const void* data, const void* indices, const void* indptr,
+                    const void* B, int64_t ldb, void* C, int64_t ldc, int64_t n_rows, int64_t n_cols, int64_t n_dense,
+                    int64_t nnz, int algo, const int32_t* tile_row, void* scratch, size_t scratch_bytes,
+                    int32_t* status, cudaStream_t st) {
+  if ((itype != FSB_I32 && itype != FSB_I64) || (ptype != FSB_I32 && ptype != FSB_I64)) return FSB_EINVAL;
+  const bool accumulate = (algo & FSB_SPMM_ACCUMULATE) != 0;
+  const bool long_rows = (algo & FSB_SPMM_LONG_ROWS) != 0;
+  algo &= ~(FSB_SPMM_ACCUMULATE | FSB_SPMM_LONG_ROWS);
+  if (algo != FSB_SPMM_AUTO && algo != FSB_SPMM_PLAIN && algo != FSB_SPMM_BULK) return FSB_EINVAL;
+  if (n_rows < 0 || n_cols < 0 || n_dense < 0 || nnz < 0) return FSB_EINVAL;
+  if (n_rows >= INT32_MAX || n_cols >= INT32_MAX || n_dense >= (1 << 24)) return FSB_ERANGE;
+  if (ptype == FSB_I32 && nnz > INT32_MAX) return FSB_ERANGE;
+  if (n_rows == 0 || n_dense == 0) return FSB_OK;
+  if (C == nullptr || indptr == nullptr || ldc < n_dense) return FSB_EINVAL;
+  const size_t sv = stored_size(vtype), si = itype == FSB_I32 ? 4 : 8, sp = ptype == FSB_I32 ? 4 : 8;
+  if (!aligned_to(C, sv) || !aligned_to(indptr, sp)) return FSB_EALIGN;
+  FSB_WALK_FIRST(check_csr(itype, ptype, indices, indptr, n_rows, n_cols, nnz, st));
+  if (nnz == 0 && accumulate) return FSB_OK;   // nothing to add
+  if (nnz == 0) {
+    const int64_t words = sv < 4 ? 1 : (int64_t)(sv / 4);    // 2- or 4-byte words per element
+    const int64_t g = (n_rows * n_dense * words + kMmThreads - 1) / kMmThreads;
+    if (g >= INT32_MAX) return FSB_ERANGE;
+    if (sv == 2)
+      zero_rows_kernel<uint16_t><<<(unsigned)g, kMmThreads, 0, st>>>((uint16_t*)C, ldc, n_rows, n_dense);
+    else
+      zero_rows_kernel<uint32_t><<<(unsigned)g, kMmThreads, 0, st>>>((uint32_t*)C, ldc * words, n_rows, n_dense * words);
+    FSB_RETURN_IF_LAUNCH_FAILED();
+    return FSB_OK;
+  }
+  if (data == nullptr || indices == nullptr || B == nullptr || ldb < n_dense) return FSB_EINVAL;
+  if (!aligned_to(data, sv) || !aligned_to(B, sv) || !aligned_to(indices, si)) return FSB_EALIGN;
+  if (tile_row == nullptr || scratch == nullptr) return FSB_EINVAL;
+  if (scratch_bytes < spmm_scratch_bytes(vtype, nnz, n_dense)) return FSB_ESCRATCH;
+  if (!aligned_to(scratch, 16)) return FSB_EALIGN;
+  if (fsb_csr_num_tiles(nnz, kMmTile) >= 65535LL * 32768LL) return FSB_ERANGE;
+
+  SpmmArgs a{data, indices, indptr, B, ldb, C, ldc, n_rows, n_dense, nnz, algo, ptype, accumulate, long_rows, tile_row,
+             scratch, status, st};
+  if (vtype == FSB_F32) return itype == FSB_I32 ? spmm_typed<float, int32_t>(a) : spmm_typed<float, int64_t>(a);
+  if (vtype == FSB_F64) return itype == FSB_I32 ? spmm_typed<double, int32_t>(a) : spmm_typed<double, int64_t>(a);
+  if (itype != FSB_I32) return FSB_EINVAL;
+  if (vtype == FSB_F16) return spmm_typed<__half, int32_t>(a);
+  if (vtype == FSB_BF16) return spmm_typed<__nv_bfloat16, int32_t>(a);
+  if (vtype == FSB_C64) return spmm_typed<float2, int32_t>(a);
+  return spmm_typed<double2, int32_t>(a);
 }
 
 }  // namespace fsb
@@ -302,10 +612,7 @@ extern "C" int fsb_spmm_tile_nnz(int vtype) {
 }
 
 extern "C" size_t fsb_spmm_csr_scratch_bytes(int vtype, int64_t nnz, int64_t n_dense) {
-  const int64_t n_tiles = fsb_csr_num_tiles(nnz, kMmTile);
-  const size_t sv = vtype == FSB_F32 ? 4 : 8;
-  size_t b = (size_t)n_tiles * 2 * (size_t)(n_dense > 0 ? n_dense : 0) * sv;
-  return (b + 255) & ~(size_t)255;
+  return spmm_scratch_bytes(vtype, nnz, n_dense);
 }
 
 extern "C" int fsb_spmm_csr(int vtype, int itype, int ptype, const void* data, const void* indices,
@@ -313,52 +620,36 @@ extern "C" int fsb_spmm_csr(int vtype, int itype, int ptype, const void* data, c
                             int64_t n_rows, int64_t n_cols, int64_t n_dense, int64_t nnz, int algo,
                             const int32_t* tile_row, void* scratch, size_t scratch_bytes, int32_t* status,
                             void* stream_) {
-  cudaStream_t st = static_cast<cudaStream_t>(stream_);
-  if ((vtype != FSB_F32 && vtype != FSB_F64) || (itype != FSB_I32 && itype != FSB_I64) ||
-      (ptype != FSB_I32 && ptype != FSB_I64))
-    return FSB_EINVAL;
-  const bool accumulate = (algo & FSB_SPMM_ACCUMULATE) != 0;
-  algo &= ~FSB_SPMM_ACCUMULATE;
-  if (algo != FSB_SPMM_AUTO && algo != FSB_SPMM_PLAIN && algo != FSB_SPMM_BULK) return FSB_EINVAL;
-  if (n_rows < 0 || n_cols < 0 || n_dense < 0 || nnz < 0) return FSB_EINVAL;
-  if (n_rows >= INT32_MAX || n_cols >= INT32_MAX || n_dense >= (1 << 24)) return FSB_ERANGE;
-  if (ptype == FSB_I32 && nnz > INT32_MAX) return FSB_ERANGE;
-  if (n_rows == 0 || n_dense == 0) return FSB_OK;
-  if (C == nullptr || indptr == nullptr || ldc < n_dense) return FSB_EINVAL;
-  const size_t sv = vtype == FSB_F32 ? 4 : 8, si = itype == FSB_I32 ? 4 : 8, sp = ptype == FSB_I32 ? 4 : 8;
-  if (!aligned_to(C, sv) || !aligned_to(indptr, sp)) return FSB_EALIGN;
-  FSB_WALK_FIRST(check_csr(itype, ptype, indices, indptr, n_rows, n_cols, nnz, st));
-  if (nnz == 0 && accumulate) return FSB_OK;   // nothing to add
-  if (nnz == 0) {
-    const int64_t n = n_rows * n_dense;
-    const int64_t g = (n + kMmThreads - 1) / kMmThreads;
-    if (g >= INT32_MAX) return FSB_ERANGE;
-    if (vtype == FSB_F32)
-      zero_rows_kernel<float><<<(unsigned)g, kMmThreads, 0, st>>>((float*)C, ldc, n_rows, (int)n_dense);
-    else
-      zero_rows_kernel<double><<<(unsigned)g, kMmThreads, 0, st>>>((double*)C, ldc, n_rows, (int)n_dense);
-    FSB_RETURN_IF_LAUNCH_FAILED();
-    return FSB_OK;
-  }
-  if (data == nullptr || indices == nullptr || B == nullptr || ldb < n_dense) return FSB_EINVAL;
-  if (!aligned_to(data, sv) || !aligned_to(B, sv) || !aligned_to(indices, si)) return FSB_EALIGN;
-  if (tile_row == nullptr || scratch == nullptr) return FSB_EINVAL;
-  if (scratch_bytes < fsb_spmm_csr_scratch_bytes(vtype, nnz, n_dense)) return FSB_ESCRATCH;
-  if (!aligned_to(scratch, 16)) return FSB_EALIGN;
-  if (fsb_csr_num_tiles(nnz, kMmTile) >= 65535LL * 32768LL) return FSB_ERANGE;
+  if (vtype != FSB_F32 && vtype != FSB_F64) return FSB_EINVAL;
+  return spmm_run(vtype, itype, ptype, data, indices, indptr, B, ldb, C, ldc, n_rows, n_cols, n_dense, nnz, algo,
+                  tile_row, scratch, scratch_bytes, status, static_cast<cudaStream_t>(stream_));
+}
 
-  SpmmArgs a{data, indices, indptr, B, ldb, C, ldc, n_rows, n_dense, nnz, algo, accumulate, tile_row, scratch,
-             status, st};
-#define FSB_CASE(VT, V, IT, I, PT, P) \
-  if (vtype == VT && itype == IT && ptype == PT) return spmm_typed<V, I, P>(a);
-  FSB_CASE(FSB_F32, float, FSB_I32, int32_t, FSB_I32, int32_t)
-  FSB_CASE(FSB_F32, float, FSB_I32, int32_t, FSB_I64, int64_t)
-  FSB_CASE(FSB_F32, float, FSB_I64, int64_t, FSB_I32, int32_t)
-  FSB_CASE(FSB_F32, float, FSB_I64, int64_t, FSB_I64, int64_t)
-  FSB_CASE(FSB_F64, double, FSB_I32, int32_t, FSB_I32, int32_t)
-  FSB_CASE(FSB_F64, double, FSB_I32, int32_t, FSB_I64, int64_t)
-  FSB_CASE(FSB_F64, double, FSB_I64, int64_t, FSB_I32, int32_t)
-  FSB_CASE(FSB_F64, double, FSB_I64, int64_t, FSB_I64, int64_t)
-#undef FSB_CASE
-  return FSB_EINVAL;
+extern "C" size_t fsb_spmm_stored_scratch_bytes(int vtype, int64_t nnz, int64_t n_dense) {
+  const size_t plan = ((size_t)fsb_csr_num_tiles(nnz, kMmTile) + 1) * sizeof(int32_t);
+  return spmm_scratch_bytes(vtype, nnz, n_dense) + ((plan + 255) & ~(size_t)255);
+}
+
+extern "C" int fsb_spmm_csr_stored(int vtype, int ptype, const void* data, const int32_t* indices, const void* indptr,
+                                   const void* B, int64_t ldb, void* C, int64_t ldc, int64_t n_rows, int64_t n_cols,
+                                   int64_t n_dense, int64_t nnz, int long_rows, void* scratch, size_t scratch_bytes,
+                                   void* stream_) {
+  if (vtype != FSB_F16 && vtype != FSB_BF16 && vtype != FSB_C64 && vtype != FSB_C128) return FSB_EINVAL;
+  int32_t* tile_row = nullptr;
+  size_t parts_bytes = 0;
+  if (nnz > 0 && n_rows > 0 && n_dense > 0) {
+    if (n_rows >= INT32_MAX || n_dense >= (1 << 24)) return FSB_ERANGE;
+    if (scratch == nullptr || indptr == nullptr) return FSB_EINVAL;
+    if (scratch_bytes < fsb_spmm_stored_scratch_bytes(vtype, nnz, n_dense)) return FSB_ESCRATCH;
+    if (!aligned_to(scratch, 16)) return FSB_EALIGN;
+    FSB_WALK_FIRST(check_csr(FSB_I32, ptype, indices, indptr, n_rows, n_cols, nnz, static_cast<cudaStream_t>(stream_)));
+    parts_bytes = spmm_scratch_bytes(vtype, nnz, n_dense);
+    tile_row = (int32_t*)((char*)scratch + parts_bytes);
+    const int rc = fsb_csr_tile_plan(ptype, indptr, n_rows, nnz, kMmTile, tile_row, stream_);
+    if (rc != FSB_OK) return rc;
+  }
+  // staged by ordinary loads: no copy whose end would have to be waited for and reported
+  return spmm_run(vtype, FSB_I32, ptype, data, indices, indptr, B, ldb, C, ldc, n_rows, n_cols, n_dense, nnz,
+                  FSB_SPMM_PLAIN | (long_rows ? FSB_SPMM_LONG_ROWS : 0), tile_row, scratch, parts_bytes, nullptr,
+                  static_cast<cudaStream_t>(stream_));
 }

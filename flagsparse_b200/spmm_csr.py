@@ -27,6 +27,8 @@ from ._common import (
     _tile_plan,
 )
 
+_STORED_VTYPE = {torch.float16: _lib.FSB_F16, torch.bfloat16: _lib.FSB_BF16, torch.complex64: _lib.FSB_C64,
+                 torch.complex128: _lib.FSB_C128}
 _SPMM_ALGO_NAMES = {"auto": _lib.FSB_SPMM_AUTO, "plain": _lib.FSB_SPMM_PLAIN, "bulk": _lib.FSB_SPMM_BULK}
 
 # A product whose gathers range over more of B than stays in L2 can be split: A into column panels (each panel's
@@ -37,6 +39,9 @@ _SPMM_ALGO_NAMES = {"auto": _lib.FSB_SPMM_AUTO, "plain": _lib.FSB_SPMM_PLAIN, "b
 # of its read-add-write of C, not by the bytes it saves.  FSB_SPMM_PANEL_MB=<MiB> or FSB_SPMM_PANELS=<n> turn it on.
 PANEL_BYTES = 0
 COL_TILE_BYTES = 128
+# rows longer than this get FSB_SPMM_LONG_ROWS (include/fsb.h): about where a group that walks one alone takes longer
+# than its neighbours take for their share of a 1024-entry tile
+LONG_ROW_NNZ = 256
 SPAN_WINDOW = 1 << 20        # consecutive entries over which the column span is sampled
 
 
@@ -339,7 +344,7 @@ def prepare_spmm_csr_opt(data, indices, indptr, shape):
     )
     nnz = data.numel()
     if data.dtype in widetypes.WIDE_DTYPES:
-        # read as stored by fsb_spmm_csr_wide: nothing to plan, no second copy of the matrix
+        # read as stored by fsb_spmm_csr_stored, which plans its tiles itself: no second copy of the matrix
         return PreparedCsrSpmmOpt(data, kernel_indices, kernel_indptr, shape, n_rows, n_cols, stats, 0, None,
                                   wide=("native", []))
     tile_nnz, tile_row = 0, None
@@ -362,6 +367,8 @@ def _spmm_launch(prepared, B, C):
     algo = _SPMM_ALGO_NAMES.get(os.environ.get("FSB_SPMM_ALGO", "auto").strip().lower(), _lib.FSB_SPMM_AUTO)
     status = p.status_word()
     status.poll()
+    if p.max_row_nnz > LONG_ROW_NNZ:
+        algo |= _lib.FSB_SPMM_LONG_ROWS
     sv = B.element_size()
     vt, it, pt = _VTYPE[p.data.dtype], _ITYPE[p.kernel_indices.dtype], _ITYPE[p.kernel_indptr.dtype]
     ldb, ldc = B.stride(0), C.stride(0)
@@ -409,10 +416,30 @@ def _spmm_launch_wide(prepared, B, C):
     _lib.check(rc, "fsb_spmm_csr_wide")
 
 
+def _spmm_launch_stored(prepared, B, C):
+    """Enqueue C = A B for float16 / bfloat16 / complex values with B and C in the matrix's own type: the tiled kernel,
+    which reads 2-byte values as they are and rounds every element of C once."""
+    p = prepared
+    dev = p.data.device
+    n_dense, nnz = int(B.shape[1]), p.data.numel()
+    if p.n_rows == 0 or n_dense == 0:
+        return
+    L = _lib.lib()
+    vt = _STORED_VTYPE[p.data.dtype]
+    scratch = torch.empty(int(L.fsb_spmm_stored_scratch_bytes(vt, nnz, n_dense)), dtype=torch.uint8, device=dev)
+    with torch.cuda.device(dev):
+        rc = L.fsb_spmm_csr_stored(
+            vt, _ITYPE[p.kernel_indptr.dtype], _ptr(p.data), _ptr(p.kernel_indices), p.kernel_indptr.data_ptr(),
+            _ptr(B), B.stride(0) if B.shape[0] > 1 else n_dense, C.data_ptr(), n_dense, p.n_rows, p.n_cols, n_dense, nnz,
+            int(p.max_row_nnz > LONG_ROW_NNZ), scratch.data_ptr(), scratch.numel(), _stream_ptr(dev),
+        )
+    _lib.check(rc, "fsb_spmm_csr_stored")
+
+
 def _run_spmm(prepared, B, out, return_time):
     dev, dtype = prepared.data.device, prepared.data.dtype
     shape = (prepared.n_rows, int(B.shape[1]))
-    if prepared.wide is not None:
+    if prepared.wide is not None and B.device.type != "cuda":   # host stand-ins take fsb_spmm_csr_wide's operands
         t0 = None
         if return_time:
             torch.cuda.synchronize(dev)
@@ -426,13 +453,17 @@ def _run_spmm(prepared, B, out, return_time):
             out.copy_(C)
             C = out
         return (C, elapsed_ms) if return_time else C
-    direct = out is not None and out.is_contiguous()
+    # float16 / bfloat16 / complex products never write into `out` while B is still read: it may be B itself there
+    direct = out is not None and out.is_contiguous() and prepared.wide is None
     C = out if direct else torch.empty(shape, dtype=dtype, device=dev)
     t0 = None
     if return_time:
         torch.cuda.synchronize(dev)
         t0 = time.perf_counter()
-    _spmm_launch(prepared, B, C)
+    if prepared.wide is not None:
+        _spmm_launch_stored(prepared, _row_major(B), C)
+    else:
+        _spmm_launch(prepared, B, C)
     elapsed_ms = None
     if return_time:
         torch.cuda.synchronize(dev)

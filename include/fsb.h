@@ -34,7 +34,7 @@ extern "C" {
 /* dtype tags */
 #define FSB_F32 0
 #define FSB_F64 1
-#define FSB_F16 2             /* fsb_spmv_csr_wide / fsb_spmm_csr_wide only */
+#define FSB_F16 2             /* the *_wide and *_stored entry points only */
 #define FSB_BF16 3
 #define FSB_C64 4             /* interleaved (re, im) float32 pairs */
 #define FSB_C128 5            /* interleaved (re, im) float64 pairs */
@@ -61,6 +61,7 @@ extern "C" {
 #define FSB_SPMM_PLAIN 1     /* tile of data/indices staged in shared memory by ordinary loads   */
 #define FSB_SPMM_BULK 2      /* tile staged by cp.async.bulk (TMA 1-D bulk copy) + mbarrier       */
 #define FSB_SPMM_ACCUMULATE 16 /* or-ed into the selector: C += A B instead of C = A B            */
+#define FSB_SPMM_LONG_ROWS 32  /* or-ed into the selector: some rows are long (see fsb_spmm_csr)  */
 
 int fsb_version(void);
 
@@ -288,7 +289,10 @@ int fsb_spmv_csr_noalloc(int vtype, int itype, int ptype, const void* data, cons
  *             holds (rows of A without entries leave their row of C untouched).  The host code uses it to
  *             multiply by column panels of A one after the other, each panel's slice of B small enough to stay
  *             in L2 while it is gathered from, and by column tiles of B / C (pass the tile's first element and the
- *             full leading dimensions).
+ *             full leading dimensions).  FSB_SPMM_LONG_ROWS: the part of a row that lies in a tile is shared by the
+ *             whole block where it has more than 64 entries (128 with 32 lanes per row); right for any
+ *             matrix, and worth its shared memory where rows are longer than that.  It changes the order in which
+ *             the entries of such rows are added.
  *   tile_row  from fsb_csr_tile_plan(tile_nnz = fsb_spmm_tile_nnz(vtype)).
  *   scratch   at least fsb_spmm_csr_scratch_bytes() bytes, 16-byte aligned (per-tile partial rows of
  *             rows that cross a tile boundary -- the counterpart of the reference's split workspace).
@@ -320,6 +324,17 @@ int fsb_spmv_csr_wide(int vtype, int ptype, const void* data, const int32_t* ind
 int fsb_spmm_csr_wide(int vtype, int ptype, const void* data, const int32_t* indices, const void* indptr,
                       const void* B, int64_t ldb, void* C, int64_t ldc, int64_t n_rows, int64_t n_cols,
                       int64_t n_dense, int64_t nnz, void* stream);
+
+/*
+ * C = A B for the same four value types with B and C in the matrix's own type (half precisions: 2-byte values read as
+ * they are stored, products and sums in float32, every element of C rounded once).  The tiled kernel of fsb_spmm_csr,
+ * its tile plan made in scratch (fsb_spmm_stored_scratch_bytes() bytes, 16-byte aligned); long_rows != 0 is
+ * FSB_SPMM_LONG_ROWS.
+ */
+size_t fsb_spmm_stored_scratch_bytes(int vtype, int64_t nnz, int64_t n_dense);
+int fsb_spmm_csr_stored(int vtype, int ptype, const void* data, const int32_t* indices, const void* indptr,
+                        const void* B, int64_t ldb, void* C, int64_t ldc, int64_t n_rows, int64_t n_cols,
+                        int64_t n_dense, int64_t nnz, int long_rows, void* scratch, size_t scratch_bytes, void* stream);
 
 /*
  * Sampled dense-dense product on a CSR pattern: out[p] = alpha * dot(X[row(p), :], Y[indices[p], :]) + beta * data[p]
