@@ -78,6 +78,9 @@ SIGNATURES = {
     "fsb_spmm_csr_stored": (
         _i32, [_i32, _i32, _vp, _vp, _vp, _vp, _i64, _vp, _i64, _i64, _i64, _i64, _i64, _i32, _vp, _sz, _vp],
     ),
+    "fsb_spmv_stored_tile_nnz": (_i32, [_i32]),
+    "fsb_spmv_stored_scratch_bytes": (_sz, [_i32, _i64]),
+    "fsb_spmv_csr_stored": (_i32, [_i32, _i32, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _vp, _vp, _sz, _vp]),
     "fsb_spmv_csr_wide": (_i32, [_i32, _i32, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _vp]),
     "fsb_spmm_csr_wide": (_i32, [_i32, _i32, _vp, _vp, _vp, _vp, _i64, _vp, _i64, _i64, _i64, _i64, _i64, _vp]),
     "fsb_sddmm_csr": (_i32, [_i32, _vp, _vp, _vp, _i64, _vp, _i64, _vp, _vp, _i64, _i64, _i64, _i64, _c.c_double,

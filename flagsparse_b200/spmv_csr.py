@@ -41,6 +41,8 @@ def _long_rows_enabled():
     return os.environ.get("FSB_SPMV_LONG_ROWS", "1") != "0"
 
 
+_WIDE_VTYPE = {torch.float16: _lib.FSB_F16, torch.bfloat16: _lib.FSB_BF16, torch.complex64: _lib.FSB_C64,
+               torch.complex128: _lib.FSB_C128}
 _ALGO_NAMES = {"auto": _lib.FSB_SPMV_AUTO, "vector": _lib.FSB_SPMV_VECTOR, "stream": _lib.FSB_SPMV_STREAM,
                "panel": _lib.FSB_SPMV_PANEL}
 
@@ -75,6 +77,13 @@ def _select_spmv_algo(n_rows, nnz, max_row_nnz):
     if max_row_nnz <= _UNIFORM_ROW_FACTOR * mean + _UNIFORM_ROW_SLACK:
         return _lib.FSB_SPMV_VECTOR
     return _lib.FSB_SPMV_STREAM
+
+
+def _uneven_rows(n_rows, nnz, max_row_nnz):
+    """Whether the longest row leaves the lanes-per-row kernel for float16 / bfloat16 / complex values waiting for it.
+    A row of n entries takes its 2 to 32 lanes about n / (4 lanes) trips to memory, one after the other; the tiled
+    kernel costs a second launch and the products' way through shared memory."""
+    return max_row_nnz > _UNIFORM_ROW_FACTOR * (nnz / max(n_rows, 1)) + _UNIFORM_ROW_SLACK
 
 
 class PreparedCsrSpmv:
@@ -237,13 +246,21 @@ def _prepare_spmv_csr(data, indices, indptr, shape, block_nnz, max_segments, reu
     block_nnz_use, max_segments_use = _resolve_block_nnz(max_row_nnz, block_nnz, max_segments)
     nnz = data.numel()
     if data.dtype in widetypes.WIDE_DTYPES:
-        # float16 / bfloat16 / complex values are read as they are stored by a kernel of their own (fsb_spmv_csr_wide):
-        # nothing to plan, no second copy of the matrix
+        # float16 / bfloat16 / complex values are read as they are stored by kernels of their own (fsb_spmv_csr_stored):
+        # no second copy of the matrix, and a tile plan where the row lengths call for one
+        tile_nnz, tile_row, scratch = 0, None, None
+        if (nnz > 0 and n_rows > 0 and data.device.type == "cuda"
+                and _uneven_rows(n_rows, nnz, max_row_nnz)):
+            L = _lib.lib()
+            tile_nnz = int(L.fsb_spmv_stored_tile_nnz(_WIDE_VTYPE[data.dtype]))
+            tile_row = _tile_plan(kernel_indptr, n_rows, nnz, tile_nnz)
+            scratch = torch.empty(int(L.fsb_spmv_stored_scratch_bytes(_WIDE_VTYPE[data.dtype], nnz)),
+                                  dtype=torch.uint8, device=data.device)
         return PreparedCsrSpmv(
             data=data, kernel_indices=kernel_indices, kernel_indptr=kernel_indptr, shape=shape, n_rows=n_rows,
             n_cols=n_cols, block_nnz=block_nnz_use, max_segments=max_segments_use, max_row_nnz=max_row_nnz,
-            stats=stats, algo=_lib.FSB_SPMV_VECTOR, tuning=0, tile_nnz=0, tile_row=None, scratch=None,
-            wide=("native", []),
+            stats=stats, algo=_lib.FSB_SPMV_VECTOR if tile_row is None else _lib.FSB_SPMV_STREAM, tuning=0,
+            tile_nnz=tile_nnz, tile_row=tile_row, scratch=scratch, wide=("native", []),
         )
     algo = _select_spmv_algo(n_rows, nnz, max_row_nnz)
     tuning = int(os.environ.get("FSB_SPMV_TUNING", "0"))
@@ -315,10 +332,6 @@ def _spmv_launch(prepared, x, y):
     _lib.check(rc, "fsb_spmv_csr")
 
 
-_WIDE_VTYPE = {torch.float16: _lib.FSB_F16, torch.bfloat16: _lib.FSB_BF16, torch.complex64: _lib.FSB_C64,
-               torch.complex128: _lib.FSB_C128}
-
-
 def _spmv_launch_wide(prepared, x, y):
     """Enqueue y = A x for float16 / bfloat16 / complex values (fsb_spmv_csr_wide): x and y are float32 for the
     half precisions and of the matrix's own type for complex values.  Stands in for the reference's base launch
@@ -333,6 +346,22 @@ def _spmv_launch_wide(prepared, x, y):
             p.kernel_indptr.data_ptr(), _ptr(x), _ptr(y), p.n_rows, p.n_cols, p.data.numel(), _stream_ptr(dev),
         )
     _lib.check(rc, "fsb_spmv_csr_wide")
+
+
+def _spmv_launch_stored(prepared, x, y):
+    """Enqueue y = A x for float16 / bfloat16 / complex values with x and y in the matrix's own type."""
+    p = prepared
+    dev = p.data.device
+    if p.n_rows == 0:
+        return
+    with torch.cuda.device(dev):
+        rc = _lib.lib().fsb_spmv_csr_stored(
+            _WIDE_VTYPE[p.data.dtype], _ITYPE[p.kernel_indptr.dtype], _ptr(p.data), _ptr(p.kernel_indices),
+            p.kernel_indptr.data_ptr(), _ptr(x), _ptr(y), p.n_rows, p.n_cols, p.data.numel(),
+            None if p.tile_row is None else p.tile_row.data_ptr(), _ptr(p.scratch),
+            0 if p.scratch is None else p.scratch.numel(), _stream_ptr(dev),
+        )
+    _lib.check(rc, "fsb_spmv_csr_stored")
 
 
 def flagsparse_spmv_csr(data=None, indices=None, indptr=None, x=None, shape=None, block_nnz=256,
@@ -358,7 +387,11 @@ def flagsparse_spmv_csr(data=None, indices=None, indptr=None, x=None, shape=None
         if return_time:
             torch.cuda.synchronize(dev)
             t0 = time.perf_counter()
-        y = widetypes.run(prepared, x, _spmv_launch_wide, (prepared.n_rows,))
+        if x.device.type == "cuda":
+            y = torch.empty(prepared.n_rows, dtype=dtype, device=dev)   # not `out`, which may be x itself
+            _spmv_launch_stored(prepared, x, y)
+        else:                                     # host stand-ins take fsb_spmv_csr_wide's operands
+            y = widetypes.run(prepared, x, _spmv_launch_wide, (prepared.n_rows,))
         elapsed_ms = None
         if return_time:
             torch.cuda.synchronize(dev)

@@ -317,6 +317,19 @@ int fsb_spmv_csr_wide(int vtype, int ptype, const void* data, const int32_t* ind
                       const void* x, void* y, int64_t n_rows, int64_t n_cols, int64_t nnz, void* stream);
 
 /*
+ * y = A x for the same four value types with x and y in the matrix's own type (half precisions: products and sums in
+ * float32, every element of y rounded once).  Without a plan (tile_row NULL) a group of 2 to 32 lanes walks each row:
+ * for rows of about equal length.  With tile_row (fsb_csr_tile_plan, tile_nnz = fsb_spmv_stored_tile_nnz(vtype)) the work
+ * of a block does not depend on the row lengths; scratch then holds fsb_spmv_stored_scratch_bytes() bytes, 16-byte
+ * aligned.  Bit-reproducible either way.
+ */
+int fsb_spmv_stored_tile_nnz(int vtype);
+size_t fsb_spmv_stored_scratch_bytes(int vtype, int64_t nnz);
+int fsb_spmv_csr_stored(int vtype, int ptype, const void* data, const int32_t* indices, const void* indptr,
+                        const void* x, void* y, int64_t n_rows, int64_t n_cols, int64_t nnz,
+                        const int32_t* tile_row, void* scratch, size_t scratch_bytes, void* stream);
+
+/*
  * C = A B for the same four value types, with the same conventions (B and C float32 for the half precisions, of the
  * matrix's own interleaved type for complex values; row-major with leading dimensions ldb / ldc in elements of that
  * type).  Replaces the launch in _triton_spmm_csr_impl for these types (spmm_csr.py:525-599, complex kernel :138-195).
