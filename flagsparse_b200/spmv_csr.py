@@ -32,6 +32,7 @@ _VECTOR_MAX_ROW_NNZ = 4096
 # "uniform" rows: the longest row is within this factor (plus a small allowance) of the mean row length
 _UNIFORM_ROW_FACTOR = 8
 _UNIFORM_ROW_SLACK = 64
+_SMALL_ROW_SLACK = 256       # the same for matrices of less than _STREAM_MIN_NNZ entries
 # regroup banded matrices for the panel kernel (costs a second copy of the entries); FSB_SPMV_PANEL=0 turns it off
 _PANEL_ENABLED = os.environ.get("FSB_SPMV_PANEL", "1") != "0"
 
@@ -71,9 +72,11 @@ def _select_spmv_algo(n_rows, nnz, max_row_nnz):
         return _ALGO_NAMES[forced]
     if max_row_nnz > _VECTOR_MAX_ROW_NNZ:
         return _lib.FSB_SPMV_STREAM
-    if nnz < _STREAM_MIN_NNZ:
-        return _lib.FSB_SPMV_VECTOR
     mean = nnz / max(n_rows, 1)
+    if nnz < _STREAM_MIN_NNZ:
+        # one launch against two (8 us against 13 us); a row of n entries takes its two or more lanes about 0.05 n us
+        # (2274 entries, two lanes: 126 us in all, the stream kernel 15 us)
+        return _lib.FSB_SPMV_VECTOR if max_row_nnz <= _UNIFORM_ROW_FACTOR * mean + _SMALL_ROW_SLACK else _lib.FSB_SPMV_STREAM
     if max_row_nnz <= _UNIFORM_ROW_FACTOR * mean + _UNIFORM_ROW_SLACK:
         return _lib.FSB_SPMV_VECTOR
     return _lib.FSB_SPMV_STREAM
