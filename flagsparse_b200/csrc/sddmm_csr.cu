@@ -95,20 +95,39 @@ sddmm_kernel(const int32_t* __restrict__ indices, const int32_t* __restrict__ ro
     V acc[E];
 #pragma unroll
     for (int e = 0; e < E; ++e) acc[e] = (V)0;
-    // Row ids never decrease along a CSR pattern, so the batch lies in one row of X iff its first and last ids
-    // agree.  Then one slice of X serves all eight gathers, which leave together.  Otherwise every entry gets its
-    // own slice of X, four entries at a time (reloading X only where the row changes would make each gather wait
-    // for the previous entry's arithmetic).
-    if (rows[0] == rows[E - 1]) {
+    // Row ids never decrease along a CSR pattern.  Most batches meet one row of X or two: a slice of each then serves all
+    // eight gathers, which leave together.  Where a batch meets more rows every entry gets its own slice of X, four
+    // entries at a time (reloading X only where the row changes would make each gather wait for the previous entry's
+    // arithmetic).  float64, and float32 with a whole warp per entry, have no registers for a second slice beside eight
+    // gathers of 16 bytes: there only a batch of one row takes the first form.  (2^19 rows of 16 entries, K 64, float32:
+    // 459 us when a batch of two rows took the second form, 350 us now; 300000 rows of 5, K 33: 171 us, 112 us.  With
+    // TWO everywhere float64, 50000 rows of 40, K 64 goes from 115 us to 168 us.)
+    constexpr bool TWO = sizeof(V) == 4 && (LG <= 16 || VW == 1);
+    const int32_t row_a = rows[0], row_b = rows[E - 1];
+    bool few = row_a == row_b;
+    unsigned in_a = 0;
+    if constexpr (TWO) {
+      few = true;
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        few = few && (rows[e] == row_a || rows[e] == row_b);
+        in_a |= (rows[e] == row_a ? 1u : 0u) << e;
+      }
+    }
+    if (few) {
       for (int k = lane * VW; k < k_dim; k += step) {
-        V xr[VW], yv[E][VW];
-        ld_dense<V, VW>(X + (int64_t)rows[0] * ldx + k, xr);
+        V xa[VW], xb[VW], yv[E][VW];
+        ld_dense<V, VW>(X + (int64_t)row_a * ldx + k, xa);
+        if constexpr (TWO) ld_dense<V, VW>(X + (int64_t)row_b * ldx + k, xb);
 #pragma unroll
         for (int e = 0; e < E; ++e) ld_dense<V, VW>(Y + (int64_t)cols[e] * ldy + k, yv[e]);
 #pragma unroll
         for (int e = 0; e < E; ++e)
 #pragma unroll
-          for (int i = 0; i < VW; ++i) acc[e] += xr[i] * yv[e][i];
+          for (int i = 0; i < VW; ++i) {
+            if constexpr (TWO) acc[e] += ((in_a >> e) & 1 ? xa[i] : xb[i]) * yv[e][i];
+            else acc[e] += xa[i] * yv[e][i];
+          }
       }
     } else {
       for (int k = lane * VW; k < k_dim; k += step) {

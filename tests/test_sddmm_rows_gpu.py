@@ -1,0 +1,29 @@
+"""SDDMM where batches of eight entries meet one, two and more rows, for the lane counts and access widths whose kernels
+treat them differently.  Bound: a dot product of K terms in any order, (K + 1) u sum |x y|."""
+
+import numpy as np
+import pytest
+import torch
+
+import flagsparse_b200 as fs
+from helpers import handmade_csr
+
+pytestmark = pytest.mark.gpu
+
+LENS = {"one": [8] * 40, "two": [5, 11, 8, 7, 9, 4, 12] * 9, "more": [1, 2, 0, 3, 1, 1, 0, 0, 4] * 21, "odd": [13, 0, 6, 1, 2, 30, 3]}
+
+
+@pytest.mark.parametrize("dtype,u", [(torch.float32, 2.0 ** -24), (torch.float64, 2.0 ** -53)], ids=str)
+@pytest.mark.parametrize("name", sorted(LENS))
+def test_batches_over_rows(cuda, fsb_lib, dtype, u, name):
+    n_cols = 200
+    _, i, p = handmade_csr(2, LENS[name], n_cols)
+    n_rows = len(p) - 1
+    row = np.repeat(np.arange(n_rows), np.diff(p))
+    prep = fs.prepare_sddmm_csr(torch.from_numpy(i).to(cuda), torch.from_numpy(p).to(cuda), (n_rows, n_cols))
+    for k in (1, 3, 4, 8, 33, 64, 66, 128, 130):
+        rng = np.random.default_rng(k)
+        x, y = (torch.from_numpy(rng.uniform(-1, 1, (n, k))).to(dtype) for n in (n_rows, n_cols))
+        out = fs.flagsparse_sddmm_csr(x=x.to(cuda), y=y.to(cuda), prepared=prep).cpu().double().numpy()
+        xd, yd = x.double().numpy()[row], y.double().numpy()[i]
+        assert np.all(np.abs(out - (xd * yd).sum(1)) <= (k + 1) * u * 1.0001 * np.abs(xd * yd).sum(1))
