@@ -42,8 +42,31 @@ def _tolerance_for_dtype(value_dtype):
     return 1e-6, 1e-5
 
 
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _stream_ptr(device):
+    if _raw_stream is not None and device.index is not None:
+        return _raw_stream(device.index)         # the handle alone, without a Stream object around it
     return torch.cuda.current_stream(device).cuda_stream
+
+
+class _Here:
+    __slots__ = ()
+
+    def __enter__(self):
+        return self
+
+    def __exit__(self, *exc):
+        return False
+
+
+_HERE = _Here()
+
+
+def _on_device(device):
+    """Context in which `device` is the current one: nothing to enter where it already is."""
+    return _HERE if torch.cuda.current_device() == device.index else torch.cuda.device(device)
 
 
 def _ptr(t):
@@ -66,7 +89,7 @@ def _analyze_csr(indices, indptr, n_rows):
     syncs, spmv_csr.py:404-427); returns CsrStats."""
     L = _lib.lib()
     stats = torch.empty(8, dtype=torch.int64, device=indptr.device)
-    with torch.cuda.device(indptr.device):
+    with _on_device(indptr.device):
         rc = L.fsb_csr_analyze(
             _ITYPE[indices.dtype], _ITYPE[indptr.dtype], _ptr(indices), indptr.data_ptr(),
             n_rows, indices.numel(), stats.data_ptr(), _stream_ptr(indptr.device),
@@ -80,7 +103,7 @@ def _tile_plan(indptr, n_rows, nnz, tile_nnz):
     L = _lib.lib()
     n_tiles = int(L.fsb_csr_num_tiles(nnz, tile_nnz))
     plan = torch.empty(n_tiles + 1, dtype=torch.int32, device=indptr.device)
-    with torch.cuda.device(indptr.device):
+    with _on_device(indptr.device):
         rc = L.fsb_csr_tile_plan(
             _ITYPE[indptr.dtype], indptr.data_ptr(), n_rows, nnz, tile_nnz, plan.data_ptr(),
             _stream_ptr(indptr.device),

@@ -18,7 +18,7 @@ import time
 import torch
 
 from ._common import SUPPORTED_INDEX_DTYPES, _INDEX_LIMIT_INT32, _check_value_dtype
-from .spmm_csr import _alg1_shape, _check_out, _run_spmm, prepare_spmm_csr_opt
+from .spmm_csr import _alg1_shape, _check_out, _prepare_spmm, _run_spmm
 from .spmv_csr import _prepare_spmv_csr, _spmv_launch
 
 
@@ -265,6 +265,5 @@ def flagsparse_spmm_coo(data, row, col, B, shape, block_n=None, block_nnz=256, o
     # Grouped by row is all the product needs: a stable sort of 32-bit row ids (four passes) instead of one of the
     # combined 64-bit key (eight); entries of a row are added in the caller's order, the same on every call
     row_s, order = torch.sort(row64.to(torch.int32), stable=True)
-    prepared = prepare_spmm_csr_opt(data[order], col64[order].to(torch.int32), _row_pointer(row_s, n_rows),
-                                    (n_rows, n_cols))
+    prepared = _prepare_spmm(data[order], col64[order], _row_pointer(row_s, n_rows), (n_rows, n_cols), once=True)
     return _run_spmm(prepared, B.contiguous(), out, return_time)

@@ -12,7 +12,7 @@ import time
 import torch
 
 from . import _lib
-from ._common import _VTYPE, _stream_ptr
+from ._common import _VTYPE, _on_device, _stream_ptr
 
 SUPPORTED_SDDMM_VALUE_DTYPES = (torch.float32, torch.float64)
 
@@ -140,7 +140,7 @@ def _sddmm_launch(prepared, x, y, data, alpha, beta, out):
     """Enqueue the product on the current stream; `out` may be a strided-free 1-D tensor only (contiguous)."""
     p = prepared
     dev = x.device
-    with torch.cuda.device(dev):
+    with _on_device(dev):
         rc = _lib.lib().fsb_sddmm_csr(
             _VTYPE[x.dtype], p.indices.data_ptr(), p.row_ids.data_ptr(), x.data_ptr(), x.stride(0), y.data_ptr(),
             y.stride(0), None if data is None else data.data_ptr(), out.data_ptr(), p.n_rows, p.n_cols, p.nnz,

@@ -21,6 +21,7 @@ from ._common import (
     _VTYPE,
     _analyze_csr,
     _check_value_dtype,
+    _on_device,
     _ptr,
     StatusWord,
     _stream_ptr,
@@ -88,7 +89,7 @@ def split_by_column_panels(data, indices, indptr, n_rows, n_cols, n_panels):
     return out
 
 
-def _prepare_spmm_csr_matrix(data, indices, indptr, shape):
+def _prepare_spmm_csr_matrix(data, indices, indptr, shape, narrow=True):
     """Checks of the reference's function of this name (spmm_csr.py:197-255), in its order.  Returns
     (data, kernel_indices, kernel_indptr, n_rows, n_cols, stats); unlike the reference the indptr keeps
     its 32-bit width when it has one (the kernels read either)."""
@@ -129,7 +130,10 @@ def _prepare_spmm_csr_matrix(data, indices, indptr, shape):
             raise IndexError("indices out of range for n_cols")
         if stats.max_index > _INDEX_LIMIT_INT32:
             raise ValueError("column indices exceed the int32 range supported by the kernel")
-    kernel_indices = indices.to(torch.int32) if indices.dtype == torch.int64 else indices
+    # a product that uses the matrix once (narrow=False) reads 64-bit indices as they are: the kernels take either, and a
+    # pass that narrows them moves more than it saves
+    keep = indices.dtype == torch.int32 or (not narrow and data.dtype in _VTYPE)
+    kernel_indices = indices if keep else indices.to(torch.int32)
     return data, kernel_indices, indptr, n_rows, n_cols, stats
 
 
@@ -198,6 +202,11 @@ def _select_spmm_opt_block_n(n_dense_cols):
     return 128
 
 
+_SPLIT_TABLES = {"long_part_rows": (0, torch.int32), "long_part_starts": (0, torch.int64),
+                 "long_part_ends": (0, torch.int64), "long_row_ids": (0, torch.int32),
+                 "long_row_part_ptr": (1, torch.int64)}
+
+
 class PreparedCsrSpmmOpt:
     """Cached CSR metadata for repeated SpMM calls on the same sparse matrix.
 
@@ -211,12 +220,11 @@ class PreparedCsrSpmmOpt:
         "data", "kernel_indices", "kernel_indptr", "shape", "n_rows", "n_cols", "max_row_nnz",
         "row_buckets", "supports_opt", "long_part_rows", "long_part_starts", "long_part_ends",
         "long_row_ids", "long_row_part_ptr", "long_row_fallback_only", "stats", "tile_nnz", "tile_row",
-        "_scratch", "_status", "_row_lengths", "wide", "_whole", "_panels", "_span",
+        "_scratch", "_status", "_row_lengths", "wide", "_whole", "_panels", "_span", "_once",
     )
 
     def __init__(self, data, kernel_indices, kernel_indptr, shape, n_rows, n_cols, stats, tile_nnz, tile_row,
                  wide=None):
-        dev = data.device
         self.data = data
         self.kernel_indices = kernel_indices
         self.kernel_indptr = kernel_indptr
@@ -231,19 +239,24 @@ class PreparedCsrSpmmOpt:
         self.row_buckets = [{"kind": "tiles", "tile_nnz": tile_nnz, "n_tiles": n_tiles, "n_rows": self.n_rows}]
         self._scratch = None
         self.supports_opt = data.dtype in (torch.float32, torch.float64)
-        self.long_part_rows = torch.empty((0,), dtype=torch.int32, device=dev)
-        self.long_part_starts = torch.empty((0,), dtype=torch.int64, device=dev)
-        self.long_part_ends = torch.empty((0,), dtype=torch.int64, device=dev)
-        self.long_row_ids = torch.empty((0,), dtype=torch.int32, device=dev)
-        self.long_row_part_ptr = torch.zeros(1, dtype=torch.int64, device=dev)
         self.long_row_fallback_only = False
         self._status = None
         self._row_lengths = None
+        self._once = False
         self._whole = None       # the matrix as one _CsrPart (shares the tile plan)
         self._panels = {}        # number of column panels -> list of _CsrPart
         self._span = None        # columns spanned by a window of consecutive entries (median over samples)
         # float16 / bfloat16 / complex values: ("native", []) -- the product goes through fsb_spmm_csr_wide
         self.wide = wide
+
+    def __getattr__(self, name):
+        # the reference's tables of split rows, always empty here: made when somebody looks at them
+        if name in _SPLIT_TABLES:
+            n, dtype = _SPLIT_TABLES[name]
+            value = torch.zeros(n, dtype=dtype, device=self.data.device)
+            setattr(self, name, value)
+            return value
+        raise AttributeError(f"{type(self).__name__!r} object has no attribute {name!r}")
 
     @property
     def row_lengths(self):
@@ -339,8 +352,14 @@ class PreparedCsrSpmmOpt:
 
 def prepare_spmm_csr_opt(data, indices, indptr, shape):
     """Analyse a CSR matrix once for repeated SpMM calls (reference: spmm_csr.py:480-522)."""
+    return _prepare_spmm(data, indices, indptr, shape, once=False)
+
+
+def _prepare_spmm(data, indices, indptr, shape, once):
+    """once: for a single product -- 64-bit indices stay, and the tiles are staged by ordinary loads, which have no
+    wait that could run out and so need no status word (a page-locked allocation and an event)."""
     data, kernel_indices, kernel_indptr, n_rows, n_cols, stats = _prepare_spmm_csr_matrix(
-        data, indices, indptr, shape
+        data, indices, indptr, shape, narrow=not once
     )
     nnz = data.numel()
     if data.dtype in widetypes.WIDE_DTYPES:
@@ -351,7 +370,9 @@ def prepare_spmm_csr_opt(data, indices, indptr, shape):
     if nnz > 0 and n_rows > 0:
         tile_nnz = int(_lib.lib().fsb_spmm_tile_nnz(_VTYPE[data.dtype]))
         tile_row = _tile_plan(kernel_indptr, n_rows, nnz, tile_nnz)
-    return PreparedCsrSpmmOpt(data, kernel_indices, kernel_indptr, shape, n_rows, n_cols, stats, tile_nnz, tile_row)
+    prepared = PreparedCsrSpmmOpt(data, kernel_indices, kernel_indptr, shape, n_rows, n_cols, stats, tile_nnz, tile_row)
+    prepared._once = once
+    return prepared
 
 
 def _spmm_launch(prepared, B, C):
@@ -365,15 +386,19 @@ def _spmm_launch(prepared, B, C):
     if p.n_rows == 0 or n_dense == 0:
         return
     algo = _SPMM_ALGO_NAMES.get(os.environ.get("FSB_SPMM_ALGO", "auto").strip().lower(), _lib.FSB_SPMM_AUTO)
-    status = p.status_word()
-    status.poll()
+    status = None
+    if p._once and algo == _lib.FSB_SPMM_AUTO:
+        algo = _lib.FSB_SPMM_PLAIN
+    else:
+        status = p.status_word()
+        status.poll()
     if p.max_row_nnz > LONG_ROW_NNZ:
         algo |= _lib.FSB_SPMM_LONG_ROWS
     sv = B.element_size()
     vt, it, pt = _VTYPE[p.data.dtype], _ITYPE[p.kernel_indices.dtype], _ITYPE[p.kernel_indptr.dtype]
     ldb, ldc = B.stride(0), C.stride(0)
     stream = _stream_ptr(dev)
-    with torch.cuda.device(dev):
+    with _on_device(dev):
         for part, c0, width, accumulate in p.passes_for(n_dense):
             scratch = part.scratch_for(width) if part.tile_row is not None else None
             rc = L.fsb_spmm_csr(
@@ -382,10 +407,11 @@ def _spmm_launch(prepared, B, C):
                 part.data.numel(), algo | (_lib.FSB_SPMM_ACCUMULATE if accumulate else 0),
                 None if part.tile_row is None else part.tile_row.data_ptr(),
                 None if scratch is None else scratch.data_ptr(), 0 if scratch is None else scratch.numel(),
-                status.data_ptr(), stream,
+                None if status is None else status.data_ptr(), stream,
             )
             _lib.check(rc, "fsb_spmm_csr")
-    status.posted("fsb_spmm_csr")
+    if status is not None:
+        status.posted("fsb_spmm_csr")
 
 
 def _check_out(out, device, shape, dtype, device_msg):
@@ -407,7 +433,7 @@ def _spmm_launch_wide(prepared, B, C):
     dev = p.data.device
     if p.n_rows == 0 or B.shape[1] == 0:
         return
-    with torch.cuda.device(dev):
+    with _on_device(dev):
         rc = _lib.lib().fsb_spmm_csr_wide(
             _WIDE_VTYPE[p.data.dtype], _ITYPE[p.kernel_indptr.dtype], _ptr(p.data), _ptr(p.kernel_indices),
             p.kernel_indptr.data_ptr(), _ptr(B), B.stride(0) if B.shape[0] > 1 else B.shape[1], _ptr(C), C.stride(0),
@@ -427,7 +453,7 @@ def _spmm_launch_stored(prepared, B, C):
     L = _lib.lib()
     vt = _STORED_VTYPE[p.data.dtype]
     scratch = torch.empty(int(L.fsb_spmm_stored_scratch_bytes(vt, nnz, n_dense)), dtype=torch.uint8, device=dev)
-    with torch.cuda.device(dev):
+    with _on_device(dev):
         rc = L.fsb_spmm_csr_stored(
             vt, _ITYPE[p.kernel_indptr.dtype], _ptr(p.data), _ptr(p.kernel_indices), p.kernel_indptr.data_ptr(),
             _ptr(B), B.stride(0) if B.shape[0] > 1 else n_dense, C.data_ptr(), n_dense, p.n_rows, p.n_cols, n_dense, nnz,
@@ -494,7 +520,7 @@ def flagsparse_spmm_csr(data, indices, indptr, B, shape, block_n=None, block_nnz
         raise ValueError("max_segments must be positive when provided")
     if B.ndim != 2:
         raise ValueError("B must be a 2D dense tensor")
-    prepared = prepare_spmm_csr_opt(data, indices, indptr, shape)
+    prepared = _prepare_spmm(data, indices, indptr, shape, once=True)
     B = _check_spmm_dense(B, prepared.data, prepared.n_cols)
     n_dense_cols = int(B.shape[1])
     _check_launch_overrides(n_dense_cols, prepared.max_row_nnz, block_n=block_n, block_nnz=block_nnz,
@@ -513,7 +539,7 @@ def flagsparse_spmm_csr_opt(data=None, indices=None, indptr=None, B=None, shape=
     if prepared is None:
         if any(arg is None for arg in (data, indices, indptr, shape)):
             raise ValueError("data, indices, indptr, and shape are required when prepared is not provided")
-        prepared = prepare_spmm_csr_opt(data, indices, indptr, shape)
+        prepared = _prepare_spmm(data, indices, indptr, shape, once=True)
     elif shape is not None:
         resolved_shape = (int(shape[0]), int(shape[1]))
         if resolved_shape != prepared.shape:

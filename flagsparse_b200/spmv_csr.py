@@ -20,6 +20,7 @@ from ._common import (
     _VTYPE,
     _analyze_csr,
     _check_value_dtype,
+    _on_device,
     _ptr,
     _stream_ptr,
     _tile_plan,
@@ -150,9 +151,11 @@ class PreparedCsrSpmv:
             word.check()
 
 
-def _prepare_spmv_csr_matrix(data, indices, indptr, shape):
+def _prepare_spmv_csr_matrix(data, indices, indptr, shape, narrow=True):
     """Validate and normalise the CSR arrays; same checks, order and exception types as the reference's
-    function of this name (spmv_csr.py:379-436).  Returns (data, kernel_indices, kernel_indptr, n_rows,
+    function of this name (spmv_csr.py:379-436).  narrow=False leaves the indices of float32 / float64 matrices at their
+    width (a one-shot product reads them once: the kernels take either, and a pass that narrows them moves more than it
+    saves).  Returns (data, kernel_indices, kernel_indptr, n_rows,
     n_cols, stats)."""
     if not all(torch.is_tensor(t) for t in (data, indices, indptr)):
         raise TypeError("data, indices and indptr have to be torch.Tensor objects")
@@ -189,6 +192,8 @@ def _prepare_spmv_csr_matrix(data, indices, indptr, shape):
             raise IndexError(f"column indices span [{stats.min_index}, {stats.max_index}], the matrix has {n_cols} columns")
         if stats.max_index > _INDEX_LIMIT_INT32:
             raise ValueError(f"int64 column index {stats.max_index} exceeds the int32 kernel range")
+    if not narrow and data.dtype in _VTYPE:
+        return data, indices, indptr, n_rows, n_cols, stats
     # same narrowing as the reference (:422-425): 32-bit column indices always, 32-bit indptr when it fits
     kernel_indices = indices.to(torch.int32) if indices.dtype == torch.int64 else indices
     kernel_indptr = indptr.to(torch.int32) if nnz <= _INDEX_LIMIT_INT32 else indptr.to(torch.int64)
@@ -201,6 +206,8 @@ def _validate_spmv_x(x, prepared):
     if not torch.is_tensor(x):            # None included
         raise TypeError("x has to be a torch.Tensor")
     a = prepared.data
+    if x.ndim == 1 and x.is_cuda and x.dtype == a.dtype and x.shape[0] == prepared.n_cols and x.device == a.device:
+        return x.contiguous()
     for failed, exc, why in (
         (x.ndim != 1, ValueError, "x has to be one-dimensional"),
         (not x.is_cuda, ValueError, "x has to live on a CUDA device"),
@@ -243,7 +250,7 @@ def _prepare_spmv_csr(data, indices, indptr, shape, block_nnz, max_segments, reu
     """reuse_expected=False (a one-shot product) skips the panel regrouping, which costs about as much as a
     hundred products and only pays when the prepared matrix is used again."""
     data, kernel_indices, kernel_indptr, n_rows, n_cols, stats = _prepare_spmv_csr_matrix(
-        data, indices, indptr, shape
+        data, indices, indptr, shape, narrow=reuse_expected
     )
     max_row_nnz = stats.max_row_nnz
     block_nnz_use, max_segments_use = _resolve_block_nnz(max_row_nnz, block_nnz, max_segments)
@@ -251,19 +258,15 @@ def _prepare_spmv_csr(data, indices, indptr, shape, block_nnz, max_segments, reu
     if data.dtype in widetypes.WIDE_DTYPES:
         # float16 / bfloat16 / complex values are read as they are stored by kernels of their own (fsb_spmv_csr_stored):
         # no second copy of the matrix, and a tile plan where the row lengths call for one
-        tile_nnz, tile_row, scratch = 0, None, None
-        if (nnz > 0 and n_rows > 0 and data.device.type == "cuda"
-                and _uneven_rows(n_rows, nnz, max_row_nnz)):
-            L = _lib.lib()
-            tile_nnz = int(L.fsb_spmv_stored_tile_nnz(_WIDE_VTYPE[data.dtype]))
+        tile_nnz, tile_row = 0, None
+        if nnz > 0 and n_rows > 0 and data.device.type == "cuda" and _uneven_rows(n_rows, nnz, max_row_nnz):
+            tile_nnz = int(_lib.lib().fsb_spmv_stored_tile_nnz(_WIDE_VTYPE[data.dtype]))
             tile_row = _tile_plan(kernel_indptr, n_rows, nnz, tile_nnz)
-            scratch = torch.empty(int(L.fsb_spmv_stored_scratch_bytes(_WIDE_VTYPE[data.dtype], nnz)),
-                                  dtype=torch.uint8, device=data.device)
         return PreparedCsrSpmv(
             data=data, kernel_indices=kernel_indices, kernel_indptr=kernel_indptr, shape=shape, n_rows=n_rows,
             n_cols=n_cols, block_nnz=block_nnz_use, max_segments=max_segments_use, max_row_nnz=max_row_nnz,
             stats=stats, algo=_lib.FSB_SPMV_VECTOR if tile_row is None else _lib.FSB_SPMV_STREAM, tuning=0,
-            tile_nnz=tile_nnz, tile_row=tile_row, scratch=scratch, wide=("native", []),
+            tile_nnz=tile_nnz, tile_row=tile_row, scratch=None, wide=("native", []),
         )
     algo = _select_spmv_algo(n_rows, nnz, max_row_nnz)
     tuning = int(os.environ.get("FSB_SPMV_TUNING", "0"))
@@ -309,7 +312,7 @@ def _spmv_launch(prepared, x, y):
     if p.algo == _lib.FSB_SPMV_PANEL and p.panel is not None:
         from . import panel
 
-        with torch.cuda.device(dev):
+        with _on_device(dev):
             panel.launch_panel(p.panel, x, y, p.n_rows, p.n_cols, _stream_ptr(dev))
         return
     if p.long_rows is not None:
@@ -317,20 +320,24 @@ def _spmv_launch(prepared, x, y):
 
         short, layout = p.long_rows
         _spmv_launch(short, x, y)      # every row of y; the long rows get zeros here
-        with torch.cuda.device(dev):
+        with _on_device(dev):
             longrows.launch_long_rows(layout, x, y, p.n_cols, _stream_ptr(dev))
         return
     algo = p.algo if p.tile_row is not None else _lib.FSB_SPMV_VECTOR
+    # calls on a small matrix may overlap in several streams, whichever kernel its rows get: scratch of the call's own
+    scratch = p.scratch
+    if scratch is not None and p.data.numel() < _STREAM_MIN_NNZ:
+        scratch = torch.empty_like(scratch)
     lanes = p.tuning & 0xFF
     tuning = p.tuning if algo == _lib.FSB_SPMV_STREAM else (lanes if lanes in (2, 4, 8, 16, 32) else 0)
-    with torch.cuda.device(dev):
+    with _on_device(dev):
         rc = L.fsb_spmv_csr(
             _VTYPE[p.data.dtype], _ITYPE[p.kernel_indices.dtype], _ITYPE[p.kernel_indptr.dtype],
             _ptr(p.data), _ptr(p.kernel_indices), p.kernel_indptr.data_ptr(), _ptr(x), _ptr(y),
             p.n_rows, p.n_cols, p.data.numel(), algo, tuning,
             None if p.tile_row is None else p.tile_row.data_ptr(),
-            None if p.scratch is None else p.scratch.data_ptr(),
-            0 if p.scratch is None else p.scratch.numel(), _stream_ptr(dev),
+            None if scratch is None else scratch.data_ptr(),
+            0 if scratch is None else scratch.numel(), _stream_ptr(dev),
         )
     _lib.check(rc, "fsb_spmv_csr")
 
@@ -343,7 +350,7 @@ def _spmv_launch_wide(prepared, x, y):
     dev = p.data.device
     if p.n_rows == 0:
         return
-    with torch.cuda.device(dev):
+    with _on_device(dev):
         rc = _lib.lib().fsb_spmv_csr_wide(
             _WIDE_VTYPE[p.data.dtype], _ITYPE[p.kernel_indptr.dtype], _ptr(p.data), _ptr(p.kernel_indices),
             p.kernel_indptr.data_ptr(), _ptr(x), _ptr(y), p.n_rows, p.n_cols, p.data.numel(), _stream_ptr(dev),
@@ -357,12 +364,17 @@ def _spmv_launch_stored(prepared, x, y):
     dev = p.data.device
     if p.n_rows == 0:
         return
-    with torch.cuda.device(dev):
-        rc = _lib.lib().fsb_spmv_csr_stored(
+    L = _lib.lib()
+    scratch = None
+    if p.tile_row is not None:       # the call's own: calls on one matrix may overlap in several streams
+        scratch = torch.empty(int(L.fsb_spmv_stored_scratch_bytes(_WIDE_VTYPE[p.data.dtype], p.data.numel())),
+                              dtype=torch.uint8, device=dev)
+    with _on_device(dev):
+        rc = L.fsb_spmv_csr_stored(
             _WIDE_VTYPE[p.data.dtype], _ITYPE[p.kernel_indptr.dtype], _ptr(p.data), _ptr(p.kernel_indices),
             p.kernel_indptr.data_ptr(), _ptr(x), _ptr(y), p.n_rows, p.n_cols, p.data.numel(),
-            None if p.tile_row is None else p.tile_row.data_ptr(), _ptr(p.scratch),
-            0 if p.scratch is None else p.scratch.numel(), _stream_ptr(dev),
+            None if p.tile_row is None else p.tile_row.data_ptr(), _ptr(scratch),
+            0 if scratch is None else scratch.numel(), _stream_ptr(dev),
         )
     _lib.check(rc, "fsb_spmv_csr_stored")
 
