@@ -1,17 +1,22 @@
 // CSR SpMV and SpMM for the value types the float32 / float64 kernels do not stream themselves: float16 and bfloat16
-// values (2 bytes per entry in memory, products and sums in float32, the dense operand and the result in float32: the
-// caller widens x / B once per call and rounds y / C once, as the reference's base path does) and complex64 /
-// complex128 values (interleaved real and imaginary parts, one pass over the matrix, complex multiply-add in the
-// component precision).  The values are read as they are stored -- no widened or split copy of the matrix exists
-// anywhere.  Rows are summed in a fixed order: bit-reproducible.
+// values (2 bytes per entry in memory, products and sums in float32) and complex64 / complex128 values (interleaved real
+// and imaginary parts, one pass over the matrix, complex multiply-add in the component precision).  The values are read
+// as they are stored -- no widened or split copy of the matrix exists anywhere.  Rows are summed in a fixed order:
+// bit-reproducible.
 //
-// SpMV: L lanes per row (L = 2 .. 32 from the mean row length), every lane walks the row with stride L, two partial
-// sums, a shuffle tree, lane 0 stores.  SpMM: a group of LN lanes per row (LN = dense width rounded up to a power of
-// two, at most 32; wider B in column tiles of 32 along gridDim.y), every lane owns one column of C, walks the row's
-// entries (value and column index are the same address for the whole group: one broadcast load) and gathers its
-// element of B's row, two entries in flight.
+// fsb_spmv_csr_stored (second half of this file): x and y in the matrix's own type too; lanes per row for even rows, tiles
+// for uneven ones.  SpMM with operands as stored runs through the tiled kernel of spmm_csr.cu.
+//
+// fsb_spmv_csr_wide / fsb_spmm_csr_wide: one launch without scratch, dense operand and result in float32 for the half
+// precisions (the caller widens x / B once per call and rounds y / C once, as the reference's base path does).  SpMV: L
+// lanes per row (L = 2 .. 32 from the mean row length), every lane walks the row with stride L, two partial sums, a
+// shuffle tree, lane 0 stores.  SpMM: a group of LN lanes per row (LN = dense width rounded up to a power of two, at most
+// 32; wider B in column tiles of 32 along gridDim.y), every lane owns one column of C, walks the row's entries (value and
+// column index are the same address for the whole group: one broadcast load) and gathers its element of B's row, two
+// entries in flight.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
+#include <string.h>
 
 #include "fsb_common.cuh"
 
