@@ -107,6 +107,15 @@ __device__ __forceinline__ void st_dense_stream(V* p, const V (&v)[VW]) {
   __stcs(reinterpret_cast<VT*>(p), t);
 }
 
+// Neumaier-compensated running sum in double: exact enough for every value type whatever the number of terms.  The total is
+// sum + comp_term(sum, comp): once the sum is infinite or NaN it stays so, and comp, inf - inf by then, must not be added.
+__device__ __forceinline__ void comp_add(double& sum, double& comp, double v) {
+  const double s2 = sum + v;
+  comp += (fabs(sum) >= fabs(v)) ? ((sum - s2) + v) : ((v - s2) + sum);
+  sum = s2;
+}
+__device__ __forceinline__ double comp_term(double sum, double comp) { return isfinite(sum) ? comp : 0.0; }
+
 __device__ __forceinline__ int pow2_floor(int v) { return v <= 1 ? 1 : (1 << (31 - __clz(v))); }
 
 }  // namespace fsb

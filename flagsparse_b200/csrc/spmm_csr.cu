@@ -388,13 +388,9 @@ spmm_fixup_kernel(const P* __restrict__ ptr, const int32_t* __restrict__ tile_ro
   if (p >= (t << log2_tile)) return;
   const int64_t t0 = p >> log2_tile;
   double sum = (double)head[t * n_dense + j], comp = 0.0;
-  for (int64_t u = t0; u < t; ++u) {
-    const double v = (double)carry[u * n_dense + j];
-    const double s2 = sum + v;
-    comp += (fabs(sum) >= fabs(v)) ? ((sum - s2) + v) : ((v - s2) + sum);
-    sum = s2;
-  }
+  for (int64_t u = t0; u < t; ++u) comp_add(sum, comp, (double)carry[u * n_dense + j]);
   D* dst = C + (int64_t)ra * ldc + j;
+  comp = comp_term(sum, comp);
   // rounded to the accumulator type first, like every other row
   const R r = accumulate ? (R)(((double)MmOps<D>::widen(*dst) + sum) + comp) : (R)(sum + comp);
   *dst = MmOps<D>::narrow(r);

@@ -346,13 +346,6 @@ spmv_stream_kernel(const V* __restrict__ data, const I* __restrict__ idx, const 
   }
 }
 
-// Neumaier-compensated running sum in double: exact enough for either value type whatever the row length
-__device__ __forceinline__ void comp_add(double& sum, double& comp, double v) {
-  const double s2 = sum + v;
-  comp += (fabs(sum) >= fabs(v)) ? ((sum - s2) + v) : ((v - s2) + sum);
-  sum = s2;
-}
-
 constexpr int kFixupSerial = 32;   // a row that crossed more tiles than this is summed by its whole warp
 
 // one thread per tile t >= 1: if the first row written by tile t started in an earlier tile, finish it.
