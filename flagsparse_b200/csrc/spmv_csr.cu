@@ -375,7 +375,7 @@ spmv_fixup_kernel(const P* __restrict__ ptr, const int32_t* __restrict__ tile_ro
   if (need && !wide) {
     double sum = (double)head[t], comp = 0.0;
     for (int64_t u = t0; u < t; ++u) comp_add(sum, comp, (double)carry[u]);
-    out.store((int64_t)ra, (V)(sum + comp));
+    out.store((int64_t)ra, (V)(sum + comp_term(sum, comp)));
   }
   unsigned todo = __ballot_sync(0xffffffffu, wide);
   while (todo) {
@@ -396,7 +396,7 @@ spmv_fixup_kernel(const P* __restrict__ ptr, const int32_t* __restrict__ tile_ro
     comp = __shfl_sync(0xffffffffu, comp, 0);
     if (lane == src) {
       comp_add(sum, comp, (double)head[t]);
-      out.store((int64_t)ra, (V)(sum + comp));
+      out.store((int64_t)ra, (V)(sum + comp_term(sum, comp)));
     }
   }
 }

@@ -6,6 +6,7 @@ import pytest
 import torch
 
 import flagsparse_b200 as fs
+from gpu_util import env
 from helpers import handmade_csr
 
 pytestmark = pytest.mark.gpu
@@ -64,3 +65,32 @@ def test_spmm(cuda, fsb_lib, dtype, plant):
             if dtype in (torch.float32, torch.float64):
                 prep = fs.prepare_spmm_csr_opt(*args, shape)
                 _check(fs.flagsparse_spmm_csr_opt(B=B.to(cuda), prepared=prep), vals, i, p, B)
+
+
+@pytest.mark.parametrize("dtype", DTYPES, ids=str)
+@pytest.mark.parametrize("plant", sorted(PLANTS))
+def test_spmv(cuda, fsb_lib, dtype, plant):
+    shape = (len(LENS), N_COLS)
+    for at in (0, 1):
+        vals, i, p = _matrix(dtype, plant, at)
+        args = [t.to(cuda) for t in (vals, torch.from_numpy(i), torch.from_numpy(p))]
+        x = _operand((N_COLS,), dtype)
+        for algo in (None, "vector", "stream") if dtype in (torch.float32, torch.float64) else (None,):
+            with env(FSB_SPMV_ALGO=algo):
+                _check(fs.flagsparse_spmv_csr(*args, x.to(cuda), shape), vals, i, p, x)
+                prep = fs.prepare_spmv_csr(*args, shape)
+                _check(fs.flagsparse_spmv_csr(x=x.to(cuda), prepared=prep), vals, i, p, x)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64], ids=str)
+@pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan])
+def test_spmv_row_of_many_tiles(cuda, fsb_lib, dtype, value):
+    """A row across more tiles than one thread of the fix-up adds up by itself (its warp does, lane by lane)."""
+    _, i, p = handmade_csr(8, [7, 150000, 9], 200000)
+    x = _operand((200000,), dtype)
+    for at in (7, 60000, 150006):
+        vals = torch.from_numpy(np.random.default_rng(9).uniform(-1, 1, i.size)).to(dtype)
+        vals[at] = value
+        y = fs.flagsparse_spmv_csr(vals.to(cuda), torch.from_numpy(i).to(cuda), torch.from_numpy(p).to(cuda), x.to(cuda),
+                                   (3, 200000))
+        _check(y, vals, i, p, x)
