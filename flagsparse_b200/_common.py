@@ -69,6 +69,12 @@ def _on_device(device):
     return _HERE if torch.cuda.current_device() == device.index else torch.cuda.device(device)
 
 
+def _resolved(t):
+    """t with the conjugation or negation that torch keeps as a flag of the tensor (x.conj(), z.conj().imag) carried out:
+    the kernels read the memory, and contiguous() leaves the flag as it is."""
+    return t.resolve_conj().resolve_neg() if t.is_conj() or t.is_neg() else t
+
+
 def _ptr(t):
     return t.data_ptr() if t is not None and t.numel() > 0 else None
 

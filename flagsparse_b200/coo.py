@@ -17,7 +17,7 @@ import time
 
 import torch
 
-from ._common import SUPPORTED_INDEX_DTYPES, _INDEX_LIMIT_INT32, _check_value_dtype
+from ._common import SUPPORTED_INDEX_DTYPES, _INDEX_LIMIT_INT32, _check_value_dtype, _resolved
 from .spmm_csr import _alg1_shape, _check_out, _prepare_spmm, _run_spmm
 from .spmv_csr import _prepare_spmv_csr, _spmv_launch
 
@@ -94,6 +94,7 @@ def _prepare_coo_tensors(data, row, col, shape, sort_by_row, reuse_expected):
         raise ValueError(f"{data.numel()} values, {row.numel()} row ids, {col.numel()} column ids: the counts differ")
     if data.dtype not in (torch.float32, torch.float64):
         raise TypeError(f"COO SpMV takes float32 or float64 values, not {data.dtype} (the CSR entry points take more)")
+    data = _resolved(data)
     row64 = row.to(torch.int64)
     col64 = col.to(torch.int64)
     _check_index_range(row64, col64, n_rows, n_cols)
@@ -161,7 +162,7 @@ def flagsparse_spmv_coo(data=None, row=None, col=None, x=None, shape=None, out=N
     dev, dtype = prepared.data.device, prepared.data.dtype
     if out is not None and (out.shape != (prepared.n_rows,) or out.dtype != dtype):
         raise ValueError("out shape/dtype must match result")
-    direct = out is not None and out.is_cuda and out.device == dev and out.is_contiguous()
+    direct = out is not None and out.is_cuda and out.device == dev and out.is_contiguous() and not out.is_neg()
     y = out if direct else torch.empty(prepared.n_rows, dtype=dtype, device=dev)
     t0 = None
     if return_time:
@@ -225,7 +226,7 @@ def _prepare_spmm_coo_inputs(data, row, col, B, shape):
             raise ValueError("row indices exceed the int32 range supported by the kernels")
         if max_col > _INDEX_LIMIT_INT32:
             raise ValueError("column indices exceed the int32 range supported by the kernels")
-    return data.contiguous(), row64, col64, n_rows, n_cols, int(B.shape[1])
+    return _resolved(data).contiguous(), row64, col64, n_rows, n_cols, int(B.shape[1])
 
 
 def _resolve_spmm_coo_launch_config(n_dense_cols, nnz, block_n=None, block_nnz=256):
@@ -266,4 +267,4 @@ def flagsparse_spmm_coo(data, row, col, B, shape, block_n=None, block_nnz=256, o
     # combined 64-bit key (eight); entries of a row are added in the caller's order, the same on every call
     row_s, order = torch.sort(row64.to(torch.int32), stable=True)
     prepared = _prepare_spmm(data[order], col64[order], _row_pointer(row_s, n_rows), (n_rows, n_cols), once=True)
-    return _run_spmm(prepared, B.contiguous(), out, return_time)
+    return _run_spmm(prepared, _resolved(B).contiguous(), out, return_time)

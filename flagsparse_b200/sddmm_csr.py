@@ -12,7 +12,7 @@ import time
 import torch
 
 from . import _lib
-from ._common import _VTYPE, _on_device, _stream_ptr
+from ._common import _VTYPE, _on_device, _resolved, _stream_ptr
 
 SUPPORTED_SDDMM_VALUE_DTYPES = (torch.float32, torch.float64)
 
@@ -130,6 +130,7 @@ def _resolve_out(prepared, x, out):
 
 def _unit_rows(t):
     """t as the kernel reads it: unit stride along a row, any stride between rows."""
+    t = _resolved(t)
     if t.shape[1] <= 1 or t.stride(1) == 1:
         if t.shape[0] <= 1 or t.stride(0) >= t.shape[1]:
             return t
@@ -183,12 +184,13 @@ def flagsparse_sddmm_csr(data=None, indices=None, indptr=None, x=None, y=None, s
             else:
                 result.copy_(data * beta)
     else:
-        target = result if result.is_contiguous() else torch.empty_like(result, memory_format=torch.contiguous_format)
+        direct = result.is_contiguous() and not result.is_neg()
+        target = result if direct else torch.empty_like(result, memory_format=torch.contiguous_format)
         if return_time:
             torch.cuda.synchronize(x.device)
             t0 = time.perf_counter()
-        _sddmm_launch(prepared, _unit_rows(x), _unit_rows(y), None if data is None else data.contiguous(), alpha,
-                      beta, target)
+        _sddmm_launch(prepared, _unit_rows(x), _unit_rows(y), None if data is None else _resolved(data).contiguous(),
+                      alpha, beta, target)
         if return_time:
             torch.cuda.synchronize(x.device)
             elapsed_ms = (time.perf_counter() - t0) * 1000.0

@@ -23,6 +23,7 @@ from ._common import (
     _check_value_dtype,
     _on_device,
     _ptr,
+    _resolved,
     StatusWord,
     _stream_ptr,
     _tile_plan,
@@ -114,7 +115,7 @@ def _prepare_spmm_csr_matrix(data, indices, indptr, shape, narrow=True):
     if indptr.dtype not in SUPPORTED_INDEX_DTYPES:
         raise TypeError("indptr dtype must be torch.int32 or torch.int64")
 
-    data = data.contiguous()
+    data = _resolved(data).contiguous()
     indices = indices.contiguous()
     indptr = indptr.contiguous()
     nnz = data.numel()
@@ -153,6 +154,7 @@ def _check_spmm_dense(B, data, n_cols):
 def _row_major(B):
     """B as the kernel can read it: unit stride along a row, any stride between rows (the reference copies every
     non-contiguous B, spmm_csr.py:280; a row-strided view needs no copy here)."""
+    B = _resolved(B)
     if B.shape[1] <= 1 or B.stride(1) == 1:
         if B.shape[0] <= 1 or B.stride(0) >= B.shape[1]:
             return B
@@ -480,7 +482,7 @@ def _run_spmm(prepared, B, out, return_time):
             C = out
         return (C, elapsed_ms) if return_time else C
     # float16 / bfloat16 / complex products never write into `out` while B is still read: it may be B itself there
-    direct = out is not None and out.is_contiguous() and prepared.wide is None
+    direct = out is not None and out.is_contiguous() and not out.is_neg() and prepared.wide is None
     C = out if direct else torch.empty(shape, dtype=dtype, device=dev)
     t0 = None
     if return_time:

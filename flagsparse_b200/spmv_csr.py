@@ -22,6 +22,7 @@ from ._common import (
     _check_value_dtype,
     _on_device,
     _ptr,
+    _resolved,
     _stream_ptr,
     _tile_plan,
 )
@@ -172,7 +173,7 @@ def _prepare_spmv_csr_matrix(data, indices, indptr, shape, narrow=True):
     if indices.dtype not in SUPPORTED_INDEX_DTYPES:
         raise TypeError(f"indices are {indices.dtype}; int32 or int64 is needed")
 
-    data = data.contiguous()
+    data = _resolved(data).contiguous()
     indices = indices.contiguous()
     indptr = indptr.contiguous()
     if indptr.dtype not in SUPPORTED_INDEX_DTYPES:
@@ -207,7 +208,7 @@ def _validate_spmv_x(x, prepared):
         raise TypeError("x has to be a torch.Tensor")
     a = prepared.data
     if x.ndim == 1 and x.is_cuda and x.dtype == a.dtype and x.shape[0] == prepared.n_cols and x.device == a.device:
-        return x.contiguous()
+        return _resolved(x).contiguous()
     for failed, exc, why in (
         (x.ndim != 1, ValueError, "x has to be one-dimensional"),
         (not x.is_cuda, ValueError, "x has to live on a CUDA device"),
@@ -217,7 +218,7 @@ def _validate_spmv_x(x, prepared):
     ):
         if failed:
             raise exc(why)
-    return x.contiguous()
+    return _resolved(x).contiguous()
 
 
 def prepare_spmv_csr(data, indices, indptr, shape, block_nnz=256, max_segments=None):
@@ -416,7 +417,7 @@ def flagsparse_spmv_csr(data=None, indices=None, indptr=None, x=None, shape=None
             y = out
         return (y, elapsed_ms) if return_time else y
     # write straight into `out` when that is safe, else into a fresh vector that is copied over
-    direct = out is not None and out.is_cuda and out.device == dev and out.is_contiguous()
+    direct = out is not None and out.is_cuda and out.device == dev and out.is_contiguous() and not out.is_neg()
     y = out if direct else torch.empty(prepared.n_rows, dtype=dtype, device=dev)
     t0 = None
     if return_time:
