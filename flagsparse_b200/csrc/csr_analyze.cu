@@ -160,6 +160,9 @@ extern "C" int fsb_csr_analyze(int itype, int ptype, const void* indices, const 
   if ((itype != FSB_I32 && itype != FSB_I64) || (ptype != FSB_I32 && ptype != FSB_I64)) return FSB_EINVAL;
   if (n_rows < 0 || nnz < 0 || stats == nullptr || indptr == nullptr) return FSB_EINVAL;
   if (nnz > 0 && indices == nullptr) return FSB_EINVAL;
+  if (!aligned_to(indptr, ptype == FSB_I32 ? 4 : 8) || !aligned_to(indices, itype == FSB_I32 ? 4 : 8) ||
+      !aligned_to(stats, 8))
+    return FSB_EALIGN;
   if (n_rows >= INT32_MAX) return FSB_ERANGE;
   stats_init_kernel<<<1, 1, 0, stream>>>(stats);
   FSB_RETURN_IF_LAUNCH_FAILED();
@@ -194,6 +197,7 @@ extern "C" int fsb_csr_tile_plan(int ptype, const void* indptr, int64_t n_rows, 
   if (ptype != FSB_I32 && ptype != FSB_I64) return FSB_EINVAL;
   if (n_rows < 0 || nnz < 0 || tile_nnz <= 0 || (tile_nnz & (tile_nnz - 1)) != 0) return FSB_EINVAL;
   if (indptr == nullptr || tile_row == nullptr) return FSB_EINVAL;
+  if (!aligned_to(indptr, ptype == FSB_I32 ? 4 : 8) || !aligned_to(tile_row, 4)) return FSB_EALIGN;
   if (n_rows >= INT32_MAX) return FSB_ERANGE;
   const int64_t n_tiles = fsb_csr_num_tiles(nnz, tile_nnz);
   if (n_tiles >= INT32_MAX) return FSB_ERANGE;

@@ -413,6 +413,7 @@ struct SpmmArgs {
   int algo, ptype;
   bool accumulate, long_rows;
   const int32_t* tile_row;
+  int32_t* own_plan;      // the plan has to be made first, here (tile_row is the same address)
   void* scratch;
   int32_t* status;
   cudaStream_t st;
@@ -437,7 +438,13 @@ static int launch_spmm(const SpmmArgs& a, int LR, int piece) {
   const int n_dense = (int)a.n_dense;
   const int width = LR * NC * VW;
   const int64_t col_tiles = (n_dense + width - 1) / width;
-  if (col_tiles > 65535) return FSB_ERANGE;
+  const int cols = n_dense * RealOf<S>::parts;
+  const int64_t fix_blocks = n_tiles > 1 ? ((n_tiles - 1) * cols + kMmThreads - 1) / kMmThreads : 0;
+  if (col_tiles > 65535 || fix_blocks >= INT32_MAX) return FSB_ERANGE;
+  if (a.own_plan != nullptr) {      // the first launch: whatever a call can be refused for has been looked at by now
+    const int rc = fsb_csr_tile_plan(a.ptype, a.ptr, a.n_rows, a.nnz, T, a.own_plan, a.st);
+    if (rc != FSB_OK) return rc;
+  }
   A* carry = (A*)a.scratch;
   A* head = carry + n_tiles * n_dense;
   const int bulk = a.algo != FSB_SPMM_PLAIN && aligned_to(a.data, 16) && aligned_to(a.idx, 16);
@@ -459,15 +466,12 @@ static int launch_spmm(const SpmmArgs& a, int LR, int piece) {
   }
 #undef FSB_SPMM_LAUNCH
   FSB_RETURN_IF_LAUNCH_FAILED();
-  if (n_tiles > 1) {
+  if (fix_blocks > 0) {
     typedef RealOf<S> R;
     int log2_tile = 0;
     while ((1 << log2_tile) < T) ++log2_tile;
-    const int cols = n_dense * R::parts;
-    const int64_t g = ((n_tiles - 1) * cols + kMmThreads - 1) / kMmThreads;
-    if (g >= INT32_MAX) return FSB_ERANGE;
 #define FSB_SPMM_FIXUP(P_)                                                                                          \
-  spmm_fixup_kernel<typename R::Acc, typename R::Out, P_><<<(unsigned)g, kMmThreads, 0, a.st>>>(                   \
+  spmm_fixup_kernel<typename R::Acc, typename R::Out, P_><<<(unsigned)fix_blocks, kMmThreads, 0, a.st>>>(          \
       (const P_*)a.ptr, a.tile_row, (const typename R::Acc*)carry, (const typename R::Acc*)head,                   \
       (typename R::Out*)a.C, a.ldc * R::parts, n_tiles, cols, log2_tile, a.accumulate)
     if (a.ptype == FSB_I64) FSB_SPMM_FIXUP(int64_t); else FSB_SPMM_FIXUP(int32_t);
@@ -551,10 +555,15 @@ static size_t spmm_scratch_bytes(int vtype, int64_t nnz, int64_t n_dense) {
   return (b + 255) & ~(size_t)255;
 }
 
+static size_t spmm_plan_bytes(int64_t nnz) {
+  return (((size_t)fsb_csr_num_tiles(nnz, kMmTile) + 1) * sizeof(int32_t) + 255) & ~(size_t)255;
+}
+
+// plan_in_scratch: no tile_row; the plan is made behind the partial rows, in the last spmm_plan_bytes() of the scratch
 static int spmm_run(int vtype, int itype, int ptype, const void* data, const void* indices, const void* indptr,
                     const void* B, int64_t ldb, void* C, int64_t ldc, int64_t n_rows, int64_t n_cols, int64_t n_dense,
-                    int64_t nnz, int algo, const int32_t* tile_row, void* scratch, size_t scratch_bytes,
-                    int32_t* status, cudaStream_t st) {
+                    int64_t nnz, int algo, const int32_t* tile_row, bool plan_in_scratch, void* scratch,
+                    size_t scratch_bytes, int32_t* status, cudaStream_t st) {
   if ((itype != FSB_I32 && itype != FSB_I64) || (ptype != FSB_I32 && ptype != FSB_I64)) return FSB_EINVAL;
   const bool accumulate = (algo & FSB_SPMM_ACCUMULATE) != 0;
   const bool long_rows = (algo & FSB_SPMM_LONG_ROWS) != 0;
@@ -582,13 +591,15 @@ static int spmm_run(int vtype, int itype, int ptype, const void* data, const voi
   }
   if (data == nullptr || indices == nullptr || B == nullptr || ldb < n_dense) return FSB_EINVAL;
   if (!aligned_to(data, sv) || !aligned_to(B, sv) || !aligned_to(indices, si)) return FSB_EALIGN;
-  if (tile_row == nullptr || scratch == nullptr) return FSB_EINVAL;
-  if (scratch_bytes < spmm_scratch_bytes(vtype, nnz, n_dense)) return FSB_ESCRATCH;
+  if ((tile_row == nullptr && !plan_in_scratch) || scratch == nullptr) return FSB_EINVAL;
+  const size_t parts_bytes = spmm_scratch_bytes(vtype, nnz, n_dense);
+  if (scratch_bytes < parts_bytes + (plan_in_scratch ? spmm_plan_bytes(nnz) : 0)) return FSB_ESCRATCH;
   if (!aligned_to(scratch, 16)) return FSB_EALIGN;
   if (fsb_csr_num_tiles(nnz, kMmTile) >= 65535LL * 32768LL) return FSB_ERANGE;
 
-  SpmmArgs a{data, indices, indptr, B, ldb, C, ldc, n_rows, n_dense, nnz, algo, ptype, accumulate, long_rows, tile_row,
-             scratch, status, st};
+  int32_t* own_plan = plan_in_scratch ? (int32_t*)((char*)scratch + parts_bytes) : nullptr;
+  SpmmArgs a{data, indices, indptr, B, ldb, C, ldc, n_rows, n_dense, nnz, algo, ptype, accumulate, long_rows,
+             plan_in_scratch ? own_plan : tile_row, own_plan, scratch, status, st};
   if (vtype == FSB_F32) return itype == FSB_I32 ? spmm_typed<float, int32_t>(a) : spmm_typed<float, int64_t>(a);
   if (vtype == FSB_F64) return itype == FSB_I32 ? spmm_typed<double, int32_t>(a) : spmm_typed<double, int64_t>(a);
   if (itype != FSB_I32) return FSB_EINVAL;
@@ -618,12 +629,11 @@ extern "C" int fsb_spmm_csr(int vtype, int itype, int ptype, const void* data, c
                             void* stream_) {
   if (vtype != FSB_F32 && vtype != FSB_F64) return FSB_EINVAL;
   return spmm_run(vtype, itype, ptype, data, indices, indptr, B, ldb, C, ldc, n_rows, n_cols, n_dense, nnz, algo,
-                  tile_row, scratch, scratch_bytes, status, static_cast<cudaStream_t>(stream_));
+                  tile_row, false, scratch, scratch_bytes, status, static_cast<cudaStream_t>(stream_));
 }
 
 extern "C" size_t fsb_spmm_stored_scratch_bytes(int vtype, int64_t nnz, int64_t n_dense) {
-  const size_t plan = ((size_t)fsb_csr_num_tiles(nnz, kMmTile) + 1) * sizeof(int32_t);
-  return spmm_scratch_bytes(vtype, nnz, n_dense) + ((plan + 255) & ~(size_t)255);
+  return spmm_scratch_bytes(vtype, nnz, n_dense) + spmm_plan_bytes(nnz);
 }
 
 extern "C" int fsb_spmm_csr_stored(int vtype, int ptype, const void* data, const int32_t* indices, const void* indptr,
@@ -631,21 +641,8 @@ extern "C" int fsb_spmm_csr_stored(int vtype, int ptype, const void* data, const
                                    int64_t n_dense, int64_t nnz, int long_rows, void* scratch, size_t scratch_bytes,
                                    void* stream_) {
   if (vtype != FSB_F16 && vtype != FSB_BF16 && vtype != FSB_C64 && vtype != FSB_C128) return FSB_EINVAL;
-  int32_t* tile_row = nullptr;
-  size_t parts_bytes = 0;
-  if (nnz > 0 && n_rows > 0 && n_dense > 0) {
-    if (n_rows >= INT32_MAX || n_dense >= (1 << 24)) return FSB_ERANGE;
-    if (scratch == nullptr || indptr == nullptr) return FSB_EINVAL;
-    if (scratch_bytes < fsb_spmm_stored_scratch_bytes(vtype, nnz, n_dense)) return FSB_ESCRATCH;
-    if (!aligned_to(scratch, 16)) return FSB_EALIGN;
-    FSB_WALK_FIRST(check_csr(FSB_I32, ptype, indices, indptr, n_rows, n_cols, nnz, static_cast<cudaStream_t>(stream_)));
-    parts_bytes = spmm_scratch_bytes(vtype, nnz, n_dense);
-    tile_row = (int32_t*)((char*)scratch + parts_bytes);
-    const int rc = fsb_csr_tile_plan(ptype, indptr, n_rows, nnz, kMmTile, tile_row, stream_);
-    if (rc != FSB_OK) return rc;
-  }
   // staged by ordinary loads: no copy whose end would have to be waited for and reported
   return spmm_run(vtype, FSB_I32, ptype, data, indices, indptr, B, ldb, C, ldc, n_rows, n_cols, n_dense, nnz,
-                  FSB_SPMM_PLAIN | (long_rows ? FSB_SPMM_LONG_ROWS : 0), tile_row, scratch, parts_bytes, nullptr,
+                  FSB_SPMM_PLAIN | (long_rows ? FSB_SPMM_LONG_ROWS : 0), nullptr, true, scratch, scratch_bytes, nullptr,
                   static_cast<cudaStream_t>(stream_));
 }
