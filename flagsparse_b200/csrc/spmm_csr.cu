@@ -62,9 +62,14 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t phase)
 
 // ---- stored value types: what is accumulated, and how a value enters a sum ---------------------------------------
 // half precisions are accumulated in float32 and rounded once when a row of C is stored
+// chains: partial sums per element of C that the entries of a segment take in turn.  Two for complex values: half as many
+// roundings behind one another (complex64, rows of 16 / 60 / 200 entries: one sum with both products fused into it has 1.48 /
+// 1.76 / 1.86 times the rms error).  One for the others: float32 / float64 have always had one, and the half precisions have
+// no registers for two of their eight sums per lane, which the rounding of the result would hide.
 template <typename S>
 struct MmOps {
   typedef S Acc;
+  static constexpr int chains = 1;
   static __device__ __forceinline__ void fma(Acc& acc, S a, S b) { acc += a * b; }
   static __device__ __forceinline__ Acc add(Acc a, Acc b) { return a + b; }
   static __device__ __forceinline__ Acc widen(S v) { return v; }
@@ -74,6 +79,7 @@ struct MmOps {
 template <>
 struct MmOps<__half> {
   typedef float Acc;
+  static constexpr int chains = 1;
   static __device__ __forceinline__ void fma(Acc& acc, __half a, __half b) {
     acc = fmaf(__half2float(a), __half2float(b), acc);
   }
@@ -85,6 +91,7 @@ struct MmOps<__half> {
 template <>
 struct MmOps<__nv_bfloat16> {
   typedef float Acc;
+  static constexpr int chains = 1;
   static __device__ __forceinline__ void fma(Acc& acc, __nv_bfloat16 a, __nv_bfloat16 b) {
     acc = fmaf(__bfloat162float(a), __bfloat162float(b), acc);
   }
@@ -96,10 +103,12 @@ struct MmOps<__nv_bfloat16> {
 template <typename C2>
 struct MmComplex {
   typedef C2 Acc;
+  static constexpr int chains = 2;
   static __device__ __forceinline__ void fma(Acc& acc, C2 a, C2 b) {
-    // written out: which products the compiler would fuse differs between the kernels
-    acc.x = ::fma(-a.y, b.y, ::fma(a.x, b.x, acc.x));
-    acc.y = ::fma(a.y, b.x, ::fma(a.x, b.y, acc.y));
+    // the product first, then one rounding at the size of the sum; written out, as what the compiler would fuse differs
+    // between the kernels
+    acc.x += ::fma(a.x, b.x, -(a.y * b.y));
+    acc.y += ::fma(a.x, b.y, a.y * b.x);
   }
   static __device__ __forceinline__ Acc add(Acc a, Acc b) {
     a.x += b.x;
@@ -221,8 +230,25 @@ spmm_tile_kernel(const S* __restrict__ data, const I* __restrict__ idx, const vo
 #pragma unroll
       for (int j = 0; j < VW; ++j) acc[i][j] = Ops::zero();
   };
-  // acc += sum over the entries p .. e-1 of value * row of B
+  constexpr int CHAINS = Ops::chains;
+  // acc += value * row of B for entry p
+  auto one = [&](int p, A (&acc)[NC][VW]) {
+    const S* row = B + (int64_t)s_idx[p] * ldb + col0;
+    const S v = s_val[p];
+#pragma unroll
+    for (int i = 0; i < NC; ++i) {
+      if (i == 0 || col0 + i * LR * VW < n_dense) {
+        Pack<S, VW> b;
+        b.gather(row + i * LR * VW);
+#pragma unroll
+        for (int j = 0; j < VW; ++j) Ops::fma(acc[i][j], v, b.get(j));
+      }
+    }
+  };
+  // acc = sum over the entries p .. e-1 of value * row of B (acc comes in cleared)
   auto walk = [&](int p, int e, A (&acc)[NC][VW]) {
+    A odd[NC][VW];                         // every other entry, where there are two partial sums
+    if (CHAINS == 2) clear(odd);
     for (; p + U <= e; p += U) {
       Pack<S, VW> b[U][NC];
 #pragma unroll
@@ -238,21 +264,18 @@ spmm_tile_kernel(const S* __restrict__ data, const I* __restrict__ idx, const vo
 #pragma unroll
         for (int i = 0; i < NC; ++i)
 #pragma unroll
-          for (int j = 0; j < VW; ++j) Ops::fma(acc[i][j], v, b[u][i].get(j));
+          for (int j = 0; j < VW; ++j) Ops::fma(CHAINS == 2 && (u & 1) ? odd[i][j] : acc[i][j], v, b[u][i].get(j));
       }
     }
     for (; p < e; ++p) {
-      const S* row = B + (int64_t)s_idx[p] * ldb + col0;
-      const S v = s_val[p];
+      one(p, acc);
+      if (CHAINS == 2 && ++p < e) one(p, odd);
+    }
+    if (CHAINS == 2) {
 #pragma unroll
-      for (int i = 0; i < NC; ++i) {
-        if (i == 0 || col0 + i * LR * VW < n_dense) {
-          Pack<S, VW> b;
-          b.gather(row + i * LR * VW);
+      for (int i = 0; i < NC; ++i)
 #pragma unroll
-          for (int j = 0; j < VW; ++j) Ops::fma(acc[i][j], v, b.get(j));
-        }
-      }
+        for (int j = 0; j < VW; ++j) acc[i][j] = Ops::add(acc[i][j], odd[i][j]);
     }
   };
   // the sum of segment g: to C, or to the arrays that the fix-up adds up
