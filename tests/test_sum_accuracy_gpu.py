@@ -40,18 +40,23 @@ def _rms(got, exact):
 def test_no_less_accurate_than_two_sums_over_a_row(cuda, fsb_lib, dtype, length):
     n_cols, n_rows = 3000, 6000 if length < 100 else 2000
     st = torch.cuda.current_stream().cuda_stream
-    n_dense = 16
-    idx = np.random.default_rng(length).integers(0, n_cols, n_rows * length).astype(np.int32)
-    vals = _values((n_rows * length,), dtype, 1)
-    operand = _values((n_cols, n_dense) if n_dense else (n_cols,), dtype, 2)
-    exact = _exact(vals, idx, operand, length)
-    d, i = vals.to(cuda), torch.from_numpy(idx).to(cuda)
-    p = torch.arange(n_rows + 1, dtype=torch.int32, device=cuda) * length
-    dense = operand.to(cuda).to(W.dense_dtype(dtype))
-    old = torch.empty((n_rows,) + tuple(operand.shape[1:]), dtype=dense.dtype, device=cuda)
-    new = fs.flagsparse_spmm_csr(d, i, p, operand.to(cuda), (n_rows, n_cols))
-    rc = fsb_lib.fsb_spmm_csr_wide(VT[dtype], 0, d.data_ptr(), i.data_ptr(), p.data_ptr(), dense.data_ptr(), n_dense,
-                                   old.data_ptr(), n_dense, n_rows, n_cols, n_dense, d.numel(), st)
-    assert rc == 0
-    a, b = _rms(new, exact), _rms(old.to(dtype), exact)
-    assert a <= 1.03 * b, (n_dense, a, b)
+    for n_dense, n_rows in ((16, n_rows), (0, 10 * n_rows)):
+        idx = np.random.default_rng(length).integers(0, n_cols, n_rows * length).astype(np.int32)
+        vals = _values((n_rows * length,), dtype, 1)
+        operand = _values((n_cols, n_dense) if n_dense else (n_cols,), dtype, 2)
+        exact = _exact(vals, idx, operand, length)
+        d, i = vals.to(cuda), torch.from_numpy(idx).to(cuda)
+        p = torch.arange(n_rows + 1, dtype=torch.int32, device=cuda) * length
+        dense = operand.to(cuda).to(W.dense_dtype(dtype))
+        old = torch.empty((n_rows,) + tuple(operand.shape[1:]), dtype=dense.dtype, device=cuda)
+        if n_dense:
+            new = fs.flagsparse_spmm_csr(d, i, p, operand.to(cuda), (n_rows, n_cols))
+            rc = fsb_lib.fsb_spmm_csr_wide(VT[dtype], 0, d.data_ptr(), i.data_ptr(), p.data_ptr(), dense.data_ptr(), n_dense,
+                                           old.data_ptr(), n_dense, n_rows, n_cols, n_dense, d.numel(), st)
+        else:
+            new = fs.flagsparse_spmv_csr(d, i, p, operand.to(cuda), (n_rows, n_cols))
+            rc = fsb_lib.fsb_spmv_csr_wide(VT[dtype], 0, d.data_ptr(), i.data_ptr(), p.data_ptr(), dense.data_ptr(),
+                                           old.data_ptr(), n_rows, n_cols, d.numel(), st)
+        assert rc == 0
+        a, b = _rms(new, exact), _rms(old.to(dtype), exact)
+        assert a <= 1.03 * b, (n_dense, a, b)
