@@ -145,10 +145,17 @@ struct Pack {
   __device__ __forceinline__ void set(int i, S v) { reinterpret_cast<S*>(&raw)[i] = v; }
 };
 
-// Resident CTAs the register budget is set for: 40 registers hold the four gathers of one access per lane; left to itself
-// the compiler fits 32 and issues them one after the other (54 columns, 28386 rows of 45 entries, float32: 60 us, 44 us).
+// Resident CTAs the register budget is set for.  One access per lane: 40 registers hold four gathers of 4-byte values; left
+// to itself the compiler fits 32 and issues them one after the other (54 columns, 28386 rows of 45 entries, float32: 60 us,
+// 44 us).  Four gathers and the sums of 8-byte values take 48 (float64, 60000 rows of 31, 40 / 64 / 128 columns with 40
+// registers: 70.6 / 77.8 / 145 us, with 48: 59.6 / 67.7 / 130 us; with 64: 66 / 74 / 146 us).  Several accesses: 64 (60000
+// rows of 31, 65 columns with 80 registers: float32 80.0 us, float64 114 us; with 64: 78.0 us, 98.8 us), four of them 80, which
+// 64 would spill.  With long rows the pieces' arithmetic comes on top (float64, 33 columns, one row of 300 among 60000 of 31:
+// 102 us with 128 registers, 82 us with 80, 88 us with 64).
 __host__ __device__ constexpr int mm_ctas(int nc, size_t size, bool with_long) {
-  return nc == 1 ? (size == 16 ? 4 : with_long ? 5 : 6) : with_long ? 2 : nc == 2 ? 4 : 3;
+  if (nc == 1) return size == 16 ? 4 : size == 8 ? 5 : 6;
+  if (with_long) return nc == 4 || (nc == 3 && size == 4) ? 2 : 3;
+  return nc < 4 ? 4 : 3;
 }
 
 // A group of LR lanes takes one segment (the part of a row that lies in the tile) at a time, four gathers of B on their
@@ -478,14 +485,21 @@ static int launch_spmm(const SpmmArgs& a, int LR, int piece) {
       carry, head, a.nnz, n_dense, LR, piece, bulk, a.status)
   // the long segments of a tile (more than 2 * piece entries each) have at most T / piece + T / (2 * piece) pieces
   const size_t parts = a.long_rows ? (size_t)(T / piece + T / (2 * piece)) * width * sizeof(A) : 0;
-  if (a.accumulate) {
-    if constexpr (REAL) {
-      if (a.long_rows) FSB_SPMM_LAUNCH(true, true, parts); else FSB_SPMM_LAUNCH(false, true, 0);
+  if (a.accumulate && !REAL) return FSB_EINVAL;
+  if (a.long_rows) {
+    if constexpr (NC == 1 || VW * (int)sizeof(S) < 16) {       // spmm_shape gives long rows no other
+      if constexpr (REAL) {
+        if (a.accumulate) FSB_SPMM_LAUNCH(true, true, parts);
+      }
+      if (!a.accumulate) FSB_SPMM_LAUNCH(true, false, parts);
     } else {
       return FSB_EINVAL;
     }
   } else {
-    if (a.long_rows) FSB_SPMM_LAUNCH(true, false, parts); else FSB_SPMM_LAUNCH(false, false, 0);
+    if constexpr (REAL) {
+      if (a.accumulate) FSB_SPMM_LAUNCH(false, true, 0);
+    }
+    if (!a.accumulate) FSB_SPMM_LAUNCH(false, false, 0);
   }
 #undef FSB_SPMM_LAUNCH
   FSB_RETURN_IF_LAUNCH_FAILED();
@@ -507,14 +521,17 @@ static int launch_spmm(const SpmmArgs& a, int LR, int piece) {
 // Lanes per entry (LR, a power of two) and accesses per lane (NC).  Up to 32 accesses there is one per lane (5 columns as
 // 2 lanes x 3: 66 us, as 8 lanes: 48 us, 200000 rows of 20 entries).  Beyond, the pair with the fewest idle lanes: 33
 // single columns take 16 lanes x 3 instead of two passes over the matrix with 32 lanes.  NC is bounded by what a lane
-// accumulates in registers (32 bytes).
+// accumulates in registers (32 bytes); 8-byte values in 16-byte accesses take one, as two leave too few CTAs in flight
+// (float64, 60000 rows of 31, 96 columns: 126 us and 113 us; 262144 rows of 16, 128 columns: 563 us and 455 us), and so do
+// other 16-byte accesses where rows are long (float32, 160 columns, 262144 rows of 16 and one of 300: 427 us and 322 us).
 template <typename S, typename I, int VW>
 static int spmm_shape(const SpmmArgs& a) {
   typedef typename MmOps<S>::Acc A;
   constexpr int VMAX = 16 / (int)sizeof(S);
   constexpr int HELD = VW * (int)sizeof(A);      // accumulator bytes of one access
   // (16-byte values: one, or the pieces of long segments would not fit beside the staged tile)
-  constexpr int NC_MAX = sizeof(S) == 16 || HELD >= 32 ? 1 : (32 / HELD < 4 ? 32 / HELD : 4);
+  constexpr int NC_TYPE = sizeof(S) == 16 || HELD >= 32 || (sizeof(S) == 8 && VW == VMAX) ? 1 : (32 / HELD < 4 ? 32 / HELD : 4);
+  const int nc_max = VW == VMAX && a.long_rows ? 1 : NC_TYPE;
   const int64_t need = (a.n_dense + VW - 1) / VW;
   const int64_t need_widest = (a.n_dense + VMAX - 1) / VMAX;
   const int LR_min = pow2_at_least((int)(need_widest < 32 ? need_widest : 32));   // what a 16-byte access would use
@@ -526,7 +543,7 @@ static int spmm_shape(const SpmmArgs& a) {
     LR = pow2_at_least((int)need);
   } else {
     int64_t best = -1;
-    for (int nc = 1; nc <= NC_MAX; ++nc)
+    for (int nc = 1; nc <= nc_max; ++nc)
       for (int lr = LR_min; lr <= 32; lr <<= 1) {
         const int64_t passes = (need + lr * nc - 1) / (lr * nc);
         const int64_t cost = passes * lr * nc * 64 + passes;   // idle lanes first, then passes over the matrix
@@ -537,10 +554,10 @@ static int spmm_shape(const SpmmArgs& a) {
         }
       }
   }
-  if constexpr (NC_MAX >= 2) {
+  if constexpr (NC_TYPE >= 2) {
     if (NC == 2) return launch_spmm<S, I, VW, 2>(a, LR, piece);
   }
-  if constexpr (NC_MAX >= 4) {
+  if constexpr (NC_TYPE >= 4) {
     if (NC == 3) return launch_spmm<S, I, VW, 3>(a, LR, piece);
     if (NC == 4) return launch_spmm<S, I, VW, 4>(a, LR, piece);
   }

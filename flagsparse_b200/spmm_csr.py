@@ -41,9 +41,17 @@ _SPMM_ALGO_NAMES = {"auto": _lib.FSB_SPMM_AUTO, "plain": _lib.FSB_SPMM_PLAIN, "b
 # of its read-add-write of C, not by the bytes it saves.  FSB_SPMM_PANEL_MB=<MiB> or FSB_SPMM_PANELS=<n> turn it on.
 PANEL_BYTES = 0
 COL_TILE_BYTES = 128
-# rows longer than this get FSB_SPMM_LONG_ROWS (include/fsb.h): about where a group that walks one alone takes longer
-# than its neighbours take for their share of a 1024-entry tile
+# A matrix with a row longer than this gets FSB_SPMM_LONG_ROWS (include/fsb.h).  A group that walks a row alone takes about
+# 0.06 us per entry (float32) to 0.12 us (half precisions), up to the 1024 of a tile; sharing it costs 1 to 4 % where it
+# brings nothing.  One row of 260 / 400 / 1030 entries, alone against shared: 262144 rows of 16, 16 columns, float32: 50 / 57 /
+# 93 us against 46 / 41 / 47 us; 4096 rows of 16, 64 columns, bfloat16: 90 / 111 / 190 us against 62 us; 60000 rows of 31, 64
+# columns, float64: 67 / 68 / 91 us against 70 us.
 LONG_ROW_NNZ = 256
+# The same where a lane takes several accesses per entry (odd widths beyond 32), whose shared form has fewer CTAs in flight:
+# 262144 rows of 16, 33 columns, one row of 400 / 600 / 1030: float32 88 / 93 / 120 us alone against 98 / 101 / 105 us, float64
+# 174 / 176 / 200 us against 218 / 220 / 222 us; 60000 rows of 31: float64 73 / 74 / 91 us against 83 us, bfloat16 138 / 150 / 174 us
+# against 144 us.
+LONG_ROW_NNZ_SEVERAL = 640
 SPAN_WINDOW = 1 << 20        # consecutive entries over which the column span is sampled
 
 
@@ -377,6 +385,13 @@ def _prepare_spmm(data, indices, indptr, shape, once):
     return prepared
 
 
+def _shares_long_rows(max_row_nnz, n_dense, element_size):
+    """Whether a product of this width gets FSB_SPMM_LONG_ROWS."""
+    vw = min(16 // element_size, n_dense & -n_dense)      # widest access that divides a row of B
+    several = n_dense > 32 * vw and vw * element_size < 16
+    return max_row_nnz > (LONG_ROW_NNZ_SEVERAL if several else LONG_ROW_NNZ)
+
+
 def _spmm_launch(prepared, B, C):
     """Enqueue C = A B on the current stream.  Stands in for _triton_spmm_csr_impl (spmm_csr.py:525-599)
     and _triton_spmm_csr_impl_opt_prepared (:1033-1055).  One launch of the tiled kernel per pass: the whole
@@ -394,9 +409,9 @@ def _spmm_launch(prepared, B, C):
     else:
         status = p.status_word()
         status.poll()
-    if p.max_row_nnz > LONG_ROW_NNZ:
-        algo |= _lib.FSB_SPMM_LONG_ROWS
     sv = B.element_size()
+    if _shares_long_rows(p.max_row_nnz, n_dense, sv):
+        algo |= _lib.FSB_SPMM_LONG_ROWS
     vt, it, pt = _VTYPE[p.data.dtype], _ITYPE[p.kernel_indices.dtype], _ITYPE[p.kernel_indptr.dtype]
     ldb, ldc = B.stride(0), C.stride(0)
     stream = _stream_ptr(dev)
@@ -459,7 +474,7 @@ def _spmm_launch_stored(prepared, B, C):
         rc = L.fsb_spmm_csr_stored(
             vt, _ITYPE[p.kernel_indptr.dtype], _ptr(p.data), _ptr(p.kernel_indices), p.kernel_indptr.data_ptr(),
             _ptr(B), B.stride(0) if B.shape[0] > 1 else n_dense, C.data_ptr(), n_dense, p.n_rows, p.n_cols, n_dense, nnz,
-            int(p.max_row_nnz > LONG_ROW_NNZ), scratch.data_ptr(), scratch.numel(), _stream_ptr(dev),
+            int(_shares_long_rows(p.max_row_nnz, n_dense, B.element_size())), scratch.data_ptr(), scratch.numel(), _stream_ptr(dev),
         )
     _lib.check(rc, "fsb_spmm_csr_stored")
 

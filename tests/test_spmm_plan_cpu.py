@@ -2,6 +2,7 @@
 B and C.  Host logic only (CPU tensors, no launch)."""
 
 import numpy as np
+import pytest
 import scipy.sparse as sp
 import torch
 
@@ -70,3 +71,12 @@ def test_pass_plan(monkeypatch):
     monkeypatch.setattr(M, "SPAN_WINDOW", 4096)
     band = _prepared_on_cpu(S.CsrSpec("band", 1 << 14, 1 << 14, ("const", 16), ("band", 64), False, 0))
     assert band.column_span() < 1024 and band.n_panels_for(128) == 1
+
+
+@pytest.mark.parametrize("size", [2, 4, 8, 16])
+def test_long_rows_are_shared_from_a_length_that_follows_the_accesses_per_lane(size):
+    one, several = M.LONG_ROW_NNZ, M.LONG_ROW_NNZ_SEVERAL
+    for n_dense, limit in ((1, one), (31, one), (32, one), (33, one if size == 16 else several), (64, one), (128, one),
+                           (127, one if size == 16 else several), (16 // size * 40, one)):
+        assert not M._shares_long_rows(limit, n_dense, size)
+        assert M._shares_long_rows(limit + 1, n_dense, size)
