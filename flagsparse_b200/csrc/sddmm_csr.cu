@@ -6,8 +6,8 @@
 // entries; the row of an entry comes from the row-id array built at prepare time, 4 bytes per entry) into shared
 // memory, so that the only trip to global memory inside the loop over batches is the gather; every lane then
 // requests its slice of all eight rows of Y through the read-only path before it uses any of them, so a group has
-// eight gathers in flight; a batch that lies inside one row (the common case) needs one slice of X's row, a batch
-// that crosses rows loads a slice of X per entry.  Each lane ends with eight partial sums (one per entry);
+// eight gathers in flight; a batch that lies inside one row needs one slice of X's row, one that meets two rows a slice of
+// each, a batch that crosses more loads a slice of X per entry.  Each lane ends with eight partial sums (one per entry);
 // they are reduced across the group by a transposed exchange (halve the entries a lane is responsible for at every
 // step: 7 shuffles for 8 entries x 8 lanes instead of 24), after which the results of consecutive entries sit in
 // consecutive lanes and leave as one contiguous streaming store.  Rows of X longer than LG * VW elements are
@@ -42,6 +42,7 @@ sddmm_kernel(const int32_t* __restrict__ indices, const int32_t* __restrict__ ro
   constexpr int T = sddmm_tile(LG);
   constexpr int kHeld = (LG >= E) ? 1 : E / LG;   // results a lane ends up with
   constexpr int kDup = (LG > E) ? LG / E : 1;     // lanes that end up with the same result
+  constexpr bool VOTE = sizeof(V) == 4 && VW == 4 && (LG == 8 || LG == 16);   // see the loop
   __shared__ __align__(16) int32_t s_cols[T];
   __shared__ __align__(16) int32_t s_rows[T];
 
@@ -66,9 +67,11 @@ sddmm_kernel(const int32_t* __restrict__ indices, const int32_t* __restrict__ ro
   const int lane = threadIdx.x & (LG - 1);
   const int group = threadIdx.x / LG;
   const unsigned gmask = LG == 32 ? 0xffffffffu : (((1u << LG) - 1u) << ((threadIdx.x & 31) & ~(LG - 1)));
+  unsigned active = 0xffffffffu;   // lanes of the warp that have a batch
 #pragma unroll 1
   for (int j = 0; j < J; ++j) {
     const int local = (j * kGroups + group) * E;
+    if constexpr (VOTE) active = __ballot_sync(active, local < left);
     if (local >= left) break;   // whole groups leave together: the shuffles below stay inside a group
     const int64_t p0 = tile0 + local;
     const int n = (int)((left - local) < E ? (left - local) : E);
@@ -100,34 +103,56 @@ sddmm_kernel(const int32_t* __restrict__ indices, const int32_t* __restrict__ ro
     // entries at a time (reloading X only where the row changes would make each gather wait for the previous entry's
     // arithmetic).  float64, and float32 with a whole warp per entry, have no registers for a second slice beside eight
     // gathers of 16 bytes: there only a batch of one row takes the first form.  (2^19 rows of 16 entries, K 64, float32:
-    // 459 us when a batch of two rows took the second form, 350 us now; 300000 rows of 5, K 33: 171 us, 112 us.  With
-    // TWO everywhere float64, 50000 rows of 40, K 64 goes from 115 us to 168 us.)
+    // 456 us when a batch of two rows took the second form, 343 us with a slice of each; 300000 rows of 5, K 33: 162 us,
+    // 105 us.  With TWO everywhere float64, 50000 rows of 40, K 64 goes from 115 us to 168 us.)
+    // VOTE (two to four groups in a warp, 16-byte gathers): the groups agree on the form that all of their batches fit, as a
+    // warp whose groups differ runs one form after the other; single rows have a form of their own.  Without it uneven
+    // rows lost what even ones had gained (2^19 rows of 16, K 64: even 343 us, Zipf lengths 392 us where 316 us had been
+    // measured with the first and last form alone; with it 292 us and 320 us.  300000 rows of 5: 98.6 us, 88 us, 86.3 us).
+    // With eight groups and more, or smaller gathers, agreeing costs more than it saves (K 16: 98 us, with it 109 us; K 33: 558
+    // us, 614 us).
     constexpr bool TWO = sizeof(V) == 4 && (LG <= 16 || VW == 1);
     const int32_t row_a = rows[0], row_b = rows[E - 1];
-    bool few = row_a == row_b;
+    bool one = row_a == row_b, few = TWO;
     unsigned in_a = 0;
     if constexpr (TWO) {
-      few = true;
 #pragma unroll
       for (int e = 0; e < E; ++e) {
         few = few && (rows[e] == row_a || rows[e] == row_b);
         in_a |= (rows[e] == row_a ? 1u : 0u) << e;
       }
     }
-    if (few) {
+    if constexpr (VOTE) {
+      one = __all_sync(active, one);
+      few = __all_sync(active, few);
+    }
+    if ((!TWO || VOTE) && one) {
       for (int k = lane * VW; k < k_dim; k += step) {
-        V xa[VW], xb[VW], yv[E][VW];
+        V xa[VW], yv[E][VW];
         ld_dense<V, VW>(X + (int64_t)row_a * ldx + k, xa);
-        if constexpr (TWO) ld_dense<V, VW>(X + (int64_t)row_b * ldx + k, xb);
 #pragma unroll
         for (int e = 0; e < E; ++e) ld_dense<V, VW>(Y + (int64_t)cols[e] * ldy + k, yv[e]);
 #pragma unroll
         for (int e = 0; e < E; ++e)
 #pragma unroll
-          for (int i = 0; i < VW; ++i) {
-            if constexpr (TWO) acc[e] += ((in_a >> e) & 1 ? xa[i] : xb[i]) * yv[e][i];
-            else acc[e] += xa[i] * yv[e][i];
-          }
+          for (int i = 0; i < VW; ++i) acc[e] += xa[i] * yv[e][i];
+      }
+    } else if (few) {
+      for (int k = lane * VW; k < k_dim; k += step) {
+        V xa[VW], xb[VW], yv[E][VW];
+        ld_dense<V, VW>(X + (int64_t)row_a * ldx + k, xa);
+        if (!VOTE || row_b != row_a) {
+          ld_dense<V, VW>(X + (int64_t)row_b * ldx + k, xb);
+        } else {
+#pragma unroll
+          for (int i = 0; i < VW; ++i) xb[i] = xa[i];
+        }
+#pragma unroll
+        for (int e = 0; e < E; ++e) ld_dense<V, VW>(Y + (int64_t)cols[e] * ldy + k, yv[e]);
+#pragma unroll
+        for (int e = 0; e < E; ++e)
+#pragma unroll
+          for (int i = 0; i < VW; ++i) acc[e] += ((in_a >> e) & 1 ? xa[i] : xb[i]) * yv[e][i];
       }
     } else {
       for (int k = lane * VW; k < k_dim; k += step) {

@@ -10,7 +10,9 @@ from helpers import handmade_csr
 
 pytestmark = pytest.mark.gpu
 
-LENS = {"one": [8] * 40, "two": [5, 11, 8, 7, 9, 4, 12] * 9, "more": [1, 2, 0, 3, 1, 1, 0, 0, 4] * 21, "odd": [13, 0, 6, 1, 2, 30, 3]}
+LENS = {"one": [8] * 40, "two": [5, 11, 8, 7, 9, 4, 12] * 9, "more": [1, 2, 0, 3, 1, 1, 0, 0, 4] * 21, "odd": [13, 0, 6, 1, 2, 30, 3],
+        # batches of one row, of two and of more beside each other, in every order that the groups of a warp can meet
+        "mixed": ([16, 5, 3, 1, 2, 1, 4, 8, 8, 1, 1, 6, 24, 7, 9, 2, 2, 2, 2] * 5 + [40] * 3 + [1] * 50) * 2}
 
 
 @pytest.mark.parametrize("dtype,u", [(torch.float32, 2.0 ** -24), (torch.float64, 2.0 ** -53)], ids=str)
@@ -21,7 +23,7 @@ def test_batches_over_rows(cuda, fsb_lib, dtype, u, name):
     n_rows = len(p) - 1
     row = np.repeat(np.arange(n_rows), np.diff(p))
     prep = fs.prepare_sddmm_csr(torch.from_numpy(i).to(cuda), torch.from_numpy(p).to(cuda), (n_rows, n_cols))
-    for k in (1, 3, 4, 8, 33, 64, 66, 128, 130):
+    for k in (1, 3, 4, 8, 16, 24, 32, 33, 64, 66, 128, 130):
         rng = np.random.default_rng(k)
         x, y = (torch.from_numpy(rng.uniform(-1, 1, (n, k))).to(dtype) for n in (n_rows, n_cols))
         out = fs.flagsparse_sddmm_csr(x=x.to(cuda), y=y.to(cuda), prepared=prep).cpu().double().numpy()
