@@ -84,11 +84,24 @@ def _select_spmv_algo(n_rows, nnz, max_row_nnz):
     return _lib.FSB_SPMV_STREAM
 
 
-def _uneven_rows(n_rows, nnz, max_row_nnz):
-    """Whether the longest row leaves the lanes-per-row kernel for float16 / bfloat16 / complex values waiting for it.
-    A row of n entries takes its 2 to 32 lanes about n / (4 lanes) trips to memory, one after the other; the tiled
-    kernel costs a second launch and the products' way through shared memory."""
-    return max_row_nnz > _UNIFORM_ROW_FACTOR * (nnz / max(n_rows, 1)) + _UNIFORM_ROW_SLACK
+# Longest row from which the tiled kernel for float16 / bfloat16 / complex values is taken, whatever the mean: a row of n
+# entries takes its few lanes 0.03 to 0.04 us per entry (0.07 us while others keep memory busy), the tiled kernel a second
+# launch, and complex values their way through shared memory: 6 % of complex64, 25 % of complex128.  So the line rises with the
+# number of entries, one per _UNEVEN_ENTRIES[bytes per value].  Lanes per row against tiles, longest row 200 / 300 / 400 / 600
+# / 1000 / 2000: 30000 rows of 16, bfloat16: 14 / 19 / 22 / 31 / 45 / 81 us against 16 us, complex128: 14 / 17 / 21 / 29 / 47 / 86 us
+# against 16 us; 500009 rows of 24, complex64: 70 / 70 / 76 / 88 / 112 / 182 us against 74 us, complex128: 87 / 87 / 87 / 101 / 139
+# / 221 us against 113 us; 2000000 rows of 20, complex64: 210 / 210 / 211 / 211 / 219 / 273 us against 225 us, complex128: 292 /
+# 294 / 301 / 300 / 299 / 357 us against 359 us.
+_UNEVEN_MIN = 288
+_UNEVEN_ENTRIES = {8: 35000, 16: 18000}
+
+
+def _uneven_rows(n_rows, nnz, max_row_nnz, element_size):
+    """Whether the longest row leaves the lanes-per-row kernel for float16 / bfloat16 / complex values waiting for it."""
+    line = max(_UNEVEN_MIN, _UNIFORM_ROW_FACTOR * (nnz / max(n_rows, 1)) + _UNIFORM_ROW_SLACK)
+    if element_size in _UNEVEN_ENTRIES:
+        line = max(line, nnz / _UNEVEN_ENTRIES[element_size])
+    return max_row_nnz > line
 
 
 class PreparedCsrSpmv:
@@ -260,7 +273,7 @@ def _prepare_spmv_csr(data, indices, indptr, shape, block_nnz, max_segments, reu
         # float16 / bfloat16 / complex values are read as they are stored by kernels of their own (fsb_spmv_csr_stored):
         # no second copy of the matrix, and a tile plan where the row lengths call for one
         tile_nnz, tile_row = 0, None
-        if nnz > 0 and n_rows > 0 and data.device.type == "cuda" and _uneven_rows(n_rows, nnz, max_row_nnz):
+        if nnz > 0 and n_rows > 0 and data.device.type == "cuda" and _uneven_rows(n_rows, nnz, max_row_nnz, data.element_size()):
             tile_nnz = int(_lib.lib().fsb_spmv_stored_tile_nnz(_WIDE_VTYPE[data.dtype]))
             tile_row = _tile_plan(kernel_indptr, n_rows, nnz, tile_nnz)
         return PreparedCsrSpmv(
