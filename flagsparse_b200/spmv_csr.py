@@ -34,7 +34,11 @@ _VECTOR_MAX_ROW_NNZ = 4096
 # "uniform" rows: the longest row is within this factor (plus a small allowance) of the mean row length
 _UNIFORM_ROW_FACTOR = 8
 _UNIFORM_ROW_SLACK = 64
-_SMALL_ROW_SLACK = 256       # the same for matrices of less than _STREAM_MIN_NNZ entries
+# The same for matrices of less than _STREAM_MIN_NNZ entries, by bytes per value.  Lanes per row against the stream kernel,
+# longest row 120 / 200 / 250 / 300 / 400 / 600: 4096 rows of 16, float32: 10.2 / 10.4 / 11.3 / 12.7 / 16.4 / 22.6 us against 15.1 us,
+# float64: 10.3 / 14.4 / 16.4 / 18.5 / 24.6 / 33.9 us; 10000 rows of 24, float32: 10.3 / 12.3 / 13.0 / 14.4 / 18.5 / 24.7 us, float64:
+# 12.3 / 16.4 / 18.7 / 22.6 / 28.7 / 39.0 us; 4096 rows of 48, from 600 and from 400 on.
+_SMALL_ROW_SLACK = {4: 256, 8: 64}
 # regroup banded matrices for the panel kernel (costs a second copy of the entries); FSB_SPMV_PANEL=0 turns it off
 _PANEL_ENABLED = os.environ.get("FSB_SPMV_PANEL", "1") != "0"
 
@@ -64,7 +68,7 @@ def _resolve_block_nnz(max_row_nnz, block_nnz, max_segments):
     return block_nnz_use, max_segments_use
 
 
-def _select_spmv_algo(n_rows, nnz, max_row_nnz):
+def _select_spmv_algo(n_rows, nnz, max_row_nnz, element_size=4):
     """Kernel choice from indptr statistics.  Rows of about equal length (longest row within a small
     factor of the mean) go to the lanes-per-row vector kernel, which needs one launch, no scratch, and leaves
     the whole L1 to the gathers of x; skewed row lengths go to the nnz-tiled stream kernel, whose work per
@@ -76,9 +80,9 @@ def _select_spmv_algo(n_rows, nnz, max_row_nnz):
         return _lib.FSB_SPMV_STREAM
     mean = nnz / max(n_rows, 1)
     if nnz < _STREAM_MIN_NNZ:
-        # one launch against two (8 us against 13 us); a row of n entries takes its two or more lanes about 0.05 n us
-        # (2274 entries, two lanes: 126 us in all, the stream kernel 15 us)
-        return _lib.FSB_SPMV_VECTOR if max_row_nnz <= _UNIFORM_ROW_FACTOR * mean + _SMALL_ROW_SLACK else _lib.FSB_SPMV_STREAM
+        # one launch against two, until the longest row takes its lanes longer than that
+        even = max_row_nnz <= _UNIFORM_ROW_FACTOR * mean + _SMALL_ROW_SLACK[element_size]
+        return _lib.FSB_SPMV_VECTOR if even else _lib.FSB_SPMV_STREAM
     if max_row_nnz <= _UNIFORM_ROW_FACTOR * mean + _UNIFORM_ROW_SLACK:
         return _lib.FSB_SPMV_VECTOR
     return _lib.FSB_SPMV_STREAM
@@ -282,7 +286,7 @@ def _prepare_spmv_csr(data, indices, indptr, shape, block_nnz, max_segments, reu
             stats=stats, algo=_lib.FSB_SPMV_VECTOR if tile_row is None else _lib.FSB_SPMV_STREAM, tuning=0,
             tile_nnz=tile_nnz, tile_row=tile_row, scratch=None, wide=("native", []),
         )
-    algo = _select_spmv_algo(n_rows, nnz, max_row_nnz)
+    algo = _select_spmv_algo(n_rows, nnz, max_row_nnz, data.element_size())
     tuning = int(os.environ.get("FSB_SPMV_TUNING", "0"))
     tile_nnz, tile_row, scratch, panel_layout = 0, None, None, None
     # rows of about equal length whose columns stay within a few chunks: regroup once, keep x in shared memory

@@ -2,7 +2,7 @@
 
 import pytest
 
-from flagsparse_b200 import spmv_csr as M
+from flagsparse_b200 import _lib, spmv_csr as M
 
 
 @pytest.mark.parametrize("size", [2, 8, 16])
@@ -11,3 +11,11 @@ def test_stored_types(size):
     for n_rows, nnz, line in ((4096, 1 << 16, 288), (1000, 200000, 1664), (0, 0, 288),
                               (2000000, 40000000, {2: 288, 8: 1142, 16: 2222}[size])):
         assert not M._uneven_rows(n_rows, nnz, line, size) and M._uneven_rows(n_rows, nnz, line + 1, size)
+
+
+@pytest.mark.parametrize("size,line", [(4, 256), (8, 64)])
+def test_small_matrices_of_native_types(size, line):
+    for n_rows, mean in ((2000, 4), (4096, 16), (4096, 48)):
+        longest = 8 * mean + line
+        assert M._select_spmv_algo(n_rows, n_rows * mean, longest, size) == _lib.FSB_SPMV_VECTOR
+        assert M._select_spmv_algo(n_rows, n_rows * mean, longest + 1, size) == _lib.FSB_SPMV_STREAM
