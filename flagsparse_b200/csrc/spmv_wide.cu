@@ -304,10 +304,11 @@ __device__ __forceinline__ void ld_four(const double2* p, double2 (&v)[4]) {
 // Even rows: L lanes per row.  GROUPS (half precisions on aligned arrays): a lane reads whole groups of four entries, one
 // request for the columns and one for the values, from the group that holds the row's first entry on, and masks what
 // belongs to the neighbours; a walk entry by entry asks for 2 bytes at a time.  x is read and y written as they are, in
-// this one pass (float16, 2e6 rows of 20 entries in a band: 165 us with the passes that widen x and round y, here 145 us;
-// 2e6 rows of 5: 71 us and 58 us).  Otherwise one entry at a time: the lanes of a row then read neighbouring 8- or 16-byte
-// values, and groups of four would spread each request over four times the lines (complex64, 500009 rows of 24: 90 us in
-// groups, 74 us entry by entry with four gathers on their way, 84 us with two).
+// this one pass (float16, 2e6 rows of 20 entries in a band of 2^15: 138 us with the passes that widen x and round y, here
+// 90 us; 2e6 rows of 5, columns anywhere: 58 us and 49 us).  Otherwise one entry at a time: the lanes of a row then read neighbouring 8- or 16-byte
+// values, and groups of four would spread each request over four times the lines (complex64, 500009 rows of 24,
+// columns anywhere: 80 us in groups, 70 us entry by entry with four gathers on their way, 74 us with two; in a band of 2^15:
+// 72 us, 63 us, 68 us).
 template <typename S, typename P, int L, bool GROUPS>
 __global__ void __launch_bounds__(kWideThreads)
 spmv_stored_vector_kernel(const S* __restrict__ data, const int32_t* __restrict__ idx, const P* __restrict__ ptr,
@@ -361,8 +362,8 @@ spmv_stored_vector_kernel(const S* __restrict__ data, const int32_t* __restrict_
     }
   } else {
     int64_t p = s + lane;
-    // (16-byte values: two at a time measured better, 70 us against 74 us, 300000 rows of 30 entries)
-    for (; sizeof(S) < 16 && p + 3 * L < e; p += 4 * L) {
+    // (complex128: 2000000 rows of 20, 298 us with two gathers on their way, 289 us with four; 100000 rows of 60: 43 us, 41 us)
+    for (; p + 3 * L < e; p += 4 * L) {
       S a[4];
       int32_t c[4];
 #pragma unroll
@@ -393,8 +394,8 @@ spmv_stored_vector_kernel(const S* __restrict__ data, const int32_t* __restrict_
 // Uneven rows: tiles of a fixed number of entries, as in spmv_stream_kernel (spmv_csr.cu): products to shared memory,
 // L lanes per segment, segments much longer than the tile's mean by whole warps; the rows that cross tiles leave
 // partial sums for spmv_stored_fixup_kernel.  The lanes-per-row kernel gives a row of 2^17 entries the 2 to 32 lanes that
-// the mean row length asks for (complex64, 3e6 rows of Zipf lengths, 36 M entries: 15.1 ms, here 241 us; complex128,
-// 252377 such rows: 7.9 ms and 36 us; bfloat16, 27496 rows: 304 us and 17 us).
+// the mean row length asks for (complex64, 3e6 rows of Zipf lengths, 36 M entries: 15.9 ms, here 226 us; complex128,
+// 252377 such rows: 7.3 ms and 37 us; bfloat16, 27496 rows: 223 us and 16 us).
 template <typename S>
 __host__ __device__ constexpr int stored_tile() { return sizeof(S) == 16 ? 1024 : 2048; }
 
@@ -571,7 +572,8 @@ static int stored_launch(const void* data_, const int32_t* idx, const void* ptr_
     return FSB_OK;
   }
   // two to four groups of four entries per lane, as in the float32 / float64 kernel; entry by entry, four to eight
-  // (complex64, 500009 rows of 24 entries: at most 4 per lane 75 us, 8: 74 us, 16: 107 us)
+  // (complex64, columns anywhere, at most 4 / 8 / 16 per lane: 500009 rows of 24: 64 / 70 / 87 us, 300000 rows of 30: 51 / 47 /
+  // 55 us, 2000000 rows of 20: 212 / 209 / 270 us; complex128: 78 / 84 / 97 us, 64 / 58 / 66 us, 294 / 289 / 344 us)
   const int64_t mean = n_rows > 0 ? nnz / n_rows : 0;
   int L = 2;
   while (L < 32 && (groups ? 16 : 8) * L < mean + 3) L <<= 1;
