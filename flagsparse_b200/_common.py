@@ -1,9 +1,9 @@
 """Dtype tables, limits and tolerances shared by the CSR SpMV / SpMM host code.
 
 Mirrors the conventions of the reference's src/flagsparse/sparse_operations/_common.py:22-31 (dtype
-whitelists, int32 index limit) and :76-85 (allclose tolerances).  The CUDA kernels compute float32 and float64;
-the other four value dtypes of the reference's whitelist run through them by widening or by splitting complex
-values into real and imaginary matrices (widetypes.py), on the entry points where the reference accepts them.
+whitelists, int32 index limit) and :76-85 (allclose tolerances).  float32 and float64 values have kernels with plans of
+their own; the other four value dtypes of the reference's whitelist run through kernels that read them as they are
+stored (widetypes.py), on the entry points where the reference accepts them.
 """
 
 import torch
@@ -12,8 +12,6 @@ from . import _lib
 
 SUPPORTED_VALUE_DTYPES = (torch.float16, torch.bfloat16, torch.float32, torch.float64, torch.complex64,
                           torch.complex128)
-# what the kernels themselves compute in; the other value dtypes are widened or split on the host
-NATIVE_VALUE_DTYPES = (torch.float32, torch.float64)
 SUPPORTED_INDEX_DTYPES = (torch.int32, torch.int64)
 _INDEX_LIMIT_INT32 = 2**31 - 1
 

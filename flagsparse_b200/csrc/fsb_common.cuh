@@ -72,7 +72,7 @@ __device__ __forceinline__ void st_shared4(double* p, const double (&v)[4]) {
   *(reinterpret_cast<double2*>(p) + 1) = make_double2(v[2], v[3]);
 }
 
-// ---- dense-row vector access for SpMM (VW elements, VW*sizeof(V) <= 16 bytes) ---------------------
+// ---- dense-row vector access (VW elements, VW*sizeof(V) <= 16 bytes) ---------------------
 template <typename V, int VW>
 struct Vec;
 template <> struct Vec<float, 1> { typedef float type; };
@@ -88,23 +88,6 @@ __device__ __forceinline__ void ld_dense(const V* p, V (&v)[VW]) {
   const V* e = reinterpret_cast<const V*>(&t);
 #pragma unroll
   for (int i = 0; i < VW; ++i) v[i] = e[i];
-}
-template <typename V, int VW>
-__device__ __forceinline__ void ld_dense_stream(const V* p, V (&v)[VW]) {
-  typedef typename Vec<V, VW>::type VT;
-  VT t = __ldcs(reinterpret_cast<const VT*>(p));
-  const V* e = reinterpret_cast<const V*>(&t);
-#pragma unroll
-  for (int i = 0; i < VW; ++i) v[i] = e[i];
-}
-template <typename V, int VW>
-__device__ __forceinline__ void st_dense_stream(V* p, const V (&v)[VW]) {
-  typedef typename Vec<V, VW>::type VT;
-  VT t;
-  V* e = reinterpret_cast<V*>(&t);
-#pragma unroll
-  for (int i = 0; i < VW; ++i) e[i] = v[i];
-  __stcs(reinterpret_cast<VT*>(p), t);
 }
 
 // Neumaier-compensated running sum in double: exact enough for every value type whatever the number of terms.  The total is

@@ -223,7 +223,8 @@ class PreparedCsrSpmmOpt:
     Attribute names follow the reference's class (spmm_csr.py:337-392).  `row_buckets` describes the tile
     plan; the `long_*` split tables of the reference stay empty because rows of any length go through the
     same tiles.  Scratch (two partial rows per tile) depends on the width of B and is cached per width:
-    calls that share a prepared object must not overlap on the GPU.
+    calls that share a prepared object must not overlap on the GPU (float16 / bfloat16 / complex values: each
+    call brings its own, so they may).
     """
 
     __slots__ = (
@@ -256,7 +257,7 @@ class PreparedCsrSpmmOpt:
         self._whole = None       # the matrix as one _CsrPart (shares the tile plan)
         self._panels = {}        # number of column panels -> list of _CsrPart
         self._span = None        # columns spanned by a window of consecutive entries (median over samples)
-        # float16 / bfloat16 / complex values: ("native", []) -- the product goes through fsb_spmm_csr_wide
+        # float16 / bfloat16 / complex values: ("native", []) -- the product goes through fsb_spmm_csr_stored
         self.wide = wide
 
     def __getattr__(self, name):
@@ -440,28 +441,10 @@ def _check_out(out, device, shape, dtype, device_msg):
         raise ValueError("out shape/dtype must match result")
 
 
-def _spmm_launch_wide(prepared, B, C):
-    """Enqueue C = A B for float16 / bfloat16 / complex values (fsb_spmm_csr_wide): B and C are float32 for the half
-    precisions and of the matrix's own type for complex values; B may have any row stride.  Stands in for the
-    reference's base launch helper on these types (_triton_spmm_csr_impl, spmm_csr.py:525-599)."""
-    from .spmv_csr import _WIDE_VTYPE
-
-    p = prepared
-    dev = p.data.device
-    if p.n_rows == 0 or B.shape[1] == 0:
-        return
-    with _on_device(dev):
-        rc = _lib.lib().fsb_spmm_csr_wide(
-            _WIDE_VTYPE[p.data.dtype], _ITYPE[p.kernel_indptr.dtype], _ptr(p.data), _ptr(p.kernel_indices),
-            p.kernel_indptr.data_ptr(), _ptr(B), B.stride(0) if B.shape[0] > 1 else B.shape[1], _ptr(C), C.stride(0),
-            p.n_rows, p.n_cols, int(B.shape[1]), p.data.numel(), _stream_ptr(dev),
-        )
-    _lib.check(rc, "fsb_spmm_csr_wide")
-
-
 def _spmm_launch_stored(prepared, B, C):
     """Enqueue C = A B for float16 / bfloat16 / complex values with B and C in the matrix's own type: the tiled kernel,
-    which reads 2-byte values as they are and rounds every element of C once."""
+    which reads 2-byte values as they are and rounds every element of C once.  Stands in for the reference's base launch
+    on these types (_triton_spmm_csr_impl, spmm_csr.py:525-599)."""
     p = prepared
     dev = p.data.device
     n_dense, nnz = int(B.shape[1]), p.data.numel()
@@ -482,20 +465,6 @@ def _spmm_launch_stored(prepared, B, C):
 def _run_spmm(prepared, B, out, return_time):
     dev, dtype = prepared.data.device, prepared.data.dtype
     shape = (prepared.n_rows, int(B.shape[1]))
-    if prepared.wide is not None and B.device.type != "cuda":   # host stand-ins take fsb_spmm_csr_wide's operands
-        t0 = None
-        if return_time:
-            torch.cuda.synchronize(dev)
-            t0 = time.perf_counter()
-        C = widetypes.run(prepared, B, _spmm_launch_wide, shape)
-        elapsed_ms = None
-        if return_time:
-            torch.cuda.synchronize(dev)
-            elapsed_ms = (time.perf_counter() - t0) * 1000.0
-        if out is not None:
-            out.copy_(C)
-            C = out
-        return (C, elapsed_ms) if return_time else C
     # float16 / bfloat16 / complex products never write into `out` while B is still read: it may be B itself there
     direct = out is not None and out.is_contiguous() and not out.is_neg() and prepared.wide is None
     C = out if direct else torch.empty(shape, dtype=dtype, device=dev)

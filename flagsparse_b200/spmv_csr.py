@@ -113,7 +113,10 @@ class PreparedCsrSpmv:
 
     Carries the attributes of the reference's class (spmv_csr.py:9-58) plus the tile plan and scratch of
     the stream kernel.  `opt_buckets` describes the plan (the reference lists row ids per length bucket
-    there).  One prepared object owns one scratch buffer: calls that share it must not overlap on the GPU.
+    there).  Calls on one prepared matrix may overlap in several streams where each brings the scratch it needs: matrices
+    of less than _STREAM_MIN_NNZ entries, float16 / bfloat16 / complex values, and every matrix that takes the
+    lanes-per-row or the panel kernel, which need none.  Larger matrices on the stream kernel, and matrices whose long rows
+    were split off, own one buffer that their calls share: these calls must not overlap on the GPU.
     """
 
     __slots__ = (
@@ -143,7 +146,7 @@ class PreparedCsrSpmv:
         self.scratch = scratch
         self.panel = panel
         self.long_rows = long_rows   # (prepared short-row part, LongRowLayout) when the long rows were split off
-        # float16 / bfloat16 / complex values: ("native", []) -- the product goes through fsb_spmv_csr_wide
+        # float16 / bfloat16 / complex values: ("native", []) -- the product goes through fsb_spmv_csr_stored
         self.wide = wide
         n_tiles = 0 if tile_row is None else tile_row.numel() - 1
         kind = {_lib.FSB_SPMV_STREAM: "stream", _lib.FSB_SPMV_PANEL: "panel"}.get(algo, "vector")
@@ -157,9 +160,6 @@ class PreparedCsrSpmv:
         if self.long_rows is not None:
             yield self.long_rows[1].status
             yield from self.long_rows[0]._status_words()
-        if self.wide is not None:
-            for part in self.wide[1]:
-                yield from part._status_words()
 
     def check_status(self):
         """Wait for the last product on this matrix and raise RuntimeError if one of its kernels gave up on a
@@ -277,7 +277,7 @@ def _prepare_spmv_csr(data, indices, indptr, shape, block_nnz, max_segments, reu
         # float16 / bfloat16 / complex values are read as they are stored by kernels of their own (fsb_spmv_csr_stored):
         # no second copy of the matrix, and a tile plan where the row lengths call for one
         tile_nnz, tile_row = 0, None
-        if nnz > 0 and n_rows > 0 and data.device.type == "cuda" and _uneven_rows(n_rows, nnz, max_row_nnz, data.element_size()):
+        if nnz > 0 and n_rows > 0 and _uneven_rows(n_rows, nnz, max_row_nnz, data.element_size()):
             tile_nnz = int(_lib.lib().fsb_spmv_stored_tile_nnz(_WIDE_VTYPE[data.dtype]))
             tile_row = _tile_plan(kernel_indptr, n_rows, nnz, tile_nnz)
         return PreparedCsrSpmv(
@@ -360,24 +360,9 @@ def _spmv_launch(prepared, x, y):
     _lib.check(rc, "fsb_spmv_csr")
 
 
-def _spmv_launch_wide(prepared, x, y):
-    """Enqueue y = A x for float16 / bfloat16 / complex values (fsb_spmv_csr_wide): x and y are float32 for the
-    half precisions and of the matrix's own type for complex values.  Stands in for the reference's base launch
-    helper on these types (_triton_spmv_csr_impl_prepared, :510-554)."""
-    p = prepared
-    dev = p.data.device
-    if p.n_rows == 0:
-        return
-    with _on_device(dev):
-        rc = _lib.lib().fsb_spmv_csr_wide(
-            _WIDE_VTYPE[p.data.dtype], _ITYPE[p.kernel_indptr.dtype], _ptr(p.data), _ptr(p.kernel_indices),
-            p.kernel_indptr.data_ptr(), _ptr(x), _ptr(y), p.n_rows, p.n_cols, p.data.numel(), _stream_ptr(dev),
-        )
-    _lib.check(rc, "fsb_spmv_csr_wide")
-
-
 def _spmv_launch_stored(prepared, x, y):
-    """Enqueue y = A x for float16 / bfloat16 / complex values with x and y in the matrix's own type."""
+    """Enqueue y = A x for float16 / bfloat16 / complex values with x and y in the matrix's own type.  Stands in for the
+    reference's base launch on these types (spmv_csr.py:510-554)."""
     p = prepared
     dev = p.data.device
     if p.n_rows == 0:
@@ -420,11 +405,8 @@ def flagsparse_spmv_csr(data=None, indices=None, indptr=None, x=None, shape=None
         if return_time:
             torch.cuda.synchronize(dev)
             t0 = time.perf_counter()
-        if x.device.type == "cuda":
-            y = torch.empty(prepared.n_rows, dtype=dtype, device=dev)   # not `out`, which may be x itself
-            _spmv_launch_stored(prepared, x, y)
-        else:                                     # host stand-ins take fsb_spmv_csr_wide's operands
-            y = widetypes.run(prepared, x, _spmv_launch_wide, (prepared.n_rows,))
+        y = torch.empty(prepared.n_rows, dtype=dtype, device=dev)   # not `out`, which may be x itself
+        _spmv_launch_stored(prepared, x, y)
         elapsed_ms = None
         if return_time:
             torch.cuda.synchronize(dev)

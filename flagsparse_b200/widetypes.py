@@ -5,14 +5,9 @@ half precisions run its float32 kernel on `data.to(float32)` and `x.to(float32)`
 (src/flagsparse/sparse_operations/spmv_csr.py:496-535, spmm_csr.py:525-560 of the reference), complex values run a
 kernel over the interleaved real view (spmv_csr.py:123-155, 536-554; spmm_csr.py:138-195).  On the GPU the entry points
 hand matrix and dense operand to fsb_spmv_csr_stored / fsb_spmm_csr_stored as they are (2 bytes per half-precision
-value, interleaved pairs for complex values; sums in float32, one rounding).  This module is the contract of
-fsb_spmv_csr_wide / fsb_spmm_csr_wide, whose dense operands the caller widens:
-  * float16 / bfloat16: the dense operand is widened to float32 once per call, products and sums are float32, the
-    float32 result is rounded once to the caller's type;
-  * complex: operand and result stay in the caller's type.
-`dense_dtype` says which type the kernel's dense operand and result have; `run` does the widening, the launch and
-the rounding around a caller-supplied `launch(prepared, dense operand, dense result)`, which is the CUDA launch or a
-host stand-in in the CPU tests.
+value, interleaved pairs for complex values; sums in float32, one rounding).  `dense_dtype` is the type that the C entry
+points fsb_spmv_csr_wide / fsb_spmm_csr_wide take their dense operand and result in: float32 for the half precisions
+(the caller widens the one and rounds the other), the caller's type for complex values.
 """
 
 import torch
@@ -29,16 +24,3 @@ def dense_dtype(dtype):
     if dtype in COMPLEX_DTYPES:
         return dtype
     raise TypeError(f"{dtype} has kernels of its own")
-
-
-def run(prepared, operand, launch, out_shape):
-    """prepared.data @ operand for a matrix of one of the four types; operand is x (1-D) or B (2-D, unit stride
-    along a row) of the matrix's dtype.  Returns a new tensor of that dtype."""
-    dtype = prepared.data.dtype
-    dense = dense_dtype(dtype)
-    o = operand if operand.dtype == dense else operand.to(dense)
-    if o.ndim == 1 or o.stride(-1) != 1 or (o.shape[0] > 1 and o.stride(0) < o.shape[1]):
-        o = o.contiguous()
-    result = torch.empty(out_shape, dtype=dense, device=operand.device)
-    launch(prepared, o, result)
-    return result if dense == dtype else result.to(dtype)

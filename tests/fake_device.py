@@ -47,7 +47,7 @@ class Launches:
     """Stand-ins for _spmv_launch / _spmm_launch that also record what they were asked to run."""
 
     def __init__(self):
-        self.spmv, self.spmm = [], []
+        self.spmv, self.spmm, self.spmm_operands = [], [], []
 
     def spmv_launch(self, prepared, x, y):
         assert prepared.data.dtype in (torch.float32, torch.float64), "the kernels compute float32 / float64 only"
@@ -59,30 +59,33 @@ class Launches:
         if prepared.n_rows:
             y.copy_(torch.from_numpy(np.asarray(_matrix(prepared) @ x.numpy(), dtype=x.numpy().dtype)))
 
-    def spmv_launch_wide(self, prepared, x, y):
-        """Stand-in for fsb_spmv_csr_wide: the matrix as stored, x and y float32 (half precisions) or complex."""
+    @staticmethod
+    def _stored_product(prepared, operand, result):
+        """Half precisions: float32 products and sums of the stored values, rounded once; complex: in their own type."""
         dt = prepared.data.dtype
-        half = dt in (torch.float16, torch.bfloat16)
         assert dt in (torch.float16, torch.bfloat16, torch.complex64, torch.complex128)
-        assert x.dtype == y.dtype == (torch.float32 if half else dt) and x.is_contiguous() and y.is_contiguous()
-        self.spmv.append("wide")
-        vals = prepared.data.to(torch.float32 if half else dt).numpy()
-        a = sp.csr_matrix((vals, prepared.kernel_indices.numpy(), prepared.kernel_indptr.numpy()),
+        assert operand.dtype == result.dtype == dt and prepared.kernel_indices.dtype == torch.int32
+        assert result.is_contiguous() and result.data_ptr() != operand.data_ptr()
+        acc = torch.float32 if dt in (torch.float16, torch.bfloat16) else dt
+        a = sp.csr_matrix((prepared.data.to(acc).numpy(), prepared.kernel_indices.numpy(), prepared.kernel_indptr.numpy()),
                           shape=(prepared.n_rows, prepared.n_cols))
-        if prepared.n_rows:
-            y.copy_(torch.from_numpy(np.asarray(a @ x.numpy(), dtype=x.numpy().dtype)))
+        if result.numel():
+            o = operand.to(acc).numpy()
+            result.copy_(torch.from_numpy(np.asarray(a @ o, dtype=o.dtype)))
 
-    def spmm_launch_wide(self, prepared, B, C):
-        """Stand-in for fsb_spmm_csr_wide."""
-        dt = prepared.data.dtype
-        half = dt in (torch.float16, torch.bfloat16)
-        assert B.dtype == C.dtype == (torch.float32 if half else dt) and B.stride(-1) == 1
+    def spmv_launch_stored(self, prepared, x, y):
+        """Stand-in for fsb_spmv_csr_stored: matrix, x and y as stored."""
+        assert x.is_contiguous() and x.shape == (prepared.n_cols,) and y.shape == (prepared.n_rows,)
+        self.spmv.append("wide")
+        self._stored_product(prepared, x, y)
+
+    def spmm_launch_stored(self, prepared, B, C):
+        """Stand-in for fsb_spmm_csr_stored: B with unit stride along a row and any stride between rows."""
+        assert (B.shape[1] <= 1 or B.stride(1) == 1) and (B.shape[0] <= 1 or B.stride(0) >= B.shape[1])
+        assert C.shape == (prepared.n_rows, B.shape[1])
         self.spmm.append(("wide", int(B.shape[1])))
-        vals = prepared.data.to(torch.float32 if half else dt).numpy()
-        a = sp.csr_matrix((vals, prepared.kernel_indices.numpy(), prepared.kernel_indptr.numpy()),
-                          shape=(prepared.n_rows, prepared.n_cols))
-        if prepared.n_rows and B.shape[1]:
-            C.copy_(torch.from_numpy(np.asarray(a @ B.numpy(), dtype=B.numpy().dtype)))
+        self.spmm_operands.append((B.dtype, B.is_contiguous(), B.stride()))
+        self._stored_product(prepared, B, C)
 
     def spmm_launch(self, prepared, B, C):
         assert prepared.data.dtype in (torch.float32, torch.float64)
@@ -102,10 +105,10 @@ def fake_cuda():
         mock.patch.object(spmv_csr, "_tile_plan", fake_tile_plan),
         mock.patch.object(spmm_csr, "_tile_plan", fake_tile_plan),
         mock.patch.object(spmv_csr, "_spmv_launch", launches.spmv_launch),
-        mock.patch.object(spmv_csr, "_spmv_launch_wide", launches.spmv_launch_wide),
+        mock.patch.object(spmv_csr, "_spmv_launch_stored", launches.spmv_launch_stored),
         mock.patch.object(coo, "_spmv_launch", launches.spmv_launch),
         mock.patch.object(spmm_csr, "_spmm_launch", launches.spmm_launch),
-        mock.patch.object(spmm_csr, "_spmm_launch_wide", launches.spmm_launch_wide),
+        mock.patch.object(spmm_csr, "_spmm_launch_stored", launches.spmm_launch_stored),
         mock.patch.object(torch.cuda, "synchronize", lambda *a, **k: None),
     ]
     for p in patches:

@@ -1,6 +1,5 @@
-"""float16 / bfloat16 / complex values on CPU: the host side of the entry points (flagsparse_b200/widetypes.py:
-widening of the dense operand, one launch, one rounding) with host stand-ins for fsb_spmv_csr_wide /
-fsb_spmm_csr_wide, against exact products of the stored values and against outputs of the reference's own base
+"""float16 / bfloat16 / complex values on CPU: the host side of the entry points with host stand-ins for
+fsb_spmv_csr_stored / fsb_spmm_csr_stored, against exact products of the stored values and against outputs of the reference's own base
 paths (tests/golden/wide_*.npz)."""
 
 import numpy as np
@@ -72,20 +71,14 @@ def test_dense_types_and_strided_operands():
         with pytest.raises(TypeError):
             W.dense_dtype(dt)
 
-    class P:
-        data = torch.ones(2, dtype=torch.complex64)
-
-    seen = []
-
-    def launch(prepared, o, r):
-        seen.append((o.dtype, o.is_contiguous(), o.stride(-1)))
-        r.zero_()
-
+    data, idx, ptr = torch.ones(2, dtype=torch.complex64), torch.tensor([0, 3]), torch.tensor([0, 1, 2])
     wide = torch.zeros(6, 8, dtype=torch.complex64)
-    W.run(P, wide[:, :5], launch, (2, 5))                 # a row stride: handed on as it is
-    W.run(P, wide.t()[:5], launch, (2, 6))                # column-major: copied
-    W.run(P, wide[0, ::2], launch, (2,))                  # strided vector: copied
-    assert seen == [(torch.complex64, False, 1), (torch.complex64, True, 1), (torch.complex64, True, 1)]
+    with fake_cuda() as launches:
+        fs.flagsparse_spmm_csr(data, idx, ptr, wide[:, :5], (2, 6))               # a row stride: handed on as it is
+        fs.flagsparse_spmm_csr(data, idx, ptr, wide.t()[:6], (2, 6))              # column-major: copied
+        fs.flagsparse_spmv_csr(data, idx, ptr, wide[:, 0], (2, 6))                # strided vector: copied
+    assert launches.spmm_operands == [(torch.complex64, False, (8, 1)), (torch.complex64, True, (6, 1))]
+    assert launches.spmv == ["wide"]
 
 
 # ---- against outputs of the reference's own base paths (tests/golden/wide_*.npz) ----------------------------------

@@ -93,7 +93,7 @@ def test_spmv(cuda, fsb_lib, dtype, rows):
     assert torch.equal(fs.flagsparse_spmv_csr(d, ti, tp, tx, shape, use_opt=True), y)   # same kernels either way
     prep = fs.prepare_spmv_csr(d, ti, tp, shape)
     assert prep.data.dtype == dtype and not prep.supports_opt and prep.shape == shape
-    assert prep.wide == ("native", [])          # read as stored by fsb_spmv_csr_wide: no widened or split copy
+    assert prep.wide == ("native", [])          # read as stored by fsb_spmv_csr_stored: no widened or split copy
     y2, ms = fs.flagsparse_spmv_csr(x=tx, prepared=prep, return_time=True)
     _check(y2, vals, i, p, shape, x, dtype, "prepared")
     assert ms >= 0 and torch.equal(y2, fs.flagsparse_spmv_csr(x=tx, prepared=prep))
