@@ -252,7 +252,10 @@ def flagsparse_spmm_coo(data, row, col, B, shape, block_n=None, block_nnz=256, o
 
     The reference merges duplicate (row, col) entries, sorts and runs a kernel per row run, computing
     float32 inputs in float64.  Here the entries are sorted into row-pointer form and the SpMM kernel sums
-    duplicates as it goes, in the value dtype.  No device synchronisation unless return_time is set.
+    duplicates as it goes, in the value dtype.  The entries of a row are added in the order in which they are given: the
+    same triples give the same result on every call, the same matrix with its triples in another order gives one that
+    may differ in the rounding of the sums (flagsparse_spmv_coo orders them by column too).  No device synchronisation
+    unless return_time is set.
     """
     if block_n is not None and block_n <= 0:
         raise ValueError("block_n must be positive when provided")

@@ -38,8 +38,8 @@ __device__ __forceinline__ long long warp_sum(long long v) {
   return v;
 }
 
-// One pass over the row pointer and one over the indices, grid-stride, in one launch.  Read at 16 bytes per thread and
-// request; the statistics meet in shared memory, so that a block sends one atomic per statistic: one per warp, on six
+// One pass over the row pointer and one over the indices, grid-stride, in one launch.  Aligned indices are read at 16 bytes
+// per thread and request; the statistics meet in shared memory, so that a block sends one atomic per statistic: one per warp, on six
 // words that every block of the device shares, used to take longer than the reading (3 M entries,
 // 250007 rows, 64-bit: two launches, 33 us; 10 us in this one; 2.1 M entries, 150001 rows: 30 us and 7 us).
 template <typename I, typename P>

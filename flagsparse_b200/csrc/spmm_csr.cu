@@ -4,9 +4,9 @@
 // `data` and of `indices` is one contiguous, 16-byte aligned block.  A CTA stages its tile in shared
 // memory -- with one cp.async.bulk (TMA 1-D bulk copy) per array completing on an mbarrier, or with
 // ordinary coalesced loads -- and loads indptr[ra .. rb] as tile-relative offsets.  Then groups of LR
-// lanes (LR = columns / VW rounded up to a power of two, VW = elements per 128-bit access) each take one
-// row segment: the (value, column) pairs come from shared memory as broadcasts, each lane gathers VW
-// consecutive elements of B's row through the read-only path, and the accumulators stay in registers.
+// lanes each take one row segment (VW elements per access of at most 128 bits, LR lanes and NC accesses per
+// lane picked by spmm_shape below): the (value, column) pairs come from shared memory as broadcasts, each lane
+// gathers its elements of B's row through the read-only path, and the accumulators stay in registers.
 // This is CUDA-core work on purpose: the operand is an irregular gather with at most 0.5 flop per byte.
 // Rows ending in the tile are written to C with streaming stores; a row continuing into the next tile
 // leaves its partial row in carry[t, :], a row that began in an earlier tile leaves it in head[t, :],
@@ -146,8 +146,8 @@ struct Pack {
 };
 
 // Resident CTAs the register budget is set for.  One access per lane: 40 registers hold four gathers of 4-byte values; left
-// to itself the compiler fits 32 and issues them one after the other (54 columns, 28386 rows of 45 entries, float32: 60 us,
-// 44 us).  Four gathers and the sums of 8-byte values take 48 (float64, 60000 rows of 31, 40 / 64 / 128 columns with 40
+// to itself the compiler fits 32 at times and issues them one after the other (54 columns, 28386 rows of 45 entries, float32:
+// 39 us, 37 us).  Four gathers and the sums of 8-byte values take 48 (float64, 60000 rows of 31, 40 / 64 / 128 columns with 40
 // registers: 70.6 / 77.8 / 145 us, with 48: 59.6 / 67.7 / 130 us; with 64: 66 / 74 / 146 us).  Several accesses: 64 (60000
 // rows of 31, 65 columns with 80 registers: float32 80.0 us, float64 114 us; with 64: 78.0 us, 98.8 us), four of them 80, which
 // 64 would spill.  With long rows the pieces' arithmetic comes on top (float64, 33 columns, one row of 300 among 60000 of 31:
@@ -161,9 +161,9 @@ __host__ __device__ constexpr int mm_ctas(int nc, size_t size, bool with_long) {
 // A group of LR lanes takes one segment (the part of a row that lies in the tile) at a time, four gathers of B on their
 // way.  LONG: segments of more than 2 * piece entries are left to a second pass: cut into pieces, dealt to all groups of
 // the CTA, their partial rows added in shared memory.  Without it the group that meets a long row of a skewed matrix
-// walks it alone while the others wait (float32, 300000 rows of Zipf lengths, 3.6 M entries, 128 columns: 413 us, with it
-// 300 us; bfloat16, 200003 such rows, 4 M entries, 128 columns, through a kernel of whole rows on widened copies of B and
-// C: 6490 us, here 291 us).  Handing out equal slices of the tile instead, whatever rows they cross,
+// walks it alone while the others wait (float32, 300000 rows of Zipf lengths, 3.6 M entries, 128 columns: 402 us, with it
+// 266 us; bfloat16, 200003 such rows, 4 M entries, 128 columns, from the CSR arrays, through a kernel of whole rows on
+// widened copies of B and C: 8.8 ms, here 219 us).  Handing out equal slices of the tile instead, whatever rows they cross,
 // balances as well but pays a row-end test per entry, and an even matrix then loses what a skewed one gains (2^20 rows
 // of 16 entries, 64 columns, float32: 615 us against 531 us).  `piece` depends on the number of columns and the value
 // type only (not on the alignment, which picks VW and LR), so the order of additions does too.

@@ -290,8 +290,8 @@ int fsb_spmv_csr_noalloc(int vtype, int itype, int ptype, const void* data, cons
  *             multiply by column panels of A one after the other, each panel's slice of B small enough to stay
  *             in L2 while it is gathered from, and by column tiles of B / C (pass the tile's first element and the
  *             full leading dimensions).  FSB_SPMM_LONG_ROWS: the part of a row that lies in a tile is shared by the
- *             whole block where it has more than 64 entries (128 with 32 lanes per row); right for any
- *             matrix, and worth its shared memory where rows are longer than that.  It changes the order in which
+ *             whole block where it has more than 64 entries (128 where a row of C is longer than 256 bytes);
+ *             right for any matrix, and worth its shared memory where rows are longer than that.  It changes the order in which
  *             the entries of such rows are added.
  *   tile_row  from fsb_csr_tile_plan(tile_nnz = fsb_spmm_tile_nnz(vtype)).
  *   scratch   at least fsb_spmm_csr_scratch_bytes() bytes, 16-byte aligned (per-tile partial rows of
