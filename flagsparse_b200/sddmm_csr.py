@@ -130,7 +130,8 @@ def _resolve_out(prepared, x, out):
 
 def _unit_rows(t):
     """t as the kernel reads it: unit stride along a row, any stride between rows."""
-    t = _resolved(t)
+    if t.is_neg():                       # float32 / float64 only: nothing to conjugate
+        t = _resolved(t)
     if t.shape[1] <= 1 or t.stride(1) == 1:
         if t.shape[0] <= 1 or t.stride(0) >= t.shape[1]:
             return t

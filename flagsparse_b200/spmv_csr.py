@@ -221,11 +221,11 @@ def _prepare_spmv_csr_matrix(data, indices, indptr, shape, narrow=True):
 def _validate_spmv_x(x, prepared):
     """x against a prepared matrix: the checks of the reference's _validate_spmv_x (spmv_csr.py:439-452) in its
     order, each with the exception type it raises there.  Returns x, contiguous."""
-    if not torch.is_tensor(x):            # None included
+    if not isinstance(x, torch.Tensor):   # None included
         raise TypeError("x has to be a torch.Tensor")
     a = prepared.data
-    if x.ndim == 1 and x.is_cuda and x.dtype == a.dtype and x.shape[0] == prepared.n_cols and x.device == a.device:
-        return _resolved(x).contiguous()
+    if x.ndim == 1 and x.dtype == a.dtype and x.numel() == prepared.n_cols and x.device == a.device:
+        return (_resolved(x) if x.is_neg() or x.is_conj() else x).contiguous()
     for failed, exc, why in (
         (x.ndim != 1, ValueError, "x has to be one-dimensional"),
         (not x.is_cuda, ValueError, "x has to live on a CUDA device"),
