@@ -113,9 +113,9 @@ def _prepare_spmm_csr_matrix(data, indices, indptr, shape, narrow=True):
         raise ValueError(f"indptr length must be n_rows+1={n_rows + 1}, got {indptr.numel()}")
     if data.numel() != indices.numel():
         raise ValueError("data and indices must have the same length (nnz)")
-    if not all(t.is_cuda for t in (data, indices, indptr)):
+    if not (data.is_cuda and indices.is_cuda and indptr.is_cuda):
         raise ValueError("data, indices, and indptr must be CUDA tensors")
-    if not all(t.device == data.device for t in (indices, indptr)):
+    if indices.device != data.device or indptr.device != data.device:
         raise ValueError("data, indices, and indptr must be on the same CUDA device")
     _check_value_dtype(data.dtype)
     if indices.dtype not in SUPPORTED_INDEX_DTYPES:
@@ -162,7 +162,8 @@ def _check_spmm_dense(B, data, n_cols):
 def _row_major(B):
     """B as the kernel can read it: unit stride along a row, any stride between rows (the reference copies every
     non-contiguous B, spmm_csr.py:280; a row-strided view needs no copy here)."""
-    B = _resolved(B)
+    if B.is_neg() or B.is_conj():
+        B = _resolved(B)
     if B.shape[1] <= 1 or B.stride(1) == 1:
         if B.shape[0] <= 1 or B.stride(0) >= B.shape[1]:
             return B
@@ -411,7 +412,7 @@ def _spmm_launch(prepared, B, C):
         status = p.status_word()
         status.poll()
     sv = B.element_size()
-    if _shares_long_rows(p.max_row_nnz, n_dense, sv):
+    if p.max_row_nnz > LONG_ROW_NNZ and _shares_long_rows(p.max_row_nnz, n_dense, sv):
         algo |= _lib.FSB_SPMM_LONG_ROWS
     vt, it, pt = _VTYPE[p.data.dtype], _ITYPE[p.kernel_indices.dtype], _ITYPE[p.kernel_indptr.dtype]
     ldb, ldc = B.stride(0), C.stride(0)

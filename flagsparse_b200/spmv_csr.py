@@ -175,7 +175,7 @@ def _prepare_spmv_csr_matrix(data, indices, indptr, shape, narrow=True):
     width (a one-shot product reads them once: the kernels take either, and a pass that narrows them moves more than it
     saves).  Returns (data, kernel_indices, kernel_indptr, n_rows,
     n_cols, stats)."""
-    if not all(torch.is_tensor(t) for t in (data, indices, indptr)):
+    if not (torch.is_tensor(data) and torch.is_tensor(indices) and torch.is_tensor(indptr)):
         raise TypeError("data, indices and indptr have to be torch.Tensor objects")
     if data.ndim != 1 or indices.ndim != 1 or indptr.ndim != 1:
         raise ValueError("data, indices and indptr have to be one-dimensional")
@@ -184,7 +184,7 @@ def _prepare_spmv_csr_matrix(data, indices, indptr, shape, narrow=True):
         raise ValueError(f"indptr has {indptr.numel()} entries, {n_rows} rows need {n_rows + 1}")
     if data.numel() != indices.numel():
         raise ValueError(f"{data.numel()} values but {indices.numel()} column indices")
-    if not all(t.is_cuda for t in (data, indices, indptr)):
+    if not (data.is_cuda and indices.is_cuda and indptr.is_cuda):
         raise ValueError("data, indices and indptr have to live on a CUDA device")
     _check_value_dtype(data.dtype)
     if indices.dtype not in SUPPORTED_INDEX_DTYPES:
