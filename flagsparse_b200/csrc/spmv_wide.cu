@@ -571,12 +571,13 @@ static int stored_launch(const void* data_, const int32_t* idx, const void* ptr_
     }
     return FSB_OK;
   }
-  // two to four groups of four entries per lane, as in the float32 / float64 kernel; entry by entry, four to eight
-  // (complex64, columns anywhere, at most 4 / 8 / 16 per lane: 500009 rows of 24: 64 / 70 / 87 us, 300000 rows of 30: 51 / 47 /
-  // 55 us, 2000000 rows of 20: 212 / 209 / 270 us; complex128: 78 / 84 / 97 us, 64 / 58 / 66 us, 294 / 289 / 344 us)
+  // two to four groups of four entries per lane, as in the float32 / float64 kernel; entry by entry, three to six
+  // (columns anywhere, 4 / 8 / 16 lanes a row: complex64, 500009 rows of 24: 70 / 64 / - us, 300000 rows of 30: 55 / 47 / 51 us,
+  // 2000000 rows of 20: 209 / 212 / - us, 100000 rows of 60: - / 35 / 31 us; complex128: 84 / 78 / - us, 66 / 58 / 64 us, 289 / 294
+  // / - us, - / 41 / 37 us)
   const int64_t mean = n_rows > 0 ? nnz / n_rows : 0;
   int L = 2;
-  while (L < 32 && (groups ? 16 : 8) * L < mean + 3) L <<= 1;
+  while (L < 32 && (groups ? 16 : 6) * L < mean + 3) L <<= 1;
   const int64_t blocks = (n_rows * L + kWideThreads - 1) / kWideThreads;
   if (blocks >= INT32_MAX) return FSB_ERANGE;
 #define FSB_STORED_CASE(L_)                                                                                           \
