@@ -19,9 +19,10 @@ from ._common import StatusWord, _VTYPE
 SM_COUNT_FALLBACK = 148
 CTAS_PER_SM = 1              # one 1024-thread CTA (row block) per SM
 # the kernel is worth its second copy of the matrix only when the extra reads of x and the padding stay small
-# bytes of x chunks loaded / bytes of entries streamed.  float32: measured on a band of +-2^20 columns (0.89: 319 G
-# entries/s against 231 G/s of the vector kernel; the SM's intake of about 37 GB/s is what bounds it, which puts the
-# break-even near 1.9).  float64 entries are 12 bytes and their chunks hold half the columns: estimate, not measured.
+# bytes of x chunks loaded / bytes of entries streamed.  float32: a band of +-2^20 columns has 0.89 (319 G entries/s against
+# 231 G/s of the vector kernel; bound by the shared-memory work per entry and the barrier per unit, not by these bytes: half
+# of every chunk left out changes the time by 3 to 4 %).  Both lines are estimates above that, the break-even is not measured;
+# float64 entries are 12 bytes and their chunks hold half the columns.
 MAX_X_OVERHEAD = 1.3
 MAX_X_OVERHEAD_F64 = 0.8
 MAX_SLOT_OVERHEAD = 1.25    # slots stored / entries
