@@ -88,24 +88,32 @@ def _select_spmv_algo(n_rows, nnz, max_row_nnz, element_size=4):
     return _lib.FSB_SPMV_STREAM
 
 
-# Longest row from which the tiled kernel for float16 / bfloat16 / complex values is taken, whatever the mean: a row of n
-# entries takes its few lanes 0.03 to 0.04 us per entry (0.07 us while others keep memory busy), the tiled kernel a second
-# launch, and complex values their way through shared memory: 6 % of complex64, 25 % of complex128.  So the line rises with the
-# number of entries, one per _UNEVEN_ENTRIES[bytes per value].  Lanes per row against tiles, longest row 200 / 300 / 400 / 600
-# / 1000 / 2000: 30000 rows of 16, bfloat16: 14 / 19 / 22 / 31 / 45 / 81 us against 16 us, complex128: 14 / 17 / 21 / 29 / 47 / 86 us
-# against 16 us; 500009 rows of 24, complex64: 70 / 70 / 76 / 88 / 112 / 182 us against 74 us, complex128: 87 / 87 / 87 / 101 / 139
-# / 221 us against 113 us; 2000000 rows of 20, complex64: 210 / 210 / 211 / 211 / 219 / 273 us against 225 us, complex128: 292 /
-# 294 / 301 / 300 / 299 / 357 us against 359 us.
+# Longest row from which the tiled kernel for float16 / bfloat16 / complex values is taken.  A row of n entries takes its L
+# lanes about 0.15 n / L us (complex), and twice that while others keep memory busy; the tiled kernel takes a second launch,
+# and complex values their way through shared memory: 6 to 15 % of complex64, 25 to 45 % of complex128.  So the line for
+# complex values is a number of entries per lane, or a share of all entries where that is more (_UNEVEN_ENTRIES[bytes per
+# value], for four lanes).  Lanes per row against tiles, longest row 200 / 300 / 400 / 600 / 1000 / 2000:
+# 30000 rows of 16, complex64: 12 / 16 / 19 / 25 / 39 / 74 us against 15 us, complex128: 14 / 18 / 23 / 29 / 47 / 88 us against 15 us,
+# bfloat16: 14 / 19 / 22 / 31 / 45 / 81 us against 16 us;
+# 500009 rows of 24, complex64: 64 / 64 / 64 / 66 / 82 / 124 us against 74 us, complex128: 80 / 81 / 84 / 83 / 101 / 158 us against
+# 113 us, bfloat16: 64 / 69 / 76 / 92 / 119 / 197 us against 60 us;
+# 2000000 rows of 20, complex64: 209 / 214 / 213 / 213 / 220 / 272 us against 223 us, complex128: 295 / 305 / 303 / 300 / 302 / 362 us
+# against 359 us, bfloat16: 187 / 187 / 187 / 187 / 215 / 290 us against 176 us.
 _UNEVEN_MIN = 288
+_UNEVEN_PER_LANE = 72
 _UNEVEN_ENTRIES = {8: 35000, 16: 18000}
 
 
 def _uneven_rows(n_rows, nnz, max_row_nnz, element_size):
     """Whether the longest row leaves the lanes-per-row kernel for float16 / bfloat16 / complex values waiting for it."""
-    line = max(_UNEVEN_MIN, _UNIFORM_ROW_FACTOR * (nnz / max(n_rows, 1)) + _UNIFORM_ROW_SLACK)
-    if element_size in _UNEVEN_ENTRIES:
-        line = max(line, nnz / _UNEVEN_ENTRIES[element_size])
-    return max_row_nnz > line
+    mean = nnz / max(n_rows, 1)
+    line = _UNIFORM_ROW_FACTOR * mean + _UNIFORM_ROW_SLACK
+    if element_size not in _UNEVEN_ENTRIES:
+        return max_row_nnz > max(line, _UNEVEN_MIN)
+    lanes = 2                            # as stored_launch in csrc/spmv_wide.cu gives them to a row
+    while lanes < 32 and 6 * lanes < int(mean) + 3:
+        lanes *= 2
+    return max_row_nnz > max(line, _UNEVEN_PER_LANE * lanes, nnz / _UNEVEN_ENTRIES[element_size] * lanes / 4)
 
 
 class PreparedCsrSpmv:

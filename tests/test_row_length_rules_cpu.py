@@ -7,9 +7,10 @@ from flagsparse_b200 import _lib, spmv_csr as M
 
 @pytest.mark.parametrize("size", [2, 8, 16])
 def test_stored_types(size):
-    # (rows, entries) -> longest row that still goes to lanes per row: a floor, a multiple of the mean, a share of the entries
-    for n_rows, nnz, line in ((4096, 1 << 16, 288), (1000, 200000, 1664), (0, 0, 288),
-                              (2000000, 40000000, {2: 288, 8: 1142, 16: 2222}[size])):
+    # (rows, entries) -> longest row that still goes to lanes per row
+    for n_rows, nnz, half, c64, c128 in ((4096, 1 << 16, 288, 288, 288), (1000, 200000, 1664, 2304, 2304), (0, 0, 288, 144, 144),
+                                         (500000, 12000000, 288, 685, 1333), (2000000, 40000000, 288, 1142, 2222)):
+        line = {2: half, 8: c64, 16: c128}[size]
         assert not M._uneven_rows(n_rows, nnz, line, size) and M._uneven_rows(n_rows, nnz, line + 1, size)
 
 
