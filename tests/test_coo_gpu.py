@@ -173,3 +173,17 @@ def test_coo_argument_contract(cuda, fsb_lib):
     y = fs.flagsparse_spmv_coo(d, r, c, x, (2, 2))
     assert y.tolist() == [1.0, 5.0]
     assert fs.flagsparse_spmm_coo(d, r, c, B, (2, 2)).tolist() == [[1.0] * 3, [5.0] * 3]
+
+
+@pytest.mark.parametrize("vt", [np.float32, np.float64])
+def test_spmm_coo_in_any_order_of_the_triples(vt, cuda, fsb_lib):
+    """The entries of a row are added in the order given: the same bits for the same triples, the bound for any order."""
+    val, row, col = _random_coo(21, 300, 400, 9000, vt=vt, ct=np.int64, skew=True)
+    B = np.random.default_rng(22).uniform(-1, 1, (400, 9)).astype(vt)
+    d, i, p = _rowptr_form(val, row, col, 300)
+    for seed in range(3):
+        order = np.random.default_rng(seed).permutation(val.size)
+        args = [torch.from_numpy(a[order]).to(cuda) for a in (val, row, col)]
+        C = fs.flagsparse_spmm_coo(*args, torch.from_numpy(B).to(cuda), (300, 400))
+        assert torch.equal(fs.flagsparse_spmm_coo(*args, torch.from_numpy(B).to(cuda), (300, 400)), C)
+        assert_spmm_ok(C.cpu().numpy(), d, i, p, (300, 400), B, what=f"order {seed}")
