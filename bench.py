@@ -552,10 +552,11 @@ class SingleGpuWorkload:
             self.nbytes = spmv_bytes(spec.n_rows, spec.n_cols, self.nnz, sv, si, sp_)
             self.flops = 2.0 * self.nnz
             self.kernel = self.prep.opt_buckets[0]["kind"]
-            self.launches = 2 if self.prep.algo == _lib.FSB_SPMV_STREAM else 1
+            self.launches = 2 if self.prep.algo == _lib.FSB_SPMV_STREAM or self.prep.bins is not None else 1
             if self.prep.long_rows is not None:
                 short = self.prep.long_rows[0]
-                self.launches = (2 if short.algo == _lib.FSB_SPMV_STREAM and short.tile_row is not None else 1) + 2
+                self.launches = (2 if short.bins is not None
+                                 or (short.algo == _lib.FSB_SPMV_STREAM and short.tile_row is not None) else 1) + 2
 
     def describe(self):
         """Layout facts of the prepared matrix for the JSON line."""
@@ -797,7 +798,7 @@ def run_sharded(args, workload, torch, device, rank, world):
         si, sp_ = op.prepared.kernel_indices.element_size(), op.prepared.kernel_indptr.element_size()
         nbytes = spmv_bytes(spec.n_rows, spec.n_cols, nnz, dense.element_size(), si, sp_)
         flops = 2.0 * nnz
-        launches = 2 if op.prepared.algo == _lib.FSB_SPMV_STREAM else 1
+        launches = 2 if op.prepared.algo == _lib.FSB_SPMV_STREAM or op.prepared.bins is not None else 1
         if op._slices is not None and op.prepared.algo == _lib.FSB_SPMV_PANEL:
             launches = len(op._slices)
             extra["slices"] = [e - b for b, e, _, _ in op._slices]

@@ -1,0 +1,152 @@
+"""Prepare-time regrouping of a CSR matrix for the two-pass SpMV (csrc/spmv_bins.cu): for matrices whose columns lie all
+over a long x and whose rows have nothing to share in a chunk of it.
+
+The reference's prepare step builds row-length buckets (src/flagsparse/sparse_operations/spmv_csr.py:281-327); this one
+stores the entries a second time, by (chunk of columns, block of rows), so that the product reads x from shared memory and
+everything else in order.  One count and one placing kernel, a cumulative sum over the units between them.
+"""
+
+import os
+
+import torch
+
+from . import _lib
+from ._common import _ITYPE, _VTYPE
+
+# Where the two passes win, each line with both sides measured (us, one pass against two; columns anywhere unless said).
+# Rows of about equal length against the lanes-per-row kernel, float32: 2^27 entries in 33.6 M / 16.8 M / 4.2 M rows: 1324 / 627 /
+# 551 against 631 / 534 / 479; 2^24 entries in 4.2 M / 1 M / 0.5 M rows: 94 / 76 / 76 against 74 / 64 / 65; 2^23 entries: 48 / 41 / 40
+# against 42 / 39 / 39, which a few hundred microseconds of prepare would not be worth; 2^22: 25 / 22 / 21 against 27 / 27 / 24.
+EVEN_MIN_NNZ = 1 << 24
+EVEN_MIN_SPAN = 2 << 20
+# Uneven rows (the short rows of a skewed matrix, mostly), float32: 107 M entries 640 against 444; 10.8 M entries in 2.1 M rows 87
+# against 45; 2.3 M entries in 0.3 M rows 20.7 against 18.6; 2.0 M entries in 0.1 M rows 18.0 against 18.6.
+UNEVEN_MIN_NNZ = 5 << 19
+UNEVEN_MIN_SPAN = 1 << 20
+# float64 moves 28.5 bytes an entry instead of 12, so it takes an x that L2 does not hold: 2^27 entries in 33.6 M / 16.8 M / 8.4 M
+# rows: 2157 / 1335 / 724 against 1502 / 1194 / 1017; uneven, 2^26 entries in 16.8 M / 8.4 M rows: 471 / 254 against 398 / 274.
+F64_MIN_SPAN = 120 << 20
+# ... or uneven rows of a few entries that would have gone to the lanes-per-row kernel, whose warps wait for their longest row:
+# 4.0 M entries in 2.1 M rows 62 against 45, 3.0 M in 1 M rows 41 against 33; 2.6 M in 0.5 M rows 29.5 against 29.4.
+F64_SHORT_MEAN = 4
+# mean entries of a unit below which the packs would mostly be padding (measured down to 36 and 9 entries, float32 and float64)
+MIN_UNIT = {4: 16, 8: 8}
+
+
+def _enabled():
+    """FSB_SPMV_BINS=0 keeps the one-pass kernels."""
+    return os.environ.get("FSB_SPMV_BINS", "1") != "0"
+
+
+def min_span(nnz, n_rows, max_row_nnz, element_size, lanes_per_row):
+    """Bytes of x that a row block has to reach for the two passes to pay, or None where they never do.  lanes_per_row: the
+    matrix would otherwise go to the lanes-per-row kernel."""
+    mean = nnz / max(n_rows, 1)
+    uneven = max_row_nnz > 2 * mean + 16
+    if element_size == 4:
+        if nnz >= EVEN_MIN_NNZ and not uneven:
+            return EVEN_MIN_SPAN
+        return UNEVEN_MIN_SPAN if uneven and nnz >= UNEVEN_MIN_NNZ else None
+    if uneven and lanes_per_row and mean <= F64_SHORT_MEAN and nnz >= UNEVEN_MIN_NNZ:
+        return UNEVEN_MIN_SPAN
+    return F64_MIN_SPAN if nnz >= EVEN_MIN_NNZ else None
+
+class BinsLayout:
+    """Device arrays of the regrouped matrix (include/fsb.h, fsb_spmv_csr_bins)."""
+
+    __slots__ = ("val", "col", "place", "dst", "ends", "chunk_pack", "block_pack", "block_row", "row_slot", "n_blocks", "n_chunks",
+                 "chunk_cols", "n_packs")
+
+    def nbytes(self):
+        return sum(t.numel() * t.element_size() for t in (self.val, self.col, self.place, self.dst, self.ends, self.row_slot,
+                                                          self.chunk_pack, self.block_pack, self.block_row))
+
+
+def _starts(packs):
+    """First pack of every unit (and the total) in the order of `packs`, as int32; the total again as a number (a sync)."""
+    ends = torch.cumsum(packs.reshape(-1), 0, dtype=torch.int64)
+    n = int(ends[-1])
+    out = torch.zeros(ends.numel() + 1, dtype=torch.int32, device=packs.device)
+    out[1:] = ends
+    return out, n
+
+
+def build_bins_layout(data, indices, indptr, n_rows, n_cols, max_row_nnz, span=0, chunk_cols=None):
+    """BinsLayout for float32 / float64 values on the GPU (int32 indices, at least one entry), or None when a row is too long
+    for a block, there are too many chunks or entries, or the row blocks reach less than `span` bytes of x on average (whole
+    chunks counted: then the gathers of a one-pass kernel are served close to the SM)."""
+    L = _lib.lib()
+    dev, nnz = data.device, data.numel()
+    vt, pt = _VTYPE[data.dtype], _ITYPE[indptr.dtype]
+    cap, pack, n_ends = (int(v) for v in (L.fsb_spmv_bins_cap(vt), L.fsb_spmv_bins_pack(vt), L.fsb_spmv_bins_ends()))
+    chunk_cols = chunk_cols or int(L.fsb_spmv_bins_chunk_cols(vt))
+    n_chunks = -(-n_cols // chunk_cols)
+    if max_row_nnz > cap // 4 or n_chunks > int(L.fsb_spmv_bins_max_chunks()) or n_cols * data.element_size() < span:
+        return None
+    # block b begins at the first row that starts at or behind entry b * step: at most step - 1 + max_row_nnz entries
+    step = cap - max_row_nnz + 1
+    n_blocks = -(-nnz // step)
+    if nnz // pack + n_blocks * n_chunks >= 2**31 - 1 or (indptr.dtype == torch.int32 and nnz >= 2**31 - 1 - cap):
+        return None
+    st = torch.cuda.current_stream(dev).cuda_stream
+    with torch.cuda.device(dev):
+        marks = torch.arange(n_blocks + 1, device=dev, dtype=indptr.dtype) * step
+        block_row = torch.searchsorted(indptr, marks).clamp_(max=n_rows).to(torch.int32)
+        block_row[0] = 0
+        block_row[-1] = n_rows
+        counts = torch.empty((n_blocks, n_chunks), dtype=torch.int32, device=dev)
+        _lib.check(L.fsb_spmv_bins_count(pt, indices.data_ptr(), indptr.data_ptr(), block_row.data_ptr(), n_blocks, n_chunks,
+                                         chunk_cols, n_cols, counts.data_ptr(), st), "fsb_spmv_bins_count")
+        if span and int(torch.count_nonzero(counts)) * chunk_cols * data.element_size() < span * n_blocks:   # a sync
+            return None
+        packs = (counts + (pack - 1)) // pack
+        del counts
+        unit_block, n_packs = _starts(packs)
+        by_chunk, _ = _starts(packs.t())
+        del packs
+        chunk_pack = by_chunk[::n_blocks].contiguous()
+        block_pack = unit_block[::n_chunks].contiguous()
+        unit_chunk = by_chunk[:-1].view(n_chunks, n_blocks).t().contiguous()
+        del by_chunk
+        lay = BinsLayout()
+        lay.val = torch.empty(pack * n_packs, dtype=data.dtype, device=dev)
+        lay.col = torch.empty(pack * n_packs, dtype=torch.int16, device=dev)
+        lay.place = torch.empty(n_packs, dtype=torch.int32, device=dev)
+        lay.dst = torch.empty(pack * n_packs, dtype=torch.int16, device=dev)
+        lay.ends = torch.empty(n_ends * n_blocks, dtype=torch.int32, device=dev)
+        lay.row_slot = torch.empty(n_rows, dtype=torch.int16, device=dev)
+        _lib.check(L.fsb_spmv_bins_place(vt, pt, data.data_ptr(), indices.data_ptr(), indptr.data_ptr(), block_row.data_ptr(),
+                                         n_blocks, n_chunks, chunk_cols, n_cols, unit_chunk.data_ptr(), unit_block.data_ptr(),
+                                         lay.val.data_ptr(), lay.col.data_ptr(), lay.place.data_ptr(), lay.dst.data_ptr(),
+                                         lay.ends.data_ptr(), lay.row_slot.data_ptr(), st), "fsb_spmv_bins_place")
+    lay.chunk_pack, lay.block_pack, lay.block_row = chunk_pack, block_pack, block_row
+    lay.n_blocks, lay.n_chunks, lay.chunk_cols, lay.n_packs = n_blocks, n_chunks, chunk_cols, n_packs
+    return lay
+
+
+def bins_for(data, indices, indptr, n_rows, n_cols, max_row_nnz, lanes_per_row):
+    """BinsLayout for a matrix that is multiplied again and again, or None where one pass over its entries is the better way."""
+    nnz, sv = data.numel(), data.element_size()
+    if not _enabled() or not data.is_cuda or data.device.type != "cuda" or nnz == 0 or n_rows == 0:
+        return None
+    span = min_span(nnz, n_rows, max_row_nnz, sv, lanes_per_row)
+    if span is None:
+        return None
+    L, vt = _lib.lib(), _VTYPE[data.dtype]
+    if int(L.fsb_spmv_bins_cap(vt)) * int(L.fsb_spmv_bins_chunk_cols(vt)) < MIN_UNIT[sv] * n_cols:
+        return None
+    return build_bins_layout(data, indices, indptr, n_rows, n_cols, max_row_nnz, span)
+
+
+def launch_bins(layout, x, y, n_rows, n_cols, stream_ptr):
+    """Enqueue the product on the current stream (its handle in stream_ptr).  The products' memory is the call's own: calls
+    on one matrix may overlap in several streams."""
+    la = layout
+    prod = torch.empty(32 * la.n_packs, dtype=torch.uint8, device=la.val.device)
+    rc = _lib.lib().fsb_spmv_csr_bins(
+        _VTYPE[la.val.dtype], la.val.data_ptr(), la.col.data_ptr(), la.place.data_ptr(), la.dst.data_ptr(), la.ends.data_ptr(),
+        la.row_slot.data_ptr(), la.chunk_pack.data_ptr(), la.block_pack.data_ptr(), la.block_row.data_ptr(), la.n_blocks,
+        la.n_chunks, la.chunk_cols, la.n_packs, prod.data_ptr(), prod.numel(), x.data_ptr(), y.data_ptr(), n_rows, n_cols,
+        stream_ptr,
+    )
+    _lib.check(rc, "fsb_spmv_csr_bins")

@@ -102,6 +102,50 @@ check_panel_kernel(const uint32_t* __restrict__ rc, const int32_t* __restrict__ 
   }
 }
 
+// A bins layout (spmv_bins.cu): tables first, then the entries, the places of the packs and the rows.
+__global__ void __launch_bounds__(kCheckThreads)
+check_bins_kernel(const uint16_t* __restrict__ col, const int32_t* __restrict__ place, const uint16_t* __restrict__ dst,
+                  const uint16_t* __restrict__ row_slot, const int32_t* __restrict__ chunk_pack,
+                  const int32_t* __restrict__ block_pack, const int32_t* __restrict__ block_row, int n_blocks, int n_chunks,
+                  int chunk_cols, int slots, int pack, int64_t n_packs, int64_t n_rows, int64_t n_cols) {
+  __shared__ int ok;
+  if (threadIdx.x == 0) ok = 1;
+  __syncthreads();
+  for (int c = threadIdx.x; c < n_chunks; c += kCheckThreads) {       // every CTA looks at the whole (short) tables
+    const int a = chunk_pack[c], z = chunk_pack[c + 1];
+    if (a < 0 || z < a || z > n_packs || (c == n_chunks - 1 && z != n_packs)) {
+      if (blockIdx.x == 0) note(FSB_BAD_UNIT_TABLE, c, z, a);
+      ok = 0;
+    }
+  }
+  for (int b = threadIdx.x; b < n_blocks; b += kCheckThreads) {
+    const int a = block_row[b], z = block_row[b + 1], pa = block_pack[b], pz = block_pack[b + 1];
+    if (a < 0 || z < a || z > n_rows || (b == 0 && a != 0) || (b == n_blocks - 1 && z != n_rows)) {
+      if (blockIdx.x == 0) note(FSB_BAD_ROW_ID, b, z, n_rows);
+      ok = 0;
+    }
+    if (pa < 0 || pz < pa || pz > n_packs) {
+      if (blockIdx.x == 0) note(FSB_BAD_UNIT_TABLE, b, pz, pa);
+      ok = 0;
+    }
+  }
+  __syncthreads();
+  if (!ok) return;
+  const int64_t stride = (int64_t)gridDim.x * kCheckThreads, first = (int64_t)blockIdx.x * kCheckThreads + threadIdx.x;
+  for (int64_t p = first; p < n_packs; p += stride)
+    if (place[p] < 0 || place[p] >= n_packs) note(FSB_BAD_UNIT_TABLE, p, place[p], n_packs);
+  for (int c = 0; c < n_chunks; ++c) {
+    const int64_t left = n_cols - (int64_t)c * chunk_cols;
+    const int64_t width = left < chunk_cols ? left : chunk_cols;
+    for (int64_t i = (int64_t)chunk_pack[c] * pack + first; i < (int64_t)chunk_pack[c + 1] * pack; i += stride)
+      if (col[i] >= width) note(FSB_BAD_COLUMN, i, col[i], width);
+  }
+  for (int64_t i = first; i < n_packs * pack; i += stride)
+    if (dst[i] >= slots) note(FSB_BAD_SLOT_ROW, i, dst[i], slots);
+  for (int64_t r = first; r < n_rows; r += stride)
+    if (row_slot[r] >= slots) note(FSB_BAD_SLOT_ROW, r, row_slot[r], slots);
+}
+
 static int begin_check(cudaStream_t st, void** rec) {
   cudaError_t e = cudaGetSymbolAddress(rec, g_bad);
   if (e != cudaSuccess) return cuda_rc(e);
@@ -171,6 +215,19 @@ int check_panel(const uint32_t* rc_words, const int32_t* unit_piece_ptr, const i
   check_panel_kernel<<<kCheckBlocks, kCheckThreads, 0, st>>>(rc_words, unit_piece_ptr, unit_chunk, owner_unit_ptr,
                                                             n_owners, slots, (uint32_t)max_row,
                                                             (uint32_t)(chunk_cols * n_buffers), n_chunks);
+  return end_check(st, rec);
+}
+
+int check_bins(int vtype, const uint16_t* col, const int32_t* place, const uint16_t* dst, const uint16_t* row_slot,
+               const int32_t* chunk_pack, const int32_t* block_pack, const int32_t* block_row, int n_blocks, int n_chunks,
+               int chunk_cols, int64_t n_packs, int64_t n_rows, int64_t n_cols, cudaStream_t st) {
+  void* rec = nullptr;
+  int rc = begin_check(st, &rec);
+  if (rc != FSB_OK) return rc;
+  const int slots = fsb_spmv_bins_cap(vtype) + fsb_spmv_bins_ends() + 2;
+  check_bins_kernel<<<kCheckBlocks, kCheckThreads, 0, st>>>(col, place, dst, row_slot, chunk_pack, block_pack, block_row, n_blocks,
+                                                            n_chunks, chunk_cols, slots, fsb_spmv_bins_pack(vtype), n_packs,
+                                                            n_rows, n_cols);
   return end_check(st, rec);
 }
 

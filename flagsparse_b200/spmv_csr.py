@@ -122,20 +122,20 @@ class PreparedCsrSpmv:
     Carries the attributes of the reference's class (spmv_csr.py:9-58) plus the tile plan and scratch of
     the stream kernel.  `opt_buckets` describes the plan (the reference lists row ids per length bucket
     there).  Calls on one prepared matrix may overlap in several streams where each brings the scratch it needs: matrices
-    of less than _STREAM_MIN_NNZ entries, float16 / bfloat16 / complex values, and every matrix that takes the
-    lanes-per-row or the panel kernel, which need none.  Larger matrices on the stream kernel, and matrices whose long rows
+    of less than _STREAM_MIN_NNZ entries, float16 / bfloat16 / complex values, the two-pass form, and every matrix that takes
+    the lanes-per-row or the panel kernel, which need none.  Larger matrices on the stream kernel, and matrices whose long rows
     were split off, own one buffer that their calls share: these calls must not overlap on the GPU.
     """
 
     __slots__ = (
         "data", "kernel_indices", "kernel_indptr", "shape", "n_rows", "n_cols", "block_nnz",
         "max_segments", "max_row_nnz", "opt_buckets", "supports_opt", "stats", "algo", "tuning",
-        "tile_nnz", "tile_row", "scratch", "panel", "long_rows", "wide",
+        "tile_nnz", "tile_row", "scratch", "panel", "long_rows", "wide", "bins",
     )
 
     def __init__(self, data, kernel_indices, kernel_indptr, shape, n_rows, n_cols, block_nnz,
                  max_segments, max_row_nnz, stats, algo, tuning, tile_nnz, tile_row, scratch, panel=None,
-                 long_rows=None, wide=None):
+                 long_rows=None, wide=None, bins=None):
         self.data = data
         self.kernel_indices = kernel_indices
         self.kernel_indptr = kernel_indptr
@@ -156,8 +156,11 @@ class PreparedCsrSpmv:
         self.long_rows = long_rows   # (prepared short-row part, LongRowLayout) when the long rows were split off
         # float16 / bfloat16 / complex values: ("native", []) -- the product goes through fsb_spmv_csr_stored
         self.wide = wide
+        self.bins = bins             # the entries regrouped for the two-pass kernels (bins.py)
         n_tiles = 0 if tile_row is None else tile_row.numel() - 1
         kind = {_lib.FSB_SPMV_STREAM: "stream", _lib.FSB_SPMV_PANEL: "panel"}.get(algo, "vector")
+        if bins is not None:
+            kind = "bins"
         if long_rows is not None:
             kind = "long-row panel + " + long_rows[0].opt_buckets[0]["kind"]
         self.opt_buckets = [{"kind": kind, "tile_nnz": tile_nnz, "n_tiles": n_tiles, "n_rows": n_rows}]
@@ -307,24 +310,30 @@ def _prepare_spmv_csr(data, indices, indptr, shape, block_nnz, max_segments, reu
         panel_layout = panel.build_panel_layout(data, kernel_indices, kernel_indptr, n_rows, n_cols, max_row_nnz,
                                                 force=algo == _lib.FSB_SPMV_PANEL)
         algo = _lib.FSB_SPMV_PANEL if panel_layout is not None else _lib.FSB_SPMV_VECTOR
-    if algo == _lib.FSB_SPMV_STREAM and nnz > 0 and n_rows > 0:
+    automatic = reuse_expected and os.environ.get("FSB_SPMV_ALGO", "") == ""
+    # skewed rows: the long ones leave for the row-group panel kernel, the short ones are a matrix of their own
+    long_rows = bins_layout = None
+    if algo == _lib.FSB_SPMV_STREAM and allow_split and automatic and _long_rows_enabled():
+        long_rows = _split_long_rows(data, kernel_indices, kernel_indptr, n_rows, n_cols, shape, block_nnz,
+                                     max_segments)
+    # columns all over a long x: two streaming passes instead of a gather per entry
+    if algo in (_lib.FSB_SPMV_VECTOR, _lib.FSB_SPMV_STREAM) and long_rows is None and automatic:
+        from . import bins
+
+        bins_layout = bins.bins_for(data, kernel_indices, kernel_indptr, n_rows, n_cols, max_row_nnz,
+                                    algo == _lib.FSB_SPMV_VECTOR)
+    if algo == _lib.FSB_SPMV_STREAM and bins_layout is None and nnz > 0 and n_rows > 0:
         L = _lib.lib()
         vt = _VTYPE[data.dtype]
         tile_nnz = int(L.fsb_spmv_tile_nnz(vt, tuning))
         tile_row = _tile_plan(kernel_indptr, n_rows, nnz, tile_nnz)
         scratch = torch.empty(int(L.fsb_spmv_csr_scratch_bytes(vt, nnz, tuning)), dtype=torch.uint8,
                               device=data.device)
-    # skewed rows: the long ones leave for the row-group panel kernel, the CSR kernels keep the short ones
-    long_rows = None
-    if (algo == _lib.FSB_SPMV_STREAM and allow_split and reuse_expected and _long_rows_enabled()
-            and os.environ.get("FSB_SPMV_ALGO", "") == ""):
-        long_rows = _split_long_rows(data, kernel_indices, kernel_indptr, n_rows, n_cols, shape, block_nnz,
-                                     max_segments)
     return PreparedCsrSpmv(
         data=data, kernel_indices=kernel_indices, kernel_indptr=kernel_indptr, shape=shape, n_rows=n_rows,
         n_cols=n_cols, block_nnz=block_nnz_use, max_segments=max_segments_use, max_row_nnz=max_row_nnz,
         stats=stats, algo=algo, tuning=tuning, tile_nnz=tile_nnz, tile_row=tile_row, scratch=scratch,
-        panel=panel_layout, long_rows=long_rows,
+        panel=panel_layout, long_rows=long_rows, bins=bins_layout,
     )
 
 
@@ -348,6 +357,12 @@ def _spmv_launch(prepared, x, y):
         _spmv_launch(short, x, y)      # every row of y; the long rows get zeros here
         with _on_device(dev):
             longrows.launch_long_rows(layout, x, y, p.n_cols, _stream_ptr(dev))
+        return
+    if p.bins is not None:
+        from . import bins
+
+        with _on_device(dev):
+            bins.launch_bins(p.bins, x, y, p.n_rows, p.n_cols, _stream_ptr(dev))
         return
     algo = p.algo if p.tile_row is not None else _lib.FSB_SPMV_VECTOR
     # calls on a small matrix may overlap in several streams, whichever kernel its rows get: scratch of the call's own

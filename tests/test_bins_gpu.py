@@ -1,0 +1,119 @@
+"""The two-pass SpMV (csrc/spmv_bins.cu): rows that end on, straddle and fill the slices, blocks and chunks, against the
+float64 oracle; the same bits on every call and whatever the chunks; infinities stay in their rows."""
+
+import numpy as np
+import pytest
+import torch
+
+import flagsparse_b200 as fs
+from flagsparse_b200 import _lib, bins
+from gpu_util import dev
+from helpers import assert_spmv_ok, handmade_csr
+
+pytestmark = pytest.mark.gpu
+
+
+def _layout(d, i, p, shape, chunk_cols=None):
+    lens = np.diff(p)
+    return bins.build_bins_layout(dev(d), dev(i), dev(p), shape[0], shape[1], int(lens.max()), chunk_cols=chunk_cols)
+
+
+def _product(lay, x, shape, shift=0):
+    """y into a vector that starts `shift` elements behind a 256-byte boundary."""
+    y = torch.full((shape[0] + shift,), float("nan"), dtype=x.dtype, device=x.device)[shift:]
+    bins.launch_bins(lay, x, y, shape[0], shape[1], torch.cuda.current_stream().cuda_stream)
+    return y
+
+
+_LENS = {
+    "one entry": [1],
+    "empty rows around": [0] * 9 + [3, 0, 0, 1] + [0] * 5,
+    "slice edges": [31, 1, 32, 33, 15, 1, 16, 17, 64, 0, 95, 5],
+    "rows over many threads": [2000, 1, 0, 3000, 33, 2500] * 9,
+    "one block exactly": {4: [512] * 48, 8: [256] * 48},
+    "one entry more than a block": {4: [512] * 48 + [1], 8: [256] * 48 + [1]},
+    "many blocks, short rows": list(np.random.default_rng(5).integers(0, 12, 30001)),
+    "no row ends in a warp": [3001] + [1] * 40,
+}
+
+
+@pytest.mark.parametrize("name", sorted(_LENS))
+@pytest.mark.parametrize("vdt,pdt", [("float32", "int32"), ("float64", "int64")])
+def test_edges(cuda, fsb_lib, name, vdt, pdt):
+    lens = _LENS[name]
+    lens = lens[np.dtype(vdt).itemsize] if isinstance(lens, dict) else lens
+    n_cols = 3001
+    d, i, p = handmade_csr(11, lens, n_cols, value_dtype=vdt, indptr_dtype=pdt, replace=True, sort=False)
+    shape = (len(lens), n_cols)
+    x = np.random.default_rng(3).uniform(-1, 1, n_cols + 1).astype(vdt)
+    want = None
+    for chunk_cols, shift in ((None, 0), (400, 1), (3004, 3)):     # one chunk; eight, the last one ragged; x and y off 16 bytes
+        lay = _layout(d, i, p, shape, chunk_cols)
+        tx = dev(x)[1:] if shift else dev(x[1:])
+        y = _product(lay, tx, shape, shift)
+        assert_spmv_ok(y.cpu().numpy(), d, i, p, shape, x[1:], what=f"{name} {chunk_cols}")
+        assert torch.equal(y, _product(lay, tx, shape))
+        want = y if want is None else want
+        assert torch.equal(y, want)
+
+
+def test_infinities_stay_in_their_rows(cuda, fsb_lib):
+    lens = [40, 3, 70, 1, 5] * 300
+    d, i, p = handmade_csr(2, lens, 5000)
+    x = np.random.default_rng(1).uniform(0.5, 1, 5000).astype(np.float32)
+    rows = [0, 2, 601, 1499]
+    for r in rows:
+        d[p[r]] = np.inf
+    d[p[7]], d[p[7] + 1] = np.inf, -np.inf
+    y = _product(_layout(d, i, p, (1500, 5000), 1000), dev(x), (1500, 5000)).cpu().numpy()
+    assert np.isposinf(y[rows]).all() and np.isnan(y[7])
+    rest = np.setdiff1d(np.arange(1500), rows + [7])
+    assert np.isfinite(y[rest]).all()
+    x[0] = np.nan                       # what fills the packs up has column 0 of its chunk: no row may see it
+    y2 = _product(_layout(d, i, p, (1500, 5000), 1000), dev(x), (1500, 5000)).cpu().numpy()
+    keep = np.setdiff1d(rest, [r for r in range(1500) if (i[p[r]:p[r + 1]] == 0).any()])
+    assert np.array_equal(y2[keep], y[keep])
+
+
+def test_what_is_left_to_one_pass(cuda, fsb_lib):
+    d, i, p = handmade_csr(4, [7000] + [2] * 50, 9000)
+    assert _layout(d, i, p, (51, 9000)) is None                        # a row too long for a block
+    d, i, p = handmade_csr(4, [4] * 500, 9000)
+    assert bins.build_bins_layout(dev(d), dev(i), dev(p), 500, 9000, 4, span=9000 * 4 + 1) is None
+    assert bins.build_bins_layout(dev(d), dev(i), dev(p), 500, 9000, 4, span=9000 * 4, chunk_cols=1000) is not None
+    # the units are looked at, not only the width of the matrix: a band reaches few chunks
+    i = (i % 40).astype(np.int32)
+    assert bins.build_bins_layout(dev(d), dev(i), dev(p), 500, 9000, 4, span=9000 * 4, chunk_cols=1000) is None
+
+
+def test_prepared_matrix_takes_the_two_passes(cuda, fsb_lib, monkeypatch):
+    monkeypatch.setattr(bins, "UNEVEN_MIN_NNZ", 1 << 17)
+    monkeypatch.setattr(bins, "UNEVEN_MIN_SPAN", 1 << 10)
+    lens = np.random.default_rng(7).integers(0, 9, 60000)
+    lens[::5000] = 700
+    d, i, p = handmade_csr(8, lens.tolist(), 50000)
+    x = np.random.default_rng(9).uniform(-1, 1, 50000).astype(np.float32)
+    prep = fs.prepare_spmv_csr(dev(d), dev(i.astype(np.int64)), dev(p), (60000, 50000))
+    assert prep.bins is not None and prep.opt_buckets[0]["kind"] == "bins"
+    y = fs.flagsparse_spmv_csr(x=dev(x), prepared=prep)
+    assert_spmv_ok(y.cpu().numpy(), d, i, p, (60000, 50000), x)
+    graph, got = torch.cuda.CUDAGraph(), None
+    tx = dev(x)
+    with torch.cuda.graph(graph):
+        got = fs.flagsparse_spmv_csr(x=tx, prepared=prep)
+    graph.replay()
+    assert torch.equal(got, y)
+    monkeypatch.setenv("FSB_SPMV_BINS", "0")
+    assert fs.prepare_spmv_csr(dev(d), dev(i), dev(p), (60000, 50000)).bins is None
+
+
+def test_refused_calls(fsb_lib):
+    """Argument errors are found on the host, before anything is launched."""
+    L = fsb_lib
+    one = [1 << 20] * 9
+    call = lambda vt=0, chunks=1, width=64, cols=64, packs=1, nbytes=32, rows=1, ptrs=one: L.fsb_spmv_csr_bins(  # noqa: E731
+        vt, *ptrs, 1, chunks, width, packs, 1 << 20, nbytes, 1 << 20, 1 << 20, rows, cols, None)
+    assert call(vt=_lib.FSB_BF16) == -1 and call(chunks=2) == -1 and call(cols=65) == -1 and call(ptrs=[None] + one[1:]) == -1
+    assert call(width=65, cols=65) == -2 and call(packs=2**31) == -2
+    assert call(nbytes=31) == -4
+    assert call(ptrs=[(1 << 20) + 4] + one[1:]) == -3
