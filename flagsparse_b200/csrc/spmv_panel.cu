@@ -11,7 +11,7 @@
 // An entry is a value plus one packed word (local row << 16 | x buffer * CW + local column): 8 bytes for
 // float32, the same as CSR with 32-bit indices.  One CTA owns one row block:
 //   - the CW elements of x a unit needs arrive in shared memory by a cp.async.bulk copy (mbarrier
-//     completion), n_buffers - 1 units ahead of their use;
+//     completion), n_buffers - 1 units ahead of their use (n_buffers, where a warp of its own fetches them);
 //   - a warp takes a whole piece: lane l owns slots R*l .. R*l+R-1 (stored interleaved so that each 128-bit
 //     load of the warp is contiguous).  In round k every lane handles its k-th slot: value * x[column] is added
 //     to the row's accumulator in shared memory.  Two slots of one round are R positions apart and a row has at
@@ -30,8 +30,7 @@
 
 namespace fsb {
 
-constexpr int kPanelWarps = 32;
-constexpr int kPanelThreads = kPanelWarps * 32;
+constexpr int kPanelMaxWarps = 32;
 constexpr int kPanelWaitSpins = 1 << 22;
 constexpr int kPanelWaitSpinsDebug = 1 << 10;   // FSB_PANEL_DEBUG_TIMEOUT: give up quickly
 
@@ -58,6 +57,12 @@ __device__ __forceinline__ bool p_wait_bounded(uint64_t* bar, uint32_t phase, in
     if (p_try_wait(bar, phase)) return true;
   return false;
 }
+
+__device__ __forceinline__ void p_arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.release.cta.shared::cta.b64 _, [%0];" ::"r"(p_smem_addr(bar)) : "memory");
+}
+// the first `threads` threads of the CTA
+__device__ __forceinline__ void p_sync(int threads) { asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory"); }
 
 // G consecutive slots of one lane (G = 4 or 8): rounds G*g .. G*g+G-1 of a piece.
 template <typename V, int G>
@@ -168,10 +173,11 @@ constexpr int kUnitLookahead = kMaxXBuffers;
 // The shared-memory state of one CTA: the x buffers, the row accumulators, the copy barriers, the unit tables.
 template <typename V>
 struct PanelShared {
-  V* xs;      // n_buf * chunk_cols
+  V* xs;      // n_buf * chunk_cols, and 16 bytes
   V* y_part;  // one accumulator per (virtual) row of the CTA
-  uint64_t* bars;
-  int* failed;
+  uint64_t* bars;      // one per buffer: its chunk has landed
+  uint64_t* gathered;  // one per buffer: every warp is done with the chunk in it
+  volatile int* failed;
   int32_t* upp;   // unit_piece_ptr of the current window of units (kUnitWindow + 1 entries)
   int32_t* uch;   // unit_chunk of the window and of the next few units (kUnitWindow + kUnitLookahead)
 };
@@ -184,13 +190,29 @@ struct PanelGeom {
   uint32_t pad_row;  // accumulator index carried by unused slots (one past the CTA's real accumulators)
 };
 
+// Warps that add products.  Where every slot costs a trip to an accumulator (kModeDirect: about one entry per row and unit,
+// wide bands) one more warp does nothing but fetch x.  A unit is short there (4400 entries, about a microsecond), and a chunk
+// asked for at the barrier that opens a unit lands hardly before the one that closes it: the copies alone, one after the
+// other, took 755 us of the product's 1026 us (2^24 rows of 32, band of +-2^20, float32; the entries alone 749 us, the
+// arithmetic alone 665 us).  Asked for as soon as the last warp is done with the buffer they run ahead of the barriers: 955 us,
+// and 924 us with hardly more warps than a unit has pieces (17; FSB_PANEL_FEW_PIECES): fewer wait at the barriers.
+constexpr int kFewWarps = 20;
+__host__ __device__ constexpr int panel_workers(int mode, bool few) {
+  return mode != kModeDirect ? kPanelMaxWarps : few ? kFewWarps : kPanelMaxWarps - 1;
+}
+__host__ __device__ constexpr int panel_threads(int mode, bool few) {
+  return 32 * (panel_workers(mode, few) + (mode == kModeDirect ? 1 : 0));
+}
+
 // Units u0 .. u1-1 of one CTA, in order: chunk of x in, pieces added into y_part.  Returns false when a bounded
 // wait ran out (every thread of the CTA gets the same answer).
-//   - x chunks are fetched n_buf - 1 units ahead into n_buf buffers (unit number `ord` of the CTA uses buffer
-//     ord % n_buf; the packed word of a slot already holds buffer * chunk_cols + local column);
-//   - piece p goes to warp (p - first piece of the CTA) % 32; a warp walks its pieces in groups of G slots per
+//   - x chunks are fetched ahead into n_buf buffers (unit number `ord` of the CTA uses buffer ord % n_buf; the packed word
+//     of a slot already holds buffer * chunk_cols + local column).  kModeDirect: by a warp of its own, n_buf units ahead, as
+//     soon as all warps are done with the buffer (mbarriers that only this warp looks at); else by thread 0, n_buf - 1
+//     units ahead, at the barrier that closes the unit;
+//   - piece p goes to warp (p - first piece of the CTA) % W; a warp walks its pieces in groups of G slots per
 //     lane (group q % (R/G) of its piece number q / (R/G)) and always has the next group on its way.
-template <typename V, int R, int G, int MODE>
+template <typename V, int R, int G, int MODE, int W>
 __device__ __forceinline__ bool panel_run_units(const V* __restrict__ val, const uint32_t* __restrict__ rc,
                                                 const int32_t* __restrict__ unit_piece_ptr,
                                                 const int32_t* __restrict__ unit_chunk, int u0, int u1,
@@ -198,152 +220,189 @@ __device__ __forceinline__ bool panel_run_units(const V* __restrict__ val, const
                                                 const PanelShared<V>& sh) {
   constexpr int GPP = R / G;          // groups per piece
   constexpr int SLOTS = 32 * R;
+  constexpr int THREADS = 32 * W;     // of the warps that add
+  constexpr bool RING = MODE == kModeDirect;
+  constexpr int E = 16 / (int)sizeof(V);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int chunk_cols = gm.chunk_cols, n_buf = gm.n_buf;
   const int spins = gm.debug ? kPanelWaitSpinsDebug : kPanelWaitSpins;
-  V* xs = sh.xs;
+  // an x that does not start on a 16-byte boundary is kept as far from one in the buffers, so that the body of every chunk
+  // can be copied in bulk
+  const int shift = (int)((reinterpret_cast<uintptr_t>(x) / sizeof(V)) % E);
+  V* xs = sh.xs + shift;
   V* y_part = sh.y_part;
   uint64_t* bars = sh.bars;
   if (u0 >= u1) return true;
 
-  // chunk `c` of x into buffer `b`: bulk copy when the byte count is a multiple of 16, else plain loads
+  // chunk `c` of x into buffer `b`, by one thread: what lies between the first and the last 16-byte boundary as a bulk copy,
+  // the up to three elements on either side one by one
   auto load_chunk = [&](int c, int b, bool first) {
     const int64_t c0 = (int64_t)c * chunk_cols;
     const int n = (int)((gm.n_cols - c0) < (int64_t)chunk_cols ? (gm.n_cols - c0) : (int64_t)chunk_cols);
-    const uint32_t bytes = (uint32_t)(n * sizeof(V));
-    if ((bytes & 15u) == 0 && aligned_to_dev(x + c0)) {
-      if (tid == 0) {
-        p_expect_tx(&bars[b], bytes + ((first && gm.debug) ? 16u : 0u));
-        p_bulk_g2s(xs + (size_t)b * chunk_cols, x + c0, bytes, &bars[b]);
-      }
-      return false;
-    }
-    for (int i = tid; i < n; i += kPanelThreads) xs[(size_t)b * chunk_cols + i] = __ldg(x + c0 + i);
-    if (tid == 0) p_expect_tx(&bars[b], (first && gm.debug) ? 16u : 0u);  // completes as soon as this arrival lands
-    return true;
+    V* dst = xs + (size_t)b * chunk_cols;
+    const V* src = x + c0;
+    int lo = shift ? E - shift : 0;
+    lo = lo < n ? lo : n;
+    const int hi = lo + (n - lo) / E * E;
+    for (int i = 0; i < lo; ++i) dst[i] = src[i];
+    for (int i = hi; i < n; ++i) dst[i] = src[i];
+    const uint32_t bytes = (uint32_t)((hi - lo) * sizeof(V));
+    p_expect_tx(&bars[b], bytes + ((first && gm.debug) ? 16u : 0u));     // releases the elements written here, too
+    if (bytes) p_bulk_g2s(dst + lo, src + lo, bytes, &bars[b]);
   };
 
-  const int p_first = unit_piece_ptr[u0];
-  const int p_cta_end = unit_piece_ptr[u1];
-  int pc = p_first + warp;            // this warp's next piece
-  // The entries do not depend on x: the warp's first group(s) are requested before anything else.
-  //   RING   two groups in a register ring, refilled as soon as a group has been consumed (the request for
-  //          group q + 2 leaves after group q); measured best where every slot costs a trip to an accumulator
-  //   else   the next group is requested right before the current one is used, into registers that are dead
-  //          otherwise; measured best for the run-summing rounds, which need the registers themselves
-  constexpr bool RING = MODE == kModeDirect;
-  const int n_my = (p_cta_end - p_first - warp + kPanelWarps - 1) / kPanelWarps;   // pieces of this warp (may be <= 0)
-  const int n_groups = n_my > 0 ? n_my * GPP : 0;
-  Group<V, G> ring[2];
-  auto request = [&](int q, Group<V, G>& slot) {
-    if (q < n_groups) {
-      const size_t piece = (size_t)(p_first + warp + kPanelWarps * (q / GPP));
-      ld_group(val + piece * SLOTS, rc + piece * SLOTS, lane, q % GPP, slot);
-    }
-  };
-  int q = 0, phase = 0;
-  if (RING) {
-    request(0, ring[0]);
-    request(1, ring[1]);
-  } else if (pc < p_cta_end) {
-    ld_group(val + (size_t)pc * SLOTS, rc + (size_t)pc * SLOTS, lane, 0, ring[0]);
-  }
-
-  // chunks of the first n_buf - 1 units (a chunk written with ordinary stores is also at least one CTA barrier
-  // ahead of its first use)
-  for (int a = 0; a < n_buf - 1 && u0 + a < u1; ++a) load_chunk(unit_chunk[u0 + a], a, a == 0);
-
-  int b = 0, par = 0;                  // buffer and barrier parity of the current unit
-  // One thread waits for a chunk of x; the CTA barrier that follows hands what it has seen on to everybody
-  // (1023 threads polling the same mbarrier cost more issue slots than the products themselves).
-  if (tid == 0 && !p_wait_bounded(&bars[0], 0u, spins)) *sh.failed = 1;
-  for (int w0 = u0; w0 < u1; w0 += kUnitWindow) {
-    const int nwin = (u1 - w0) < kUnitWindow ? (u1 - w0) : kUnitWindow;
-    const int nch = (u1 - w0) < (kUnitWindow + kUnitLookahead) ? (u1 - w0) : (kUnitWindow + kUnitLookahead);
-    if (w0 > u0) __syncthreads();  // the previous window's tables are no longer read
-    for (int i = tid; i <= nwin; i += kPanelThreads) sh.upp[i] = unit_piece_ptr[w0 + i];
-    for (int i = tid; i < nch; i += kPanelThreads) sh.uch[i] = unit_chunk[w0 + i];
-    __syncthreads();               // also: the first chunk has landed (or the wait for it was given up)
-    for (int u = w0; u < w0 + nwin; ++u) {
-      if (*sh.failed) {
-        // leave no copy in flight into this CTA's shared memory: one more bounded wait per chunk requested ahead
-        int bb = b, pp = par;
-        for (int a = 1; a < n_buf - 1 && u + a < u1; ++a) {
-          if (++bb == n_buf) { bb = 0; pp ^= 1; }
-          p_wait_bounded(&bars[bb], (uint32_t)pp, spins);
+  if (RING && warp == W) {
+    if (lane == 0) {
+      int last = u0 - 1;              // last unit whose chunk was asked for
+      for (int u = u0; u < u1; ++u) {
+        const int c = unit_chunk[u];  // (read before the wait)
+        const int ord = u - u0;
+        if (ord >= n_buf) {           // the buffer was used by unit u - n_buf
+          bool ok = false;
+          for (int i = 0; i < spins && !ok && !*sh.failed; ++i)
+            ok = p_try_wait(&sh.gathered[ord % n_buf], (uint32_t)((ord / n_buf - 1) & 1));
+          if (!ok) break;             // thread 0 will miss the chunk and say so: all warps then learn of it at one barrier
         }
-        return false;
+        load_chunk(c, ord % n_buf, ord == 0);
+        last = u;
       }
-      // the buffer of the previous unit was last read before the barrier that closed it: free to refill
-      if (u + n_buf - 1 < u1) {
-        int bn = b + n_buf - 1;
-        bn = bn >= n_buf ? bn - n_buf : bn;
-        load_chunk(sh.uch[u + n_buf - 1 - w0], bn, false);
+      // no copy may be in flight when the CTA ends: wait (bounded) for the last ones
+      for (int u = last - n_buf + 1 < u0 ? u0 : last - n_buf + 1; u <= last; ++u)
+        p_wait_bounded(&bars[(u - u0) % n_buf], (uint32_t)(((u - u0) / n_buf) & 1), spins);
+    }
+    __syncwarp();
+  } else {
+    const int p_first = unit_piece_ptr[u0];
+    const int p_cta_end = unit_piece_ptr[u1];
+    int pc = p_first + warp;            // this warp's next piece
+    // The entries do not depend on x: the warp's first group(s) are requested before anything else.
+    //   RING   two groups in a register ring, refilled as soon as a group has been consumed (the request for
+    //          group q + 2 leaves after group q); measured best where every slot costs a trip to an accumulator
+    //   else   the next group is requested right before the current one is used, into registers that are dead
+    //          otherwise; measured best for the run-summing rounds, which need the registers themselves
+    const int n_my = (p_cta_end - p_first - warp + W - 1) / W;   // pieces of this warp (may be <= 0)
+    const int n_groups = n_my > 0 ? n_my * GPP : 0;
+    Group<V, G> ring[2];
+    auto request = [&](int q, Group<V, G>& slot) {
+      if (q < n_groups) {
+        const size_t piece = (size_t)(p_first + warp + W * (q / GPP));
+        ld_group(val + piece * SLOTS, rc + piece * SLOTS, lane, q % GPP, slot);
       }
-      const int p_end = sh.upp[u - w0 + 1];
-      while (pc < p_end) {
-        V acc = (V)0;
-#pragma unroll
-        for (int g = 0; g < GPP; ++g) {
-          if (RING) {
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-              if (phase == i) {
-                panel_rounds_direct<V, G>(ring[i], xs, y_part);
-                request(q + 2, ring[i]);
-              }
-            }
-            phase ^= 1;
-            ++q;
-          } else {
-            // the next group (of this piece, or the first one of this warp's next piece, whichever unit that
-            // piece belongs to) is in flight while this one is used
-            Group<V, G> nxt;
-            const bool more = g + 1 < GPP;
-            const int np = more ? pc : pc + kPanelWarps;
-            const bool have = np < p_cta_end;
-            if (have) ld_group(val + (size_t)np * SLOTS, rc + (size_t)np * SLOTS, lane, more ? g + 1 : 0, nxt);
-            // a lane's run ends with its last slot of the piece; inside the piece the next group tells
-            const uint32_t next_word = more ? nxt.w[0] : (gm.pad_row << 16);
-            panel_rounds_runs<V, G, MODE == kModeRunsClash>(ring[0], next_word, !more, acc, xs, y_part, lane,
-                                                             gm.pad_row);
-            if (have) ring[0] = nxt;
+    };
+    int q = 0, phase = 0;
+    if (RING) {
+      request(0, ring[0]);
+      request(1, ring[1]);
+    } else if (pc < p_cta_end) {
+      ld_group(val + (size_t)pc * SLOTS, rc + (size_t)pc * SLOTS, lane, 0, ring[0]);
+    }
+
+    // chunks of the first n_buf - 1 units
+    if (!RING && tid == 0)
+      for (int a = 0; a < n_buf - 1 && u0 + a < u1; ++a) load_chunk(unit_chunk[u0 + a], a, a == 0);
+
+    int b = 0, par = 0;                  // buffer and barrier parity of the current unit
+    // One thread waits for a chunk of x; the barrier that follows hands what it has seen on to everybody
+    // (1023 threads polling the same mbarrier cost more issue slots than the products themselves).
+    if (tid == 0 && !p_wait_bounded(&bars[0], 0u, spins)) *sh.failed = 1;
+    bool ok = true;
+    for (int w0 = u0; w0 < u1 && ok; w0 += kUnitWindow) {
+      const int nwin = (u1 - w0) < kUnitWindow ? (u1 - w0) : kUnitWindow;
+      const int nch = (u1 - w0) < (kUnitWindow + kUnitLookahead) ? (u1 - w0) : (kUnitWindow + kUnitLookahead);
+      if (w0 > u0) p_sync(THREADS);  // the previous window's tables are no longer read
+      for (int i = tid; i <= nwin; i += THREADS) sh.upp[i] = unit_piece_ptr[w0 + i];
+      if (!RING)
+        for (int i = tid; i < nch; i += THREADS) sh.uch[i] = unit_chunk[w0 + i];
+      p_sync(THREADS);               // also: the first chunk has landed (or the wait for it was given up)
+      for (int u = w0; u < w0 + nwin; ++u) {
+        if (*sh.failed) {            // set by thread 0 before a barrier: all see it in the same unit
+          // leave no copy in flight into this CTA's shared memory: one more bounded wait per chunk requested ahead
+          for (int a = 1; !RING && a < n_buf - 1 && u + a < u1; ++a) {
+            if (++b == n_buf) { b = 0; par ^= 1; }
+            p_wait_bounded(&bars[b], (uint32_t)par, spins);
           }
+          ok = false;
+          break;
         }
-        pc += kPanelWarps;
+        // the buffer of the previous unit was last read before the barrier that closed it: free to refill
+        if (!RING && tid == 0 && u + n_buf - 1 < u1) load_chunk(sh.uch[u + n_buf - 1 - w0], b == 0 ? n_buf - 1 : b - 1, false);
+        const int p_end = sh.upp[u - w0 + 1];
+        if (RING && pc >= p_end && lane == 0) p_arrive(&sh.gathered[b]);     // no piece in this unit
+        while (pc < p_end) {
+          V acc = (V)0;
+#pragma unroll
+          for (int g = 0; g < GPP; ++g) {
+            if (RING) {
+#pragma unroll
+              for (int i = 0; i < 2; ++i) {
+                if (phase == i) {
+                  panel_rounds_direct<V, G>(ring[i], xs, y_part);
+                  // The warp is done with this chunk.  Not before the rounds: the sums are what shows that the gathers have
+                  // come back (told right behind them, the copy of the next chunk overtook some).
+                  if (g == GPP - 1 && pc + W >= p_end) {
+                    __syncwarp();
+                    if (lane == 0) p_arrive(&sh.gathered[b]);
+                  }
+                  request(q + 2, ring[i]);
+                }
+              }
+              phase ^= 1;
+              ++q;
+            } else {
+              // the next group (of this piece, or the first one of this warp's next piece, whichever unit that
+              // piece belongs to) is in flight while this one is used
+              Group<V, G> nxt;
+              const bool more = g + 1 < GPP;
+              const int np = more ? pc : pc + W;
+              const bool have = np < p_cta_end;
+              if (have) ld_group(val + (size_t)np * SLOTS, rc + (size_t)np * SLOTS, lane, more ? g + 1 : 0, nxt);
+              // a lane's run ends with its last slot of the piece; inside the piece the next group tells
+              const uint32_t next_word = more ? nxt.w[0] : (gm.pad_row << 16);
+              panel_rounds_runs<V, G, MODE == kModeRunsClash>(ring[0], next_word, !more, acc, xs, y_part, lane,
+                                                               gm.pad_row);
+              if (have) ring[0] = nxt;
+            }
+          }
+          pc += W;
+        }
+        if (++b == n_buf) { b = 0; par ^= 1; }
+        // the next unit's chunk must have landed before anybody gathers from it
+        if (tid == 0 && u + 1 < u1 && !p_wait_bounded(&bars[b], (uint32_t)par, spins)) *sh.failed = 1;
+        p_sync(THREADS);  // every add of this unit is done (its x buffer may be refilled); the next chunk is in
       }
-      if (++b == n_buf) { b = 0; par ^= 1; }
-      // the next unit's chunk must have landed before anybody gathers from it
-      if (tid == 0 && u + 1 < u1 && !p_wait_bounded(&bars[b], (uint32_t)par, spins)) *sh.failed = 1;
-      __syncthreads();  // every add of this unit is done (its x buffer may be refilled); the next chunk is in
     }
   }
-  if (*sh.failed) return false;
-  return true;
+  __syncthreads();
+  return !*sh.failed;
 }
 
 struct PanelStatic {
   uint64_t bars[kMaxXBuffers];
+  uint64_t gathered[kMaxXBuffers];
   int32_t upp[kUnitWindow + 1];
   int32_t uch[kUnitWindow + kUnitLookahead];
   int failed;
 };
 
-template <typename V>
+template <typename V, int THREADS>
 __device__ __forceinline__ void panel_setup(PanelShared<V>& sh, unsigned char* smem, PanelStatic* st, int chunk_cols,
-                                            int n_buf, int n_acc, uint32_t pad_row) {
+                                            int n_buf, int n_acc, uint32_t pad_row, int workers) {
   sh.xs = reinterpret_cast<V*>(smem);
-  sh.y_part = sh.xs + (size_t)n_buf * chunk_cols;
+  sh.y_part = sh.xs + (size_t)n_buf * chunk_cols + 16 / sizeof(V);   // the last buffer may be shifted by up to 16 bytes
   sh.bars = st->bars;
+  sh.gathered = st->gathered;
   sh.failed = &st->failed;
   sh.upp = st->upp;
   sh.uch = st->uch;
   const int tid = threadIdx.x;
-  for (int i = tid; i < n_acc; i += kPanelThreads) sh.y_part[i] = (V)0;
+  for (int i = tid; i < n_acc; i += THREADS) sh.y_part[i] = (V)0;
   if (tid == 0) {
     st->failed = 0;
     sh.y_part[pad_row] = (V)0;
-    for (int b = 0; b < n_buf; ++b) p_mbar_init(&st->bars[b], 1);
+    for (int b = 0; b < n_buf; ++b) {
+      p_mbar_init(&st->bars[b], 1);
+      p_mbar_init(&st->gathered[b], workers);
+    }
     p_fence_init();
   }
   __syncthreads();
@@ -351,21 +410,22 @@ __device__ __forceinline__ void panel_setup(PanelShared<V>& sh, unsigned char* s
 
 // One CTA per block of rb_rows consecutive rows (block block_begin + blockIdx.x); every row of y the launch
 // covers is written exactly once.
-template <typename V, int R, int G, int MODE>
-__global__ void __launch_bounds__(kPanelThreads, 1)
+template <typename V, int R, int G, int MODE, bool FEW>
+__global__ void __launch_bounds__(panel_threads(MODE, FEW), 1)
 spmv_panel_kernel(const V* __restrict__ val, const uint32_t* __restrict__ rc, const int32_t* __restrict__ unit_piece_ptr,
                   const int32_t* __restrict__ unit_chunk, const int32_t* __restrict__ rb_unit_ptr,
                   const V* __restrict__ x, V* __restrict__ y, int block_begin, int64_t n_rows, int rb_rows,
                   PanelGeom gm, int32_t* __restrict__ status) {
   extern __shared__ __align__(128) unsigned char p_smem[];
   __shared__ __align__(8) PanelStatic p_static;
+  constexpr int W = panel_workers(MODE, FEW), THREADS = panel_threads(MODE, FEW);
   const int tid = threadIdx.x;
   const int rb = block_begin + (int)blockIdx.x;
   const int64_t r0 = (int64_t)rb * rb_rows;
   const int nr = (int)((n_rows - r0) < (int64_t)rb_rows ? (n_rows - r0) : (int64_t)rb_rows);
   PanelShared<V> sh;
-  panel_setup<V>(sh, p_smem, &p_static, gm.chunk_cols, gm.n_buf, nr, gm.pad_row);
-  if (!panel_run_units<V, R, G, MODE>(val, rc, unit_piece_ptr, unit_chunk, rb_unit_ptr[rb], rb_unit_ptr[rb + 1], x,
+  panel_setup<V, THREADS>(sh, p_smem, &p_static, gm.chunk_cols, gm.n_buf, nr, gm.pad_row, W);
+  if (!panel_run_units<V, R, G, MODE, W>(val, rc, unit_piece_ptr, unit_chunk, rb_unit_ptr[rb], rb_unit_ptr[rb + 1], x,
                                        gm, sh)) {
     if (tid == 0 && status != nullptr) *reinterpret_cast<volatile int32_t*>(status) = 2;  // may be host memory
     return;
@@ -377,10 +437,10 @@ spmv_panel_kernel(const V* __restrict__ val, const uint32_t* __restrict__ rc, co
     const int nv = nr / E;
     const float4* src4 = reinterpret_cast<const float4*>(sh.y_part);
     float4* dst4 = reinterpret_cast<float4*>(dst);
-    for (int i = tid; i < nv; i += kPanelThreads) dst4[i] = src4[i];
-    for (int i = nv * E + tid; i < nr; i += kPanelThreads) dst[i] = sh.y_part[i];
+    for (int i = tid; i < nv; i += THREADS) dst4[i] = src4[i];
+    for (int i = nv * E + tid; i < nr; i += THREADS) dst[i] = sh.y_part[i];
   } else {
-    for (int i = tid; i < nr; i += kPanelThreads) dst[i] = sh.y_part[i];
+    for (int i = tid; i < nr; i += THREADS) dst[i] = sh.y_part[i];
   }
 }
 
@@ -391,8 +451,8 @@ spmv_panel_kernel(const V* __restrict__ val, const uint32_t* __restrict__ rc, co
 // unit" still holds).  The units of a group are dealt to several CTAs by column range, so a CTA ends with
 // partial sums of its group's rows: it writes them to part[cta_part_ptr[cta] + (q - first q of the group)],
 // and panel_group_reduce_kernel adds the partial sums of each row in CTA order.
-template <typename V, int R, int G, int MODE>
-__global__ void __launch_bounds__(kPanelThreads, 1)
+template <typename V, int R, int G, int MODE, bool FEW>
+__global__ void __launch_bounds__(panel_threads(MODE, FEW), 1)
 spmv_panel_groups_kernel(const V* __restrict__ val, const uint32_t* __restrict__ rc,
                          const int32_t* __restrict__ unit_piece_ptr, const int32_t* __restrict__ unit_chunk,
                          const int32_t* __restrict__ cta_unit_ptr, const int32_t* __restrict__ cta_group,
@@ -401,6 +461,7 @@ spmv_panel_groups_kernel(const V* __restrict__ val, const uint32_t* __restrict__
                          PanelGeom gm, int32_t* __restrict__ status) {
   extern __shared__ __align__(128) unsigned char p_smem[];
   __shared__ __align__(8) PanelStatic p_static;
+  constexpr int W = panel_workers(MODE, FEW), THREADS = panel_threads(MODE, FEW);
   const int tid = threadIdx.x;
   const int cta = blockIdx.x;
   const int g = cta_group[cta];
@@ -408,14 +469,14 @@ spmv_panel_groups_kernel(const V* __restrict__ val, const uint32_t* __restrict__
   const int vb0 = vbase[q0];
   const int n_acc = vbase[q1] - vb0;
   PanelShared<V> sh;
-  panel_setup<V>(sh, p_smem, &p_static, gm.chunk_cols, gm.n_buf, n_acc, gm.pad_row);
-  if (!panel_run_units<V, R, G, MODE>(val, rc, unit_piece_ptr, unit_chunk, cta_unit_ptr[cta], cta_unit_ptr[cta + 1],
+  panel_setup<V, THREADS>(sh, p_smem, &p_static, gm.chunk_cols, gm.n_buf, n_acc, gm.pad_row, W);
+  if (!panel_run_units<V, R, G, MODE, W>(val, rc, unit_piece_ptr, unit_chunk, cta_unit_ptr[cta], cta_unit_ptr[cta + 1],
                                        x, gm, sh)) {
     if (tid == 0 && status != nullptr) *reinterpret_cast<volatile int32_t*>(status) = 2;  // may be host memory
     return;
   }
   V* out = part + cta_part_ptr[cta];
-  for (int i = tid; i < q1 - q0; i += kPanelThreads) {
+  for (int i = tid; i < q1 - q0; i += THREADS) {
     const int a = vbase[q0 + i] - vb0, b = vbase[q0 + i + 1] - vb0;
     V s = (V)0;
     for (int v = a; v < b; ++v) s += sh.y_part[v];
@@ -456,7 +517,7 @@ extern "C" int fsb_spmv_panel_piece_slots(int rounds) {
 extern "C" size_t fsb_spmv_panel_smem_bytes(int vtype, int rb_rows, int chunk_cols, int n_buffers) {
   const size_t sv = vtype == FSB_F32 ? 4 : 8;
   // the accumulators of the CTA plus the spare one that unused slots add their zeros to
-  return (size_t)n_buffers * (size_t)chunk_cols * sv + (((size_t)rb_rows + 1 + 3) & ~(size_t)3) * sv;
+  return (size_t)n_buffers * (size_t)chunk_cols * sv + 16 + (((size_t)rb_rows + 1 + 3) & ~(size_t)3) * sv;
 }
 
 extern "C" size_t fsb_spmv_panel_static_smem_bytes(void) { return sizeof(PanelStatic); }
@@ -468,9 +529,10 @@ static bool panel_buffers_ok(int n_buffers, int chunk_cols) {
 // FN<V, R, G, MODE> for the runtime (vtype, rounds, mode)
 #define FSB_PANEL_CASE(FN, V, R_, LAUNCH)                                                        \
   do {                                                                                           \
-    if (mode == kModeRunsClash) LAUNCH((FN<V, R_, Shape<V, R_>::G, kModeRunsClash>));            \
-    else if (mode == kModeRuns) LAUNCH((FN<V, R_, Shape<V, R_>::G, kModeRuns>));                 \
-    else LAUNCH((FN<V, R_, Shape<V, R_>::G, kModeDirect>));                                      \
+    if (mode == kModeRunsClash) LAUNCH((FN<V, R_, Shape<V, R_>::G, kModeRunsClash, false>));     \
+    else if (mode == kModeRuns) LAUNCH((FN<V, R_, Shape<V, R_>::G, kModeRuns, false>));          \
+    else if (few) LAUNCH((FN<V, R_, Shape<V, R_>::G, kModeDirect, true>));                       \
+    else LAUNCH((FN<V, R_, Shape<V, R_>::G, kModeDirect, false>));                               \
   } while (0)
 #define FSB_PANEL_DISPATCH(FN, V, LAUNCH)                                                        \
   do {                                                                                           \
@@ -502,11 +564,12 @@ extern "C" int fsb_spmv_csr_panel(int vtype, const void* val, const uint32_t* rc
   const int mode = (flags & FSB_PANEL_LONG_RUNS) ? kModeRunsClash : ((flags & FSB_PANEL_RUNS) ? kModeRuns : kModeDirect);
   const PanelGeom gm{n_cols, chunk_cols, n_buffers, (flags & FSB_PANEL_DEBUG_TIMEOUT) ? 1 : 0, (uint32_t)rb_rows};
   const unsigned grid = (unsigned)(block_end - block_begin);
+  const bool few = (flags & FSB_PANEL_FEW_PIECES) != 0;
 #define FSB_PANEL_LAUNCH_(K)                                                                                    \
   do {                                                                                                          \
     cudaError_t e = cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);           \
     if (e != cudaSuccess) return cuda_rc(e);                                                                    \
-    K<<<grid, kPanelThreads, smem, st>>>((const VT_*)val, rc, unit_piece_ptr, unit_chunk, rb_unit_ptr,          \
+    K<<<grid, panel_threads(mode, few), smem, st>>>((const VT_*)val, rc, unit_piece_ptr, unit_chunk, rb_unit_ptr,          \
                                          (const VT_*)x, (VT_*)y, block_begin, n_rows, rb_rows, gm, status);     \
   } while (0)
   if (vtype == FSB_F32) {
@@ -548,11 +611,12 @@ extern "C" int fsb_spmv_csr_panel_groups(int vtype, const void* val, const uint3
   const PanelGeom gm{n_cols, chunk_cols, n_buffers, (flags & FSB_PANEL_DEBUG_TIMEOUT) ? 1 : 0,
                      (uint32_t)max_group_acc};
   const unsigned rgrid = (unsigned)((n_long + 255) / 256);
+  const bool few = (flags & FSB_PANEL_FEW_PIECES) != 0;
 #define FSB_GROUPS_LAUNCH_(K)                                                                                    \
   do {                                                                                                           \
     cudaError_t e = cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);            \
     if (e != cudaSuccess) return cuda_rc(e);                                                                     \
-    K<<<(unsigned)n_ctas, kPanelThreads, smem, st>>>((const VT_*)val, rc, unit_piece_ptr, unit_chunk,            \
+    K<<<(unsigned)n_ctas, panel_threads(mode, few), smem, st>>>((const VT_*)val, rc, unit_piece_ptr, unit_chunk,            \
                                                      cta_unit_ptr, cta_group, group_q_ptr, vbase, cta_part_ptr,  \
                                                      (VT_*)part, (const VT_*)x, gm, status);                     \
   } while (0)

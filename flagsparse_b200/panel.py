@@ -30,12 +30,22 @@ N_BUFFERS = 2               # chunks of x in shared memory (fetched N_BUFFERS - 
 ROUNDS = (4, 8, 16)         # slots per lane and piece the kernel is built for (see csrc/spmv_panel.cu)
 FLAG_LONG_RUNS = 1          # FSB_PANEL_LONG_RUNS
 FLAG_RUNS = 2               # FSB_PANEL_RUNS
+FLAG_FEW_PIECES = 4         # FSB_PANEL_FEW_PIECES
+# Mean pieces of a unit up to which 20 warps are enough: with 17.6 pieces 20 / 31 warps take 457 / 471 us (2^23 rows of 32, band of
+# +-2^20), with 21.4 (2^26 rows) 5056 / 4135 us.
+FEW_PIECES = 18
 # mean entries of a row inside one unit from which summing a run in a register beats one accumulator update per entry
 RUNS_MIN_MEAN = 1.5
 FLAG_DEBUG_TIMEOUT = 256    # FSB_PANEL_DEBUG_TIMEOUT
 MAX_ROW_NNZ = 512
 MIN_NNZ = 1 << 22
 ACC_BANKS = {4: 32, 8: 16}   # accumulators that sit in different shared-memory banks (32 banks of 4 bytes), by value size
+
+
+def kernel_flags(nnz, n_runs, max_run, rounds, n_pieces, n_units):
+    """FSB_PANEL_* of a layout."""
+    few = FLAG_FEW_PIECES if n_pieces <= FEW_PIECES * n_units else 0
+    return (FLAG_LONG_RUNS if max_run > rounds else 0) | (FLAG_RUNS if nnz >= RUNS_MIN_MEAN * n_runs else 0) | few
 
 
 class PanelLayout:
@@ -564,7 +574,7 @@ def _build_fused(data, indices, indptr, n_rows, n_cols, geometry, NB, rounds, fo
     lay.unit_piece_ptr, lay.unit_chunk, lay.rb_unit_ptr = upiece, u_ch, rb_unit_ptr
     lay.n_row_blocks, lay.rb_rows, lay.chunk_cols, lay.n_buffers = n_rb, RB, CW, NB
     lay.rounds, lay.max_run, lay.pad_row = rounds, max_run, RB
-    lay.flags = (FLAG_LONG_RUNS if max_run > rounds else 0) | (FLAG_RUNS if nnz >= RUNS_MIN_MEAN * n_runs else 0)
+    lay.flags = kernel_flags(nnz, n_runs, max_run, rounds, n_pieces, n_units)
     lay.n_units, lay.n_pieces = n_units, n_pieces
     lay.x_overhead = n_units * CW * sv / float(nnz * (sv + 4))
     lay.slot_overhead = n_pieces * SLOTS / float(nnz)
@@ -648,7 +658,7 @@ def build_panel_layout(data, indices, indptr, n_rows, n_cols, max_row_nnz, force
     lay.rb_unit_ptr = rb_unit_ptr.to(torch.int32)
     lay.n_row_blocks, lay.rb_rows, lay.chunk_cols, lay.n_buffers = n_rb, RB, CW, NB
     lay.rounds, lay.max_run, lay.pad_row = rounds, max_run, RB
-    lay.flags = (FLAG_LONG_RUNS if max_run > rounds else 0) | (FLAG_RUNS if nnz >= RUNS_MIN_MEAN * n_runs else 0)
+    lay.flags = kernel_flags(nnz, n_runs, max_run, rounds, n_pieces, n_units)
     lay.n_units, lay.n_pieces = n_units, n_pieces
     lay.x_overhead = n_units * CW * sv / float(nnz * (sv + 4))
     lay.slot_overhead = n_pieces * SLOTS / float(nnz)

@@ -147,7 +147,10 @@ int fsb_spmv_csr_scatter(int vtype, int itype, int ptype, const void* data, cons
  *                        per entry, with no predicates).  Only speed depends on this flag.
  *                        FSB_PANEL_LONG_RUNS: some row has more than `rounds` entries inside one unit (never
  *                        more than a piece holds); the kernel then also combines the lanes that finish on the
- *                        same row.  Must be set for such layouts.  FSB_PANEL_DEBUG_TIMEOUT (tests only): the first copy of x of every CTA is made to
+ *                        same row.  Must be set for such layouts.
+ *                        FSB_PANEL_FEW_PIECES: units have 20 pieces or fewer, mostly; without the other two the kernel
+ *                        then runs with fewer warps.  Only speed depends on this flag.
+ *                        FSB_PANEL_DEBUG_TIMEOUT (tests only): the first copy of x of every CTA is made to
  *                        look incomplete and the wait limit is lowered, so that the kernel takes its time-out
  *                        path -- it reports through `status` and returns without touching y
  *   n_buffers            2..8 chunks of x in shared memory (n_buffers * chunk_cols <= 65536): chunks are
@@ -166,6 +169,7 @@ int fsb_spmv_csr_scatter(int vtype, int itype, int ptype, const void* data, cons
  */
 #define FSB_PANEL_LONG_RUNS 1
 #define FSB_PANEL_RUNS 2
+#define FSB_PANEL_FEW_PIECES 4
 #define FSB_PANEL_DEBUG_TIMEOUT 256
 int fsb_spmv_panel_piece_slots(int rounds);
 size_t fsb_spmv_panel_smem_bytes(int vtype, int rb_rows, int chunk_cols, int n_buffers);
