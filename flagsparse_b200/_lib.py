@@ -83,6 +83,8 @@ SIGNATURES = {
     "fsb_spmv_csr_stored": (_i32, [_i32, _i32, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _vp, _vp, _sz, _vp]),
     "fsb_spmv_csr_wide": (_i32, [_i32, _i32, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _vp]),
     "fsb_spmm_csr_wide": (_i32, [_i32, _i32, _vp, _vp, _vp, _vp, _i64, _vp, _i64, _i64, _i64, _i64, _i64, _vp]),
+    "fsb_coo_scratch_bytes": (_sz, [_i64]),
+    "fsb_coo_group": (_i32, [_i32, _i32, _i32, _vp, _vp, _vp, _i64, _i64, _i64, _i32, _vp, _vp, _vp, _vp, _vp, _vp, _sz, _vp]),
     "fsb_spmv_bins_max_chunks": (_i32, []),
     "fsb_spmv_bins_chunk_cols": (_i32, [_i32]),
     "fsb_spmv_bins_cap": (_i32, [_i32]),

@@ -16,7 +16,7 @@ CSRC = os.path.join(os.path.dirname(os.path.abspath(__file__)), "csrc")
 INCLUDE = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "include")
 LIB = os.path.join(CSRC, "libfsb.so")
 CHECK_LIB = os.path.join(CSRC, "libfsb_check.so")
-SOURCES = ("csr_analyze.cu", "spmv_csr.cu", "spmv_panel.cu", "spmv_bins.cu", "spmv_wide.cu", "spmm_csr.cu", "sddmm_csr.cu",
+SOURCES = ("csr_analyze.cu", "spmv_csr.cu", "spmv_panel.cu", "spmv_bins.cu", "spmv_wide.cu", "spmm_csr.cu", "sddmm_csr.cu", "coo_group.cu",
            "bounds_check.cu", "panel_build.cu")
 NVCC_FLAGS = (
     "-O3",

@@ -367,12 +367,16 @@ def prepare_spmm_csr_opt(data, indices, indptr, shape):
     return _prepare_spmm(data, indices, indptr, shape, once=False)
 
 
-def _prepare_spmm(data, indices, indptr, shape, once):
+def _prepare_spmm(data, indices, indptr, shape, once, known=None):
     """once: for a single product -- 64-bit indices stay, and the tiles are staged by ordinary loads, which have no
-    wait that could run out and so need no status word (a page-locked allocation and an event)."""
-    data, kernel_indices, kernel_indptr, n_rows, n_cols, stats = _prepare_spmm_csr_matrix(
-        data, indices, indptr, shape, narrow=not once
-    )
+    wait that could run out and so need no status word (a page-locked allocation and an event).  known: the statistics of
+    arrays that were made here (contiguous, 32-bit column ids): nothing is left to check."""
+    if known is None:
+        data, kernel_indices, kernel_indptr, n_rows, n_cols, stats = _prepare_spmm_csr_matrix(
+            data, indices, indptr, shape, narrow=not once
+        )
+    else:
+        kernel_indices, kernel_indptr, (n_rows, n_cols), stats = indices, indptr, shape, known
     nnz = data.numel()
     if data.dtype in widetypes.WIDE_DTYPES:
         # read as stored by fsb_spmm_csr_stored, which plans its tiles itself: no second copy of the matrix

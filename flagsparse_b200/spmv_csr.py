@@ -275,12 +275,17 @@ def _split_long_rows(data, kernel_indices, kernel_indptr, n_rows, n_cols, shape,
     return short, layout
 
 
-def _prepare_spmv_csr(data, indices, indptr, shape, block_nnz, max_segments, reuse_expected, allow_split=True):
-    """reuse_expected=False (a one-shot product) skips the panel regrouping, which costs about as much as a
+def _prepare_spmv_csr(data, indices, indptr, shape, block_nnz, max_segments, reuse_expected, allow_split=True,
+                      known=None):
+    """known: the statistics of arrays that were made here (contiguous, 32-bit column ids): nothing is left to check.
+    reuse_expected=False (a one-shot product) skips the panel regrouping, which costs about as much as a
     hundred products and only pays when the prepared matrix is used again."""
-    data, kernel_indices, kernel_indptr, n_rows, n_cols, stats = _prepare_spmv_csr_matrix(
-        data, indices, indptr, shape, narrow=reuse_expected
-    )
+    if known is None:
+        data, kernel_indices, kernel_indptr, n_rows, n_cols, stats = _prepare_spmv_csr_matrix(
+            data, indices, indptr, shape, narrow=reuse_expected
+        )
+    else:
+        kernel_indices, kernel_indptr, (n_rows, n_cols), stats = indices, indptr, shape, known
     max_row_nnz = stats.max_row_nnz
     block_nnz_use, max_segments_use = _resolve_block_nnz(max_row_nnz, block_nnz, max_segments)
     nnz = data.numel()

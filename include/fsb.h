@@ -354,6 +354,22 @@ int fsb_spmm_csr_stored(int vtype, int ptype, const void* data, const int32_t* i
                         int64_t n_dense, int64_t nnz, int long_rows, void* scratch, size_t scratch_bytes, void* stream);
 
 /*
+ * COO triples grouped by row (nnz > 0): values and columns in row order -- entries of a row in the order in which they are
+ * given, or with by_column != 0 in column order, equal (row, column) pairs in the order given --, the sorted row ids and the
+ * row pointer (int32, n_rows + 1).  Takes the place of the sorts of the reference
+ * (_sort_coo_lex, src/flagsparse/sparse_operations/spmv_coo.py:153-165; spmm_coo.py:21-105).
+ *   value_bytes   2, 4, 8 or 16 bytes per value; rtype, ctype: FSB_I32 / FSB_I64 of row and col
+ *   stats         ten int64 on the device: the eight of fsb_csr_analyze, then the smallest and largest row id.  Nothing is
+ *                 checked on the way: ids outside the matrix touch no memory outside the arrays, and what the other outputs
+ *                 hold is then meaningless.
+ *   scratch       fsb_coo_scratch_bytes(nnz) bytes, 16-byte aligned
+ */
+size_t fsb_coo_scratch_bytes(int64_t nnz);
+int fsb_coo_group(int value_bytes, int rtype, int ctype, const void* data, const void* row, const void* col, int64_t nnz,
+                  int64_t n_rows, int64_t n_cols, int by_column, void* out_data, int32_t* out_row, int32_t* out_col,
+                  int32_t* indptr, int64_t* stats, void* scratch, size_t scratch_bytes, void* stream);
+
+/*
  * y = A x in two streaming passes (float32 / float64), for matrices whose columns lie all over a long x: every entry is
  * multiplied where its chunk of x is in shared memory, the products go through memory once, and every row block adds up
  * its rows in CSR order, in double.  Bit-reproducible.  Takes the place of the launches in
