@@ -10,7 +10,7 @@
 // ids out of range lead nowhere but to a place inside the arrays, and the caller reads the statistics once, at the end.
 // 2.1 M triples in no order, 150001 rows, 64-bit ids: 110 us of kernels -- first count with the checks 16 us, moves 26 and 45 us
 // (the latency of one wave of tiles; the last one waits for values and columns from anywhere), row pointer 10 us -- where a
-// library sort, gathers and passes for the checks took 210 us and five looks from the host.
+// library sort, gathers, passes for the checks and an analysis took 210 us and two read-backs.
 #include "fsb_common.cuh"
 
 namespace fsb {
