@@ -10,7 +10,7 @@
 //   sum       a CTA owns a row block: it fetches the block's run of packs from every chunk (one 32-bit pack number per pack),
 //             puts each product at its entry's CSR position in shared memory (16 bits per entry), and adds up the rows.
 // Per float32 entry 4 + 2 bytes in and 4 out, then 4 + 2 + 0.5 in: twice the bytes of one pass, all of them streamed.  Rows
-// are summed in CSR order, in double, so results do not depend on the order of the entries inside a unit and are
+// are summed in CSR order, in double (float64: compensated inside a slice), so results do not depend on the order of the entries inside a unit and are
 // bit-reproducible.  107 M entries in 16.7 M rows of Zipf lengths, columns anywhere in 2^24, float32: 640 us through
 // spmv_stream_kernel, 443 us here: multiply 215 us (1.2 GB, memory), sum 225 us (0.85 GB; a block's products arrive, are added
 // up and leave in turn, and two blocks an SM cover each other's phases in part).  With the products written to block order by
@@ -170,15 +170,27 @@ bins_sum_kernel(const V* __restrict__ prod, const int32_t* __restrict__ place, c
   }
   __syncthreads();
   V* slice = s_prod + tid * (S + 1);
-  double tail = 0;
+  // float64: what every addition rounds off is kept beside the sum, or slot after slot would lose more than the lanes' tree of
+  // the one-pass kernel (rows of 4 entries: rms error 8.9e-17 without it, 7.7e-17 in one pass)
+  constexpr bool COMP = sizeof(V) == 8;
+  double tail = 0, off = 0;
 #pragma unroll
   for (int j = 0; j < S; ++j) {
-    tail += (double)slice[j];
+    const double v = (double)slice[j];
+    if (COMP) {
+      const double t = tail + v, u = t - tail;
+      off += (tail - (t - u)) + (v - u);
+      tail = t;
+    } else {
+      tail += v;
+    }
     if (mask & (1u << j)) {
-      slice[j] = (V)tail;
+      slice[j] = (V)(COMP ? tail + comp_term(tail, off) : tail);
       tail = 0;
+      off = 0;
     }
   }
+  if (COMP) tail += comp_term(tail, off);
   // inclusive segmented scan over the lanes: what lane l and the lanes before have of the row that goes on behind lane l
   const uint32_t closed = __ballot_sync(0xffffffffu, mask != 0);     // lanes in which a row ends
 #pragma unroll
