@@ -57,10 +57,11 @@ def test_edges(cuda, fsb_lib, name, vdt, pdt):
         assert torch.equal(y, want)
 
 
-def test_infinities_stay_in_their_rows(cuda, fsb_lib):
+@pytest.mark.parametrize("vdt", ["float32", "float64"])
+def test_infinities_stay_in_their_rows(cuda, fsb_lib, vdt):
     lens = [40, 3, 70, 1, 5] * 300
-    d, i, p = handmade_csr(2, lens, 5000)
-    x = np.random.default_rng(1).uniform(0.5, 1, 5000).astype(np.float32)
+    d, i, p = handmade_csr(2, lens, 5000, value_dtype=vdt)
+    x = np.random.default_rng(1).uniform(0.5, 1, 5000).astype(vdt)
     rows = [0, 2, 601, 1499]
     for r in rows:
         d[p[r]] = np.inf
