@@ -91,8 +91,7 @@ SIGNATURES = {
     "fsb_spmv_bins_pack": (_i32, [_i32]),
     "fsb_spmv_bins_ends": (_i32, []),
     "fsb_spmv_bins_count": (_i32, [_i32, _vp, _vp, _vp, _i32, _i32, _i32, _i64, _vp, _vp]),
-    "fsb_spmv_bins_place": (_i32, [_i32, _i32, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp,
-                                   _vp]),
+    "fsb_spmv_bins_place": (_i32, [_i32, _i32, _vp, _vp, _vp, _i32, _i32, _i32, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp]),
     "fsb_spmv_csr_bins": (_i32, [_i32, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i64, _vp, _sz, _vp, _vp,
                                  _i64, _i64, _vp]),
     "fsb_sddmm_csr": (_i32, [_i32, _vp, _vp, _vp, _i64, _vp, _i64, _vp, _vp, _i64, _i64, _i64, _i64, _c.c_double,

@@ -2,8 +2,9 @@
 over a long x and whose rows have nothing to share in a chunk of it.
 
 The reference's prepare step builds row-length buckets (src/flagsparse/sparse_operations/spmv_csr.py:281-327); this one
-stores the entries a second time, by (chunk of columns, block of rows), so that the product reads x from shared memory and
-everything else in order.  One count and one placing kernel, a cumulative sum over the units between them.
+stores the columns a second time, by (chunk of columns, block of rows), so that the product reads x from shared memory and
+everything else in order; the values are read where the caller has them.  One count and one placing kernel, a cumulative sum
+over the units between them.
 """
 
 import os
@@ -14,20 +15,20 @@ from . import _lib
 from ._common import _ITYPE, _VTYPE
 
 # Where the two passes win, each line with both sides measured (us, one pass against two; columns anywhere unless said).
-# Rows of about equal length against the lanes-per-row kernel, float32: 2^27 entries in 33.6 M / 16.8 M / 4.2 M rows: 1324 / 627 /
-# 551 against 631 / 534 / 479; 2^24 entries in 4.2 M / 1 M / 0.5 M rows: 94 / 76 / 76 against 74 / 64 / 65; 2^23 entries: 48 / 41 / 40
-# against 42 / 39 / 39, which a few hundred microseconds of prepare would not be worth; 2^22: 25 / 22 / 21 against 27 / 27 / 24.
+# Rows of about equal length against the lanes-per-row kernel, float32: 2^27 entries in 33.6 M / 16.8 M / 4.2 M rows: 1330 / 626 /
+# 549 against 609 / 533 / 472; 2^24 entries in 4.2 M / 1 M / 0.5 M rows: 92 / 74 / 74 against 75 / 66 / 64; 2^23 entries in 2.1 M /
+# 0.5 M rows: 45 / 35 against 43 / 39.
 EVEN_MIN_NNZ = 1 << 24
 EVEN_MIN_SPAN = 2 << 20
-# Uneven rows (the short rows of a skewed matrix, mostly), float32: 107 M entries 640 against 444; 10.8 M entries in 2.1 M rows 87
-# against 45; 2.3 M entries in 0.3 M rows 20.7 against 18.6; 2.0 M entries in 0.1 M rows 18.0 against 18.6.
+# Uneven rows (the short rows of a skewed matrix, mostly), float32: 10.4 M entries in 2.1 M rows 91 against 46; 3.1 M in 0.5 M rows
+# 24.2 against 22.1; 2.7 M in 0.3 M rows 22.0 against 19.5; 2.6 M in 0.25 M rows 20.7 against 19.8.
 UNEVEN_MIN_NNZ = 5 << 19
 UNEVEN_MIN_SPAN = 1 << 20
-# float64 moves 28.5 bytes an entry instead of 12, so it takes an x that L2 does not hold: 2^27 entries in 33.6 M / 16.8 M / 8.4 M
-# rows: 2157 / 1335 / 724 against 1502 / 1194 / 1017; uneven, 2^26 entries in 16.8 M / 8.4 M rows: 471 / 254 against 398 / 274.
+# float64 moves 29 bytes an entry instead of 12, so it takes an x that L2 does not hold: 2^27 entries in 33.6 M / 16.8 M / 8.4 M
+# rows: 2155 / 1335 / 716 against 1461 / 1178 / 1030; uneven, 2^26 entries in 16.8 M / 8.4 M rows: 780 / 464 against 648 / 546.
 F64_MIN_SPAN = 120 << 20
 # ... or uneven rows of a few entries that would have gone to the lanes-per-row kernel, whose warps wait for their longest row:
-# 4.0 M entries in 2.1 M rows 62 against 45, 3.0 M in 1 M rows 41 against 33; 2.6 M in 0.5 M rows 29.5 against 29.4.
+# 4.8 M entries in 2.1 M rows 66 against 49, 3.3 M in 1 M rows 42 against 35; by tiles, 2.6 M in 0.5 M rows 23.6 against 30.1.
 F64_SHORT_MEAN = 4
 # mean entries of a unit below which the packs would mostly be padding (measured down to 36 and 9 entries, float32 and float64)
 MIN_UNIT = {4: 16, 8: 8}
@@ -54,12 +55,12 @@ def min_span(nnz, n_rows, max_row_nnz, element_size, lanes_per_row):
 class BinsLayout:
     """Device arrays of the regrouped matrix (include/fsb.h, fsb_spmv_csr_bins)."""
 
-    __slots__ = ("val", "col", "place", "dst", "ends", "chunk_pack", "block_pack", "block_row", "row_slot", "n_blocks", "n_chunks",
-                 "chunk_cols", "n_packs")
+    __slots__ = ("data", "col", "place", "dst", "ends", "chunk_pack", "block_pack", "block_start", "row_slot", "n_blocks",
+                 "n_chunks", "chunk_cols", "n_packs")
 
     def nbytes(self):
-        return sum(t.numel() * t.element_size() for t in (self.val, self.col, self.place, self.dst, self.ends, self.row_slot,
-                                                          self.chunk_pack, self.block_pack, self.block_row))
+        return sum(t.numel() * t.element_size() for t in (self.col, self.place, self.dst, self.ends, self.row_slot,
+                                                          self.chunk_pack, self.block_pack, self.block_start))
 
 
 def _starts(packs):
@@ -109,17 +110,18 @@ def build_bins_layout(data, indices, indptr, n_rows, n_cols, max_row_nnz, span=0
         unit_chunk = by_chunk[:-1].view(n_chunks, n_blocks).t().contiguous()
         del by_chunk
         lay = BinsLayout()
-        lay.val = torch.empty(pack * n_packs, dtype=data.dtype, device=dev)
+        lay.data = data                       # the caller's own: the product reads the values there
         lay.col = torch.empty(pack * n_packs, dtype=torch.int16, device=dev)
         lay.place = torch.empty(n_packs, dtype=torch.int32, device=dev)
         lay.dst = torch.empty(pack * n_packs, dtype=torch.int16, device=dev)
         lay.ends = torch.empty(n_ends * n_blocks, dtype=torch.int32, device=dev)
         lay.row_slot = torch.empty(n_rows, dtype=torch.int16, device=dev)
-        _lib.check(L.fsb_spmv_bins_place(vt, pt, data.data_ptr(), indices.data_ptr(), indptr.data_ptr(), block_row.data_ptr(),
+        _lib.check(L.fsb_spmv_bins_place(vt, pt, indices.data_ptr(), indptr.data_ptr(), block_row.data_ptr(),
                                          n_blocks, n_chunks, chunk_cols, n_cols, unit_chunk.data_ptr(), unit_block.data_ptr(),
-                                         lay.val.data_ptr(), lay.col.data_ptr(), lay.place.data_ptr(), lay.dst.data_ptr(),
+                                         lay.col.data_ptr(), lay.place.data_ptr(), lay.dst.data_ptr(),
                                          lay.ends.data_ptr(), lay.row_slot.data_ptr(), st), "fsb_spmv_bins_place")
-    lay.chunk_pack, lay.block_pack, lay.block_row = chunk_pack, block_pack, block_row
+        lay.block_start = torch.stack((block_row.to(torch.int64), indptr[block_row.long()].to(torch.int64)), 1).contiguous()
+    lay.chunk_pack, lay.block_pack = chunk_pack, block_pack
     lay.n_blocks, lay.n_chunks, lay.chunk_cols, lay.n_packs = n_blocks, n_chunks, chunk_cols, n_packs
     return lay
 
@@ -138,15 +140,17 @@ def bins_for(data, indices, indptr, n_rows, n_cols, max_row_nnz, lanes_per_row):
     return build_bins_layout(data, indices, indptr, n_rows, n_cols, max_row_nnz, span)
 
 
-def launch_bins(layout, x, y, n_rows, n_cols, stream_ptr):
-    """Enqueue the product on the current stream (its handle in stream_ptr).  The products' memory is the call's own: calls
-    on one matrix may overlap in several streams."""
+def launch_bins(layout, x, y, n_rows, n_cols, stream_ptr, data=None):
+    """Enqueue the product on the current stream (its handle in stream_ptr).  data: the values, in CSR order, instead of those
+    that the layout was made with.  The memory between the passes is the call's own: calls on one matrix may overlap in
+    several streams."""
     la = layout
-    prod = torch.empty(32 * la.n_packs, dtype=torch.uint8, device=la.val.device)
+    data = la.data if data is None else data
+    xg = torch.empty(32 * la.n_packs, dtype=torch.uint8, device=data.device)
     rc = _lib.lib().fsb_spmv_csr_bins(
-        _VTYPE[la.val.dtype], la.val.data_ptr(), la.col.data_ptr(), la.place.data_ptr(), la.dst.data_ptr(), la.ends.data_ptr(),
-        la.row_slot.data_ptr(), la.chunk_pack.data_ptr(), la.block_pack.data_ptr(), la.block_row.data_ptr(), la.n_blocks,
-        la.n_chunks, la.chunk_cols, la.n_packs, prod.data_ptr(), prod.numel(), x.data_ptr(), y.data_ptr(), n_rows, n_cols,
-        stream_ptr,
+        _VTYPE[data.dtype], la.col.data_ptr(), la.place.data_ptr(), la.dst.data_ptr(), la.ends.data_ptr(),
+        la.row_slot.data_ptr(), la.chunk_pack.data_ptr(), la.block_pack.data_ptr(), la.block_start.data_ptr(), data.data_ptr(),
+        la.n_blocks, la.n_chunks, la.chunk_cols, la.n_packs, xg.data_ptr(), xg.numel(), x.data_ptr(), y.data_ptr(), n_rows,
+        n_cols, stream_ptr,
     )
     _lib.check(rc, "fsb_spmv_csr_bins")

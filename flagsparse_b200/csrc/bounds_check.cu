@@ -106,7 +106,7 @@ check_panel_kernel(const uint32_t* __restrict__ rc, const int32_t* __restrict__ 
 __global__ void __launch_bounds__(kCheckThreads)
 check_bins_kernel(const uint16_t* __restrict__ col, const int32_t* __restrict__ place, const uint16_t* __restrict__ dst,
                   const uint16_t* __restrict__ row_slot, const int32_t* __restrict__ chunk_pack,
-                  const int32_t* __restrict__ block_pack, const int32_t* __restrict__ block_row, int n_blocks, int n_chunks,
+                  const int32_t* __restrict__ block_pack, const int64_t* __restrict__ block_start, int n_blocks, int n_chunks,
                   int chunk_cols, int slots, int pack, int64_t n_packs, int64_t n_rows, int64_t n_cols) {
   __shared__ int ok;
   if (threadIdx.x == 0) ok = 1;
@@ -119,7 +119,8 @@ check_bins_kernel(const uint16_t* __restrict__ col, const int32_t* __restrict__ 
     }
   }
   for (int b = threadIdx.x; b < n_blocks; b += kCheckThreads) {
-    const int a = block_row[b], z = block_row[b + 1], pa = block_pack[b], pz = block_pack[b + 1];
+    const int64_t a = block_start[2 * b], z = block_start[2 * b + 2];
+    const int pa = block_pack[b], pz = block_pack[b + 1];
     if (a < 0 || z < a || z > n_rows || (b == 0 && a != 0) || (b == n_blocks - 1 && z != n_rows)) {
       if (blockIdx.x == 0) note(FSB_BAD_ROW_ID, b, z, n_rows);
       ok = 0;
@@ -219,13 +220,13 @@ int check_panel(const uint32_t* rc_words, const int32_t* unit_piece_ptr, const i
 }
 
 int check_bins(int vtype, const uint16_t* col, const int32_t* place, const uint16_t* dst, const uint16_t* row_slot,
-               const int32_t* chunk_pack, const int32_t* block_pack, const int32_t* block_row, int n_blocks, int n_chunks,
+               const int32_t* chunk_pack, const int32_t* block_pack, const int64_t* block_start, int n_blocks, int n_chunks,
                int chunk_cols, int64_t n_packs, int64_t n_rows, int64_t n_cols, cudaStream_t st) {
   void* rec = nullptr;
   int rc = begin_check(st, &rec);
   if (rc != FSB_OK) return rc;
   const int slots = fsb_spmv_bins_cap(vtype) + fsb_spmv_bins_ends() + 2;
-  check_bins_kernel<<<kCheckBlocks, kCheckThreads, 0, st>>>(col, place, dst, row_slot, chunk_pack, block_pack, block_row, n_blocks,
+  check_bins_kernel<<<kCheckBlocks, kCheckThreads, 0, st>>>(col, place, dst, row_slot, chunk_pack, block_pack, block_start, n_blocks,
                                                             n_chunks, chunk_cols, slots, fsb_spmv_bins_pack(vtype), n_packs,
                                                             n_rows, n_cols);
   return end_check(st, rec);

@@ -3,23 +3,26 @@
 // Why: where neither L1 nor a chunk of x in shared memory serves the gathers (columns anywhere, rows too short to fill a unit
 // of the panel kernel), a one-pass kernel sends one request per entry towards L2, and once x outgrows L2 close to half of
 // them go on to memory for 32 bytes each.  Here no gather leaves the SM.  Prepare cuts the rows into blocks of at most 24 576
-// (float64: 12 288) entries and the columns into chunks, and stores the entries chunk by chunk, inside a chunk block by
-// block; what a block has in a chunk (a "unit") is filled up to whole packs of 32 bytes of values.
-//   multiply  a CTA holds one chunk of x in shared memory and walks its share of the entries in storage order: value and
-//             16-bit column inside the chunk in, product out, three streams;
+// (float64: 12 288) entries and the columns into chunks, and stores the columns of the entries a second time, chunk by chunk,
+// inside a chunk block by block; what a block has in a chunk (a "unit") is filled up to whole packs (8 entries, float64: 4).
+//   gather    a CTA holds one chunk of x in shared memory and walks its share of the entries in storage order: 16-bit column
+//             inside the chunk in, element of x out, two streams;
 //   sum       a CTA owns a row block: it fetches the block's run of packs from every chunk (one 32-bit pack number per pack),
-//             puts each product at its entry's CSR position in shared memory (16 bits per entry), and adds up the rows.
-// Per float32 entry 4 + 2 bytes in and 4 out, then 4 + 2 + 0.5 in: twice the bytes of one pass, all of them streamed.  Rows
-// are summed in CSR order, in double (float64: compensated inside a slice), so results do not depend on the order of the entries inside a unit and are
-// bit-reproducible.  107 M entries in 16.7 M rows of Zipf lengths, columns anywhere in 2^24, float32: 640 us through
-// spmv_stream_kernel, 443 us here: multiply 215 us (1.2 GB, memory), sum 225 us (0.85 GB; a block's products arrive, are added
-// up and leave in turn, and two blocks an SM cover each other's phases in part).  With the products written to block order by
-// the multiply (runs of 300 bytes on the way out, one run per block to read): 270 us and 185 us.
+//             puts each element of x at its entry's CSR position in shared memory (16 bits per entry), multiplies by the values,
+//             which lie in CSR order where the caller has them, and adds up the rows.
+// Per float32 entry 2 bytes in and 4 out, then 4 + 2 + 0.5 + 4 in (float64: 10 and 19): twice the bytes of one pass, all of
+// them streamed.  Rows are summed in CSR order, in double (float64: compensated inside a slice), so results do not depend on
+// the order of the entries inside a unit and are bit-reproducible.  107 M entries in 16.7 M rows of Zipf lengths, columns
+// anywhere in 2^24, float32: 640 us through spmv_stream_kernel, 443 us here: gather 135 us (0.64 GB), sum 306 us (1.13 GB; a
+// block's elements arrive, are multiplied and added up and leave in turn, and two blocks an SM cover each other's phases in
+// part).  With a copy of the values in storage order, multiplied by the first pass: 216 and 225 us, but 4 more bytes an entry,
+// and values that the caller writes later would not be seen.  (The values asked for ahead with prefetch.global.L2: 437 us
+// here, but 73 us instead of 70 us for 2^24 entries, which L2 holds.)
 #include "fsb_common.cuh"
 
 namespace fsb {
 
-constexpr int kBinMulThreads = 1024;
+constexpr int kBinGatherThreads = 1024;
 constexpr int kBinSumThreads = 768;
 constexpr int kBinBuildThreads = 512;
 constexpr int kBinQuad = 4;                  // entries that a thread moves together
@@ -31,7 +34,7 @@ template <typename V> __host__ __device__ constexpr int bin_pack() { return 32 /
 template <typename V> __host__ __device__ constexpr int bin_slice() { return 128 / (int)sizeof(V); }
 template <typename V> __host__ __device__ constexpr int bin_cap() { return kBinSumThreads * bin_slice<V>(); }
 template <typename V> __host__ __device__ __forceinline__ int bin_slot(int i) { return i + i / bin_slice<V>(); }
-// two more places: a zero for the rows without entries, and where the products go that fill a unit up
+// two more places: a zero for the rows without entries, and where what fills a unit up goes
 template <typename V> __host__ __device__ constexpr int bin_empty() { return kBinSumThreads * (bin_slice<V>() + 1); }
 template <typename V> __host__ __device__ constexpr int bin_fill() { return bin_empty<V>() + 1; }
 
@@ -51,12 +54,12 @@ __device__ __forceinline__ void st_quad(double* p, const double (&v)[4]) {
   reinterpret_cast<double2*>(p)[1] = make_double2(v[2], v[3]);
 }
 
-// prod[e] = val[e] * x[first column of e's chunk + col[e]] for all stored entries e.  CTA i takes the i-th equal share of the
-// packs; a share crosses few chunks, so the chunks of x cost little beside the entries.
+// xg[e] = x[first column of e's chunk + col[e]] for all stored entries e.  CTA i takes the i-th equal share of the packs; a
+// share crosses few chunks, so the chunks of x cost little beside the entries.
 template <typename V>
-__global__ void __launch_bounds__(kBinMulThreads, 1)
-bins_multiply_kernel(const V* __restrict__ val, const uint16_t* __restrict__ col, const int32_t* __restrict__ chunk_pack,
-                     int n_chunks, int chunk_cols, const V* __restrict__ x, int64_t n_cols, V* __restrict__ prod) {
+__global__ void __launch_bounds__(kBinGatherThreads, 1)
+bins_gather_kernel(const uint16_t* __restrict__ col, const int32_t* __restrict__ chunk_pack, int n_chunks, int chunk_cols,
+                   const V* __restrict__ x, int64_t n_cols, V* __restrict__ xg) {
   extern __shared__ __align__(16) unsigned char b_smem[];
   V* xs = reinterpret_cast<V*>(b_smem);
   constexpr int QP = bin_pack<V>() / kBinQuad;        // quads of a pack
@@ -80,48 +83,45 @@ bins_multiply_kernel(const V* __restrict__ val, const uint16_t* __restrict__ col
     __syncthreads();                          // the previous chunk is no longer read
     const V* src = x + c0;
     if (aligned_to_dev(src)) {
-      for (int i = tid; i < n / E; i += kBinMulThreads) cp_async16(xs + i * E, src + i * E);
-      for (int i = n / E * E + tid; i < n; i += kBinMulThreads) xs[i] = src[i];
+      for (int i = tid; i < n / E; i += kBinGatherThreads) cp_async16(xs + i * E, src + i * E);
+      for (int i = n / E * E + tid; i < n; i += kBinGatherThreads) xs[i] = src[i];
       cp_async_wait();
     } else {
-      for (int i = tid; i < n; i += kBinMulThreads) xs[i] = __ldg(src + i);
+      for (int i = tid; i < n; i += kBinGatherThreads) xs[i] = __ldg(src + i);
     }
     __syncthreads();
-    // the next U quads are requested before the current ones are multiplied: the loads never wait for the gathers
+    // the next U quads are requested before the current ones are looked up
     const int64_t end = (int64_t)p_end * QP;
-    V v[2][U][4];
     uint2 w[2][U];
     auto request = [&](int64_t k, int s) {
 #pragma unroll
       for (int u = 0; u < U; ++u) {
-        const int64_t kk = k + u * kBinMulThreads;
-        if (kk < end) {
-          ld_stream4(val + kk * kBinQuad, v[s][u]);
-          w[s][u] = __ldcs(reinterpret_cast<const uint2*>(col + kk * kBinQuad));
-        }
+        const int64_t kk = k + u * kBinGatherThreads;
+        if (kk < end) w[s][u] = __ldcs(reinterpret_cast<const uint2*>(col + kk * kBinQuad));
       }
     };
-    auto multiply = [&](int64_t k, int s) {
+    auto look_up = [&](int64_t k, int s) {
 #pragma unroll
       for (int u = 0; u < U; ++u) {
-        const int64_t kk = k + u * kBinMulThreads;
+        const int64_t kk = k + u * kBinGatherThreads;
         if (kk < end) {
           uint32_t cc[4];
+          V v[4];
           unpack16(w[s][u], cc);
 #pragma unroll
-          for (int j = 0; j < 4; ++j) v[s][u][j] *= xs[cc[j]];
-          st_quad(prod + kk * kBinQuad, v[s][u]);
+          for (int j = 0; j < 4; ++j) v[j] = xs[cc[j]];
+          st_quad(xg + kk * kBinQuad, v);
         }
       }
     };
-    constexpr int STEP = U * kBinMulThreads;
+    constexpr int STEP = U * kBinGatherThreads;
     int64_t k = (int64_t)p * QP + tid;
     request(k, 0);
     for (; k < end; k += 2 * STEP) {
       request(k + STEP, 1);
-      multiply(k, 0);
+      look_up(k, 0);
       request(k + 2 * STEP, 0);
-      multiply(k + STEP, 1);
+      look_up(k + STEP, 1);
     }
     p = p_end;
   }
@@ -133,8 +133,8 @@ bins_multiply_kernel(const V* __restrict__ val, const uint16_t* __restrict__ col
 // before have of the row that a slice begins in the middle of comes from a segmented scan over the threads.
 template <typename V>
 __global__ void __launch_bounds__(kBinSumThreads, 2)
-bins_sum_kernel(const V* __restrict__ prod, const int32_t* __restrict__ place, const uint16_t* __restrict__ dst,
-                const int32_t* __restrict__ block_pack, const int32_t* __restrict__ block_row,
+bins_sum_kernel(const V* __restrict__ data, const V* __restrict__ xg, const int32_t* __restrict__ place,
+                const uint16_t* __restrict__ dst, const int32_t* __restrict__ block_pack, const int64_t* __restrict__ block_start,
                 const uint32_t* __restrict__ ends, const uint16_t* __restrict__ row_slot, V* __restrict__ y) {
   extern __shared__ __align__(16) unsigned char b_smem[];
   V* s_prod = reinterpret_cast<V*>(b_smem);
@@ -145,7 +145,8 @@ bins_sum_kernel(const V* __restrict__ prod, const int32_t* __restrict__ place, c
   __shared__ int s_any[NW];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int b = blockIdx.x;
-  const int r0 = block_row[b], r1 = block_row[b + 1];
+  const int64_t r0 = block_start[2 * b], r1 = block_start[2 * b + 2];
+  const int n = (int)(block_start[2 * b + 3] - block_start[2 * b + 1]);
   const int64_t q0 = (int64_t)block_pack[b] * QP + tid;
   int left = (int)((int64_t)block_pack[b + 1] * QP - q0);             // quads from this thread's first one on
   const uint32_t mask = __ldcs(ends + (int64_t)b * kBinSumThreads + tid);
@@ -159,13 +160,35 @@ bins_sum_kernel(const V* __restrict__ prod, const int32_t* __restrict__ place, c
     for (; left > 0; left -= kBinSumThreads) {
       V v[4];
       uint32_t d[4];
-      ld_stream4(prod + ((int64_t)from * QP + within) * kBinQuad, v);
+      ld_stream4(xg + ((int64_t)from * QP + within) * kBinQuad, v);
       unpack16(__ldcs(reinterpret_cast<const uint2*>(to)), d);
       at += kBinSumThreads / QP;
       to += kBinSumThreads * kBinQuad;
       if (left > kBinSumThreads) from = __ldcs(at);     // the next pack's place is on its way while this one is fetched
 #pragma unroll
       for (int j = 0; j < 4; ++j) s_prod[d[j]] = v[j];
+    }
+  }
+  // times the values, which lie in CSR order: entry i of the block is kept at bin_slot(i)
+  {
+    constexpr int D = sizeof(V) == 4 ? 8 : 4;          // values of a thread on their way together
+    constexpr int STEP = kBinSumThreads + kBinSumThreads / S;
+    const V* at = data + block_start[2 * b + 1] + tid;
+    V* keep = s_prod + bin_slot<V>(tid);
+    V a[D];
+#pragma unroll
+    for (int u = 0; u < D; ++u) a[u] = tid + u * kBinSumThreads < n ? __ldcs(at + u * kBinSumThreads) : (V)0;
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < S; k += D) {
+#pragma unroll
+      for (int u = 0; u < D; ++u) {
+        if (tid + (k + u) * kBinSumThreads < n) keep[(k + u) * STEP] *= a[u];
+        if (k + D < S) {
+          const int next = k + D + u;
+          a[u] = tid + next * kBinSumThreads < n ? __ldcs(at + next * kBinSumThreads) : (V)0;
+        }
+      }
     }
   }
   __syncthreads();
@@ -217,7 +240,7 @@ bins_sum_kernel(const V* __restrict__ prod, const int32_t* __restrict__ place, c
   }
   __syncthreads();
   // four rows of a thread at a time, from a multiple of four on; what is left at both ends one by one
-  const int64_t a0 = ((int64_t)r0 + 3) & ~(int64_t)3, a1 = (int64_t)r1 & ~(int64_t)3;
+  const int64_t a0 = (r0 + 3) & ~(int64_t)3, a1 = r1 & ~(int64_t)3;
   if (a0 < a1 && aligned_to_dev(y)) {
     for (int64_t r = a0 + 4 * tid; r < a1; r += 4 * kBinSumThreads) {
       uint32_t d[4];
@@ -230,7 +253,7 @@ bins_sum_kernel(const V* __restrict__ prod, const int32_t* __restrict__ place, c
     const int64_t r = tid < 4 ? r0 + tid : a1 + (tid - 4);
     if (tid < 8 && (tid < 4 ? r < a0 : r < r1)) y[r] = s_prod[row_slot[r]];
   } else {
-    for (int64_t r = (int64_t)r0 + tid; r < r1; r += kBinSumThreads) y[r] = s_prod[row_slot[r]];
+    for (int64_t r = r0 + tid; r < r1; r += kBinSumThreads) y[r] = s_prod[row_slot[r]];
   }
 }
 
@@ -252,13 +275,13 @@ bins_count_kernel(const int32_t* __restrict__ idx, const P* __restrict__ ptr, co
 }
 
 // Every entry of block b to its unit, in any order inside the unit (the sum puts the products back in CSR order); what is
-// left of a unit's last pack is filled with zeros that no row reads.  unit_chunk[b * n_chunks + c], unit_block[...]: first
+// left of a unit's last pack is filled with first columns that no row reads.  unit_chunk[b * n_chunks + c], unit_block[...]: first
 // pack of the unit in chunk order and in block order; the last of each array is the number of packs.
 template <typename V, typename P>
 __global__ void __launch_bounds__(kBinBuildThreads)
-bins_place_kernel(const V* __restrict__ data, const int32_t* __restrict__ idx, const P* __restrict__ ptr,
+bins_place_kernel(const int32_t* __restrict__ idx, const P* __restrict__ ptr,
                   const int32_t* __restrict__ block_row, int n_chunks, int chunk_cols, const int32_t* __restrict__ unit_chunk,
-                  const int32_t* __restrict__ unit_block, V* __restrict__ val, uint16_t* __restrict__ col,
+                  const int32_t* __restrict__ unit_block, uint16_t* __restrict__ col,
                   int32_t* __restrict__ place, uint16_t* __restrict__ dst, uint32_t* __restrict__ ends,
                   uint16_t* __restrict__ row_slot) {
   constexpr int PACK = bin_pack<V>(), S = bin_slice<V>();
@@ -285,9 +308,7 @@ bins_place_kernel(const V* __restrict__ data, const int32_t* __restrict__ idx, c
   for (int64_t i = lo + threadIdx.x; i < hi; i += kBinBuildThreads) {
     const uint32_t j = (uint32_t)idx[i], c = j / (uint32_t)chunk_cols;
     const int rank = atomicAdd(&s_cells[c], 1);
-    const int64_t at = (int64_t)cm[c] * PACK + rank;
-    val[at] = data[i];
-    col[at] = (uint16_t)(j - c * (uint32_t)chunk_cols);
+    col[(int64_t)cm[c] * PACK + rank] = (uint16_t)(j - c * (uint32_t)chunk_cols);
     dst[(int64_t)bm[c] * PACK + rank] = (uint16_t)bin_slot<V>((int)(i - lo));
   }
   __syncthreads();
@@ -295,7 +316,6 @@ bins_place_kernel(const V* __restrict__ data, const int32_t* __restrict__ idx, c
     const int n = s_cells[c], packs = (n + PACK - 1) / PACK;
     for (int k = 0; k < packs; ++k) place[bm[c] + k] = cm[c] + k;
     for (int k = n; k < packs * PACK; ++k) {
-      val[(int64_t)cm[c] * PACK + k] = (V)0;
       col[(int64_t)cm[c] * PACK + k] = 0;
       dst[(int64_t)bm[c] * PACK + k] = (uint16_t)bin_fill<V>();
     }
@@ -340,23 +360,23 @@ extern "C" int fsb_spmv_bins_count(int ptype, const int32_t* indices, const void
   return FSB_OK;
 }
 
-extern "C" int fsb_spmv_bins_place(int vtype, int ptype, const void* data, const int32_t* indices, const void* indptr,
+extern "C" int fsb_spmv_bins_place(int vtype, int ptype, const int32_t* indices, const void* indptr,
                                    const int32_t* block_row, int32_t n_blocks, int32_t n_chunks, int32_t chunk_cols,
-                                   int64_t n_cols, const int32_t* unit_chunk, const int32_t* unit_block, void* val,
+                                   int64_t n_cols, const int32_t* unit_chunk, const int32_t* unit_block,
                                    uint16_t* col, int32_t* place, uint16_t* dst, uint32_t* ends, uint16_t* row_slot,
                                    void* stream_) {
   cudaStream_t st = static_cast<cudaStream_t>(stream_);
   const int rc = bins_check_shape(vtype, ptype, n_blocks, n_chunks, chunk_cols, n_cols);
   if (rc != FSB_OK) return rc;
   if (n_blocks == 0) return FSB_OK;
-  if (!data || !indices || !indptr || !block_row || !unit_chunk || !unit_block || !val || !col || !place || !dst || !ends ||
+  if (!indices || !indptr || !block_row || !unit_chunk || !unit_block || !col || !place || !dst || !ends ||
       !row_slot)
     return FSB_EINVAL;
   const size_t smem = (size_t)n_chunks * sizeof(int32_t);
 #define FSB_BINS_PLACE(V_, P_)                                                                                         \
   bins_place_kernel<V_, P_><<<(unsigned)n_blocks, kBinBuildThreads, smem, st>>>(                                       \
-      (const V_*)data, indices, (const P_*)indptr, block_row, n_chunks, chunk_cols, unit_chunk, unit_block, (V_*)val,  \
-      col, place, dst, ends, row_slot)
+      indices, (const P_*)indptr, block_row, n_chunks, chunk_cols, unit_chunk, unit_block, col, \
+      place, dst, ends, row_slot)
   if (vtype == FSB_F32) {
     if (ptype == FSB_I32) FSB_BINS_PLACE(float, int32_t); else FSB_BINS_PLACE(float, int64_t);
   } else {
@@ -367,10 +387,10 @@ extern "C" int fsb_spmv_bins_place(int vtype, int ptype, const void* data, const
   return FSB_OK;
 }
 
-extern "C" int fsb_spmv_csr_bins(int vtype, const void* val, const uint16_t* col, const int32_t* place, const uint16_t* dst,
-                                 const uint32_t* ends, const uint16_t* row_slot, const int32_t* chunk_pack,
-                                 const int32_t* block_pack, const int32_t* block_row, int32_t n_blocks, int32_t n_chunks,
-                                 int32_t chunk_cols, int64_t n_packs, void* prod, size_t prod_bytes, const void* x, void* y,
+extern "C" int fsb_spmv_csr_bins(int vtype, const uint16_t* col, const int32_t* place, const uint16_t* dst, const uint32_t* ends,
+                                 const uint16_t* row_slot, const int32_t* chunk_pack, const int32_t* block_pack,
+                                 const int64_t* block_start, const void* data, int32_t n_blocks, int32_t n_chunks,
+                                 int32_t chunk_cols, int64_t n_packs, void* xg, size_t xg_bytes, const void* x, void* y,
                                  int64_t n_rows, int64_t n_cols, void* stream_) {
   cudaStream_t st = static_cast<cudaStream_t>(stream_);
   int rc = bins_check_shape(vtype, FSB_I32, n_blocks, n_chunks, chunk_cols, n_cols);
@@ -378,18 +398,18 @@ extern "C" int fsb_spmv_csr_bins(int vtype, const void* val, const uint16_t* col
   if (n_rows < 0 || n_packs < 0) return FSB_EINVAL;
   if (n_rows >= INT32_MAX || n_packs >= INT32_MAX) return FSB_ERANGE;
   if (n_rows == 0) return FSB_OK;
-  if (n_blocks == 0 || !val || !col || !place || !dst || !ends || !row_slot || !chunk_pack || !block_pack || !block_row ||
-      !prod || !x || !y)
+  if (n_blocks == 0 || !col || !place || !dst || !ends || !row_slot || !chunk_pack || !block_pack || !block_start || !data ||
+      !xg || !x || !y)
     return FSB_EINVAL;
   const size_t sv = vtype == FSB_F32 ? 4 : 8;
-  if (prod_bytes < (size_t)n_packs * 32) return FSB_ESCRATCH;
-  if (!aligned_to(val, 16) || !aligned_to(col, 16) || !aligned_to(dst, 16) || !aligned_to(row_slot, 16) || !aligned_to(prod, 32) ||
-      !aligned_to(x, sv) || !aligned_to(y, sv))
+  if (xg_bytes < (size_t)n_packs * 32) return FSB_ESCRATCH;
+  if (!aligned_to(col, 16) || !aligned_to(dst, 16) || !aligned_to(row_slot, 16) || !aligned_to(xg, 32) ||
+      !aligned_to(data, sv) || !aligned_to(x, sv) || !aligned_to(y, sv))
     return FSB_EALIGN;
-  const size_t mul_smem = (size_t)chunk_cols * sv;
+  const size_t gather_smem = (size_t)chunk_cols * sv;
   const size_t sum_smem = (size_t)(vtype == FSB_F32 ? bin_fill<float>() + 1 : bin_fill<double>() + 1) * sv;
-  if (mul_smem > 226 * 1024) return FSB_ERANGE;
-  FSB_WALK_FIRST(check_bins(vtype, col, place, dst, row_slot, chunk_pack, block_pack, block_row, n_blocks, n_chunks,
+  if (gather_smem > 226 * 1024) return FSB_ERANGE;
+  FSB_WALK_FIRST(check_bins(vtype, col, place, dst, row_slot, chunk_pack, block_pack, block_start, n_blocks, n_chunks,
                             chunk_cols, n_packs, n_rows, n_cols, st));
   int dev = 0, sms = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -397,16 +417,15 @@ extern "C" int fsb_spmv_csr_bins(int vtype, const void* val, const uint16_t* col
   if (e != cudaSuccess) return cuda_rc(e);
 #define FSB_BINS_RUN(V_)                                                                                                    \
   do {                                                                                                                      \
-    e = cudaFuncSetAttribute(bins_multiply_kernel<V_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mul_smem);         \
+    e = cudaFuncSetAttribute(bins_gather_kernel<V_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gather_smem);        \
     if (e != cudaSuccess) return cuda_rc(e);                                                                                \
     e = cudaFuncSetAttribute(bins_sum_kernel<V_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sum_smem);              \
     if (e != cudaSuccess) return cuda_rc(e);                                                                                \
-    bins_multiply_kernel<V_><<<(unsigned)sms, kBinMulThreads, mul_smem, st>>>((const V_*)val, col, chunk_pack,              \
-                                                                              n_chunks, chunk_cols, (const V_*)x, n_cols,   \
-                                                                              (V_*)prod);                                   \
+    bins_gather_kernel<V_><<<(unsigned)sms, kBinGatherThreads, gather_smem, st>>>(col, chunk_pack, n_chunks, chunk_cols,    \
+                                                                                  (const V_*)x, n_cols, (V_*)xg);           \
     FSB_RETURN_IF_LAUNCH_FAILED();                                                                                          \
-    bins_sum_kernel<V_><<<(unsigned)n_blocks, kBinSumThreads, sum_smem, st>>>((const V_*)prod, place, dst, block_pack, block_row,  \
-                                                                              ends, row_slot, (V_*)y);                      \
+    bins_sum_kernel<V_><<<(unsigned)n_blocks, kBinSumThreads, sum_smem, st>>>(                                              \
+        (const V_*)data, (const V_*)xg, place, dst, block_pack, block_start, ends, row_slot, (V_*)y);                       \
   } while (0)
   if (vtype == FSB_F32) FSB_BINS_RUN(float); else FSB_BINS_RUN(double);
 #undef FSB_BINS_RUN

@@ -367,7 +367,7 @@ def _spmv_launch(prepared, x, y):
         from . import bins
 
         with _on_device(dev):
-            bins.launch_bins(p.bins, x, y, p.n_rows, p.n_cols, _stream_ptr(dev))
+            bins.launch_bins(p.bins, x, y, p.n_rows, p.n_cols, _stream_ptr(dev), data=p.data)
         return
     algo = p.algo if p.tile_row is not None else _lib.FSB_SPMV_VECTOR
     # calls on a small matrix may overlap in several streams, whichever kernel its rows get: scratch of the call's own

@@ -370,27 +370,30 @@ int fsb_coo_group(int value_bytes, int rtype, int ctype, const void* data, const
                   int32_t* indptr, int64_t* stats, void* scratch, size_t scratch_bytes, void* stream);
 
 /*
- * y = A x in two streaming passes (float32 / float64), for matrices whose columns lie all over a long x: every entry is
- * multiplied where its chunk of x is in shared memory, the products go through memory once, and every row block adds up
- * its rows in CSR order, in double.  Bit-reproducible.  Takes the place of the launches in
- * _triton_spmv_csr_impl_opt_prepared (spmv_csr.py:329-376) for these matrices.
+ * y = A x in two streaming passes (float32 / float64), for matrices whose columns lie all over a long x: the element of x
+ * that an entry needs is taken where its chunk of x is in shared memory and goes through memory once; every row block
+ * multiplies by the values, which stay in CSR order in the caller's array, and adds up its rows in CSR order, in double.
+ * Bit-reproducible.  Takes the place of the launches in _triton_spmv_csr_impl_opt_prepared (spmv_csr.py:329-376) for these
+ * matrices.
  *   chunk c     columns [c * chunk_cols, (c + 1) * chunk_cols); chunk_cols = fsb_spmv_bins_chunk_cols(vtype) or less, a
  *               multiple of 4; at most fsb_spmv_bins_max_chunks() chunks, the last one not empty
- *   block b     rows [block_row[b], block_row[b + 1]), at most fsb_spmv_bins_cap(vtype) entries; the blocks cover rows
- *               0 .. n_rows - 1
+ *   block b     rows block_start[2 b] .. block_start[2 b + 2] - 1, whose entries are block_start[2 b + 1] ..
+ *               block_start[2 b + 3] - 1 of data; at most fsb_spmv_bins_cap(vtype) entries; the blocks cover rows
+ *               0 .. n_rows - 1 (block_start: 2 * (n_blocks + 1) values)
  *   unit (c, b) the entries of block b in chunk c, filled up to whole packs (fsb_spmv_bins_pack(vtype) entries, 32 bytes of
- *               values).  Chunk order: chunk by chunk, inside a chunk block by block; block order: the other way round.
+ *               x).  Chunk order: chunk by chunk, inside a chunk block by block; block order: the other way round.
  *               chunk_pack[c], c = 0 .. n_chunks and block_pack[b], b = 0 .. n_blocks: first pack of a chunk in chunk order,
  *               of a block in block order; the last of both is n_packs
- *   val, col    per entry, in chunk order: value, column inside its chunk (what fills a pack up: 0 and 0)
+ *   col         per entry, in chunk order: column inside its chunk (what fills a pack up: 0)
  *   place       per pack, in block order: its number in chunk order
- *   dst         per entry, in block order: where the sum keeps its product (what fills a pack up: a place nobody reads)
+ *   dst         per entry, in block order: where the sum keeps it (what fills a pack up: a place nobody reads)
  *   ends        fsb_spmv_bins_ends() words per block, one per thread of the sum: bit j is set where entry j of the thread's
  *               slice of the block (cap / ends entries each) is the last of its row
- *   row_slot    per row: where its last product is kept (rows without entries: a zero)
- * val, col, dst and row_slot are 16-byte aligned.  fsb_spmv_bins_count writes the entries of every unit, counts[b * n_chunks + c];
+ *   row_slot    per row: where its last entry is kept (rows without entries: a zero)
+ *   data        the values, aligned to their size
+ * col, dst and row_slot are 16-byte aligned.  fsb_spmv_bins_count writes the entries of every unit, counts[b * n_chunks + c];
  * fsb_spmv_bins_place the layout, from the first pack of every unit in chunk order and in block order (unit_chunk, unit_block,
- * [b * n_chunks + c]).  prod: 32 * n_packs bytes of scratch, 32-byte aligned, a call's own while it runs.
+ * [b * n_chunks + c]).  xg: 32 * n_packs bytes of scratch, 32-byte aligned, a call's own while it runs.
  */
 int fsb_spmv_bins_max_chunks(void);
 int fsb_spmv_bins_chunk_cols(int vtype);
@@ -399,14 +402,14 @@ int fsb_spmv_bins_pack(int vtype);
 int fsb_spmv_bins_ends(void);
 int fsb_spmv_bins_count(int ptype, const int32_t* indices, const void* indptr, const int32_t* block_row, int32_t n_blocks,
                         int32_t n_chunks, int32_t chunk_cols, int64_t n_cols, int32_t* counts, void* stream);
-int fsb_spmv_bins_place(int vtype, int ptype, const void* data, const int32_t* indices, const void* indptr,
+int fsb_spmv_bins_place(int vtype, int ptype, const int32_t* indices, const void* indptr,
                         const int32_t* block_row, int32_t n_blocks, int32_t n_chunks, int32_t chunk_cols, int64_t n_cols,
-                        const int32_t* unit_chunk, const int32_t* unit_block, void* val, uint16_t* col, int32_t* place,
+                        const int32_t* unit_chunk, const int32_t* unit_block, uint16_t* col, int32_t* place,
                         uint16_t* dst, uint32_t* ends, uint16_t* row_slot, void* stream);
-int fsb_spmv_csr_bins(int vtype, const void* val, const uint16_t* col, const int32_t* place, const uint16_t* dst,
-                      const uint32_t* ends, const uint16_t* row_slot, const int32_t* chunk_pack, const int32_t* block_pack,
-                      const int32_t* block_row, int32_t n_blocks, int32_t n_chunks, int32_t chunk_cols, int64_t n_packs,
-                      void* prod, size_t prod_bytes, const void* x, void* y, int64_t n_rows, int64_t n_cols, void* stream);
+int fsb_spmv_csr_bins(int vtype, const uint16_t* col, const int32_t* place, const uint16_t* dst, const uint32_t* ends,
+                      const uint16_t* row_slot, const int32_t* chunk_pack, const int32_t* block_pack, const int64_t* block_start,
+                      const void* data, int32_t n_blocks, int32_t n_chunks, int32_t chunk_cols, int64_t n_packs, void* xg,
+                      size_t xg_bytes, const void* x, void* y, int64_t n_rows, int64_t n_cols, void* stream);
 
 /*
  * Sampled dense-dense product on a CSR pattern: out[p] = alpha * dot(X[row(p), :], Y[indices[p], :]) + beta * data[p]
