@@ -30,7 +30,13 @@ F64_MIN_SPAN = 120 << 20
 # ... or uneven rows of a few entries that would have gone to the lanes-per-row kernel, whose warps wait for their longest row:
 # 4.8 M entries in 2.1 M rows 66 against 49, 3.3 M in 1 M rows 42 against 35; by tiles, 2.6 M in 0.5 M rows 23.6 against 30.1.
 F64_SHORT_MEAN = 4
-# mean entries of a unit below which the packs would mostly be padding (measured down to 36 and 9 entries, float32 and float64)
+# Rows of a block, at most: one CTA writes them, and rows without entries count for nothing in the cut by entries.  float32, one
+# pass against two with no such line / at most 2^16 rows: 2^24 rows, 4 entries in every row of the first half 272 against 1499 /
+# 178 us; 16 in every one of the last 2^20 rows 207 against 2519 / 119; 10 M entries in the first 2 M of 30 M rows 324 against 4578 /
+# 124.  At most 2^14 / 2^18 rows: 188 / 202, 132 / 112, - / 140.
+BLOCK_ROWS = 1 << 16
+# Mean entries of a unit below which the packs would mostly be padding; near the line, one pass against two: float32 with 17 entries
+# (2^25 in all, 70 M columns) 519 against 218 us, float64 with 8.4 (2^27, 36 M columns) 2177 against 1448.
 MIN_UNIT = {4: 16, 8: 8}
 
 
@@ -51,6 +57,12 @@ def min_span(nnz, n_rows, max_row_nnz, element_size, lanes_per_row):
     if uneven and lanes_per_row and mean <= F64_SHORT_MEAN and nnz >= UNEVEN_MIN_NNZ:
         return UNEVEN_MIN_SPAN
     return F64_MIN_SPAN if nnz >= EVEN_MIN_NNZ else None
+
+
+def most_blocks(nnz, n_rows, max_row_nnz, cap):
+    """Row blocks of a matrix, at most: one per `cap` entries, less what a last row may add, and one per BLOCK_ROWS rows."""
+    return -(-nnz // (cap - max_row_nnz + 1)) + -(-n_rows // BLOCK_ROWS)
+
 
 class BinsLayout:
     """Device arrays of the regrouped matrix (include/fsb.h, fsb_spmv_csr_bins)."""
@@ -84,17 +96,18 @@ def build_bins_layout(data, indices, indptr, n_rows, n_cols, max_row_nnz, span=0
     n_chunks = -(-n_cols // chunk_cols)
     if max_row_nnz > cap // 4 or n_chunks > int(L.fsb_spmv_bins_max_chunks()) or n_cols * data.element_size() < span:
         return None
-    # block b begins at the first row that starts at or behind entry b * step: at most step - 1 + max_row_nnz entries
+    # a block begins at the first row that starts at or behind entry k * step: at most step - 1 + max_row_nnz entries; and at
+    # every BLOCK_ROWS-th row
     step = cap - max_row_nnz + 1
-    n_blocks = -(-nnz // step)
+    n_blocks = most_blocks(nnz, n_rows, max_row_nnz, cap)
     if nnz // pack + n_blocks * n_chunks >= 2**31 - 1 or (indptr.dtype == torch.int32 and nnz >= 2**31 - 1 - cap):
         return None
     st = torch.cuda.current_stream(dev).cuda_stream
     with torch.cuda.device(dev):
-        marks = torch.arange(n_blocks + 1, device=dev, dtype=indptr.dtype) * step
-        block_row = torch.searchsorted(indptr, marks).clamp_(max=n_rows).to(torch.int32)
-        block_row[0] = 0
-        block_row[-1] = n_rows
+        marks = torch.arange(1, -(-nnz // step), device=dev, dtype=indptr.dtype) * step
+        every = torch.arange(0, n_rows + BLOCK_ROWS, BLOCK_ROWS, device=dev).clamp_(max=n_rows)
+        block_row = torch.unique(torch.cat((torch.searchsorted(indptr, marks).clamp_(max=n_rows), every))).to(torch.int32)
+        n_blocks = block_row.numel() - 1
         counts = torch.empty((n_blocks, n_chunks), dtype=torch.int32, device=dev)
         _lib.check(L.fsb_spmv_bins_count(pt, indices.data_ptr(), indptr.data_ptr(), block_row.data_ptr(), n_blocks, n_chunks,
                                          chunk_cols, n_cols, counts.data_ptr(), st), "fsb_spmv_bins_count")
@@ -135,7 +148,8 @@ def bins_for(data, indices, indptr, n_rows, n_cols, max_row_nnz, lanes_per_row):
     if span is None:
         return None
     L, vt = _lib.lib(), _VTYPE[data.dtype]
-    if int(L.fsb_spmv_bins_cap(vt)) * int(L.fsb_spmv_bins_chunk_cols(vt)) < MIN_UNIT[sv] * n_cols:
+    cap, chunk_cols = int(L.fsb_spmv_bins_cap(vt)), int(L.fsb_spmv_bins_chunk_cols(vt))
+    if max_row_nnz > cap // 4 or nnz * chunk_cols < MIN_UNIT[sv] * n_cols * most_blocks(nnz, n_rows, max_row_nnz, cap):
         return None
     return build_bins_layout(data, indices, indptr, n_rows, n_cols, max_row_nnz, span)
 

@@ -87,6 +87,22 @@ def test_what_is_left_to_one_pass(cuda, fsb_lib):
     assert bins.build_bins_layout(dev(d), dev(i), dev(p), 500, 9000, 4, span=9000 * 4, chunk_cols=1000) is None
 
 
+@pytest.mark.parametrize("where", ["start", "middle", "end", "rows of one block", "one row more"])
+@pytest.mark.parametrize("vdt", ["float32", "float64"])
+def test_runs_of_empty_rows_are_shared_by_blocks(cuda, fsb_lib, where, vdt):
+    some = list(np.random.default_rng(2).integers(1, 9, 2000))
+    empty = {"rows of one block": (1 << 16) - 2000, "one row more": (1 << 16) - 1999}.get(where, 3 * 10**5)
+    cut = {"start": 0, "middle": 1000}.get(where, 2000)
+    lens = some[:cut] + [0] * empty + some[cut:]
+    d, i, p = handmade_csr(5, lens, 7000, value_dtype=vdt)
+    shape = (len(lens), 7000)
+    x = np.random.default_rng(3).uniform(-1, 1, 7000).astype(vdt)
+    lay = _layout(d, i, p, shape, 1000)
+    rows = lay.block_start.view(-1, 2)[:, 0].cpu().numpy()
+    assert rows[0] == 0 and rows[-1] == shape[0] and 0 < np.diff(rows).min() and np.diff(rows).max() <= 1 << 16
+    assert_spmv_ok(_product(lay, dev(x), shape).cpu().numpy(), d, i, p, shape, x, what=where)
+
+
 def test_prepared_matrix_takes_the_two_passes(cuda, fsb_lib, monkeypatch):
     monkeypatch.setattr(bins, "UNEVEN_MIN_NNZ", 1 << 17)
     monkeypatch.setattr(bins, "UNEVEN_MIN_SPAN", 1 << 10)
