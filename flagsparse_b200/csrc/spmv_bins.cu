@@ -13,11 +13,12 @@
 // Per float32 entry 2 bytes in and 4 out, then 4 + 2 + 0.5 + 4 in (float64: 10 and 19): twice the bytes of one pass, all of
 // them streamed.  Rows are summed in CSR order, in double (float64: compensated inside a slice), so results do not depend on
 // the order of the entries inside a unit and are bit-reproducible.  107 M entries in 16.7 M rows of Zipf lengths, columns
-// anywhere in 2^24, float32: 640 us through spmv_stream_kernel, 443 us here: gather 135 us (0.64 GB), sum 306 us (1.13 GB; a
+// anywhere in 2^24, float32: 640 us through spmv_stream_kernel, 456 us here: gather 135 us (0.64 GB), sum 318 us (1.13 GB; a
 // block's elements arrive, are multiplied and added up and leave in turn, and two blocks an SM cover each other's phases in
 // part).  With a copy of the values in storage order, multiplied by the first pass: 216 and 225 us, but 4 more bytes an entry,
-// and values that the caller writes later would not be seen.  (The values asked for ahead with prefetch.global.L2: 437 us
-// here, but 73 us instead of 70 us for 2^24 entries, which L2 holds.)
+// and values that the caller writes later would not be seen.  (Values asked for ahead with prefetch.global.L2: 6 us less
+// here, but 3 us more for 2^24 entries, which L2 holds.)  12 us of the sum keep the part of a row in the slice where it ends in
+// double until what the slices before have is there: rounded before, two parts that cancel lose what they differ by.
 #include "fsb_common.cuh"
 
 namespace fsb {
@@ -130,7 +131,8 @@ bins_gather_kernel(const uint16_t* __restrict__ col, const int32_t* __restrict__
 // y of row block b = blockIdx.x.  ends[b * kBinSumThreads + t]: bit j is set where entry j of thread t's slice is the last of
 // its row; row_slot[r]: where row r's last product is kept.  A thread adds up its slice, slot by slot, and a finished row's
 // sum takes the place of its last product: by rows, most lanes would wait for the longest row of their warp.  What the slices
-// before have of the row that a slice begins in the middle of comes from a segmented scan over the threads.
+// before have of the row that a slice begins in the middle of comes from a segmented scan over the threads, and is added to the
+// unrounded sum.
 template <typename V>
 __global__ void __launch_bounds__(kBinSumThreads, 2)
 bins_sum_kernel(const V* __restrict__ data, const V* __restrict__ xg, const int32_t* __restrict__ place,
@@ -196,7 +198,7 @@ bins_sum_kernel(const V* __restrict__ data, const V* __restrict__ xg, const int3
   // float64: what every addition rounds off is kept beside the sum, or slot after slot would lose more than the lanes' tree of
   // the one-pass kernel (rows of 4 entries: rms error 8.9e-17 without it, 7.7e-17 in one pass)
   constexpr bool COMP = sizeof(V) == 8;
-  double tail = 0, off = 0;
+  double tail = 0, off = 0, head = 0;      // head: the first row that ends here, without what the slices before have of it
 #pragma unroll
   for (int j = 0; j < S; ++j) {
     const double v = (double)slice[j];
@@ -208,7 +210,9 @@ bins_sum_kernel(const V* __restrict__ data, const V* __restrict__ xg, const int3
       tail += v;
     }
     if (mask & (1u << j)) {
-      slice[j] = (V)(COMP ? tail + comp_term(tail, off) : tail);
+      if (COMP) tail += comp_term(tail, off);
+      if ((mask & ((1u << j) - 1u)) == 0) head = tail;
+      slice[j] = (V)tail;
       tail = 0;
       off = 0;
     }
@@ -235,8 +239,7 @@ bins_sum_kernel(const V* __restrict__ data, const V* __restrict__ xg, const int3
         carry += s_tail[v];
         if (s_any[v]) break;
       }
-    V* first = slice + __ffs(mask) - 1;
-    *first = (V)(carry + (double)*first);
+    slice[__ffs(mask) - 1] = (V)(carry + head);
   }
   __syncthreads();
   // four rows of a thread at a time, from a multiple of four on; what is left at both ends one by one

@@ -7,7 +7,7 @@ import torch
 
 import flagsparse_b200 as fs
 from flagsparse_b200 import _lib, bins
-from gpu_util import dev
+from gpu_util import dev, spmv
 from helpers import assert_spmv_ok, handmade_csr
 
 pytestmark = pytest.mark.gpu
@@ -55,6 +55,47 @@ def test_edges(cuda, fsb_lib, name, vdt, pdt):
         assert torch.equal(y, _product(lay, tx, shape))
         want = y if want is None else want
         assert torch.equal(y, want)
+
+
+def test_a_row_over_two_slices_is_rounded_once(cuda, fsb_lib):
+    # the part in the slice where the row ends has 25 bits, and in the second row more than float32 can hold
+    big, huge = 2.0**30, 3e38
+    d = np.zeros(80, dtype=np.float32)
+    d[[0, 1, 32, 33]] = [big, 0.5, -big, 0.25]
+    d[[40, 64, 65]] = [-huge, huge, huge]
+    i = np.tile(np.arange(40, dtype=np.int32), 2)
+    lay = _layout(d, i, np.array([0, 40, 80], dtype=np.int32), (2, 40))
+    y = _product(lay, torch.ones(40, device=cuda), (2, 40)).cpu().numpy()
+    assert y.tolist() == [0.75, float(np.float32(huge))]
+
+
+def _two_products(a, b):
+    """a * b of float64 values as an unevaluated sum, exact (Dekker)."""
+    def halves(v):
+        t = v * 134217729.0
+        hi = t - (t - v)
+        return hi, v - hi
+
+    p, (ah, al), (bh, bl) = a * b, halves(a), halves(b)
+    return p, ((ah * bh - p) + ah * bl + al * bh) + al * bl
+
+
+@pytest.mark.parametrize("length", [2, 4, 16, 60, 700])
+@pytest.mark.parametrize("vdt", ["float32", "float64"])
+def test_no_less_accurate_than_one_pass(cuda, fsb_lib, vdt, length):
+    """Root mean square error of rows of equal length: 1.03 is left for the spread of an rms over 3 * 10^4 rows and more,
+    1.1 over the 3000 longest."""
+    n_rows, n_cols = max(3000, 200000 // length), 30000
+    rng = np.random.default_rng(length)
+    i = rng.integers(0, n_cols, n_rows * length).astype(np.int32)
+    d, x = rng.uniform(-1, 1, n_rows * length).astype(vdt), rng.uniform(-1, 1, n_cols).astype(vdt)
+    p = np.arange(n_rows + 1, dtype=np.int32) * length
+    hi, lo = _two_products(d.astype(np.float64), x.astype(np.float64)[i])
+    wide = hi.reshape(n_rows, -1).astype(np.longdouble).sum(1) + lo.reshape(n_rows, -1).astype(np.longdouble).sum(1)
+    rms = lambda y: float(np.sqrt(np.mean((y.astype(np.longdouble) - wide) ** 2)))  # noqa: E731
+    two = rms(_product(_layout(d, i, p, (n_rows, n_cols), 4096), dev(x), (n_rows, n_cols)).cpu().numpy())
+    one = min(rms(spmv(d, i, p, (n_rows, n_cols), x, algo=algo)) for algo in ("vector", "stream"))
+    assert two <= (1.03 if n_rows >= 3 * 10**4 else 1.1) * one, (two, one)
 
 
 @pytest.mark.parametrize("vdt", ["float32", "float64"])
