@@ -151,16 +151,26 @@ def bins_for(data, indices, indptr, n_rows, n_cols, max_row_nnz, lanes_per_row):
     cap, chunk_cols = int(L.fsb_spmv_bins_cap(vt)), int(L.fsb_spmv_bins_chunk_cols(vt))
     if max_row_nnz > cap // 4 or nnz * chunk_cols < MIN_UNIT[sv] * n_cols * most_blocks(nnz, n_rows, max_row_nnz, cap):
         return None
-    return build_bins_layout(data, indices, indptr, n_rows, n_cols, max_row_nnz, span)
+    try:
+        return build_bins_layout(data, indices, indptr, n_rows, n_cols, max_row_nnz, span)
+    except torch.OutOfMemoryError:       # a one-pass kernel needs none of it
+        return None
+
+
+def _between_passes(layout, device):
+    return torch.empty(32 * layout.n_packs, dtype=torch.uint8, device=device)
 
 
 def launch_bins(layout, x, y, n_rows, n_cols, stream_ptr, data=None):
     """Enqueue the product on the current stream (its handle in stream_ptr).  data: the values, in CSR order, instead of those
     that the layout was made with.  The memory between the passes is the call's own: calls on one matrix may overlap in
-    several streams."""
+    several streams.  False where it is refused: nothing was enqueued then."""
     la = layout
     data = la.data if data is None else data
-    xg = torch.empty(32 * la.n_packs, dtype=torch.uint8, device=data.device)
+    try:
+        xg = _between_passes(la, data.device)
+    except torch.OutOfMemoryError:
+        return False
     rc = _lib.lib().fsb_spmv_csr_bins(
         _VTYPE[data.dtype], la.col.data_ptr(), la.place.data_ptr(), la.dst.data_ptr(), la.ends.data_ptr(),
         la.row_slot.data_ptr(), la.chunk_pack.data_ptr(), la.block_pack.data_ptr(), la.block_start.data_ptr(), data.data_ptr(),
@@ -168,3 +178,4 @@ def launch_bins(layout, x, y, n_rows, n_cols, stream_ptr, data=None):
         n_cols, stream_ptr,
     )
     _lib.check(rc, "fsb_spmv_csr_bins")
+    return True

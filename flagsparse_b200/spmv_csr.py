@@ -122,7 +122,8 @@ class PreparedCsrSpmv:
     Carries the attributes of the reference's class (spmv_csr.py:9-58) plus the tile plan and scratch of
     the stream kernel.  `opt_buckets` describes the plan (the reference lists row ids per length bucket
     there).  Calls on one prepared matrix may overlap in several streams where each brings the scratch it needs: matrices
-    of less than _STREAM_MIN_NNZ entries, float16 / bfloat16 / complex values, the two-pass form, and every matrix that takes
+    of less than _STREAM_MIN_NNZ entries, float16 / bfloat16 / complex values, the two-pass form (a call that is refused the
+    memory between the passes takes one, with the kernel that its rows get without them), and every matrix that takes
     the lanes-per-row or the panel kernel, which need none.  Larger matrices on the stream kernel, and matrices whose long rows
     were split off, own one buffer that their calls share: these calls must not overlap on the GPU.
     """
@@ -327,7 +328,8 @@ def _prepare_spmv_csr(data, indices, indptr, shape, block_nnz, max_segments, reu
 
         bins_layout = bins.bins_for(data, kernel_indices, kernel_indptr, n_rows, n_cols, max_row_nnz,
                                     algo == _lib.FSB_SPMV_VECTOR)
-    if algo == _lib.FSB_SPMV_STREAM and bins_layout is None and nnz > 0 and n_rows > 0:
+    # (with the two-pass form, too: a product that cannot have the memory between the passes takes one)
+    if algo == _lib.FSB_SPMV_STREAM and nnz > 0 and n_rows > 0:
         L = _lib.lib()
         vt = _VTYPE[data.dtype]
         tile_nnz = int(L.fsb_spmv_tile_nnz(vt, tuning))
@@ -367,12 +369,13 @@ def _spmv_launch(prepared, x, y):
         from . import bins
 
         with _on_device(dev):
-            bins.launch_bins(p.bins, x, y, p.n_rows, p.n_cols, _stream_ptr(dev), data=p.data)
-        return
+            done = bins.launch_bins(p.bins, x, y, p.n_rows, p.n_cols, _stream_ptr(dev), data=p.data)
+        if done:
+            return
     algo = p.algo if p.tile_row is not None else _lib.FSB_SPMV_VECTOR
     # calls on a small matrix may overlap in several streams, whichever kernel its rows get: scratch of the call's own
     scratch = p.scratch
-    if scratch is not None and p.data.numel() < _STREAM_MIN_NNZ:
+    if scratch is not None and (p.data.numel() < _STREAM_MIN_NNZ or p.bins is not None):
         scratch = torch.empty_like(scratch)
     lanes = p.tuning & 0xFF
     tuning = p.tuning if algo == _lib.FSB_SPMV_STREAM else (lanes if lanes in (2, 4, 8, 16, 32) else 0)

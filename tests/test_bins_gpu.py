@@ -7,7 +7,7 @@ import torch
 
 import flagsparse_b200 as fs
 from flagsparse_b200 import _lib, bins
-from gpu_util import dev, spmv
+from gpu_util import dev, env, spmv
 from helpers import assert_spmv_ok, handmade_csr
 
 pytestmark = pytest.mark.gpu
@@ -163,6 +163,30 @@ def test_prepared_matrix_takes_the_two_passes(cuda, fsb_lib, monkeypatch):
     assert torch.equal(got, y)
     monkeypatch.setenv("FSB_SPMV_BINS", "0")
     assert fs.prepare_spmv_csr(dev(d), dev(i), dev(p), (60000, 50000)).bins is None
+
+
+@pytest.mark.parametrize("longest,form", [(40, "vector"), (700, "stream")])
+def test_memory_that_is_refused_leaves_one_pass(cuda, fsb_lib, monkeypatch, longest, form):
+    for name in ("UNEVEN_MIN_NNZ", "UNEVEN_MIN_SPAN"):
+        monkeypatch.setattr(bins, name, 1 << 10)
+    lens = np.random.default_rng(7).integers(0, 9, 60000)
+    lens[::5000] = longest
+    d, i, p = handmade_csr(8, lens.tolist(), 50000)
+    x = dev(np.random.default_rng(9).uniform(-1, 1, 50000).astype(np.float32))
+    with env(FSB_SPMV_ALGO=form):
+        want = fs.flagsparse_spmv_csr(x=x, prepared=fs.prepare_spmv_csr(dev(d), dev(i), dev(p), (60000, 50000)))
+    prep = fs.prepare_spmv_csr(dev(d), dev(i), dev(p), (60000, 50000))
+    assert prep.bins is not None
+
+    def refuse(*args):
+        raise torch.OutOfMemoryError
+
+    monkeypatch.setattr(bins, "_between_passes", refuse)
+    assert torch.equal(fs.flagsparse_spmv_csr(x=x, prepared=prep), want)
+    monkeypatch.setattr(bins, "build_bins_layout", refuse)
+    prep = fs.prepare_spmv_csr(dev(d), dev(i), dev(p), (60000, 50000))
+    assert prep.bins is None and prep.opt_buckets[0]["kind"] == form
+    assert torch.equal(fs.flagsparse_spmv_csr(x=x, prepared=prep), want)
 
 
 def test_refused_calls(fsb_lib):
