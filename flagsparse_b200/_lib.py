@@ -38,7 +38,7 @@ BAD_KINDS = {
     2: "row pointer outside [0, nnz]",
     3: "row pointer smaller than the one before it",
     4: "row id outside [0, n_rows)",
-    5: "panel slot with an accumulator beyond the spare one",
+    5: "slot whose place (panel: accumulator) is not one of its row block's",
     6: "panel slot with an x position beyond the x buffers",
     7: "unit with a column chunk beyond n_cols",
     8: "unit or piece pointer table negative or decreasing",

@@ -105,15 +105,16 @@ check_panel_kernel(const uint32_t* __restrict__ rc, const int32_t* __restrict__ 
 // A bins layout (spmv_bins.cu): tables first, then the entries, the places of the packs and the rows.
 __global__ void __launch_bounds__(kCheckThreads)
 check_bins_kernel(const uint16_t* __restrict__ col, const int32_t* __restrict__ place, const uint16_t* __restrict__ dst,
-                  const uint16_t* __restrict__ row_slot, const int32_t* __restrict__ chunk_pack,
-                  const int32_t* __restrict__ block_pack, const int64_t* __restrict__ block_start, int n_blocks, int n_chunks,
-                  int chunk_cols, int slots, int pack, int64_t n_packs, int64_t n_rows, int64_t n_cols) {
+                  const uint32_t* __restrict__ ends, const uint16_t* __restrict__ row_slot,
+                  const int32_t* __restrict__ chunk_pack, const int32_t* __restrict__ block_pack,
+                  const int64_t* __restrict__ block_start, int n_blocks, int n_chunks, int chunk_cols, int cap, int threads,
+                  int pack, int64_t n_packs, int64_t n_rows, int64_t n_cols) {
   __shared__ int ok;
   if (threadIdx.x == 0) ok = 1;
   __syncthreads();
   for (int c = threadIdx.x; c < n_chunks; c += kCheckThreads) {       // every CTA looks at the whole (short) tables
     const int a = chunk_pack[c], z = chunk_pack[c + 1];
-    if (a < 0 || z < a || z > n_packs || (c == n_chunks - 1 && z != n_packs)) {
+    if (a < 0 || z < a || z > n_packs || (c == 0 && a != 0) || (c == n_chunks - 1 && z != n_packs)) {
       if (blockIdx.x == 0) note(FSB_BAD_UNIT_TABLE, c, z, a);
       ok = 0;
     }
@@ -125,7 +126,12 @@ check_bins_kernel(const uint16_t* __restrict__ col, const int32_t* __restrict__ 
       if (blockIdx.x == 0) note(FSB_BAD_ROW_ID, b, z, n_rows);
       ok = 0;
     }
-    if (pa < 0 || pz < pa || pz > n_packs) {
+    const int64_t n = block_start[2 * b + 3] - block_start[2 * b + 1];
+    if (n < 0 || n > cap || (b == 0 && block_start[1] != 0)) {
+      if (blockIdx.x == 0) note(FSB_BAD_ROW_POINTER, b, n, cap);
+      ok = 0;
+    }
+    if (pa < 0 || pz < pa || pz > n_packs || (b == 0 && pa != 0) || (b == n_blocks - 1 && pz != n_packs)) {
       if (blockIdx.x == 0) note(FSB_BAD_UNIT_TABLE, b, pz, pa);
       ok = 0;
     }
@@ -141,8 +147,13 @@ check_bins_kernel(const uint16_t* __restrict__ col, const int32_t* __restrict__ 
     for (int64_t i = (int64_t)chunk_pack[c] * pack + first; i < (int64_t)chunk_pack[c + 1] * pack; i += stride)
       if (col[i] >= width) note(FSB_BAD_COLUMN, i, col[i], width);
   }
+  // a slice of cap / threads entries has one place more; then come the zero of the rows without entries, and the place that
+  // what fills a unit up goes to
+  const int slice = cap / threads, zero = threads * (slice + 1), slots = zero + 2;
   for (int64_t i = first; i < n_packs * pack; i += stride)
-    if (dst[i] >= slots) note(FSB_BAD_SLOT_ROW, i, dst[i], slots);
+    if (dst[i] == zero || dst[i] >= slots) note(FSB_BAD_SLOT_ROW, i, dst[i], slots);
+  for (int64_t i = first; i < (int64_t)n_blocks * threads; i += stride)
+    if (slice < 32 && (ends[i] >> (slice & 31)) != 0) note(FSB_BAD_SLOT_ROW, i, ends[i], slice);
   for (int64_t r = first; r < n_rows; r += stride)
     if (row_slot[r] >= slots) note(FSB_BAD_SLOT_ROW, r, row_slot[r], slots);
 }
@@ -219,16 +230,16 @@ int check_panel(const uint32_t* rc_words, const int32_t* unit_piece_ptr, const i
   return end_check(st, rec);
 }
 
-int check_bins(int vtype, const uint16_t* col, const int32_t* place, const uint16_t* dst, const uint16_t* row_slot,
-               const int32_t* chunk_pack, const int32_t* block_pack, const int64_t* block_start, int n_blocks, int n_chunks,
+int check_bins(int vtype, const uint16_t* col, const int32_t* place, const uint16_t* dst, const uint32_t* ends,
+               const uint16_t* row_slot, const int32_t* chunk_pack, const int32_t* block_pack, const int64_t* block_start, int n_blocks, int n_chunks,
                int chunk_cols, int64_t n_packs, int64_t n_rows, int64_t n_cols, cudaStream_t st) {
   void* rec = nullptr;
   int rc = begin_check(st, &rec);
   if (rc != FSB_OK) return rc;
-  const int slots = fsb_spmv_bins_cap(vtype) + fsb_spmv_bins_ends() + 2;
-  check_bins_kernel<<<kCheckBlocks, kCheckThreads, 0, st>>>(col, place, dst, row_slot, chunk_pack, block_pack, block_start, n_blocks,
-                                                            n_chunks, chunk_cols, slots, fsb_spmv_bins_pack(vtype), n_packs,
-                                                            n_rows, n_cols);
+  check_bins_kernel<<<kCheckBlocks, kCheckThreads, 0, st>>>(col, place, dst, ends, row_slot, chunk_pack, block_pack, block_start,
+                                                            n_blocks, n_chunks, chunk_cols, fsb_spmv_bins_cap(vtype),
+                                                            fsb_spmv_bins_ends(), fsb_spmv_bins_pack(vtype), n_packs, n_rows,
+                                                            n_cols);
   return end_check(st, rec);
 }
 

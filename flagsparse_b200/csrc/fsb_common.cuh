@@ -27,8 +27,8 @@ int check_entry_ids(const int32_t* indices, const int32_t* row_ids, int64_t n_ro
 int check_panel(const uint32_t* rc_words, const int32_t* unit_piece_ptr, const int32_t* unit_chunk,
                 const int32_t* owner_unit_ptr, int n_owners, int slots, int max_row, int chunk_cols, int n_buffers,
                 int64_t n_cols, cudaStream_t st);
-int check_bins(int vtype, const uint16_t* col, const int32_t* place, const uint16_t* dst, const uint16_t* row_slot,
-               const int32_t* chunk_pack, const int32_t* block_pack, const int64_t* block_start, int n_blocks, int n_chunks,
+int check_bins(int vtype, const uint16_t* col, const int32_t* place, const uint16_t* dst, const uint32_t* ends,
+               const uint16_t* row_slot, const int32_t* chunk_pack, const int32_t* block_pack, const int64_t* block_start, int n_blocks, int n_chunks,
                int chunk_cols, int64_t n_packs, int64_t n_rows, int64_t n_cols, cudaStream_t st);
 #define FSB_WALK_FIRST(call)                       \
   do {                                             \

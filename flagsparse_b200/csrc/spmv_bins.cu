@@ -412,7 +412,7 @@ extern "C" int fsb_spmv_csr_bins(int vtype, const uint16_t* col, const int32_t* 
   const size_t gather_smem = (size_t)chunk_cols * sv;
   const size_t sum_smem = (size_t)(vtype == FSB_F32 ? bin_fill<float>() + 1 : bin_fill<double>() + 1) * sv;
   if (gather_smem > 226 * 1024) return FSB_ERANGE;
-  FSB_WALK_FIRST(check_bins(vtype, col, place, dst, row_slot, chunk_pack, block_pack, block_start, n_blocks, n_chunks,
+  FSB_WALK_FIRST(check_bins(vtype, col, place, dst, ends, row_slot, chunk_pack, block_pack, block_start, n_blocks, n_chunks,
                             chunk_cols, n_packs, n_rows, n_cols, st));
   int dev = 0, sms = 0;
   cudaError_t e = cudaGetDevice(&dev);

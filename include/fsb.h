@@ -438,7 +438,7 @@ int fsb_sddmm_csr(int vtype, const int32_t* indices, const int32_t* row_ids, con
 #define FSB_BAD_ROW_POINTER 2         /* indptr[position] outside [0, nnz]                           */
 #define FSB_ROW_POINTER_DECREASES 3   /* indptr[position] < indptr[position - 1] (the limit)         */
 #define FSB_BAD_ROW_ID 4              /* row_ids[position] outside [0, n_rows)                       */
-#define FSB_BAD_SLOT_ROW 5            /* accumulator of slot `position` beyond the spare accumulator */
+#define FSB_BAD_SLOT_ROW 5            /* place or accumulator that is not one of its row block's      */
 #define FSB_BAD_SLOT_COLUMN 6         /* x slot of slot `position` >= n_buffers * chunk_cols         */
 #define FSB_BAD_CHUNK 7               /* unit_chunk[position] * chunk_cols >= n_cols                 */
 #define FSB_BAD_UNIT_TABLE 8          /* a unit / piece pointer table that is negative or decreases  */
