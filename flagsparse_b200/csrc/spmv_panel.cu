@@ -165,7 +165,7 @@ __device__ __forceinline__ void panel_rounds_runs(const Group<V, GS>& G, uint32_
   }
 }
 
-constexpr int kModeDirect = 0, kModeRuns = 1, kModeRunsClash = 2;
+constexpr int kModeDirect = 0, kModeRuns = 1, kModeRunsClash = 2, kModeDirectFew = 3;
 constexpr int kMaxXBuffers = 8;
 constexpr int kUnitWindow = 512;   // units whose tables are kept in shared memory at a time
 constexpr int kUnitLookahead = kMaxXBuffers;
@@ -195,19 +195,23 @@ struct PanelGeom {
 // asked for at the barrier that opens a unit lands hardly before the one that closes it: the copies alone, one after the
 // other, took 755 us of the product's 1026 us (2^24 rows of 32, band of +-2^20, float32; the entries alone 749 us, the
 // arithmetic alone 665 us).  Asked for as soon as the last warp is done with the buffer they run ahead of the barriers: 955 us,
-// and 924 us with hardly more warps than a unit has pieces (17; FSB_PANEL_FEW_PIECES): fewer wait at the barriers.
+// and 924 us with hardly more warps than a unit has pieces (17; FSB_PANEL_FEW_PIECES): fewer wait at the barriers.  31 / 20
+// warps at other sizes, float64: 7.2 pieces 294 / 244 us, 10.6: 174 / 154, 14.1: 414 / 404 (without the fetching warp 312, -, 432);
+// float32: 8.8 pieces 70 / 64, 16.8: 68 / 64, 17.6: 469 / 470, 19.8: 248 / 254, 21.9: 265 / 373, 30.5: 340 / 415, 34.7: 471 / 436
+// (without the fetching warp 494).
 constexpr int kFewWarps = 20;
-__host__ __device__ constexpr int panel_workers(int mode, bool few) {
-  return mode != kModeDirect ? kPanelMaxWarps : few ? kFewWarps : kPanelMaxWarps - 1;
+__host__ __device__ constexpr bool panel_direct(int mode) { return mode == kModeDirect || mode == kModeDirectFew; }
+__host__ __device__ constexpr int panel_workers(int mode) {
+  return !panel_direct(mode) ? kPanelMaxWarps : mode == kModeDirectFew ? kFewWarps : kPanelMaxWarps - 1;
 }
-__host__ __device__ constexpr int panel_threads(int mode, bool few) {
-  return 32 * (panel_workers(mode, few) + (mode == kModeDirect ? 1 : 0));
+__host__ __device__ constexpr int panel_threads(int mode) {
+  return 32 * (panel_workers(mode) + (panel_direct(mode) ? 1 : 0));
 }
 
 // Units u0 .. u1-1 of one CTA, in order: chunk of x in, pieces added into y_part.  Returns false when a bounded
 // wait ran out (every thread of the CTA gets the same answer).
 //   - x chunks are fetched ahead into n_buf buffers (unit number `ord` of the CTA uses buffer ord % n_buf; the packed word
-//     of a slot already holds buffer * chunk_cols + local column).  kModeDirect: by a warp of its own, n_buf units ahead, as
+//     of a slot already holds buffer * chunk_cols + local column).  Direct modes: by a warp of its own, n_buf units ahead, as
 //     soon as all warps are done with the buffer (mbarriers that only this warp looks at); else by thread 0, n_buf - 1
 //     units ahead, at the barrier that closes the unit;
 //   - piece p goes to warp (p - first piece of the CTA) % W; a warp walks its pieces in groups of G slots per
@@ -221,7 +225,7 @@ __device__ __forceinline__ bool panel_run_units(const V* __restrict__ val, const
   constexpr int GPP = R / G;          // groups per piece
   constexpr int SLOTS = 32 * R;
   constexpr int THREADS = 32 * W;     // of the warps that add
-  constexpr bool RING = MODE == kModeDirect;
+  constexpr bool RING = panel_direct(MODE);
   constexpr int E = 16 / (int)sizeof(V);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int chunk_cols = gm.chunk_cols, n_buf = gm.n_buf;
@@ -410,15 +414,15 @@ __device__ __forceinline__ void panel_setup(PanelShared<V>& sh, unsigned char* s
 
 // One CTA per block of rb_rows consecutive rows (block block_begin + blockIdx.x); every row of y the launch
 // covers is written exactly once.
-template <typename V, int R, int G, int MODE, bool FEW>
-__global__ void __launch_bounds__(panel_threads(MODE, FEW), 1)
+template <typename V, int R, int G, int MODE>
+__global__ void __launch_bounds__(panel_threads(MODE), 1)
 spmv_panel_kernel(const V* __restrict__ val, const uint32_t* __restrict__ rc, const int32_t* __restrict__ unit_piece_ptr,
                   const int32_t* __restrict__ unit_chunk, const int32_t* __restrict__ rb_unit_ptr,
                   const V* __restrict__ x, V* __restrict__ y, int block_begin, int64_t n_rows, int rb_rows,
                   PanelGeom gm, int32_t* __restrict__ status) {
   extern __shared__ __align__(128) unsigned char p_smem[];
   __shared__ __align__(8) PanelStatic p_static;
-  constexpr int W = panel_workers(MODE, FEW), THREADS = panel_threads(MODE, FEW);
+  constexpr int W = panel_workers(MODE), THREADS = panel_threads(MODE);
   const int tid = threadIdx.x;
   const int rb = block_begin + (int)blockIdx.x;
   const int64_t r0 = (int64_t)rb * rb_rows;
@@ -451,8 +455,8 @@ spmv_panel_kernel(const V* __restrict__ val, const uint32_t* __restrict__ rc, co
 // unit" still holds).  The units of a group are dealt to several CTAs by column range, so a CTA ends with
 // partial sums of its group's rows: it writes them to part[cta_part_ptr[cta] + (q - first q of the group)],
 // and panel_group_reduce_kernel adds the partial sums of each row in CTA order.
-template <typename V, int R, int G, int MODE, bool FEW>
-__global__ void __launch_bounds__(panel_threads(MODE, FEW), 1)
+template <typename V, int R, int G, int MODE>
+__global__ void __launch_bounds__(panel_threads(MODE), 1)
 spmv_panel_groups_kernel(const V* __restrict__ val, const uint32_t* __restrict__ rc,
                          const int32_t* __restrict__ unit_piece_ptr, const int32_t* __restrict__ unit_chunk,
                          const int32_t* __restrict__ cta_unit_ptr, const int32_t* __restrict__ cta_group,
@@ -461,7 +465,7 @@ spmv_panel_groups_kernel(const V* __restrict__ val, const uint32_t* __restrict__
                          PanelGeom gm, int32_t* __restrict__ status) {
   extern __shared__ __align__(128) unsigned char p_smem[];
   __shared__ __align__(8) PanelStatic p_static;
-  constexpr int W = panel_workers(MODE, FEW), THREADS = panel_threads(MODE, FEW);
+  constexpr int W = panel_workers(MODE), THREADS = panel_threads(MODE);
   const int tid = threadIdx.x;
   const int cta = blockIdx.x;
   const int g = cta_group[cta];
@@ -526,20 +530,23 @@ static bool panel_buffers_ok(int n_buffers, int chunk_cols) {
   return n_buffers >= 2 && n_buffers <= kMaxXBuffers && (int64_t)n_buffers * chunk_cols <= 65536;
 }
 
-// FN<V, R, G, MODE> for the runtime (vtype, rounds, mode)
-#define FSB_PANEL_CASE(FN, V, R_, LAUNCH)                                                        \
-  do {                                                                                           \
-    if (mode == kModeRunsClash) LAUNCH((FN<V, R_, Shape<V, R_>::G, kModeRunsClash, false>));     \
-    else if (mode == kModeRuns) LAUNCH((FN<V, R_, Shape<V, R_>::G, kModeRuns, false>));          \
-    else if (few) LAUNCH((FN<V, R_, Shape<V, R_>::G, kModeDirect, true>));                       \
-    else LAUNCH((FN<V, R_, Shape<V, R_>::G, kModeDirect, false>));                               \
+// FN<V, R, G, MODE> for the runtime (rounds, mode); kModeDirectFew has only the first form
+#define FSB_PANEL_BY_ROUNDS(FN, V, MODE_, LAUNCH)                              \
+  do {                                                                         \
+    if (rounds == 4) LAUNCH((FN<V, 4, Shape<V, 4>::G, MODE_>));                \
+    else if (rounds == 8) LAUNCH((FN<V, 8, Shape<V, 8>::G, MODE_>));           \
+    else LAUNCH((FN<V, 16, Shape<V, 16>::G, MODE_>));                          \
   } while (0)
-#define FSB_PANEL_DISPATCH(FN, V, LAUNCH)                                                        \
-  do {                                                                                           \
-    if (rounds == 4) FSB_PANEL_CASE(FN, V, 4, LAUNCH);                                           \
-    else if (rounds == 8) FSB_PANEL_CASE(FN, V, 8, LAUNCH);                                      \
-    else FSB_PANEL_CASE(FN, V, 16, LAUNCH);                                                      \
+#define FSB_PANEL_DISPATCH(FN, V, LAUNCH)                                                  \
+  do {                                                                                     \
+    if (mode == kModeRunsClash) FSB_PANEL_BY_ROUNDS(FN, V, kModeRunsClash, LAUNCH);        \
+    else if (mode == kModeRuns) FSB_PANEL_BY_ROUNDS(FN, V, kModeRuns, LAUNCH);             \
+    else FSB_PANEL_BY_ROUNDS(FN, V, kModeDirect, LAUNCH);                                  \
   } while (0)
+
+static int panel_mode(int flags) {
+  return (flags & FSB_PANEL_LONG_RUNS) ? kModeRunsClash : (flags & FSB_PANEL_RUNS) ? kModeRuns : kModeDirect;
+}
 
 extern "C" int fsb_spmv_csr_panel(int vtype, const void* val, const uint32_t* rc, const int32_t* unit_piece_ptr,
                                   const int32_t* unit_chunk, const int32_t* rb_unit_ptr, int32_t n_row_blocks,
@@ -561,23 +568,25 @@ extern "C" int fsb_spmv_csr_panel(int vtype, const void* val, const uint32_t* rc
   if (!aligned_to(val, 16) || !aligned_to(rc, 16)) return FSB_EALIGN;
   FSB_WALK_FIRST(check_panel(rc, unit_piece_ptr, unit_chunk, rb_unit_ptr, n_row_blocks,
                              fsb_spmv_panel_piece_slots(rounds), rb_rows, chunk_cols, n_buffers, n_cols, st));
-  const int mode = (flags & FSB_PANEL_LONG_RUNS) ? kModeRunsClash : ((flags & FSB_PANEL_RUNS) ? kModeRuns : kModeDirect);
+  int mode = panel_mode(flags);
+  if (mode == kModeDirect && (flags & FSB_PANEL_FEW_PIECES)) mode = kModeDirectFew;
   const PanelGeom gm{n_cols, chunk_cols, n_buffers, (flags & FSB_PANEL_DEBUG_TIMEOUT) ? 1 : 0, (uint32_t)rb_rows};
   const unsigned grid = (unsigned)(block_end - block_begin);
-  const bool few = (flags & FSB_PANEL_FEW_PIECES) != 0;
 #define FSB_PANEL_LAUNCH_(K)                                                                                    \
   do {                                                                                                          \
     cudaError_t e = cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);           \
     if (e != cudaSuccess) return cuda_rc(e);                                                                    \
-    K<<<grid, panel_threads(mode, few), smem, st>>>((const VT_*)val, rc, unit_piece_ptr, unit_chunk, rb_unit_ptr,          \
+    K<<<grid, panel_threads(mode), smem, st>>>((const VT_*)val, rc, unit_piece_ptr, unit_chunk, rb_unit_ptr,          \
                                          (const VT_*)x, (VT_*)y, block_begin, n_rows, rb_rows, gm, status);     \
   } while (0)
   if (vtype == FSB_F32) {
     typedef float VT_;
-    FSB_PANEL_DISPATCH(spmv_panel_kernel, float, FSB_PANEL_LAUNCH_);
+    if (mode == kModeDirectFew) FSB_PANEL_BY_ROUNDS(spmv_panel_kernel, float, kModeDirectFew, FSB_PANEL_LAUNCH_);
+    else FSB_PANEL_DISPATCH(spmv_panel_kernel, float, FSB_PANEL_LAUNCH_);
   } else {
     typedef double VT_;
-    FSB_PANEL_DISPATCH(spmv_panel_kernel, double, FSB_PANEL_LAUNCH_);
+    if (mode == kModeDirectFew) FSB_PANEL_BY_ROUNDS(spmv_panel_kernel, double, kModeDirectFew, FSB_PANEL_LAUNCH_);
+    else FSB_PANEL_DISPATCH(spmv_panel_kernel, double, FSB_PANEL_LAUNCH_);
   }
 #undef FSB_PANEL_LAUNCH_
   FSB_RETURN_IF_LAUNCH_FAILED();
@@ -607,16 +616,15 @@ extern "C" int fsb_spmv_csr_panel_groups(int vtype, const void* val, const uint3
   if (!aligned_to(val, 16) || !aligned_to(rc, 16)) return FSB_EALIGN;
   FSB_WALK_FIRST(check_panel(rc, unit_piece_ptr, unit_chunk, cta_unit_ptr, n_ctas, fsb_spmv_panel_piece_slots(rounds),
                              max_group_acc, chunk_cols, n_buffers, n_cols, st));
-  const int mode = (flags & FSB_PANEL_LONG_RUNS) ? kModeRunsClash : ((flags & FSB_PANEL_RUNS) ? kModeRuns : kModeDirect);
+  const int mode = panel_mode(flags);
   const PanelGeom gm{n_cols, chunk_cols, n_buffers, (flags & FSB_PANEL_DEBUG_TIMEOUT) ? 1 : 0,
                      (uint32_t)max_group_acc};
   const unsigned rgrid = (unsigned)((n_long + 255) / 256);
-  const bool few = (flags & FSB_PANEL_FEW_PIECES) != 0;
 #define FSB_GROUPS_LAUNCH_(K)                                                                                    \
   do {                                                                                                           \
     cudaError_t e = cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);            \
     if (e != cudaSuccess) return cuda_rc(e);                                                                     \
-    K<<<(unsigned)n_ctas, panel_threads(mode, few), smem, st>>>((const VT_*)val, rc, unit_piece_ptr, unit_chunk,            \
+    K<<<(unsigned)n_ctas, panel_threads(mode), smem, st>>>((const VT_*)val, rc, unit_piece_ptr, unit_chunk,            \
                                                      cta_unit_ptr, cta_group, group_q_ptr, vbase, cta_part_ptr,  \
                                                      (VT_*)part, (const VT_*)x, gm, status);                     \
   } while (0)

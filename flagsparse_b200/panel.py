@@ -20,19 +20,19 @@ SM_COUNT_FALLBACK = 148
 CTAS_PER_SM = 1              # one 1024-thread CTA (row block) per SM
 # the kernel is worth its second copy of the matrix only when the extra reads of x and the padding stay small
 # bytes of x chunks loaded / bytes of entries streamed.  float32: a band of +-2^20 columns has 0.89 (319 G entries/s against
-# 231 G/s of the vector kernel; bound by the shared-memory work per entry and the barrier per unit, not by these bytes: half
-# of every chunk left out changes the time by 3 to 4 %).  Both lines are estimates above that, the break-even is not measured;
+# 231 G/s of the vector kernel; bound by the shared-memory work per entry, the barrier per unit and how soon a copy of x lands,
+# not by these bytes: half of every chunk left out changes the time by 3 to 4 %).  Both lines are estimates above that, the break-even is not measured;
 # float64 entries are 12 bytes and their chunks hold half the columns.
 MAX_X_OVERHEAD = 1.3
 MAX_X_OVERHEAD_F64 = 0.8
 MAX_SLOT_OVERHEAD = 1.25    # slots stored / entries
-N_BUFFERS = 2               # chunks of x in shared memory (fetched N_BUFFERS - 1 units ahead)
+N_BUFFERS = 2               # chunks of x in shared memory (fetched N_BUFFERS - 1 units ahead, by the warp of its own N_BUFFERS)
 ROUNDS = (4, 8, 16)         # slots per lane and piece the kernel is built for (see csrc/spmv_panel.cu)
 FLAG_LONG_RUNS = 1          # FSB_PANEL_LONG_RUNS
 FLAG_RUNS = 2               # FSB_PANEL_RUNS
 FLAG_FEW_PIECES = 4         # FSB_PANEL_FEW_PIECES
-# Mean pieces of a unit up to which 20 warps are enough: with 17.6 pieces 20 / 31 warps take 457 / 471 us (2^23 rows of 32, band of
-# +-2^20), with 21.4 (2^26 rows) 5056 / 4135 us.
+# Mean pieces of a unit up to which 20 warps are enough: 20 / 31 warps take, float32, band of +-2^20, with 17.6 pieces 457 / 471 us
+# (2^23 rows of 32), with 19.8 (2^22 rows of 36) 254 / 248, with 21.4 (2^26 rows) 5056 / 4135; float64 with 14.1 pieces 404 / 414.
 FEW_PIECES = 18
 # mean entries of a row inside one unit from which summing a run in a register beats one accumulator update per entry
 RUNS_MIN_MEAN = 1.5

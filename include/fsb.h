@@ -149,12 +149,13 @@ int fsb_spmv_csr_scatter(int vtype, int itype, int ptype, const void* data, cons
  *                        more than a piece holds); the kernel then also combines the lanes that finish on the
  *                        same row.  Must be set for such layouts.
  *                        FSB_PANEL_FEW_PIECES: units have 20 pieces or fewer, mostly; without the other two the kernel
- *                        then runs with fewer warps.  Only speed depends on this flag.
+ *                        then runs with fewer warps (the long-row form never does).  Only speed depends on this flag.
  *                        FSB_PANEL_DEBUG_TIMEOUT (tests only): the first copy of x of every CTA is made to
  *                        look incomplete and the wait limit is lowered, so that the kernel takes its time-out
  *                        path -- it reports through `status` and returns without touching y
  *   n_buffers            2..8 chunks of x in shared memory (n_buffers * chunk_cols <= 65536): chunks are
- *                        fetched n_buffers - 1 units ahead of their use
+ *                        fetched n_buffers - 1 units ahead of their use (without FSB_PANEL_RUNS and
+ *                        FSB_PANEL_LONG_RUNS: n_buffers, by a warp of its own)
  *   unit_piece_ptr       pieces [unit_piece_ptr[u], unit_piece_ptr[u+1]) belong to unit u
  *   unit_chunk           column chunk of unit u
  *   rb_unit_ptr          units [rb_unit_ptr[b], rb_unit_ptr[b+1]) belong to row block b, in chunk order
