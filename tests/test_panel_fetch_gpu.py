@@ -49,6 +49,24 @@ def test_fetching_warp(cuda, fsb_lib, vdt, buffers, chunk, rounds):
         assert_spmv_ok(want.cpu().numpy(), d, i, p, (n, n_cols), x[shift:shift + n_cols], what=f"x off by {shift}")
 
 
+@pytest.mark.parametrize("vdt,few", [("float32", 0), ("float32", P.FLAG_FEW_PIECES), ("float64", P.FLAG_FEW_PIECES)])
+def test_more_units_than_a_window(cuda, fsb_lib, vdt, few):
+    """The adding warps change their tables of 512 units while the fetching warp runs on: 1251 units a row block."""
+    n, n_cols = 6007, 40001
+    d, i, p = _band(n, n_cols, 18, 8)
+    d = d.astype(vdt)
+    x = np.random.default_rng(9).uniform(-1, 1, n_cols).astype(vdt)
+    with env(FSB_SPMV_ALGO="panel", FSB_PANEL_CHUNK=32, FSB_PANEL_ROUNDS=4):
+        prep = fs.prepare_spmv_csr(dev(d), dev(i), dev(p), (n, n_cols))
+    lay = prep.panel
+    assert not lay.flags & (P.FLAG_RUNS | P.FLAG_LONG_RUNS) and int((lay.rb_unit_ptr[1:] - lay.rb_unit_ptr[:-1]).max()) > 1024
+    lay.flags = (lay.flags & ~P.FLAG_FEW_PIECES) | few
+    y = fs.flagsparse_spmv_csr(x=dev(x), prepared=prep)
+    prep.check_status()
+    assert_spmv_ok(y.cpu().numpy(), d, i, p, (n, n_cols), x, what="three windows of units")
+    assert torch.equal(y, fs.flagsparse_spmv_csr(x=dev(x), prepared=prep))
+
+
 def test_a_wait_that_runs_out_is_reported(cuda, fsb_lib):
     d, i, p = _band(3000, 9000, 18, 7)
     with env(FSB_SPMV_ALGO="panel", FSB_PANEL_CHUNK=128):
