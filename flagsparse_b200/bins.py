@@ -111,8 +111,11 @@ def build_bins_layout(data, indices, indptr, n_rows, n_cols, max_row_nnz, span=0
         counts = torch.empty((n_blocks, n_chunks), dtype=torch.int32, device=dev)
         _lib.check(L.fsb_spmv_bins_count(pt, indices.data_ptr(), indptr.data_ptr(), block_row.data_ptr(), n_blocks, n_chunks,
                                          chunk_cols, n_cols, counts.data_ptr(), st), "fsb_spmv_bins_count")
-        if span and int(torch.count_nonzero(counts)) * chunk_cols * data.element_size() < span * n_blocks:   # a sync
-            return None
+        start = indptr[block_row.long()].to(torch.int64)
+        if span:
+            units, blocks = torch.stack((torch.count_nonzero(counts), torch.count_nonzero(start[1:] > start[:-1]))).tolist()  # a sync
+            if units * chunk_cols * data.element_size() < span * blocks:       # (blocks of empty rows reach nothing)
+                return None
         packs = (counts + (pack - 1)) // pack
         del counts
         unit_block, n_packs = _starts(packs)
@@ -133,7 +136,7 @@ def build_bins_layout(data, indices, indptr, n_rows, n_cols, max_row_nnz, span=0
                                          n_blocks, n_chunks, chunk_cols, n_cols, unit_chunk.data_ptr(), unit_block.data_ptr(),
                                          lay.col.data_ptr(), lay.place.data_ptr(), lay.dst.data_ptr(),
                                          lay.ends.data_ptr(), lay.row_slot.data_ptr(), st), "fsb_spmv_bins_place")
-        lay.block_start = torch.stack((block_row.to(torch.int64), indptr[block_row.long()].to(torch.int64)), 1).contiguous()
+        lay.block_start = torch.stack((block_row.to(torch.int64), start), 1)
     lay.chunk_pack, lay.block_pack = chunk_pack, block_pack
     lay.n_blocks, lay.n_chunks, lay.chunk_cols, lay.n_packs = n_blocks, n_chunks, chunk_cols, n_packs
     return lay

@@ -128,6 +128,13 @@ def test_what_is_left_to_one_pass(cuda, fsb_lib):
     assert bins.build_bins_layout(dev(d), dev(i), dev(p), 500, 9000, 4, span=9000 * 4, chunk_cols=1000) is None
 
 
+def test_blocks_of_empty_rows_do_not_count_for_the_reach(cuda, fsb_lib):
+    lens = [4] * 500 + [0] * 3 * 10**5
+    d, i, p = handmade_csr(4, lens, 9000)
+    build = lambda span: bins.build_bins_layout(dev(d), dev(i), dev(p), len(lens), 9000, 4, span=span, chunk_cols=1000)  # noqa: E731
+    assert build(9000 * 4) is not None and build(9000 * 4 + 1) is None
+
+
 @pytest.mark.parametrize("where", ["start", "middle", "end", "rows of one block", "one row more"])
 @pytest.mark.parametrize("vdt", ["float32", "float64"])
 def test_runs_of_empty_rows_are_shared_by_blocks(cuda, fsb_lib, where, vdt):
