@@ -15,20 +15,20 @@ from . import _lib
 from ._common import _ITYPE, _VTYPE
 
 # Where the two passes win, each line with both sides measured (us, one pass against two; columns anywhere unless said).
-# Rows of about equal length against the lanes-per-row kernel, float32: 2^27 entries in 33.6 M / 16.8 M / 4.2 M rows: 1330 / 626 /
-# 549 against 609 / 533 / 472; 2^24 entries in 4.2 M / 1 M / 0.5 M rows: 92 / 74 / 74 against 75 / 66 / 64; 2^23 entries in 2.1 M /
-# 0.5 M rows: 45 / 35 against 43 / 39.
+# Rows of about equal length against the lanes-per-row kernel, float32: 2^27 entries in 33.6 M / 16.8 M / 4.2 M rows: 1331 / 626 /
+# 549 against 636 / 542 / 474; 2^24 entries in 4.2 M / 1 M / 0.5 M rows: 92 / 74 / 74 against 78 / 69 / 66; 2^23 entries in 2.1 M /
+# 0.5 M rows: 45 / 35 against 47 / 42.
 EVEN_MIN_NNZ = 1 << 24
 EVEN_MIN_SPAN = 2 << 20
-# Uneven rows (the short rows of a skewed matrix, mostly), float32: 10.4 M entries in 2.1 M rows 91 against 46; 3.1 M in 0.5 M rows
-# 24.2 against 22.1; 2.7 M in 0.3 M rows 22.0 against 19.5; 2.6 M in 0.25 M rows 20.7 against 19.8.
+# Uneven rows (the short rows of a skewed matrix, mostly), float32: 107 M entries 1081 against 452; 10.4 M in 2.1 M rows 90 against
+# 51; 3.1 M in 0.5 M rows 24.1 against 22.5; 2.7 M in 0.3 M rows 22.1 against 20.0; 2.6 M in 0.25 M rows 20.6 against 19.8.
 UNEVEN_MIN_NNZ = 5 << 19
 UNEVEN_MIN_SPAN = 1 << 20
 # float64 moves 29 bytes an entry instead of 12, so it takes an x that L2 does not hold: 2^27 entries in 33.6 M / 16.8 M / 8.4 M
-# rows: 2155 / 1335 / 716 against 1461 / 1178 / 1030; uneven, 2^26 entries in 16.8 M / 8.4 M rows: 780 / 464 against 648 / 546.
+# rows: 2154 / 1335 / 726 against 1466 / 1143 / 998; uneven, 2^26 entries in 16.8 M / 8.4 M rows: 781 / 465 against 643 / 537.
 F64_MIN_SPAN = 120 << 20
 # ... or uneven rows of a few entries that would have gone to the lanes-per-row kernel, whose warps wait for their longest row:
-# 4.8 M entries in 2.1 M rows 66 against 49, 3.3 M in 1 M rows 42 against 35; by tiles, 2.6 M in 0.5 M rows 23.6 against 30.1.
+# 4.8 M entries in 2.1 M rows 66 against 52, 3.3 M in 1 M rows 42 against 35; by tiles, 2.6 M in 0.5 M rows 23.7 against 29.8.
 F64_SHORT_MEAN = 4
 # Rows of a block, at most: one CTA writes them, and rows without entries count for nothing in the cut by entries.  float32, one
 # pass against two with no such line / at most 2^16 rows: 2^24 rows, 4 entries in every row of the first half 272 against 1499 /

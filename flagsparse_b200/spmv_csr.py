@@ -251,7 +251,13 @@ def _validate_spmv_x(x, prepared):
 
 
 def prepare_spmv_csr(data, indices, indptr, shape, block_nnz=256, max_segments=None):
-    """Analyse a CSR matrix once for repeated SpMV calls (reference: spmv_csr.py:455-495)."""
+    """Analyse a CSR matrix once for repeated SpMV calls (reference: spmv_csr.py:455-495).
+
+    Values written into `data` afterwards are seen by the next product of matrices on the lanes-per-row, the stream and the
+    two-pass kernels, which read the array itself (opt_buckets[0]["kind"] "vector", "stream", "bins"); the panel and the
+    long-row form keep a copy of the values in their own order, made here: prepare again after a change.  `indices` and
+    `indptr` belong to what is prepared and must not change in any form.
+    """
     return _prepare_spmv_csr(data, indices, indptr, shape, block_nnz, max_segments, reuse_expected=True)
 
 
