@@ -15,25 +15,26 @@ from . import _lib
 from ._common import _ITYPE, _VTYPE
 
 # Where the two passes win, each line with both sides measured (us, one pass against two; columns anywhere unless said).
-# Rows of about equal length against the lanes-per-row kernel, float32: 2^27 entries in 33.6 M / 16.8 M / 4.2 M rows: 1331 / 626 /
-# 549 against 636 / 542 / 474; 2^24 entries in 4.2 M / 1 M / 0.5 M rows: 92 / 74 / 74 against 78 / 69 / 66; 2^23 entries in 2.1 M /
-# 0.5 M rows: 45 / 35 against 47 / 42.
+# Rows of about equal length against the lanes-per-row kernel, float32: 2^27 entries in 33.6 M / 16.8 M / 4.2 M rows: 1326 / 624 /
+# 549 against 606 / 530 / 473; 2^24 entries in 4.2 M / 1 M / 0.5 M rows: 92 / 75 / 75 against 75 / 67 / 65; 2^23 entries in 2.1 M /
+# 0.5 M rows: 45 / 35 against 43 / 40.
 EVEN_MIN_NNZ = 1 << 24
 EVEN_MIN_SPAN = 2 << 20
-# Uneven rows (the short rows of a skewed matrix, mostly), float32: 107 M entries 1081 against 452; 10.4 M in 2.1 M rows 90 against
-# 51; 3.1 M in 0.5 M rows 24.1 against 22.5; 2.7 M in 0.3 M rows 22.1 against 20.0; 2.6 M in 0.25 M rows 20.6 against 19.8.
+# Uneven rows (the short rows of a skewed matrix, mostly), float32: 107 M entries 1081 against 439; 10.4 M in 2.1 M rows 90 against
+# 47; 3.1 M in 0.5 M rows 24.1 against 22.3; 2.7 M in 0.3 M rows 22.0 against 19.8; 2.6 M in 0.25 M rows 20.6 against 20.0.
 UNEVEN_MIN_NNZ = 5 << 19
 UNEVEN_MIN_SPAN = 1 << 20
 # float64 moves 29 bytes an entry instead of 12, so it takes an x that L2 does not hold: 2^27 entries in 33.6 M / 16.8 M / 8.4 M
-# rows: 2154 / 1335 / 726 against 1466 / 1143 / 998; uneven, 2^26 entries in 16.8 M / 8.4 M rows: 781 / 465 against 643 / 537.
+# rows: 2154 / 1334 / 709 against 1420 / 1135 / 994; uneven, 2^26 entries in 16.8 M / 8.4 M rows: 780 / 465 against 630 / 530.
 F64_MIN_SPAN = 120 << 20
 # ... or uneven rows of a few entries that would have gone to the lanes-per-row kernel, whose warps wait for their longest row:
-# 4.8 M entries in 2.1 M rows 66 against 52, 3.3 M in 1 M rows 42 against 35; by tiles, 2.6 M in 0.5 M rows 23.7 against 29.8.
+# 4.8 M entries in 2.1 M rows 66 against 48, 3.3 M in 1 M rows 41 against 34; by tiles, 2.6 M in 0.5 M rows 23.3 against 29.8.
 F64_SHORT_MEAN = 4
-# Rows of a block, at most: one CTA writes them, and rows without entries count for nothing in the cut by entries.  float32, one
-# pass against two with no such line / at most 2^16 rows: 2^24 rows, 4 entries in every row of the first half 272 against 1499 /
-# 178 us; 16 in every one of the last 2^20 rows 207 against 2519 / 119; 10 M entries in the first 2 M of 30 M rows 324 against 4578 /
-# 124.  At most 2^14 / 2^18 rows: 188 / 202, 132 / 112, - / 140.
+# Rows of a block, at most (see cuts): one CTA writes them, and rows without entries count for nothing in the cut by entries.
+# float32, one pass against two with no such line / with it: 2^24 rows, 4 entries in every row of the first half 272 against 1499 /
+# 175 us; 16 in every one of the last 2^20 rows 207 against 2519 / 119; 10 M entries in the first 2 M of 30 M rows 323 against 4578 /
+# 126; with 2^14 / 2^18 instead: 177 / 204, 120 / 121, 128 / 143.  Blocks of fewer rows stay whole: cut at every 2^16th row of the
+# matrix, 107 M entries of short rows took 452 instead of 439 us, 27 M in 67 M rows 324 instead of 283.
 BLOCK_ROWS = 1 << 16
 # Mean entries of a unit below which the packs would mostly be padding; near the line, one pass against two: float32 with 17 entries
 # (2^25 in all, 70 M columns) 519 against 218 us, float64 with 8.4 (2^27, 36 M columns) 2177 against 1448.
@@ -59,9 +60,11 @@ def min_span(nnz, n_rows, max_row_nnz, element_size, lanes_per_row):
     return F64_MIN_SPAN if nnz >= EVEN_MIN_NNZ else None
 
 
-def most_blocks(nnz, n_rows, max_row_nnz, cap):
-    """Row blocks of a matrix, at most: one per `cap` entries, less what a last row may add, and one per BLOCK_ROWS rows."""
-    return -(-nnz // (cap - max_row_nnz + 1)) + -(-n_rows // BLOCK_ROWS)
+def cuts(nnz, n_rows, max_row_nnz, cap):
+    """(entries, rows) from one cut of the row blocks to the next: the row in which a cut by entries falls goes to the block
+    before it; rows as BLOCK_ROWS says, or twice what a block of a matrix of almost empty rows has on average."""
+    step = cap - max_row_nnz + 1
+    return step, max(BLOCK_ROWS, 2 * -(-n_rows // max(1024, -(-nnz // step))))
 
 
 class BinsLayout:
@@ -73,6 +76,18 @@ class BinsLayout:
     def nbytes(self):
         return sum(t.numel() * t.element_size() for t in (self.col, self.place, self.dst, self.ends, self.row_slot,
                                                           self.chunk_pack, self.block_pack, self.block_start))
+
+
+def _cut_rows(begin, n_rows, most):
+    """First rows of the blocks, and n_rows, as int32: those that begin at the rows `begin` (the first at row 0 whatever it
+    says), each cut into parts of about as many rows and `most` at most, and nothing for the empty ones."""
+    begin = torch.cat((begin.new_zeros(1), begin[1:].clamp(max=n_rows), begin.new_full((1,), n_rows)))
+    lens = begin[1:] - begin[:-1]
+    parts = (lens + (most - 1)) // most
+    block = torch.repeat_interleave(torch.arange(parts.numel(), device=begin.device), parts)      # a sync
+    part = torch.arange(block.numel(), device=begin.device) - (torch.cumsum(parts, 0) - parts)[block]
+    rows = begin[block] + lens[block] * part // parts[block]
+    return torch.cat((rows, begin[-1:])).to(torch.int32)
 
 
 def _starts(packs):
@@ -96,17 +111,16 @@ def build_bins_layout(data, indices, indptr, n_rows, n_cols, max_row_nnz, span=0
     n_chunks = -(-n_cols // chunk_cols)
     if max_row_nnz > cap // 4 or n_chunks > int(L.fsb_spmv_bins_max_chunks()) or n_cols * data.element_size() < span:
         return None
-    # a block begins at the first row that starts at or behind entry k * step: at most step - 1 + max_row_nnz entries; and at
-    # every BLOCK_ROWS-th row
-    step = cap - max_row_nnz + 1
-    n_blocks = most_blocks(nnz, n_rows, max_row_nnz, cap)
+    # a block begins at the first row that starts at or behind entry k * step: at most step - 1 + max_row_nnz entries; one of
+    # more than `rows` rows is cut into parts of as many rows each
+    step, rows = cuts(nnz, n_rows, max_row_nnz, cap)
+    n_blocks = -(-nnz // step) + -(-n_rows // rows)            # at most
     if nnz // pack + n_blocks * n_chunks >= 2**31 - 1 or (indptr.dtype == torch.int32 and nnz >= 2**31 - 1 - cap):
         return None
     st = torch.cuda.current_stream(dev).cuda_stream
     with torch.cuda.device(dev):
-        marks = torch.arange(1, -(-nnz // step), device=dev, dtype=indptr.dtype) * step
-        every = torch.arange(0, n_rows + BLOCK_ROWS, BLOCK_ROWS, device=dev).clamp_(max=n_rows)
-        block_row = torch.unique(torch.cat((torch.searchsorted(indptr, marks).clamp_(max=n_rows), every))).to(torch.int32)
+        block_row = _cut_rows(torch.searchsorted(indptr, torch.arange(-(-nnz // step), device=dev, dtype=indptr.dtype) * step),
+                              n_rows, rows)
         n_blocks = block_row.numel() - 1
         counts = torch.empty((n_blocks, n_chunks), dtype=torch.int32, device=dev)
         _lib.check(L.fsb_spmv_bins_count(pt, indices.data_ptr(), indptr.data_ptr(), block_row.data_ptr(), n_blocks, n_chunks,
@@ -151,8 +165,7 @@ def bins_for(data, indices, indptr, n_rows, n_cols, max_row_nnz, lanes_per_row):
     if span is None:
         return None
     L, vt = _lib.lib(), _VTYPE[data.dtype]
-    cap, chunk_cols = int(L.fsb_spmv_bins_cap(vt)), int(L.fsb_spmv_bins_chunk_cols(vt))
-    if max_row_nnz > cap // 4 or nnz * chunk_cols < MIN_UNIT[sv] * n_cols * most_blocks(nnz, n_rows, max_row_nnz, cap):
+    if int(L.fsb_spmv_bins_cap(vt)) * int(L.fsb_spmv_bins_chunk_cols(vt)) < MIN_UNIT[sv] * n_cols:
         return None
     try:
         return build_bins_layout(data, indices, indptr, n_rows, n_cols, max_row_nnz, span)

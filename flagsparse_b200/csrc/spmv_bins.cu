@@ -13,12 +13,12 @@
 // Per float32 entry 2 bytes in and 4 out, then 4 + 2 + 0.5 + 4 in (float64: 10 and 19): twice the bytes of one pass, all of
 // them streamed.  Rows are summed in CSR order, in double (float64: compensated inside a slice), so results do not depend on
 // the order of the entries inside a unit and are bit-reproducible.  107 M entries in 16.7 M rows of Zipf lengths, columns
-// anywhere in 2^24, float32: 640 us through spmv_stream_kernel, 456 us here: gather 135 us (0.64 GB), sum 318 us (1.13 GB; a
+// anywhere in 2^24, float32: 640 us through spmv_stream_kernel, 442 us here: gather 135 us (0.64 GB), sum 305 us (1.13 GB; a
 // block's elements arrive, are multiplied and added up and leave in turn, and two blocks an SM cover each other's phases in
 // part).  With a copy of the values in storage order, multiplied by the first pass: 216 and 225 us, but 4 more bytes an entry,
 // and values that the caller writes later would not be seen.  (Values asked for ahead with prefetch.global.L2: 3 us less
-// here, but 4 us more for 2^24 entries, which L2 holds.)  12 us of the sum keep the part of a row in the slice where it ends in
-// double until what the slices before have is there: rounded before, two parts that cancel lose what they differ by.
+// here, but 4 us more for 2^24 entries, which L2 holds.)  The part of a row in the slice where it ends stays in double until what
+// the slices before have is there: rounded before, two parts that cancel lose what they differ by.
 #include "fsb_common.cuh"
 
 namespace fsb {
