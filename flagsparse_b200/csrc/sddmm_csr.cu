@@ -9,31 +9,83 @@
 // eight gathers in flight; a batch that lies inside one row needs one slice of X's row, one that meets two rows a slice of
 // each, a batch that crosses more loads a slice of X per entry.  Each lane ends with eight partial sums (one per entry);
 // they are reduced across the group by a transposed exchange (halve the entries a lane is responsible for at every
-// step: 7 shuffles for 8 entries x 8 lanes instead of 24), after which the results of consecutive entries sit in
-// consecutive lanes and leave as one contiguous streaming store.  Rows of X longer than LG * VW elements are
-// walked in several steps.  The summation order is fixed, so results are bit-reproducible.
+// step: 7 shuffles for 8 entries x 8 lanes instead of 24), and put into shared memory, from where the tile's results leave
+// in order.  Rows of X longer than LG * VW elements are walked in several steps.  The summation order is fixed, so results are bit-reproducible.
 // CUDA-core work on purpose: one dot product per entry over gathered rows is about 0.5 flop per byte.
 #include "fsb_common.cuh"
 
 namespace fsb {
 
-#ifndef FSB_SDDMM_MIN_CTAS
-#define FSB_SDDMM_MIN_CTAS 3   // resident CTAs per SM the register budget is set for (80 registers: no spills)
-#endif
 constexpr int kSdThreads = 256;
 constexpr int kSdBatch = 8;   // consecutive entries one group handles
 
-// entries one CTA handles: J passes of (threads / LG) groups x 8 entries, at most 2048
+// Resident CTAs the register budget is set for: 64 registers, but 80 for 16-byte accesses of float64, whose eight sums take twice
+// the room (131072 rows of 16, K 200: 476 us, with 64 registers 603 us).
+__host__ __device__ constexpr int sddmm_ctas(int vw, size_t size) { return size == 8 && vw == 2 ? 3 : 4; }
+
+// entries one CTA handles: J passes of (threads / LG) groups x 8 entries, about 1024 (262144 rows of 6, K 8: 17.3 us, with 2048
+// 20.3 us, a last wave that is a quarter full; 2^19 rows of 16, K 64: 251 us, with 512 265 us)
 __host__ __device__ constexpr int sddmm_passes(int LG) {
   const int per_pass = (kSdThreads / LG) * kSdBatch;
-  return per_pass >= 2048 ? 1 : (2048 / per_pass < 8 ? 2048 / per_pass : 8);
+  return per_pass >= 1024 ? 1 : (1024 / per_pass < 8 ? 1024 / per_pass : 8);
 }
 __host__ __device__ constexpr int sddmm_tile(int LG) { return (kSdThreads / LG) * kSdBatch * sddmm_passes(LG); }
 
+// row `id` of a matrix whose rows are `stride` bytes apart, from `base` on: one wide multiply-add and one for the high word
+template <typename V>
+__device__ __forceinline__ const V* row_at(const char* base, int32_t id, uint64_t stride) {
+  return reinterpret_cast<const V*>(base + (uint64_t)(uint32_t)id * stride);
+}
+
+// dot product of what one lane holds of two rows; pairs of floats go through the packed multiply-add
+template <typename V, int VW>
+__device__ __forceinline__ V lane_dot(const V (&a)[VW], const V (&b)[VW]) {
+  V s = a[0] * b[0];
+#pragma unroll
+  for (int i = 1; i < VW; ++i) s = fma(a[i], b[i], s);
+  return s;
+}
+__device__ __forceinline__ uint64_t pack2(float x, float y) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ float lane_dot(const float (&a)[4], const float (&b)[4]) {
+  uint64_t t;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(t) : "l"(pack2(a[0], a[1])), "l"(pack2(b[0], b[1])));
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(t) : "l"(pack2(a[2], a[3])), "l"(pack2(b[2], b[3])));
+  float x, y;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(t));
+  return x + y;
+}
+
+// The form of a batch of eight entries: bit e is set where entry e lies in the row of the first one; kSdOne: all of them do;
+// kSdTwo: the others lie in the row of the last one.
+//
+// Row ids never decrease along a CSR pattern.  Most batches meet one row of X or two: a slice of each then serves all eight
+// gathers, which leave together.  Where a batch meets more rows every entry gets its own slice of X, four entries at a time
+// (reloading X only where the row changes would make each gather wait for the previous entry's arithmetic).
+// vote (two to four groups in a warp, 16-byte gathers): the groups agree on the form that all of their batches fit, as a
+// warp whose groups differ runs one form after the other (2^19 rows of 16, K 64, Zipf lengths: 392 us without it, 292 us with
+// it; float64, 2^18 such rows, K 32: 204 us, 146 us).  With eight groups and more, or smaller gathers, agreeing costs more than
+// it saves (K 16: 98 us, with it 109 us; K 33: 558 us, 614 us), and a batch of one row takes the form of two.
+//
+// What bounded the kernel before its present shape was its own arithmetic: 340 warp instructions for 16 entries (2^19 rows of
+// 16, K 64, float32), of which the gathers, the products and their sums need about a third; 4.8 of the 10.2 cycles that a
+// warp took per instruction were spent waiting for memory.  So the forms are worked out once per batch while the ids are staged
+// (not by every lane of the group), rows are found by one wide multiply-add from a stride in bytes, pairs of floats are
+// multiplied by one instruction, and the results leave through shared memory with alpha, beta and `data` at the end.
+// That case 290 us before, 251 us now (gathers at 8.6 TB/s, DRAM traffic 1.2 GB); 131072 rows of 32: 117 us, 95 us; K 33:
+// 268 us, 173 us; float64, 2^18 rows of 16, K 32: 228 us, 146 us.  A group that walks whole rows instead, as the SpMM kernel
+// does, with the next row's slice of X on its way: 309 us (groups of a warp wait for the longest row among theirs).
+constexpr uint32_t kSdOne = 1u << 8, kSdTwo = 1u << 9;
+template <typename V>
+__host__ __device__ constexpr bool sddmm_vote(int VW, int LG) { return VW * (int)sizeof(V) == 16 && (LG == 8 || LG == 16); }
+
 template <typename V, int VW, int LG>
-__global__ void __launch_bounds__(kSdThreads, FSB_SDDMM_MIN_CTAS)
+__global__ void __launch_bounds__(kSdThreads, sddmm_ctas(VW, sizeof(V)))
 sddmm_kernel(const int32_t* __restrict__ indices, const int32_t* __restrict__ row_ids, const V* __restrict__ X,
-             int64_t ldx, const V* __restrict__ Y, int64_t ldy, const V* __restrict__ data, V* __restrict__ out,
+             int64_t ldx, const V* __restrict__ Y, int64_t ldy, const V* data, V* out,
              int64_t nnz, int k_dim, V alpha, V beta, int ids_aligned) {
   constexpr int E = kSdBatch;
   constexpr int step = LG * VW;
@@ -42,9 +94,12 @@ sddmm_kernel(const int32_t* __restrict__ indices, const int32_t* __restrict__ ro
   constexpr int T = sddmm_tile(LG);
   constexpr int kHeld = (LG >= E) ? 1 : E / LG;   // results a lane ends up with
   constexpr int kDup = (LG > E) ? LG / E : 1;     // lanes that end up with the same result
-  constexpr bool VOTE = sizeof(V) == 4 && VW == 4 && (LG == 8 || LG == 16);   // see the loop
+  constexpr bool VOTE = sddmm_vote<V>(VW, LG);
+  constexpr bool ONE = VOTE || LG == 32;          // batches of one row have a form of their own
   __shared__ __align__(16) int32_t s_cols[T];
   __shared__ __align__(16) int32_t s_rows[T];
+  __shared__ __align__(16) V s_out[T];
+  __shared__ uint32_t s_form[T / E];
 
   // the tile's column and row ids go to shared memory once (entries past the end repeat the last one; they are
   // never stored), so that the loop below has one trip to global memory per batch: the gathers
@@ -63,9 +118,26 @@ sddmm_kernel(const int32_t* __restrict__ indices, const int32_t* __restrict__ ro
     }
   }
   __syncthreads();
+  for (int b = threadIdx.x; b < T / E; b += kSdThreads) {
+    const int32_t* r = s_rows + b * E;
+    const int32_t row_a = r[0], row_b = r[E - 1];
+    uint32_t form = row_a == row_b ? kSdOne : 0;
+    bool two = true;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      two = two && (r[e] == row_a || r[e] == row_b);
+      form |= (r[e] == row_a ? 1u : 0u) << e;
+    }
+    s_form[b] = form | (two ? kSdTwo : 0);
+  }
+  __syncthreads();
 
   const int lane = threadIdx.x & (LG - 1);
   const int group = threadIdx.x / LG;
+  const int k0 = lane * VW;
+  const char* Xk = reinterpret_cast<const char*>(X + k0);
+  const char* Yk = reinterpret_cast<const char*>(Y + k0);
+  const uint64_t xs = (uint64_t)ldx * sizeof(V), ys = (uint64_t)ldy * sizeof(V);
   const unsigned gmask = LG == 32 ? 0xffffffffu : (((1u << LG) - 1u) << ((threadIdx.x & 31) & ~(LG - 1)));
   unsigned active = 0xffffffffu;   // lanes of the warp that have a batch
 #pragma unroll 1
@@ -73,101 +145,57 @@ sddmm_kernel(const int32_t* __restrict__ indices, const int32_t* __restrict__ ro
     const int local = (j * kGroups + group) * E;
     if constexpr (VOTE) active = __ballot_sync(active, local < left);
     if (local >= left) break;   // whole groups leave together: the shuffles below stay inside a group
-    const int64_t p0 = tile0 + local;
-    const int n = (int)((left - local) < E ? (left - local) : E);
-    int32_t rows[E], cols[E];
-    {
-      const int4 c0 = *reinterpret_cast<const int4*>(s_cols + local);
-      const int4 c1 = *reinterpret_cast<const int4*>(s_cols + local + 4);
-      const int4 r0 = *reinterpret_cast<const int4*>(s_rows + local);
-      const int4 r1 = *reinterpret_cast<const int4*>(s_rows + local + 4);
-      cols[0] = c0.x; cols[1] = c0.y; cols[2] = c0.z; cols[3] = c0.w;
-      cols[4] = c1.x; cols[5] = c1.y; cols[6] = c1.z; cols[7] = c1.w;
-      rows[0] = r0.x; rows[1] = r0.y; rows[2] = r0.z; rows[3] = r0.w;
-      rows[4] = r1.x; rows[5] = r1.y; rows[6] = r1.z; rows[7] = r1.w;
-    }
-
-    // the values of `data` this lane will need at the end are requested before the gathers, not after them
-    const bool writer = (lane % kDup) == 0;
-    const int first = (lane / kDup) * kHeld;
-    V din[kHeld];
-#pragma unroll
-    for (int i = 0; i < kHeld; ++i)
-      din[i] = (data != nullptr && writer && first + i < n) ? __ldcs(data + p0 + first + i) : (V)0;
-
     V acc[E];
 #pragma unroll
     for (int e = 0; e < E; ++e) acc[e] = (V)0;
-    // Row ids never decrease along a CSR pattern.  Most batches meet one row of X or two: a slice of each then serves all
-    // eight gathers, which leave together.  Where a batch meets more rows every entry gets its own slice of X, four
-    // entries at a time (reloading X only where the row changes would make each gather wait for the previous entry's
-    // arithmetic).  float64, and float32 with a whole warp per entry, have no registers for a second slice beside eight
-    // gathers of 16 bytes: there only a batch of one row takes the first form.  (2^19 rows of 16 entries, K 64, float32:
-    // 456 us when a batch of two rows took the second form, 343 us with a slice of each; 300000 rows of 5, K 33: 162 us,
-    // 105 us.  With TWO everywhere float64, 50000 rows of 40, K 64 goes from 115 us to 168 us.)
-    // VOTE (two to four groups in a warp, 16-byte gathers): the groups agree on the form that all of their batches fit, as a
-    // warp whose groups differ runs one form after the other; single rows have a form of their own.  Without it uneven
-    // rows lost what even ones had gained (2^19 rows of 16, K 64: even 343 us, Zipf lengths 392 us where 316 us had been
-    // measured with the first and last form alone; with it 292 us and 320 us.  300000 rows of 5: 98.6 us, 88 us, 86.3 us).
-    // With eight groups and more, or smaller gathers, agreeing costs more than it saves (K 16: 98 us, with it 109 us; K 33: 558
-    // us, 614 us).
-    constexpr bool TWO = sizeof(V) == 4 && (LG <= 16 || VW == 1);
-    const int32_t row_a = rows[0], row_b = rows[E - 1];
-    bool one = row_a == row_b, few = TWO;
-    unsigned in_a = 0;
-    if constexpr (TWO) {
-#pragma unroll
-      for (int e = 0; e < E; ++e) {
-        few = few && (rows[e] == row_a || rows[e] == row_b);
-        in_a |= (rows[e] == row_a ? 1u : 0u) << e;
-      }
-    }
+    const uint32_t form = s_form[local / E];
+    bool one = (form & kSdOne) != 0, two = (form & kSdTwo) != 0;
     if constexpr (VOTE) {
       one = __all_sync(active, one);
-      few = __all_sync(active, few);
+      two = __all_sync(active, two);
     }
-    if ((!TWO || VOTE) && one) {
-      for (int k = lane * VW; k < k_dim; k += step) {
+    const int32_t* cols = s_cols + local;
+    const int32_t* rows = s_rows + local;
+    if (ONE && one) {
+      const char *xp = reinterpret_cast<const char*>(row_at<V>(Xk, rows[0], xs)), *yp = Yk;
+      for (int k = k0; k < k_dim; k += step, xp += step * sizeof(V), yp += step * sizeof(V)) {
         V xa[VW], yv[E][VW];
-        ld_dense<V, VW>(X + (int64_t)row_a * ldx + k, xa);
+        ld_dense<V, VW>(reinterpret_cast<const V*>(xp), xa);
 #pragma unroll
-        for (int e = 0; e < E; ++e) ld_dense<V, VW>(Y + (int64_t)cols[e] * ldy + k, yv[e]);
+        for (int e = 0; e < E; ++e) ld_dense<V, VW>(row_at<V>(yp, cols[e], ys), yv[e]);
 #pragma unroll
-        for (int e = 0; e < E; ++e)
-#pragma unroll
-          for (int i = 0; i < VW; ++i) acc[e] += xa[i] * yv[e][i];
+        for (int e = 0; e < E; ++e) acc[e] += lane_dot(xa, yv[e]);
       }
-    } else if (few) {
-      for (int k = lane * VW; k < k_dim; k += step) {
+    } else if (two) {
+      const char *xp = reinterpret_cast<const char*>(row_at<V>(Xk, rows[0], xs)), *yp = Yk;
+      const char *xq = reinterpret_cast<const char*>(row_at<V>(Xk, rows[E - 1], xs));
+      for (int k = k0; k < k_dim; k += step, xp += step * sizeof(V), xq += step * sizeof(V), yp += step * sizeof(V)) {
         V xa[VW], xb[VW], yv[E][VW];
-        ld_dense<V, VW>(X + (int64_t)row_a * ldx + k, xa);
-        if (!VOTE || row_b != row_a) {
-          ld_dense<V, VW>(X + (int64_t)row_b * ldx + k, xb);
-        } else {
+        ld_dense<V, VW>(reinterpret_cast<const V*>(xp), xa);
+        ld_dense<V, VW>(reinterpret_cast<const V*>(xq), xb);
 #pragma unroll
-          for (int i = 0; i < VW; ++i) xb[i] = xa[i];
+        for (int e = 0; e < E; ++e) ld_dense<V, VW>(row_at<V>(yp, cols[e], ys), yv[e]);
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+          V t;                       // (a branch of the group; choosing the slice first takes an instruction per element)
+          if (form >> e & 1) t = lane_dot(xa, yv[e]);
+          else t = lane_dot(xb, yv[e]);
+          acc[e] += t;
         }
-#pragma unroll
-        for (int e = 0; e < E; ++e) ld_dense<V, VW>(Y + (int64_t)cols[e] * ldy + k, yv[e]);
-#pragma unroll
-        for (int e = 0; e < E; ++e)
-#pragma unroll
-          for (int i = 0; i < VW; ++i) acc[e] += ((in_a >> e) & 1 ? xa[i] : xb[i]) * yv[e][i];
       }
     } else {
-      for (int k = lane * VW; k < k_dim; k += step) {
+      const char *xp = Xk, *yp = Yk;
+      for (int k = k0; k < k_dim; k += step, xp += step * sizeof(V), yp += step * sizeof(V)) {
 #pragma unroll
         for (int h = 0; h < E; h += E / 2) {
           V xv[E / 2][VW], yv[E / 2][VW];
 #pragma unroll
           for (int e = 0; e < E / 2; ++e) {
-            ld_dense<V, VW>(X + (int64_t)rows[h + e] * ldx + k, xv[e]);
-            ld_dense<V, VW>(Y + (int64_t)cols[h + e] * ldy + k, yv[e]);
+            ld_dense<V, VW>(row_at<V>(xp, rows[h + e], xs), xv[e]);
+            ld_dense<V, VW>(row_at<V>(yp, cols[h + e], ys), yv[e]);
           }
 #pragma unroll
-          for (int e = 0; e < E / 2; ++e)
-#pragma unroll
-            for (int i = 0; i < VW; ++i) acc[h + e] += xv[e][i] * yv[e][i];
+          for (int e = 0; e < E / 2; ++e) acc[h + e] += lane_dot(xv[e], yv[e]);
         }
       }
     }
@@ -192,18 +220,18 @@ sddmm_kernel(const int32_t* __restrict__ indices, const int32_t* __restrict__ ro
         acc[0] += __shfl_xor_sync(gmask, acc[0], off, LG);
       }
     }
-    // a lane now holds kHeld consecutive entries starting at `first`; where LG > E, kDup lanes hold the same sum
-    if (writer) {
+    // a lane now holds kHeld consecutive entries; where LG > E, kDup lanes hold the same sum
+    if (lane % kDup == 0) {
 #pragma unroll
-      for (int i = 0; i < kHeld; ++i) {
-        const int e = first + i;
-        if (e < n) {
-          V v = acc[i] * alpha;
-          if (data != nullptr) v += din[i] * beta;
-          __stcs(out + p0 + e, v);
-        }
-      }
+      for (int i = 0; i < kHeld; ++i) s_out[local + (lane / kDup) * kHeld + i] = acc[i];
     }
+  }
+  __syncthreads();
+  // results leave in order, with `data`, which may be the same array
+  for (int i = threadIdx.x; i < T && i < left; i += kSdThreads) {
+    V v = s_out[i] * alpha;
+    if (data != nullptr) v += __ldcs(data + tile0 + i) * beta;
+    __stcs(out + tile0 + i, v);
   }
 }
 

@@ -29,3 +29,22 @@ def test_batches_over_rows(cuda, fsb_lib, dtype, u, name):
         out = fs.flagsparse_sddmm_csr(x=x.to(cuda), y=y.to(cuda), prepared=prep).cpu().double().numpy()
         xd, yd = x.double().numpy()[row], y.double().numpy()[i]
         assert np.all(np.abs(out - (xd * yd).sum(1)) <= (k + 1) * u * 1.0001 * np.abs(xd * yd).sum(1))
+
+
+@pytest.mark.parametrize("dtype,u", [(torch.float32, 2.0 ** -24), (torch.float64, 2.0 ** -53)], ids=str)
+@pytest.mark.parametrize("k", [3, 4, 64, 128])          # a thread, a half warp, a warp per entry, and single elements
+def test_ends_of_tiles(cuda, fsb_lib, dtype, u, k):
+    """Tiles of 512 to 2048 entries: one less, all, one more, and out in the place of data."""
+    rng = np.random.default_rng(k)
+    for nnz in (1, 511, 512, 513, 1023, 1024, 1025, 2047, 2048, 2049):
+        ptr = np.unique(np.concatenate([[0, nnz], rng.integers(0, nnz + 1, nnz // 7)]))
+        col = rng.integers(0, 50, nnz)
+        x, y, d = (rng.uniform(-1, 1, s).astype(np.float32) for s in ((len(ptr) - 1, k), (50, k), nnz))
+        x, y, d = (torch.from_numpy(v).to(dtype) for v in (x, y, d))
+        prep = fs.prepare_sddmm_csr(torch.from_numpy(col.astype(np.int32)).to(cuda), torch.from_numpy(ptr).to(cuda), (len(ptr) - 1, 50))
+        out = d.to(cuda)
+        fs.flagsparse_sddmm_csr(out, x=x.to(cuda), y=y.to(cuda), alpha=0.5, beta=-2.0, prepared=prep, out=out)
+        xd, yd = x.double().numpy()[np.repeat(np.arange(len(ptr) - 1), np.diff(ptr))], y.double().numpy()[col]
+        # the dot product's (k + 1) u, and a rounding for beta * data and one for the sum
+        bound = (k + 1) * u * 0.5 * np.abs(xd * yd).sum(1) + 2 * u * (0.5 * np.abs((xd * yd).sum(1)) + 2 * np.abs(d.double().numpy()))
+        assert np.all(np.abs(out.cpu().double().numpy() - (0.5 * (xd * yd).sum(1) - 2 * d.double().numpy())) <= 1.0001 * bound), nnz
