@@ -18,6 +18,14 @@ inline int cuda_rc(cudaError_t e) { return e == cudaSuccess ? FSB_OK : FSB_CUDA_
 inline bool aligned_to(const void* p, size_t a) { return (reinterpret_cast<uintptr_t>(p) & (a - 1)) == 0; }
 __device__ __forceinline__ bool aligned_to_dev(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
+// SMs of the current device
+inline int sm_count(int* out) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(out, cudaDevAttrMultiProcessorCount, dev);
+  return cuda_rc(e);
+}
+
 // ---- the checking build: entry points walk their index arrays first (bounds_check.cu) ----------------
 #ifdef FSB_BOUNDS_CHECK
 int check_csr(int itype, int ptype, const void* indices, const void* indptr, int64_t n_rows, int64_t n_cols,

@@ -414,10 +414,10 @@ extern "C" int fsb_spmv_csr_bins(int vtype, const uint16_t* col, const int32_t* 
   if (gather_smem > 226 * 1024) return FSB_ERANGE;
   FSB_WALK_FIRST(check_bins(vtype, col, place, dst, ends, row_slot, chunk_pack, block_pack, block_start, n_blocks, n_chunks,
                             chunk_cols, n_packs, n_rows, n_cols, st));
-  int dev = 0, sms = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (e != cudaSuccess) return cuda_rc(e);
+  int sms = 0;
+  rc = sm_count(&sms);
+  if (rc != FSB_OK) return rc;
+  cudaError_t e;
 #define FSB_BINS_RUN(V_)                                                                                                    \
   do {                                                                                                                      \
     e = cudaFuncSetAttribute(bins_gather_kernel<V_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gather_smem);        \

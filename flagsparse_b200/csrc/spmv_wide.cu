@@ -14,11 +14,11 @@
 // 32; wider B in column tiles of 32 along gridDim.y), every lane owns one column of C, walks the row's entries (value and
 // column index are the same address for the whole group: one broadcast load) and gathers its element of B's row, two
 // entries in flight.
-#include <cuda_bf16.h>
-#include <cuda_fp16.h>
 #include <string.h>
 
 #include "fsb_common.cuh"
+#include "spmv_rows.cuh"
+#include "stored_ops.cuh"
 
 namespace fsb {
 
@@ -60,20 +60,6 @@ struct WideOps<double2> {
     acc.y += a.x * b.y + a.y * b.x;
   }
 };
-
-__device__ __forceinline__ float w_zero(float*) { return 0.f; }
-__device__ __forceinline__ float2 w_zero(float2*) { return make_float2(0.f, 0.f); }
-__device__ __forceinline__ double2 w_zero(double2*) { return make_double2(0.0, 0.0); }
-__device__ __forceinline__ float w_add(float a, float b) { return a + b; }
-__device__ __forceinline__ float2 w_add(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ double2 w_add(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ float w_down(float v, int o) { return __shfl_down_sync(0xffffffffu, v, o); }
-__device__ __forceinline__ float2 w_down(float2 v, int o) {
-  return make_float2(__shfl_down_sync(0xffffffffu, v.x, o), __shfl_down_sync(0xffffffffu, v.y, o));
-}
-__device__ __forceinline__ double2 w_down(double2 v, int o) {
-  return make_double2(__shfl_down_sync(0xffffffffu, v.x, o), __shfl_down_sync(0xffffffffu, v.y, o));
-}
 
 template <typename S, typename P, int L>
 __global__ void __launch_bounds__(kWideThreads)
@@ -236,52 +222,6 @@ namespace fsb {
 // ---------------------------------------------------------------------------------------------------
 // y = A x with x and y in the matrix's own type
 // ---------------------------------------------------------------------------------------------------
-// Products and sums in the accumulator type, every element of y rounded once.  `prod` is the product in the accumulator
-// type: exact for the half precisions, a multiplication and a fused multiply-add per component for complex values.
-template <typename S> struct StoredOps;
-template <>
-struct StoredOps<__half> {
-  typedef float A;
-  typedef float R;
-  static __device__ __forceinline__ A prod(__half a, __half b) { return __half2float(a) * __half2float(b); }
-  static __device__ __forceinline__ void fma(A& acc, __half a, __half b) {
-    acc = fmaf(__half2float(a), __half2float(b), acc);
-  }
-  static __device__ __forceinline__ __half narrow(A v) { return __float2half_rn(v); }
-};
-template <>
-struct StoredOps<__nv_bfloat16> {
-  typedef float A;
-  typedef float R;
-  static __device__ __forceinline__ A prod(__nv_bfloat16 a, __nv_bfloat16 b) {
-    return __bfloat162float(a) * __bfloat162float(b);
-  }
-  static __device__ __forceinline__ void fma(A& acc, __nv_bfloat16 a, __nv_bfloat16 b) {
-    acc = fmaf(__bfloat162float(a), __bfloat162float(b), acc);
-  }
-  static __device__ __forceinline__ __nv_bfloat16 narrow(A v) { return __float2bfloat16_rn(v); }
-};
-template <typename C2, typename Real>
-struct StoredComplex {
-  typedef C2 A;
-  typedef Real R;
-  static __device__ __forceinline__ A prod(C2 a, C2 b) {
-    C2 r;
-    r.x = ::fma(a.x, b.x, -(a.y * b.y));
-    r.y = ::fma(a.x, b.y, a.y * b.x);
-    return r;
-  }
-  // one rounding at the size of the sum: rows of 700 entries, rms error 1.11 times as large with both products fused into it
-  static __device__ __forceinline__ void fma(A& acc, C2 a, C2 b) {
-    const C2 p = prod(a, b);
-    acc.x += p.x;
-    acc.y += p.y;
-  }
-  static __device__ __forceinline__ C2 narrow(A v) { return v; }
-};
-template <> struct StoredOps<float2> : StoredComplex<float2, float> {};
-template <> struct StoredOps<double2> : StoredComplex<double2, double> {};
-
 // four consecutive stored values: 8, 32 or 64 bytes in accesses of at most 16
 __device__ __forceinline__ void ld_four(const __half* p, __half (&v)[4]) {
   const uint2 t = __ldcs(reinterpret_cast<const uint2*>(p));
@@ -571,6 +511,7 @@ static int stored_launch(const void* data_, const int32_t* idx, const void* ptr_
     }
     return FSB_OK;
   }
+  if (rows_apply(data, idx, n_rows, nnz)) return rows_run<S, int32_t, P>(data, idx, ptr, x, RowsOut<S>{y}, n_rows, nnz, st);
   // two to four groups of four entries per lane, as in the float32 / float64 kernel; entry by entry, three to six
   // (columns anywhere, 4 / 8 / 16 lanes a row: complex64, 500009 rows of 24: 70 / 64 / - us, 300000 rows of 30: 55 / 47 / 51 us,
   // 2000000 rows of 20: 209 / 212 / - us, 100000 rows of 60: - / 35 / 31 us; complex128: 84 / 78 / - us, 66 / 58 / 64 us, 289 / 294

@@ -1,0 +1,59 @@
+"""The SpMV kernel that walks neighbouring rows on one SM (from 8192 rows on): every number of lanes, rows that take one turn and
+several, shares of even and uneven weight, ends of the arrays, every value type and index width.  Reference and bound as for
+the tiled kernels: the product of the stored values in complex128."""
+
+import numpy as np
+import pytest
+import torch
+
+import flagsparse_b200 as fs
+from helpers import handmade_csr
+from test_stored_types_gpu import DTYPES, _check, _values
+
+pytestmark = pytest.mark.gpu
+
+
+def _lengths():
+    rng = np.random.default_rng(5)
+    yield "least", [k % 6 for k in range(8192)]
+    yield "one more", [k % 6 for k in range(8193)]
+    for mean in (1, 5, 13, 27, 60, 130):                       # 2, 2, 4, 8, 16, 32 lanes for four entries at a time
+        yield f"mean {mean}", rng.poisson(mean, 8200 + mean)
+    yield "several turns", np.where(np.arange(9001) % 97 == 5, 90, 4)
+    yield "empty, then rows", np.where(np.arange(30000) < 24000, 0, 9)     # uneven shares: dealt in turn
+    yield "long rows first", np.where(np.arange(20003) < 2500, 70, 8)
+    yield "last entry", [0] * 20000 + [1]
+
+
+@pytest.mark.parametrize("dtype", DTYPES, ids=str)
+def test_against_the_stored_values(cuda, fsb_lib, dtype):
+    n_cols = 12000
+    for name, lens in _lengths():
+        _, i, p = handmade_csr(7, [int(v) for v in lens], n_cols)
+        vals, x = _values(int(p[-1]), dtype, 4), _values(n_cols, dtype, 5)
+        shape = (len(p) - 1, n_cols)
+        d, ti, tp, tx = vals.to(cuda), torch.from_numpy(i).to(cuda), torch.from_numpy(p).to(cuda), x.to(cuda)
+        y = fs.flagsparse_spmv_csr(d, ti, tp, tx, shape)
+        _check(y, vals, i, p, n_cols, x, dtype)
+        for wi, wp in ((ti.long(), tp), (ti, tp.long()), (ti.long(), tp.long())):
+            assert torch.equal(fs.flagsparse_spmv_csr(d, wi, wp, tx, shape), y), name
+        prep = fs.prepare_spmv_csr(d, ti, tp, shape)
+        assert torch.equal(fs.flagsparse_spmv_csr(x=tx, prepared=prep), y), name
+        if vals.numel() > 1:                                    # arrays that start off a 16-byte boundary: lanes per row
+            off = torch.cat([d[:1], d])[1:], torch.cat([ti[:1], ti])[1:]
+            _check(fs.flagsparse_spmv_csr(*off, tp, tx, shape), vals, i, p, n_cols, x, dtype)
+
+
+def test_what_neighbours_hold_stays_out(cuda, fsb_lib):
+    """Infinite and NaN entries of one row, read along with the rows beside it, and of x, where no entry points."""
+    n, length = 9000, 7
+    d = torch.ones(n * length, device=cuda)
+    d[length * 100:length * 101] = float("inf")
+    d[length * 205] = float("nan")
+    i = (torch.arange(n * length, device=cuda, dtype=torch.int32) * 3) % 5000
+    x = torch.ones(5001, device=cuda)
+    x[5000] = float("nan")
+    y = fs.flagsparse_spmv_csr(d, i, torch.arange(n + 1, device=cuda, dtype=torch.int32) * length, x, (n, 5001))
+    want = torch.full((n,), float(length), device=cuda)
+    want[100], want[205] = float("inf"), float("nan")
+    assert torch.equal(torch.nan_to_num(y, nan=-1.0), torch.nan_to_num(want, nan=-1.0))
