@@ -6,6 +6,9 @@ their own; the other four value dtypes of the reference's whitelist run through 
 stored (widetypes.py), on the entry points where the reference accepts them.
 """
 
+import ctypes
+import threading
+
 import torch
 
 from . import _lib
@@ -88,15 +91,54 @@ class CsrStats:
          self.max_row_nnz, self.n_empty_rows, self.n_long_rows) = (int(v) for v in values)
 
 
+class _CheckSlot:
+    """What fsb_csr_check needs beside the matrix: counters on the device and page-locked memory for the answer.  One per thread
+    and device: a call is over when its answer is there, whichever stream it was enqueued on."""
+
+    __slots__ = ("work", "host", "work_ptr", "host_ptr", "_words")
+
+    def __init__(self, device):
+        self.host = torch.zeros(10, dtype=torch.int64, pin_memory=True)
+        self.work = torch.zeros(7, dtype=torch.int64, device=device)
+        torch.cuda.current_stream(device).synchronize()       # the zeros are there for whatever stream comes next
+        self.work_ptr, self.host_ptr = self.work.data_ptr(), self.host.data_ptr()
+        self._words = (ctypes.c_int64 * 8).from_address(self.host_ptr)
+
+    def stats(self):
+        return CsrStats(self._words)
+
+
+_thread = threading.local()
+
+
+def _check_slot(device):
+    """This thread's slot for `device`, or None where there can be none (not a GPU; first used while a stream is captured)."""
+    slots = getattr(_thread, "slots", None)
+    if slots is None:
+        slots = _thread.slots = {}
+    slot = slots.get(device.index)
+    if slot is None and device.type == "cuda" and device.index is not None and not torch.cuda.is_current_stream_capturing():
+        slot = slots[device.index] = _CheckSlot(device)
+    return slot
+
+
 def _analyze_csr(indices, indptr, n_rows):
     """One fused device pass over indptr and indices (the reference does six reductions with six host
     syncs, spmv_csr.py:404-427); returns CsrStats."""
     L = _lib.lib()
-    stats = torch.empty(8, dtype=torch.int64, device=indptr.device)
-    with _on_device(indptr.device):
+    dev = indptr.device
+    with _on_device(dev):
+        slot = _check_slot(dev)
+        if slot is not None:
+            rc = L.fsb_csr_check(_ITYPE[indices.dtype], _ITYPE[indptr.dtype], _ptr(indices), indptr.data_ptr(), n_rows,
+                                 indices.numel(), slot.work_ptr, slot.host_ptr, _stream_ptr(dev))
+            if rc != _lib.FSB_CAPTURING:
+                _lib.check(rc, "fsb_csr_check")
+                return slot.stats()
+        stats = torch.empty(8, dtype=torch.int64, device=dev)
         rc = L.fsb_csr_analyze(
             _ITYPE[indices.dtype], _ITYPE[indptr.dtype], _ptr(indices), indptr.data_ptr(),
-            n_rows, indices.numel(), stats.data_ptr(), _stream_ptr(indptr.device),
+            n_rows, indices.numel(), stats.data_ptr(), _stream_ptr(dev),
         )
     _lib.check(rc, "fsb_csr_analyze")
     return CsrStats(stats.cpu().tolist())

@@ -22,6 +22,7 @@ FSB_SPMV_PANEL = 3  # host-side tag only: the panel kernel has its own entry poi
 FSB_SPMM_AUTO, FSB_SPMM_PLAIN, FSB_SPMM_BULK = 0, 1, 2
 FSB_SPMM_ACCUMULATE = 16  # or-ed into the selector: C += A B
 FSB_SPMM_LONG_ROWS = 32   # or-ed into the selector: long rows are shared by a block
+FSB_OK, FSB_NOT_LAUNCHED, FSB_CAPTURING = 0, 1, 2
 FSB_CUDA_ERROR_BASE = 1000
 
 _ERRORS = {
@@ -53,6 +54,12 @@ SIGNATURES = {
     "fsb_spmv_tile_nnz": (_i32, [_i32, _i32]),
     "fsb_spmm_tile_nnz": (_i32, [_i32]),
     "fsb_csr_analyze": (_i32, [_i32, _i32, _vp, _vp, _i64, _i64, _vp, _vp]),
+    "fsb_csr_check": (_i32, [_i32, _i32, _vp, _vp, _i64, _i64, _vp, _vp, _vp]),
+    "fsb_spmv_csr_once": (_i32, [_i32, _i32, _i32, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _vp, _vp, _vp]),
+    "fsb_spmm_csr_once": (
+        _i32,
+        [_i32, _i32, _i32, _vp, _vp, _vp, _vp, _i64, _vp, _i64, _i64, _i64, _i64, _i64, _i64, _vp, _sz, _vp, _vp, _vp],
+    ),
     "fsb_csr_num_tiles": (_i64, [_i64, _i32]),
     "fsb_csr_tile_plan": (_i32, [_i32, _vp, _i64, _i64, _i32, _vp, _vp]),
     "fsb_spmv_csr_scratch_bytes": (_sz, [_i32, _i64, _i32]),

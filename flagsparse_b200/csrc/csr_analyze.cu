@@ -1,8 +1,15 @@
 // CSR structure analysis (one pass over indptr, one over indices) and the nnz-tile plan.
+#if defined(__x86_64__)
+#include <immintrin.h>
+#endif
+
+#include <atomic>
+
 #include "fsb_common.cuh"
 
 namespace fsb {
 
+constexpr int kCheckTicket = 8;      // behind the eight statistics in host memory
 enum { S_PTR_FIRST = 0, S_PTR_LAST, S_DECREASING, S_MIN_IDX, S_MAX_IDX, S_MAX_ROW, S_EMPTY, S_LONG };
 
 __global__ void stats_init_kernel(int64_t* s) {
@@ -42,10 +49,10 @@ __device__ __forceinline__ long long warp_sum(long long v) {
 // per thread and request; the statistics meet in shared memory, so that a block sends one atomic per statistic: one per warp, on six
 // words that every block of the device shares, used to take longer than the reading (3 M entries,
 // 250007 rows, 64-bit: two launches, 33 us; 10 us in this one; 2.1 M entries, 150001 rows: 30 us and 7 us).
+// Thread k < 6 of a block returns what the block found: longest row, decreasing and empty rows, long rows, smallest and largest index.
 template <typename I, typename P>
-__global__ void __launch_bounds__(256)
-csr_stats_kernel(const P* __restrict__ ptr, int64_t n_rows, int64_t long_len, const I* __restrict__ idx, int64_t nnz,
-                 int wide_loads, int64_t* __restrict__ s) {
+__device__ __forceinline__ long long csr_stats_block(const P* __restrict__ ptr, int64_t n_rows, int64_t long_len, const I* __restrict__ idx, int64_t nnz,
+                 int wide_loads) {
   constexpr int E = 16 / (int)sizeof(I);
   constexpr int U = 4;                       // requests in flight
   __shared__ long long s_part[8][6];
@@ -100,9 +107,10 @@ csr_stats_kernel(const P* __restrict__ ptr, int64_t n_rows, int64_t long_len, co
     s_part[w][4] = wide_mn; s_part[w][5] = wide_mx;
   }
   __syncthreads();
+  long long v = 0;
   if (threadIdx.x < 6) {
     const int k = threadIdx.x;
-    long long v = s_part[0][k];
+    v = s_part[0][k];
 #pragma unroll
     for (int j = 1; j < 8; ++j) {
       const long long u = s_part[j][k];
@@ -110,17 +118,68 @@ csr_stats_kernel(const P* __restrict__ ptr, int64_t n_rows, int64_t long_len, co
       else if (k == 4) v = u < v ? u : v;
       else v += u;
     }
-    if (k == 0 && v > 0) atomicMax(reinterpret_cast<long long*>(s + S_MAX_ROW), v);
-    if (k >= 1 && k <= 3 && v != 0)
-      atomicAdd(reinterpret_cast<unsigned long long*>(s + (k == 1 ? S_DECREASING : k == 2 ? S_EMPTY : S_LONG)),
-                (unsigned long long)v);
-    if (k == 4 && v != INT64_MAX) atomicMin(reinterpret_cast<long long*>(s + S_MIN_IDX), v);
-    if (k == 5 && v != INT64_MIN) atomicMax(reinterpret_cast<long long*>(s + S_MAX_IDX), v);
   }
+  return v;
+}
+
+template <typename I, typename P>
+__global__ void __launch_bounds__(256)
+csr_stats_kernel(const P* __restrict__ ptr, int64_t n_rows, int64_t long_len, const I* __restrict__ idx, int64_t nnz,
+                 int wide_loads, int64_t* __restrict__ s) {
+  const long long v = csr_stats_block<I, P>(ptr, n_rows, long_len, idx, nnz, wide_loads);
+  const int k = threadIdx.x;
+  if (k == 0 && v > 0) atomicMax(reinterpret_cast<long long*>(s + S_MAX_ROW), v);
+  if (k >= 1 && k <= 3 && v != 0)
+    atomicAdd(reinterpret_cast<unsigned long long*>(s + (k == 1 ? S_DECREASING : k == 2 ? S_EMPTY : S_LONG)),
+              (unsigned long long)v);
+  if (k == 4 && v != INT64_MAX) atomicMin(reinterpret_cast<long long*>(s + S_MIN_IDX), v);
+  if (k == 5 && v != INT64_MIN) atomicMax(reinterpret_cast<long long*>(s + S_MAX_IDX), v);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     s[S_PTR_FIRST] = (int64_t)ptr[0];
     s[S_PTR_LAST] = (int64_t)ptr[n_rows];
   }
+}
+
+// The same for a host that waits: the block that ends last writes the eight numbers to host memory (`out`, page-locked), then
+// `ticket` behind them, and leaves `work` zero, as it was found.  No launch to set up, no copy, no wait for the whole stream
+// (250007 rows, 3 M entries with 64-bit indices: 13.8 us; set-up, csr_stats_kernel and copy are 13.5 us on the GPU, but the host's
+// part of them and of the wait made a whole product of these arrays 62 us, 33 us now; 4096 rows of 16, 32 columns of B: 75 and 34).
+// work: 0 longest, 1 to 3 counts, 4 and 5 the extreme indices in an order that has zero for none, 6 blocks that are done.
+constexpr unsigned long long kSignBit = 1ull << 63;
+template <typename I, typename P>
+__global__ void __launch_bounds__(256)
+csr_check_kernel(const P* __restrict__ ptr, int64_t n_rows, int64_t long_len, const I* __restrict__ idx, int64_t nnz,
+                 int wide_loads, unsigned long long* __restrict__ work, volatile int64_t* out, int64_t ticket) {
+  const long long v = csr_stats_block<I, P>(ptr, n_rows, long_len, idx, nnz, wide_loads);
+  const int k = threadIdx.x;
+  if (k < 6) {
+    const unsigned long long bits = (unsigned long long)v;
+    if (k >= 1 && k <= 3) {
+      if (v != 0) atomicAdd(work + k, bits);
+    } else {
+      const unsigned long long w = k == 0 ? (v > 0 ? bits : 0) : k == 4 ? ~(bits ^ kSignBit) : bits ^ kSignBit;
+      if (w != 0) atomicMax(work + k, w);
+    }
+    __threadfence();
+  }
+  __syncthreads();
+  if (k != 0) return;
+  if (atomicAdd(work + 6, 1ull) != gridDim.x - 1) return;
+  __threadfence();
+  unsigned long long w[6];
+#pragma unroll
+  for (int j = 0; j < 6; ++j) w[j] = atomicExch(work + j, 0ull);
+  atomicExch(work + 6, 0ull);
+  out[S_PTR_FIRST] = (int64_t)ptr[0];
+  out[S_PTR_LAST] = (int64_t)ptr[n_rows];
+  out[S_DECREASING] = (int64_t)w[1];
+  out[S_MIN_IDX] = (int64_t)(~w[4] ^ kSignBit);
+  out[S_MAX_IDX] = (int64_t)(w[5] ^ kSignBit);
+  out[S_MAX_ROW] = (int64_t)w[0];
+  out[S_EMPTY] = (int64_t)w[2];
+  out[S_LONG] = (int64_t)w[3];
+  __threadfence_system();
+  out[kCheckTicket] = ticket;
 }
 
 // tile_row[t] = (first j with ptr[j] > t*T) - 1, i.e. the row that holds nnz number t*T
@@ -148,6 +207,75 @@ static int grid_for(int64_t n, int threads, int cap) {
   return (int)g;
 }
 
+static int stats_check_args(int itype, int ptype, const void* indices, const void* indptr, int64_t n_rows, int64_t nnz) {
+  if ((itype != FSB_I32 && itype != FSB_I64) || (ptype != FSB_I32 && ptype != FSB_I64)) return FSB_EINVAL;
+  if (n_rows < 0 || nnz < 0 || indptr == nullptr) return FSB_EINVAL;
+  if (nnz > 0 && indices == nullptr) return FSB_EINVAL;
+  if (!aligned_to(indptr, ptype == FSB_I32 ? 4 : 8) || !aligned_to(indices, itype == FSB_I32 ? 4 : 8)) return FSB_EALIGN;
+  if (n_rows >= INT32_MAX) return FSB_ERANGE;
+  return FSB_OK;
+}
+// "long" = more than 32x the mean row length (at least 64)
+static int64_t stats_long_len(int64_t n_rows, int64_t nnz) {
+  const int64_t mean_up = n_rows > 0 ? (nnz + n_rows - 1) / n_rows : 0;
+  return mean_up * 32 < 64 ? 64 : mean_up * 32;
+}
+static int stats_grid(int itype, int64_t n_rows, int64_t nnz) {
+  const int64_t per_thread = itype == FSB_I32 ? 16 : 8;      // four requests
+  const int64_t rows_blocks = (n_rows + 1023) / 1024, idx_blocks = (nnz + 256 * per_thread - 1) / (256 * per_thread);
+  return grid_for((rows_blocks > idx_blocks ? rows_blocks : idx_blocks) * 256, 256, 148 * 8);
+}
+
+int csr_check_launch(int itype, int ptype, const void* indices, const void* indptr, int64_t n_rows, int64_t nnz, void* work,
+                     int64_t* host, cudaStream_t stream) {
+  const int rc = stats_check_args(itype, ptype, indices, indptr, n_rows, nnz);
+  if (rc != FSB_OK) return rc;
+  if (work == nullptr || host == nullptr) return FSB_EINVAL;
+  if (!aligned_to(work, 8) || !aligned_to(host, 8)) return FSB_EALIGN;
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  const cudaError_t e = cudaStreamIsCapturing(stream, &capturing);
+  if (e != cudaSuccess) return cuda_rc(e);
+  if (capturing != cudaStreamCaptureStatusNone) return FSB_CAPTURING;        // nothing would run before the wait
+  const int64_t ticket = host[kCheckTicket] + 1;
+  const int wide_loads = nnz > 0 && aligned_to(indices, 16);
+#define FSB_CHECK_CSR(I_, P_)                                                                                        \
+  csr_check_kernel<I_, P_><<<stats_grid(itype, n_rows, nnz), 256, 0, stream>>>(                                      \
+      (const P_*)indptr, n_rows, stats_long_len(n_rows, nnz), (const I_*)indices, nnz, wide_loads,                   \
+      (unsigned long long*)work, host, ticket)
+  if (itype == FSB_I32) {
+    if (ptype == FSB_I32) FSB_CHECK_CSR(int32_t, int32_t); else FSB_CHECK_CSR(int32_t, int64_t);
+  } else {
+    if (ptype == FSB_I32) FSB_CHECK_CSR(int64_t, int32_t); else FSB_CHECK_CSR(int64_t, int64_t);
+  }
+#undef FSB_CHECK_CSR
+  FSB_RETURN_IF_LAUNCH_FAILED();
+  host[kCheckTicket + 1] = ticket;     // what the wait looks for
+  return FSB_OK;
+}
+
+int csr_check_wait(const int64_t* host, cudaStream_t stream) {
+  const volatile int64_t* seen = host + kCheckTicket;
+  const int64_t ticket = host[kCheckTicket + 1];
+  for (int i = 0; i < (1 << 18) && *seen != ticket; ++i) {     // about 10 ms
+#if defined(__x86_64__)
+    _mm_pause();
+#endif
+  }
+  if (*seen != ticket) {               // a long queue in front of it, or a failure: the runtime tells
+    const cudaError_t e = cudaStreamSynchronize(stream);
+    if (e != cudaSuccess) return cuda_rc(e);
+    if (*seen != ticket) return FSB_CUDA_ERROR_BASE + (int)cudaErrorUnknown;
+  }
+  std::atomic_thread_fence(std::memory_order_acquire);
+  return FSB_OK;
+}
+
+bool csr_check_passed(const int64_t* host, int64_t n_cols, int64_t nnz) {
+  return host[S_PTR_FIRST] == 0 && host[S_PTR_LAST] == nnz && host[S_DECREASING] == 0 &&
+         (nnz == 0 || (host[S_MIN_IDX] >= 0 && host[S_MAX_IDX] < n_cols));
+}
+int64_t csr_check_longest(const int64_t* host) { return host[S_MAX_ROW]; }
+
 }  // namespace fsb
 
 using namespace fsb;
@@ -157,22 +285,15 @@ extern "C" int fsb_version(void) { return FSB_VERSION; }
 extern "C" int fsb_csr_analyze(int itype, int ptype, const void* indices, const void* indptr,
                                int64_t n_rows, int64_t nnz, int64_t* stats, void* stream_) {
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
-  if ((itype != FSB_I32 && itype != FSB_I64) || (ptype != FSB_I32 && ptype != FSB_I64)) return FSB_EINVAL;
-  if (n_rows < 0 || nnz < 0 || stats == nullptr || indptr == nullptr) return FSB_EINVAL;
-  if (nnz > 0 && indices == nullptr) return FSB_EINVAL;
-  if (!aligned_to(indptr, ptype == FSB_I32 ? 4 : 8) || !aligned_to(indices, itype == FSB_I32 ? 4 : 8) ||
-      !aligned_to(stats, 8))
-    return FSB_EALIGN;
-  if (n_rows >= INT32_MAX) return FSB_ERANGE;
+  const int rc = stats_check_args(itype, ptype, indices, indptr, n_rows, nnz);
+  if (rc != FSB_OK) return rc;
+  if (stats == nullptr) return FSB_EINVAL;
+  if (!aligned_to(stats, 8)) return FSB_EALIGN;
   stats_init_kernel<<<1, 1, 0, stream>>>(stats);
   FSB_RETURN_IF_LAUNCH_FAILED();
-  // "long" = more than 32x the mean row length (at least 64)
-  int64_t mean_up = n_rows > 0 ? (nnz + n_rows - 1) / n_rows : 0;
-  int64_t long_len = mean_up * 32 < 64 ? 64 : mean_up * 32;
+  const int64_t long_len = stats_long_len(n_rows, nnz);
   const int wide_loads = nnz > 0 && aligned_to(indices, 16);
-  const int64_t per_thread = itype == FSB_I32 ? 16 : 8;      // four requests
-  const int64_t rows_blocks = (n_rows + 1023) / 1024, idx_blocks = (nnz + 256 * per_thread - 1) / (256 * per_thread);
-  const int g = grid_for((rows_blocks > idx_blocks ? rows_blocks : idx_blocks) * 256, 256, 148 * 8);
+  const int g = stats_grid(itype, n_rows, nnz);
 #define FSB_STATS(I_, P_)                                                                                           \
   csr_stats_kernel<I_, P_><<<g, 256, 0, stream>>>((const P_*)indptr, n_rows, long_len, (const I_*)indices, nnz,     \
                                                   wide_loads, stats)
@@ -184,6 +305,13 @@ extern "C" int fsb_csr_analyze(int itype, int ptype, const void* indices, const 
 #undef FSB_STATS
   FSB_RETURN_IF_LAUNCH_FAILED();
   return FSB_OK;
+}
+
+extern "C" int fsb_csr_check(int itype, int ptype, const void* indices, const void* indptr, int64_t n_rows, int64_t nnz, void* work,
+                             int64_t* host, void* stream_) {
+  const cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+  const int rc = csr_check_launch(itype, ptype, indices, indptr, n_rows, nnz, work, host, stream);
+  return rc != FSB_OK ? rc : csr_check_wait(host, stream);
 }
 
 extern "C" int64_t fsb_csr_num_tiles(int64_t nnz, int tile_nnz) {

@@ -26,6 +26,14 @@ inline int sm_count(int* out) {
   return cuda_rc(e);
 }
 
+// ---- checks of CSR arrays that the host waits for (csr_analyze.cu) ------------------------------------
+// launch, then wait; `host` (page-locked) holds the statistics of fsb_csr_analyze from then on
+int csr_check_launch(int itype, int ptype, const void* indices, const void* indptr, int64_t n_rows, int64_t nnz, void* work,
+                     int64_t* host, cudaStream_t stream);
+int csr_check_wait(const int64_t* host, cudaStream_t stream);
+bool csr_check_passed(const int64_t* host, int64_t n_cols, int64_t nnz);
+int64_t csr_check_longest(const int64_t* host);
+
 // ---- the checking build: entry points walk their index arrays first (bounds_check.cu) ----------------
 #ifdef FSB_BOUNDS_CHECK
 int check_csr(int itype, int ptype, const void* indices, const void* indptr, int64_t n_rows, int64_t n_cols,

@@ -686,3 +686,26 @@ extern "C" int fsb_spmm_csr_stored(int vtype, int ptype, const void* data, const
                   FSB_SPMM_PLAIN | (long_rows ? FSB_SPMM_LONG_ROWS : 0), nullptr, true, scratch, scratch_bytes, nullptr,
                   static_cast<cudaStream_t>(stream_));
 }
+
+extern "C" int fsb_spmm_csr_once(int vtype, int itype, int ptype, const void* data, const void* indices, const void* indptr,
+                                 const void* B, int64_t ldb, void* C, int64_t ldc, int64_t n_rows, int64_t n_cols, int64_t n_dense,
+                                 int64_t nnz, int64_t long_row, void* scratch, size_t scratch_bytes, void* work, int64_t* host,
+                                 void* stream_) {
+  const cudaStream_t st = static_cast<cudaStream_t>(stream_);
+  if (vtype < FSB_F32 || vtype > FSB_C128 || n_dense < 0 || nnz <= 0) return FSB_EINVAL;
+  const size_t parts = spmm_scratch_bytes(vtype, nnz, n_dense);
+  if (scratch == nullptr) return FSB_EINVAL;
+  if (scratch_bytes < parts + spmm_plan_bytes(nnz)) return FSB_ESCRATCH;
+  if (!aligned_to(scratch, 16)) return FSB_EALIGN;
+  int rc = csr_check_launch(itype, ptype, indices, indptr, n_rows, nnz, work, host, st);
+  if (rc != FSB_OK) return rc;
+  // the plan needs no checked row pointer: it reads n_rows + 1 numbers and writes its own array, whatever they are
+  int32_t* tile_row = (int32_t*)((char*)scratch + parts);
+  rc = fsb_csr_tile_plan(ptype, indptr, n_rows, nnz, kMmTile, tile_row, stream_);
+  const int waited = csr_check_wait(host, st);
+  if (rc != FSB_OK || waited != FSB_OK) return rc != FSB_OK ? rc : waited;
+  if (!csr_check_passed(host, n_cols, nnz)) return FSB_NOT_LAUNCHED;
+  const int algo = FSB_SPMM_PLAIN | (csr_check_longest(host) > long_row ? FSB_SPMM_LONG_ROWS : 0);
+  return spmm_run(vtype, itype, ptype, data, indices, indptr, B, ldb, C, ldc, n_rows, n_cols, n_dense, nnz, algo, tile_row, false,
+                  scratch, parts, nullptr, st);
+}

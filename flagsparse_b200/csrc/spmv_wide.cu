@@ -591,3 +591,21 @@ extern "C" int fsb_spmv_csr_stored(int vtype, int ptype, const void* data, const
   }
 #undef FSB_STORED_TYPE
 }
+
+// Check and product of arrays that are used once, whatever the value type.
+extern "C" int fsb_spmv_csr_once(int vtype, int itype, int ptype, const void* data, const void* indices, const void* indptr,
+                                 const void* x, void* y, int64_t n_rows, int64_t n_cols, int64_t nnz, int64_t longest, void* work,
+                                 int64_t* host, void* stream_) {
+  cudaStream_t st = static_cast<cudaStream_t>(stream_);
+  const bool stored = vtype != FSB_F32 && vtype != FSB_F64;
+  if (stored && itype != FSB_I32) return FSB_EINVAL;
+  int rc = csr_check_launch(itype, ptype, indices, indptr, n_rows, nnz, work, host, st);
+  if (rc == FSB_OK) rc = csr_check_wait(host, st);
+  if (rc != FSB_OK) return rc;
+  if (!csr_check_passed(host, n_cols, nnz) || csr_check_longest(host) > longest) return FSB_NOT_LAUNCHED;
+  if (stored)
+    return fsb_spmv_csr_stored(vtype, ptype, data, (const int32_t*)indices, indptr, x, y, n_rows, n_cols, nnz, nullptr, nullptr, 0,
+                               stream_);
+  return fsb_spmv_csr(vtype, itype, ptype, data, indices, indptr, x, y, n_rows, n_cols, nnz, FSB_SPMV_VECTOR, 0, nullptr, nullptr, 0,
+                      stream_);
+}

@@ -20,6 +20,7 @@ from ._common import (
     _ITYPE,
     _VTYPE,
     _analyze_csr,
+    _check_slot,
     _check_value_dtype,
     _on_device,
     _ptr,
@@ -391,11 +392,16 @@ def _prepare_spmm(data, indices, indptr, shape, once, known=None):
     return prepared
 
 
-def _shares_long_rows(max_row_nnz, n_dense, element_size):
-    """Whether a product of this width gets FSB_SPMM_LONG_ROWS."""
+def _long_row(n_dense, element_size):
+    """Longest row up to which a product of this width does without FSB_SPMM_LONG_ROWS."""
     vw = min(16 // element_size, n_dense & -n_dense)      # widest access that divides a row of B
     several = n_dense > 32 * vw and vw * element_size < 16
-    return max_row_nnz > (LONG_ROW_NNZ_SEVERAL if several else LONG_ROW_NNZ)
+    return LONG_ROW_NNZ_SEVERAL if several else LONG_ROW_NNZ
+
+
+def _shares_long_rows(max_row_nnz, n_dense, element_size):
+    """Whether a product of this width gets FSB_SPMM_LONG_ROWS."""
+    return max_row_nnz > _long_row(n_dense, element_size)
 
 
 def _spmm_launch(prepared, B, C):
@@ -494,6 +500,53 @@ def _run_spmm(prepared, B, out, return_time):
     return C
 
 
+_SPMM_SWITCHES = ("FSB_SPMM_ALGO", "FSB_SPMM_PANELS", "FSB_SPMM_PANEL_MB")
+
+
+def _spmm_once(data, indices, indptr, B, shape):
+    """C = A B straight from the arrays, where every argument is as the kernels read it, by one call that checks the arrays, plans
+    the tiles, waits for the answer and enqueues the product.  None where that was not done: the arguments are for the general
+    path, which also finds the words for what is wrong with them."""
+    if not (isinstance(data, torch.Tensor) and isinstance(indices, torch.Tensor) and isinstance(indptr, torch.Tensor)):
+        return None
+    dev, dtype = data.device, data.dtype
+    if dev.type != "cuda" or indices.device != dev or indptr.device != dev or B.device != dev or B.dtype != dtype:
+        return None
+    vt, it, pt = _VTYPE.get(dtype), _ITYPE.get(indices.dtype), _ITYPE.get(indptr.dtype)
+    if vt is None:
+        vt = _STORED_VTYPE.get(dtype)
+        if it != _lib.FSB_I32:
+            return None
+    elif any(name in os.environ for name in _SPMM_SWITCHES):
+        return None
+    if vt is None or it is None or pt is None or data.ndim != 1 or indices.ndim != 1 or indptr.ndim != 1 or len(shape) != 2:
+        return None
+    n_rows, n_cols, nnz, n_dense = int(shape[0]), int(shape[1]), data.numel(), int(B.shape[1])
+    if not (0 < nnz == indices.numel() and 0 < n_rows == indptr.numel() - 1 and B.shape[0] == n_cols < _INDEX_LIMIT_INT32
+            and n_dense > 0):
+        return None
+    if not (data.is_contiguous() and indices.is_contiguous() and indptr.is_contiguous() and B.is_contiguous()):
+        return None
+    if data.is_neg() or B.is_neg() or data.is_conj() or B.is_conj():
+        return None
+    L = _lib.lib()
+    with _on_device(dev):
+        slot = _check_slot(dev)
+        if slot is None:
+            return None
+        C = torch.empty((n_rows, n_dense), dtype=dtype, device=dev)
+        scratch = torch.empty(int(L.fsb_spmm_stored_scratch_bytes(vt, nnz, n_dense)), dtype=torch.uint8, device=dev)
+        rc = L.fsb_spmm_csr_once(
+            vt, it, pt, data.data_ptr(), indices.data_ptr(), indptr.data_ptr(), B.data_ptr(), n_dense, C.data_ptr(), n_dense, n_rows,
+            n_cols, n_dense, nnz, _long_row(n_dense, data.element_size()), scratch.data_ptr(), scratch.numel(), slot.work_ptr,
+            slot.host_ptr, _stream_ptr(dev))
+    if rc == _lib.FSB_OK:
+        return C
+    if rc not in (_lib.FSB_NOT_LAUNCHED, _lib.FSB_CAPTURING):
+        _lib.check(rc, "fsb_spmm_csr_once")
+    return None
+
+
 def flagsparse_spmm_csr(data, indices, indptr, B, shape, block_n=None, block_nnz=None, max_segments=None,
                         out=None, return_time=False):
     """CSR SpMM: C = A @ B (reference: spmm_csr.py:1057-1126, same arguments and defaults).
@@ -511,6 +564,10 @@ def flagsparse_spmm_csr(data, indices, indptr, B, shape, block_n=None, block_nnz
         raise ValueError("max_segments must be positive when provided")
     if B.ndim != 2:
         raise ValueError("B must be a 2D dense tensor")
+    if out is None and not return_time and block_n is None and block_nnz is None and max_segments is None:
+        C = _spmm_once(data, indices, indptr, B, shape)
+        if C is not None:
+            return C
     prepared = _prepare_spmm(data, indices, indptr, shape, once=True)
     B = _check_spmm_dense(B, prepared.data, prepared.n_cols)
     n_dense_cols = int(B.shape[1])

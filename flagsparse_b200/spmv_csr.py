@@ -19,6 +19,7 @@ from ._common import (
     _ITYPE,
     _VTYPE,
     _analyze_csr,
+    _check_slot,
     _check_value_dtype,
     _on_device,
     _ptr,
@@ -76,16 +77,14 @@ def _select_spmv_algo(n_rows, nnz, max_row_nnz, element_size=4):
     forced = os.environ.get("FSB_SPMV_ALGO", "").strip().lower()
     if forced in ("vector", "stream", "panel"):
         return _ALGO_NAMES[forced]
-    if max_row_nnz > _VECTOR_MAX_ROW_NNZ:
-        return _lib.FSB_SPMV_STREAM
-    mean = nnz / max(n_rows, 1)
-    if nnz < _STREAM_MIN_NNZ:
-        # one launch against two, until the longest row takes its lanes longer than that
-        even = max_row_nnz <= _UNIFORM_ROW_FACTOR * mean + _SMALL_ROW_SLACK[element_size]
-        return _lib.FSB_SPMV_VECTOR if even else _lib.FSB_SPMV_STREAM
-    if max_row_nnz <= _UNIFORM_ROW_FACTOR * mean + _UNIFORM_ROW_SLACK:
-        return _lib.FSB_SPMV_VECTOR
-    return _lib.FSB_SPMV_STREAM
+    return _lib.FSB_SPMV_VECTOR if max_row_nnz <= _longest_even(n_rows, nnz, element_size) else _lib.FSB_SPMV_STREAM
+
+
+def _longest_even(n_rows, nnz, element_size):
+    """Longest row of a float32 / float64 matrix up to which its rows are even: one launch of the kernels for such rows against two
+    of the stream kernel, until the longest row takes its lanes longer than that."""
+    slack = _SMALL_ROW_SLACK[element_size] if nnz < _STREAM_MIN_NNZ else _UNIFORM_ROW_SLACK
+    return min(_VECTOR_MAX_ROW_NNZ, int(_UNIFORM_ROW_FACTOR * (nnz / max(n_rows, 1)) + slack))
 
 
 # Longest row from which the tiled kernel for float16 / bfloat16 / complex values is taken.  A row of n entries takes its L
@@ -104,16 +103,21 @@ _UNEVEN_PER_LANE = 72
 _UNEVEN_ENTRIES = {8: 35000, 16: 18000}
 
 
-def _uneven_rows(n_rows, nnz, max_row_nnz, element_size):
-    """Whether the longest row leaves the lanes-per-row kernel for float16 / bfloat16 / complex values waiting for it."""
+def _longest_even_stored(n_rows, nnz, element_size):
+    """The same for float16 / bfloat16 / complex values."""
     mean = nnz / max(n_rows, 1)
     line = _UNIFORM_ROW_FACTOR * mean + _UNIFORM_ROW_SLACK
     if element_size not in _UNEVEN_ENTRIES:
-        return max_row_nnz > max(line, _UNEVEN_MIN)
+        return int(max(line, _UNEVEN_MIN))
     lanes = 2                            # as stored_launch in csrc/spmv_wide.cu gives them to a row
     while lanes < 32 and 6 * lanes < int(mean) + 3:
         lanes *= 2
-    return max_row_nnz > max(line, _UNEVEN_PER_LANE * lanes, nnz / _UNEVEN_ENTRIES[element_size] * lanes / 4)
+    return int(max(line, _UNEVEN_PER_LANE * lanes, nnz / _UNEVEN_ENTRIES[element_size] * lanes / 4))
+
+
+def _uneven_rows(n_rows, nnz, max_row_nnz, element_size):
+    """Whether the longest row leaves the lanes-per-row kernel for float16 / bfloat16 / complex values waiting for it."""
+    return max_row_nnz > _longest_even_stored(n_rows, nnz, element_size)
 
 
 class PreparedCsrSpmv:
@@ -181,11 +185,11 @@ class PreparedCsrSpmv:
             word.check()
 
 
-def _prepare_spmv_csr_matrix(data, indices, indptr, shape, narrow=True):
+def _prepare_spmv_csr_matrix(data, indices, indptr, shape, narrow=True, stats=None):
     """Validate and normalise the CSR arrays; same checks, order and exception types as the reference's
     function of this name (spmv_csr.py:379-436).  narrow=False leaves the indices of float32 / float64 matrices at their
     width (a one-shot product reads them once: the kernels take either, and a pass that narrows them moves more than it
-    saves).  Returns (data, kernel_indices, kernel_indptr, n_rows,
+    saves).  stats: what the analysis of these very arrays gave.  Returns (data, kernel_indices, kernel_indptr, n_rows,
     n_cols, stats)."""
     if not (torch.is_tensor(data) and torch.is_tensor(indices) and torch.is_tensor(indptr)):
         raise TypeError("data, indices and indptr have to be torch.Tensor objects")
@@ -210,7 +214,8 @@ def _prepare_spmv_csr_matrix(data, indices, indptr, shape, narrow=True):
         indptr = indptr.to(torch.int64)
 
     nnz = data.numel()
-    stats = _analyze_csr(indices, indptr, n_rows)
+    if stats is None:
+        stats = _analyze_csr(indices, indptr, n_rows)
     if stats.ptr_first != 0:
         raise ValueError("indptr[0] is not 0")
     if stats.ptr_last != nnz:
@@ -283,13 +288,13 @@ def _split_long_rows(data, kernel_indices, kernel_indptr, n_rows, n_cols, shape,
 
 
 def _prepare_spmv_csr(data, indices, indptr, shape, block_nnz, max_segments, reuse_expected, allow_split=True,
-                      known=None):
+                      known=None, stats=None):
     """known: the statistics of arrays that were made here (contiguous, 32-bit column ids): nothing is left to check.
     reuse_expected=False (a one-shot product) skips the panel regrouping, which costs about as much as a
     hundred products and only pays when the prepared matrix is used again."""
     if known is None:
         data, kernel_indices, kernel_indptr, n_rows, n_cols, stats = _prepare_spmv_csr_matrix(
-            data, indices, indptr, shape, narrow=reuse_expected
+            data, indices, indptr, shape, narrow=reuse_expected, stats=stats
         )
     else:
         kernel_indices, kernel_indptr, (n_rows, n_cols), stats = indices, indptr, shape, known
@@ -419,6 +424,55 @@ def _spmv_launch_stored(prepared, x, y):
     _lib.check(rc, "fsb_spmv_csr_stored")
 
 
+def _spmv_once(data, indices, indptr, x, shape, out):
+    """(y, stats): the product straight from the arrays, where every argument is as the kernels read it, by one call that checks the
+    arrays, waits for the answer and enqueues the kernel for even rows.  y is None where that was not done: the arguments are for
+    the general path, which also finds the words for what is wrong with them (stats None: nothing was looked at)."""
+    none = None, None
+    if not (isinstance(data, torch.Tensor) and isinstance(indices, torch.Tensor) and isinstance(indptr, torch.Tensor)
+            and isinstance(x, torch.Tensor)):
+        return none
+    dev, dtype = data.device, data.dtype
+    if dev.type != "cuda" or indices.device != dev or indptr.device != dev or x.device != dev or x.dtype != dtype:
+        return none
+    vt, it, pt = _VTYPE.get(dtype), _ITYPE.get(indices.dtype), _ITYPE.get(indptr.dtype)
+    stored = vt is None
+    if stored:
+        vt = _WIDE_VTYPE.get(dtype)
+        if out is not None or it != _lib.FSB_I32:
+            return none
+    elif "FSB_SPMV_ALGO" in os.environ or "FSB_SPMV_TUNING" in os.environ:
+        return none
+    if vt is None or it is None or pt is None or data.ndim != 1 or indices.ndim != 1 or indptr.ndim != 1 or x.ndim != 1:
+        return none
+    n_rows, n_cols, nnz = int(shape[0]), int(shape[1]), data.numel()
+    if not (0 < nnz == indices.numel() and 0 < n_rows == indptr.numel() - 1 and x.numel() == n_cols < _INDEX_LIMIT_INT32):
+        return none
+    if not (data.is_contiguous() and indices.is_contiguous() and indptr.is_contiguous() and x.is_contiguous()):
+        return none
+    if data.is_neg() or x.is_neg() or data.is_conj() or x.is_conj():
+        return none
+    if out is not None and not (out.device == dev and out.shape == (n_rows,) and out.dtype == dtype and out.is_contiguous()
+                                and not out.is_neg()):
+        return none
+    L = _lib.lib()
+    with _on_device(dev):
+        slot = _check_slot(dev)
+        if slot is None:
+            return none
+        y = out if out is not None else torch.empty(n_rows, dtype=dtype, device=dev)
+        longest = (_longest_even_stored if stored else _longest_even)(n_rows, nnz, data.element_size())
+        rc = L.fsb_spmv_csr_once(vt, it, pt, data.data_ptr(), indices.data_ptr(), indptr.data_ptr(), x.data_ptr(), y.data_ptr(),
+                                 n_rows, n_cols, nnz, longest, slot.work_ptr, slot.host_ptr, _stream_ptr(dev))
+    if rc == _lib.FSB_OK:
+        return y, None
+    if rc == _lib.FSB_NOT_LAUNCHED:
+        return None, slot.stats()
+    if rc != _lib.FSB_CAPTURING:
+        _lib.check(rc, "fsb_spmv_csr_once")
+    return none
+
+
 def flagsparse_spmv_csr(data=None, indices=None, indptr=None, x=None, shape=None, block_nnz=256,
                         max_segments=None, out=None, return_time=False, use_opt=False, prepared=None):
     """CSR SpMV: y = A @ x (reference: spmv_csr.py:557-610, same arguments and defaults).
@@ -431,7 +485,12 @@ def flagsparse_spmv_csr(data=None, indices=None, indptr=None, x=None, shape=None
     if prepared is None:
         if any(arg is None for arg in (data, indices, indptr, shape)):
             raise ValueError("data, indices, indptr, and shape are required when prepared is not provided")
-        prepared = _prepare_spmv_csr(data, indices, indptr, shape, block_nnz, max_segments, reuse_expected=False)
+        stats = None
+        if not return_time and block_nnz == 256 and max_segments is None:
+            y, stats = _spmv_once(data, indices, indptr, x, shape, out)
+            if y is not None:
+                return y
+        prepared = _prepare_spmv_csr(data, indices, indptr, shape, block_nnz, max_segments, reuse_expected=False, stats=stats)
     x = _validate_spmv_x(x, prepared)
     dev = prepared.data.device
     dtype = prepared.data.dtype

@@ -43,6 +43,8 @@ extern "C" {
 
 /* error codes (negative) */
 #define FSB_OK 0
+#define FSB_NOT_LAUNCHED 1   /* fsb_*_once: checked, but the product is left to the caller (see there)          */
+#define FSB_CAPTURING 2      /* a call that waits for the GPU, on a stream that is being captured: nothing ran  */
 #define FSB_EINVAL (-1)      /* bad enum / negative size / null pointer where one is required */
 #define FSB_ERANGE (-2)      /* n_rows, n_cols or a tile count outside the supported range   */
 #define FSB_EALIGN (-3)      /* pointer not aligned to its element size                      */
@@ -83,6 +85,28 @@ int fsb_spmm_tile_nnz(int vtype);
  */
 int fsb_csr_analyze(int itype, int ptype, const void* indices, const void* indptr, int64_t n_rows,
                     int64_t nnz, int64_t* stats, void* stream);
+
+/*
+ * The same eight numbers for a host that waits for them.  work: 7 uint64 on the device, zero before the first call and left so by
+ * every call; host: 10 int64 of page-locked memory, zero before the first call: [0..7] the statistics, [8] and [9] tickets of the
+ * last run and the last call.  Both belong to one call at a time (one pair per thread).  Returns when the numbers are there;
+ * FSB_CAPTURING, with nothing enqueued, while the stream is being captured.
+ */
+int fsb_csr_check(int itype, int ptype, const void* indices, const void* indptr, int64_t n_rows, int64_t nnz, void* work,
+                  int64_t* host, void* stream);
+
+/*
+ * Check and product of CSR arrays that are used once (fsb_csr_check, then the product of checked arrays): y = A x by the kernels for
+ * rows of about equal length, C = A B.  Returns FSB_OK with the product enqueued, FSB_CAPTURING, or FSB_NOT_LAUNCHED without the
+ * product: the arrays are not a CSR matrix of this shape (host tells why), or, y = A x, a row has more than `longest` entries.  All value types; other than float32 / float64 with 32-bit indices.  long_row: longest row up to
+ * which rows are not shared by a block (FSB_SPMM_LONG_ROWS); scratch as for fsb_spmm_csr_stored.
+ */
+int fsb_spmv_csr_once(int vtype, int itype, int ptype, const void* data, const void* indices, const void* indptr, const void* x,
+                      void* y, int64_t n_rows, int64_t n_cols, int64_t nnz, int64_t longest, void* work, int64_t* host,
+                      void* stream);
+int fsb_spmm_csr_once(int vtype, int itype, int ptype, const void* data, const void* indices, const void* indptr, const void* B,
+                      int64_t ldb, void* C, int64_t ldc, int64_t n_rows, int64_t n_cols, int64_t n_dense, int64_t nnz,
+                      int64_t long_row, void* scratch, size_t scratch_bytes, void* work, int64_t* host, void* stream);
 
 /*
  * Tile plan: tile_row[t] for t = 0..n_tiles, n_tiles = ceil(nnz / tile_nnz), int32 on the device.
