@@ -127,6 +127,10 @@ struct MmComplex {
 template <> struct MmOps<float2> : MmComplex<float2> {};
 template <> struct MmOps<double2> : MmComplex<double2> {};
 
+template <typename S> struct RealOf { typedef S Out; typedef typename MmOps<S>::Acc Acc; static constexpr int parts = 1; };
+template <> struct RealOf<float2> { typedef float Out; typedef float Acc; static constexpr int parts = 2; };
+template <> struct RealOf<double2> { typedef double Out; typedef double Acc; static constexpr int parts = 2; };
+
 template <int BYTES> struct RawVec;
 template <> struct RawVec<2> { typedef unsigned short type; };
 template <> struct RawVec<4> { typedef unsigned int type; };
@@ -231,6 +235,17 @@ spmm_tile_kernel(const S* __restrict__ data, const I* __restrict__ idx, const vo
   const int width = LR * NC * VW;                          // columns of this column tile
   const int col0 = (int)blockIdx.y * width + lane * VW;    // first column of access 0; access i is LR * VW further on
 
+  // Row c of B: one wide multiply-add from a stride in bytes, and one for the high word, where several accesses per lane or small
+  // ones leave the arithmetic in the way of the gathers (float32, 262144 rows of 16, 33 columns: 102 us, from the stride in elements
+  // 112 us; float16, 200003 rows of 20, 70 columns: 132 / 146; complex64, 32 columns: 81 / 86).  float64 and 16-byte gathers of
+  // one access lose registers to it (float64, 75 columns: 179 / 161; float32, 64 columns: 256 / 233).
+  constexpr bool FROM_BYTES = RealOf<S>::parts == 2 || (sizeof(S) <= 4 && VW * (int)sizeof(S) < 16);
+  const char* B0 = reinterpret_cast<const char*>(B + col0);
+  const uint64_t row_bytes = (uint64_t)ldb * sizeof(S);
+  auto row_of = [&](I c) {
+    if constexpr (FROM_BYTES) return reinterpret_cast<const S*>(B0 + (uint64_t)(uint32_t)c * row_bytes);
+    else return B + (int64_t)c * ldb + col0;
+  };
   auto clear = [](A (&acc)[NC][VW]) {
 #pragma unroll
     for (int i = 0; i < NC; ++i)
@@ -240,7 +255,7 @@ spmm_tile_kernel(const S* __restrict__ data, const I* __restrict__ idx, const vo
   constexpr int CHAINS = Ops::chains;
   // acc += value * row of B for entry p
   auto one = [&](int p, A (&acc)[NC][VW]) {
-    const S* row = B + (int64_t)s_idx[p] * ldb + col0;
+    const S* row = row_of(s_idx[p]);
     const S v = s_val[p];
 #pragma unroll
     for (int i = 0; i < NC; ++i) {
@@ -260,7 +275,7 @@ spmm_tile_kernel(const S* __restrict__ data, const I* __restrict__ idx, const vo
       Pack<S, VW> b[U][NC];
 #pragma unroll
       for (int u = 0; u < U; ++u) {
-        const S* row = B + (int64_t)s_idx[p + u] * ldb + col0;
+        const S* row = row_of(s_idx[p + u]);
 #pragma unroll
         for (int i = 0; i < NC; ++i)
           if (i == 0 || col0 + i * LR * VW < n_dense) b[u][i].gather(row + i * LR * VW);
@@ -400,7 +415,8 @@ spmm_tile_kernel(const S* __restrict__ data, const I* __restrict__ idx, const vo
   }
 }
 
-// one thread per (tile t >= 1, column): finish the row that started before tile t and ends in it.  R: real type of the
+// one thread per (tile t >= 1, column): finish the row that started before tile t and ends in it (bfloat16, 4 M entries in rows of
+// Zipf lengths up to 49 tiles, 128 columns: 20.5 us with every sum compensated, 9.7 us; float64, 262144 such rows, 64 columns: 26 us with one sum, 19 us).  R: real type of the
 // partial sums, D: real type of C (complex columns are taken as pairs of real ones)
 template <typename R, typename D, typename P>
 __global__ void __launch_bounds__(kMmThreads)
@@ -418,7 +434,28 @@ spmm_fixup_kernel(const P* __restrict__ ptr, const int32_t* __restrict__ tile_ro
   if (p >= (t << log2_tile)) return;
   const int64_t t0 = p >> log2_tile;
   double sum = (double)head[t * n_dense + j], comp = 0.0;
-  for (int64_t u = t0; u < t; ++u) comp_add(sum, comp, (double)carry[u * n_dense + j]);
+  if constexpr (sizeof(R) == 4) {
+    for (int64_t u = t0; u < t; ++u) carry_add<R>(sum, comp, (double)carry[u * n_dense + j]);
+  } else {
+    // four compensated sums in turn, or each would wait for the one before it
+    double sums[4] = {sum, 0.0, 0.0, 0.0}, comps[4] = {0.0, 0.0, 0.0, 0.0};
+    int64_t u = t0;
+    for (; u + 8 <= t; u += 8) {
+      R v[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] = __ldg(carry + (u + k) * n_dense + j);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) comp_add(sums[k & 3], comps[k & 3], (double)v[k]);
+    }
+    for (; u < t; ++u) comp_add(sums[0], comps[0], (double)__ldg(carry + u * n_dense + j));
+#pragma unroll
+    for (int k = 1; k < 4; ++k) {
+      comp_add(sums[0], comps[0], sums[k]);
+      comps[0] += comp_term(sums[k], comps[k]);
+    }
+    sum = sums[0];
+    comp = comps[0];
+  }
   D* dst = C + (int64_t)ra * ldc + j;
   comp = comp_term(sum, comp);
   // rounded to the accumulator type first, like every other row
@@ -448,10 +485,6 @@ struct SpmmArgs {
   int32_t* status;
   cudaStream_t st;
 };
-
-template <typename S> struct RealOf { typedef S Out; typedef typename MmOps<S>::Acc Acc; static constexpr int parts = 1; };
-template <> struct RealOf<float2> { typedef float Out; typedef float Acc; static constexpr int parts = 2; };
-template <> struct RealOf<double2> { typedef double Out; typedef double Acc; static constexpr int parts = 2; };
 
 static int pow2_at_least(int v) {
   int p = 1;

@@ -108,3 +108,16 @@ def test_long_row_hint_keeps_the_accumulating_form(cuda, fsb_lib, monkeypatch):
     prep = fs.prepare_spmm_csr_opt(vals.to(cuda), torch.from_numpy(i).to(cuda), torch.from_numpy(p).to(cuda),
                                    (len(p) - 1, n_cols))
     _check(fs.flagsparse_spmm_csr_opt(B=B.to(cuda), prepared=prep), vals, i, p, n_cols, B, torch.float32)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64, torch.bfloat16, torch.complex128], ids=str)
+def test_spmm_rows_over_many_tiles(cuda, fsb_lib, dtype):
+    """Rows that cross 7 to 25 tiles of 1024, where their partial sums are taken eight at a time and one by one."""
+    n_cols = 30000
+    for lens in ([3, 7 * 1024, 5, 8 * 1024, 1, 9 * 1024 + 1, 0, 16 * 1024], [17 * 1024 - 3, 2, 25 * 1024, 40]):
+        _, i, p = handmade_csr(3, lens, n_cols)
+        vals = _values(int(p[-1]), dtype, 4)
+        for n_dense in (1, 33, 40):
+            B = _values((n_cols, n_dense), dtype, n_dense)
+            C = fs.flagsparse_spmm_csr(vals.to(cuda), torch.from_numpy(i).to(cuda), torch.from_numpy(p).to(cuda), B.to(cuda), (len(p) - 1, n_cols))
+            _check(C, vals, i, p, n_cols, B, dtype)
