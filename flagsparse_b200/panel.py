@@ -38,7 +38,10 @@ FEW_PIECES = 18
 RUNS_MIN_MEAN = 1.5
 FLAG_DEBUG_TIMEOUT = 256    # FSB_PANEL_DEBUG_TIMEOUT
 MAX_ROW_NNZ = 512
-MIN_NNZ = 1 << 22
+# Entries from which the regrouping pays against the kernel for even rows on the caller's arrays (us, rows / panel): float32, 4.5 M
+# entries, 30 a row, band 2^13 / 2^15 13 / 19, 17 / 20; 7.5 M 19 / 19, 25 / 23; 10.8 M 25 / 23, 31 / 25; float64, 4.5 M entries, band
+# 2^13 17 / 21; 7.5 M 27 / 26.
+MIN_NNZ = 3 << 21
 ACC_BANKS = {4: 32, 8: 16}   # accumulators that sit in different shared-memory banks (32 banks of 4 bytes), by value size
 
 
@@ -75,21 +78,35 @@ def default_rounds():
     return r if r in ROUNDS else None
 
 
-def _geometry(dtype, n_rows, device, n_buffers):
+# Columns of a float64 chunk where the accumulators of one wave of row blocks leave room for them: fewer and fuller units (4096 /
+# 8192 columns; 6144 to 10240 are as good here and there: 500009 rows of 30, band 2^15 62 / 44 us; 1000000 rows of 20, band 2^13 56 / 50;
+# 500000 of 60, band 2^15 76 / 70; 700000 of 16, band 2^14 42 / 41).  Not where the rows take a second wave for it (2^22 rows of 32,
+# band 2^16 351 / 436).
+ROOMY_CHUNK_F64 = 8192
+
+
+def _geometry(dtype, n_rows, device, n_buffers, roomy=True):
     L = _lib.lib()
     vt = _VTYPE[dtype]
     sv = 4 if dtype == torch.float32 else 8
     # columns per chunk of x (any multiple of 4; two buffers of it sit beside the accumulators).  Measured on the two
     # banded benchmark matrices: 10240 beats 8192 by 2-4 % (fewer, fuller units), 12288 and more lose on the narrow
     # band (less room for accumulators)
-    chunk_cols = int(os.environ.get("FSB_PANEL_CHUNK", "0")) or (10240 if sv == 4 else 4096)
+    forced = int(os.environ.get("FSB_PANEL_CHUNK", "0"))
     try:
         sms = torch.cuda.get_device_properties(device).multi_processor_count
     except Exception:
         sms = SM_COUNT_FALLBACK
     budget = smem_budget() // CTAS_PER_SM
-    fixed = int(L.fsb_spmv_panel_smem_bytes(vt, 0, chunk_cols, n_buffers))
-    rb_cap = min(49152, (budget - fixed) // sv // 64 * 64)
+
+    def most_rows(cols):
+        fixed = int(L.fsb_spmv_panel_smem_bytes(vt, 0, cols, n_buffers))
+        return min(49152, (budget - fixed) // sv // 64 * 64)
+
+    chunk_cols = forced or (10240 if sv == 4 else 4096)
+    if sv == 8 and not forced and roomy and n_rows <= most_rows(ROOMY_CHUNK_F64) * sms * CTAS_PER_SM:
+        chunk_cols = ROOMY_CHUNK_F64
+    rb_cap = most_rows(chunk_cols)
     if rb_cap < 1024:
         return None              # the x buffers alone (nearly) fill the shared memory
     # whole waves of CTAs: the number of row blocks is a multiple of the CTAs the GPU runs at once
@@ -589,11 +606,20 @@ def build_panel_layout(data, indices, indptr, n_rows, n_cols, max_row_nnz, force
         return None
     if not force and (nnz < MIN_NNZ or max_row_nnz > MAX_ROW_NNZ):
         return None
-    dev = data.device
+    geometry = None
+    for roomy in (True, False):     # a matrix refused for how much of x its chunks take may do with smaller ones
+        tried, geometry = geometry, _geometry(data.dtype, n_rows, data.device, default_buffers(), roomy)
+        if geometry is None or geometry == tried:
+            return None
+        lay = _build_with(geometry, data, indices, indptr, n_rows, n_cols, force, rounds)
+        if lay is not None:
+            return lay
+    return None
+
+
+def _build_with(geometry, data, indices, indptr, n_rows, n_cols, force, rounds):
+    nnz, dev = data.numel(), data.device
     NB = default_buffers()
-    geometry = _geometry(data.dtype, n_rows, dev, NB)
-    if geometry is None:
-        return None
     vt, sv, CW, RB = geometry
     n_rb = -(-n_rows // RB)
     n_ch = -(-n_cols // CW)
@@ -625,7 +651,7 @@ def build_panel_layout(data, indices, indptr, n_rows, n_cols, max_row_nnz, force
             if rounds < ROUNDS[-1]:
                 # a run that does not fit in a small piece (or too much padding): the largest piece may still do
                 del vals, rcs
-                return build_panel_layout(data, indices, indptr, n_rows, n_cols, max_row_nnz, force, ROUNDS[-1])
+                return _build_with(geometry, data, indices, indptr, n_rows, n_cols, force, ROUNDS[-1])
             return None
         if part == ():
             continue                 # no entries in these rows
