@@ -2,13 +2,13 @@
 // entries are wanted in column order, too), the checks of both id arrays, and the row pointer.
 //
 // A row id of a matrix with n_rows rows has bits(n_rows - 1) digits' worth of information, not 32: 150001 rows are two passes
-// of nine bits.  One pass is three launches: counts of every digit per tile of 4096 entries; a scan over the tiles for
+// of nine bits.  One pass is three launches: counts of every digit per tile of 2048 or 4096 entries; a scan over the tiles for
 // every digit; and the move, in which a tile ranks its entries (equal digits of a warp find each other by votes, a warp
 // counts its own in shared memory), brings them into digit order in shared memory and writes each digit's run to its place.
 // The first count also takes the minimum and maximum of both id arrays, the last move fetches values and columns in their
 // new order, so that nothing but (id, position) pairs is moved before.  All of it is enqueued without a look at the checks:
 // ids out of range lead nowhere but to a place inside the arrays, and the caller reads the statistics once, at the end.
-// 2.1 M triples in no order, 150001 rows, 64-bit ids: 110 us of kernels -- first count with the checks 16 us, moves 26 and 45 us
+// 2.1 M triples in no order, 150001 rows, 64-bit ids: 105 us of kernels -- first count with the checks 14 us, moves 23 and 41 us
 // (the latency of one wave of tiles; the last one waits for values and columns from anywhere), row pointer 10 us -- where a
 // library sort, gathers, passes for the checks and an analysis took 210 us and two read-backs.
 #include "fsb_common.cuh"
@@ -17,8 +17,10 @@ namespace fsb {
 
 constexpr int kCooThreads = 256;
 constexpr int kCooWarps = kCooThreads / 32;
-constexpr int kCooItems = 16;                       // entries of a thread
-constexpr int kCooTile = kCooThreads * kCooItems;
+constexpr int kCooMost = 16;                        // entries of a thread, at most
+// Entries of a thread: 16, but 8 up to 3 M entries, which are fewer tiles of 4096 than the SMs hold at a time (1.3 M triples, four
+// passes: moves 93 us, with 16 and the scans of half as many tiles 76; 64000: 24 and 36; 5.2 M, two passes: 165 and 162).
+static int coo_items(int64_t nnz) { return nnz <= 3 << 20 ? 8 : kCooMost; }
 constexpr int kCooMaxBits = 9;                      // of a digit: 8 warps x 512 counters in shared memory
 enum { C_PTR_FIRST = 0, C_PTR_LAST, C_DECREASING, C_MIN_COL, C_MAX_COL, C_MAX_ROW_NNZ, C_EMPTY, C_LONG, C_MIN_ROW, C_MAX_ROW, C_STATS };
 
@@ -67,10 +69,11 @@ __device__ __forceinline__ long long block_extreme(long long v, long long* s_par
 }
 
 // counts[digit * n_tiles + tile]; RANGE: also the extremes of both id arrays
-template <typename Src, typename R, typename C, bool RANGE>
+template <typename Src, typename R, typename C, bool RANGE, int kCooItems>
 __global__ void __launch_bounds__(kCooThreads)
 coo_count_kernel(Src src, int64_t nnz, int shift, int bits, int32_t* __restrict__ counts, const R* __restrict__ row,
                  const C* __restrict__ col, int64_t* __restrict__ stats) {
+  constexpr int kCooTile = kCooThreads * kCooItems;
   extern __shared__ int32_t s_count[];
   __shared__ long long s_part[kCooWarps];
   const int n_digits = 1 << bits;
@@ -155,11 +158,12 @@ template <> struct CooValue<8> { typedef uint2 type; };
 template <> struct CooValue<16> { typedef uint4 type; };
 
 // The move of one pass.  LAST: values and columns go to their final places, with the sorted row ids; else the pairs do.
-template <typename Src, typename C, typename S, bool LAST>
+template <typename Src, typename C, typename S, bool LAST, int kCooItems>
 __global__ void __launch_bounds__(kCooThreads)
 coo_move_kernel(Src src, int64_t nnz, int shift, int bits, const int32_t* __restrict__ counts,
                 const int32_t* __restrict__ totals, uint32_t* __restrict__ out_ids, uint32_t* __restrict__ out_order,
                 const S* __restrict__ data, const C* __restrict__ col, S* __restrict__ out_data, int32_t* __restrict__ out_col) {
+  constexpr int kCooTile = kCooThreads * kCooItems;
   extern __shared__ int32_t s_raw[];
   const int n_digits = 1 << bits;
   int32_t* s_warp = s_raw;                            // [warp][digit]: entries of the warp, then of the warps before
@@ -299,7 +303,7 @@ struct CooScratch {
   size_t bytes;
 };
 static CooScratch coo_scratch(void* base, int64_t nnz) {
-  const int64_t n_tiles = (nnz + kCooTile - 1) / kCooTile;
+  const int64_t tile = (int64_t)kCooThreads * coo_items(nnz), n_tiles = (nnz + tile - 1) / tile;
   const size_t col = (((size_t)nnz * 4) + 255) & ~(size_t)255;
   char* p = (char*)base;
   CooScratch s;
@@ -328,8 +332,9 @@ struct CooArgs {
 struct Yes { static constexpr bool value = true; };
 struct No { static constexpr bool value = false; };
 
-template <typename R, typename C, typename S>
-static int coo_run(const CooArgs& a) {
+template <typename R, typename C, typename S, int kCooItems>
+static int coo_passes(const CooArgs& a) {
+  constexpr int kCooTile = kCooThreads * kCooItems;
   const int64_t n_tiles = (a.nnz + kCooTile - 1) / kCooTile;
   const R* row = (const R*)a.row;
   const C* col = (const C*)a.col;
@@ -348,15 +353,15 @@ static int coo_run(const CooArgs& a) {
       uint32_t* ids = last ? (uint32_t*)a.out_row : a.s.ids[side ^ 1];
       auto pass = [&](auto src, auto range) -> int {
         typedef decltype(src) Src;
-        coo_count_kernel<Src, R, C, decltype(range)::value><<<(unsigned)n_tiles, kCooThreads, count_smem, a.st>>>(
+        coo_count_kernel<Src, R, C, decltype(range)::value, kCooItems><<<(unsigned)n_tiles, kCooThreads, count_smem, a.st>>>(
             src, a.nnz, shift, width, a.s.counts, row, col, a.stats);
         FSB_RETURN_IF_LAUNCH_FAILED();
         coo_scan_kernel<<<1u << width, kCooThreads, 0, a.st>>>(a.s.counts, (int)n_tiles, a.s.totals);
         FSB_RETURN_IF_LAUNCH_FAILED();
 #define FSB_COO_MOVE(LAST_)                                                                                             \
-  e = cudaFuncSetAttribute(coo_move_kernel<Src, C, S, LAST_>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);  \
+  e = cudaFuncSetAttribute(coo_move_kernel<Src, C, S, LAST_, kCooItems>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);  \
   if (e != cudaSuccess) return cuda_rc(e);                                                                              \
-  coo_move_kernel<Src, C, S, LAST_><<<(unsigned)n_tiles, kCooThreads, move_smem, a.st>>>(                               \
+  coo_move_kernel<Src, C, S, LAST_, kCooItems><<<(unsigned)n_tiles, kCooThreads, move_smem, a.st>>>(                               \
       src, a.nnz, shift, width, a.s.counts, a.s.totals, ids, a.s.order[side ^ 1], (const S*)a.data, col, (S*)a.out_data, \
       a.out_col)
         if (last) {
@@ -381,6 +386,11 @@ static int coo_run(const CooArgs& a) {
   return FSB_OK;
 }
 
+template <typename R, typename C, typename S>
+static int coo_run(const CooArgs& a) {
+  return coo_items(a.nnz) == 8 ? coo_passes<R, C, S, 8>(a) : coo_passes<R, C, S, kCooMost>(a);
+}
+
 }  // namespace fsb
 
 using namespace fsb;
@@ -395,7 +405,7 @@ extern "C" int fsb_coo_group(int value_bytes, int rtype, int ctype, const void* 
   if ((rtype != FSB_I32 && rtype != FSB_I64) || (ctype != FSB_I32 && ctype != FSB_I64)) return FSB_EINVAL;
   if (value_bytes != 2 && value_bytes != 4 && value_bytes != 8 && value_bytes != 16) return FSB_EINVAL;
   if (nnz <= 0 || n_rows < 0 || n_cols < 0) return FSB_EINVAL;
-  if (nnz > INT32_MAX - kCooTile || n_rows >= INT32_MAX || n_cols >= INT32_MAX) return FSB_ERANGE;
+  if (nnz > INT32_MAX - kCooThreads * kCooMost || n_rows >= INT32_MAX || n_cols >= INT32_MAX) return FSB_ERANGE;
   if (!data || !row || !col || !out_data || !out_row || !out_col || !indptr || !stats || !scratch) return FSB_EINVAL;
   if (!aligned_to(data, value_bytes) || !aligned_to(out_data, value_bytes) || !aligned_to(row, rtype == FSB_I32 ? 4 : 8) ||
       !aligned_to(col, ctype == FSB_I32 ? 4 : 8) || !aligned_to(stats, 8) || !aligned_to(scratch, 16))

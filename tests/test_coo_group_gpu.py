@@ -37,6 +37,17 @@ def test_against_stable_sorts(cuda, fsb_lib, nnz, n_rows, n_cols, vdt, rt, ct, b
     assert s.n_long_rows == (lens > max(64, 32 * -(-nnz // n_rows))).sum()
 
 
+@pytest.mark.parametrize("nnz", [2047, 2048, 2049, (3 << 20) - 1, 3 << 20, (3 << 20) + 1])
+def test_tiles_of_both_sizes(cuda, fsb_lib, nnz):
+    rng = np.random.default_rng(nnz)
+    row, col = rng.integers(0, 3000, nnz), rng.integers(0, 50000, nnz)
+    for by_column in (False, True):
+        g = coo._group(dev(np.arange(nnz).astype(np.float64)), dev(row), dev(col.astype(np.int32)), 3000, 50000, by_column)
+        order = np.lexsort((col, row)) if by_column else np.argsort(row, kind="stable")
+        assert np.array_equal(g.data.cpu().numpy(), order) and np.array_equal(g.col.cpu().numpy(), col[order])
+        assert np.array_equal(np.diff(g.indptr.cpu().numpy()), np.bincount(row, minlength=3000))
+
+
 @pytest.mark.parametrize("bad_row,bad_col,message", [(-1, 0, "row"), (50, 0, "row"), (2**40, 0, "row"), (0, -5, "col"),
                                                      (0, 60, "col"), (-1, 60, "row")])
 def test_ids_out_of_range_are_refused(cuda, fsb_lib, bad_row, bad_col, message):
