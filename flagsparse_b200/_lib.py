@@ -22,6 +22,7 @@ FSB_SPMV_PANEL = 3  # host-side tag only: the panel kernel has its own entry poi
 FSB_SPMM_AUTO, FSB_SPMM_PLAIN, FSB_SPMM_BULK = 0, 1, 2
 FSB_SPMM_ACCUMULATE = 16  # or-ed into the selector: C += A B
 FSB_SPMM_LONG_ROWS = 32   # or-ed into the selector: long rows are shared by a block
+FSB_SPMM_UNEVEN_ROWS = 64 # or-ed into the selector: the longest row is above 5/4 of the mean
 FSB_OK, FSB_NOT_LAUNCHED, FSB_CAPTURING = 0, 1, 2
 FSB_CUDA_ERROR_BASE = 1000
 

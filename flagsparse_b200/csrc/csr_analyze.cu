@@ -23,7 +23,9 @@ __global__ void stats_init_kernel(int64_t* s) {
   s[S_LONG] = 0;
 }
 
+// (one instruction where all lanes hold 32-bit numbers, which is nearly always)
 __device__ __forceinline__ long long warp_max(long long v) {
+  if (__all_sync(0xffffffffu, v == (int)v)) return __reduce_max_sync(0xffffffffu, (int)v);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     long long u = __shfl_xor_sync(0xffffffffu, v, o);
@@ -32,6 +34,7 @@ __device__ __forceinline__ long long warp_max(long long v) {
   return v;
 }
 __device__ __forceinline__ long long warp_min(long long v) {
+  if (__all_sync(0xffffffffu, v == (int)v)) return __reduce_min_sync(0xffffffffu, (int)v);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     long long u = __shfl_xor_sync(0xffffffffu, v, o);
@@ -39,12 +42,6 @@ __device__ __forceinline__ long long warp_min(long long v) {
   }
   return v;
 }
-__device__ __forceinline__ long long warp_sum(long long v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-
 // One pass over the row pointer and one over the indices, grid-stride, in one launch.  Aligned indices are read at 16 bytes
 // per thread and request; the statistics meet in shared memory, so that a block sends one atomic per statistic: one per warp, on six
 // words that every block of the device shares, used to take longer than the reading (3 M entries,
@@ -58,6 +55,16 @@ __device__ __forceinline__ long long csr_stats_block(const P* __restrict__ ptr, 
   __shared__ long long s_part[8][6];
   const int64_t first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  // the rows first: their loads are on their way while the indices are looked at
+  long long longest = 0;
+  unsigned n_dec = 0, n_empty = 0, n_long = 0;         // (of one thread, fewer than 2^32 / 32)
+  for (int64_t i = first; i < n_rows; i += stride) {
+    const long long len = (long long)ptr[i + 1] - (long long)ptr[i];
+    longest = len > longest ? len : longest;
+    n_dec += len < 0;
+    n_empty += len == 0;
+    n_long += len > long_len;
+  }
   I mn = sizeof(I) == 4 ? (I)INT32_MAX : (I)INT64_MAX, mx = sizeof(I) == 4 ? (I)INT32_MIN : (I)INT64_MIN;
   int64_t done = 0;
   if (wide_loads) {
@@ -84,27 +91,17 @@ __device__ __forceinline__ long long csr_stats_block(const P* __restrict__ ptr, 
     mn = c < mn ? c : mn;
     mx = c > mx ? c : mx;
   }
-  long long longest = 0, dec = 0, empty = 0, lng = 0;
-  for (int64_t i = first; i < n_rows; i += stride) {
-    const long long len = (long long)ptr[i + 1] - (long long)ptr[i];
-    longest = len > longest ? len : longest;
-    dec += len < 0;
-    empty += len == 0;
-    lng += len > long_len;
-  }
   const bool any = nnz > 0;                  // a thread without an entry holds the neutral values of I, not of int64
-  long long wide_mn = (!any || mn > mx) ? (long long)INT64_MAX : (long long)mn;
-  long long wide_mx = (!any || mn > mx) ? (long long)INT64_MIN : (long long)mx;
+  const long long wide_mn = (!any || mn > mx) ? (long long)INT64_MAX : (long long)mn;
+  const long long wide_mx = (!any || mn > mx) ? (long long)INT64_MIN : (long long)mx;
   longest = warp_max(longest);
-  dec = warp_sum(dec);
-  empty = warp_sum(empty);
-  lng = warp_sum(lng);
-  wide_mn = warp_min(wide_mn);
-  wide_mx = warp_max(wide_mx);
+  const long long dec = __reduce_add_sync(0xffffffffu, n_dec), empty = __reduce_add_sync(0xffffffffu, n_empty),
+                  lng = __reduce_add_sync(0xffffffffu, n_long);
+  const long long low = warp_min(wide_mn), high = warp_max(wide_mx);
   const int w = threadIdx.x >> 5;
   if ((threadIdx.x & 31) == 0) {
     s_part[w][0] = longest; s_part[w][1] = dec; s_part[w][2] = empty; s_part[w][3] = lng;
-    s_part[w][4] = wide_mn; s_part[w][5] = wide_mx;
+    s_part[w][4] = low; s_part[w][5] = high;
   }
   __syncthreads();
   long long v = 0;
@@ -142,7 +139,7 @@ csr_stats_kernel(const P* __restrict__ ptr, int64_t n_rows, int64_t long_len, co
 
 // The same for a host that waits: the block that ends last writes the eight numbers to host memory (`out`, page-locked), then
 // `ticket` behind them, and leaves `work` zero, as it was found.  No launch to set up, no copy, no wait for the whole stream
-// (250007 rows, 3 M entries with 64-bit indices: 13.8 us; set-up, csr_stats_kernel and copy are 13.5 us on the GPU, but the host's
+// (250007 rows, 3 M entries with 64-bit indices: 10.7 us; set-up, csr_stats_kernel and copy were 13.5 us on the GPU, but the host's
 // part of them and of the wait made a whole product of these arrays 62 us, 33 us now; 4096 rows of 16, 32 columns of B: 75 and 34).
 // work: 0 longest, 1 to 3 counts, 4 and 5 the extreme indices in an order that has zero for none, 6 blocks that are done.
 constexpr unsigned long long kSignBit = 1ull << 63;
@@ -150,6 +147,11 @@ template <typename I, typename P>
 __global__ void __launch_bounds__(256)
 csr_check_kernel(const P* __restrict__ ptr, int64_t n_rows, int64_t long_len, const I* __restrict__ idx, int64_t nnz,
                  int wide_loads, unsigned long long* __restrict__ work, volatile int64_t* out, int64_t ticket) {
+  int64_t ptr_first = 0, ptr_last = 0;      // (asked for early: whichever block is the last one has them by then)
+  if (threadIdx.x == 0) {
+    ptr_first = (int64_t)ptr[0];
+    ptr_last = (int64_t)ptr[n_rows];
+  }
   const long long v = csr_stats_block<I, P>(ptr, n_rows, long_len, idx, nnz, wide_loads);
   const int k = threadIdx.x;
   if (k < 6) {
@@ -170,8 +172,8 @@ csr_check_kernel(const P* __restrict__ ptr, int64_t n_rows, int64_t long_len, co
 #pragma unroll
   for (int j = 0; j < 6; ++j) w[j] = atomicExch(work + j, 0ull);
   atomicExch(work + 6, 0ull);
-  out[S_PTR_FIRST] = (int64_t)ptr[0];
-  out[S_PTR_LAST] = (int64_t)ptr[n_rows];
+  out[S_PTR_FIRST] = ptr_first;
+  out[S_PTR_LAST] = ptr_last;
   out[S_DECREASING] = (int64_t)w[1];
   out[S_MIN_IDX] = (int64_t)(~w[4] ^ kSignBit);
   out[S_MAX_IDX] = (int64_t)(w[5] ^ kSignBit);
@@ -223,7 +225,7 @@ static int64_t stats_long_len(int64_t n_rows, int64_t nnz) {
 static int stats_grid(int itype, int64_t n_rows, int64_t nnz) {
   const int64_t per_thread = itype == FSB_I32 ? 16 : 8;      // four requests
   const int64_t rows_blocks = (n_rows + 1023) / 1024, idx_blocks = (nnz + 256 * per_thread - 1) / (256 * per_thread);
-  return grid_for((rows_blocks > idx_blocks ? rows_blocks : idx_blocks) * 256, 256, 148 * 8);
+  return grid_for((rows_blocks > idx_blocks ? rows_blocks : idx_blocks) * 256, 256, 148 * 4);   // (8 an SM: 13.3 us, 4: 10.7)
 }
 
 int csr_check_launch(int itype, int ptype, const void* indices, const void* indptr, int64_t n_rows, int64_t nnz, void* work,

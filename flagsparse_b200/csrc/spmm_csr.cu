@@ -21,6 +21,7 @@ namespace fsb {
 constexpr int kMmThreads = 256;
 constexpr int kMmTile = 1024;  // nnz per tile
 constexpr int kMmMinPiece = 32; // shortest piece of a long segment
+constexpr int kMmBuckets = 64;  // of segment lengths: two entries each, the last for all that are longer
 constexpr int kWaitSpins = 1 << 22;
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -173,6 +174,11 @@ __host__ __device__ constexpr int mm_ctas(int nc, size_t size, bool with_long) {
 // balances as well but pays a row-end test per entry, and an even matrix then loses what a skewed one gains (2^20 rows
 // of 16 entries, 64 columns, float32: 615 us against 531 us).  `piece` depends on the number of columns and the value
 // type only (not on the alignment, which picks VW and LR), so the order of additions does too.
+// by_length: the segments of a tile are taken in the order of their lengths, the longest first: two to four groups share a warp, and
+// those whose segment is shorter wait for the longest among them (us, in the order of the rows / by length: float32, 32 columns,
+// 300000 rows of 5 37 / 33, 262144 Zipf rows of 16 87 / 81; 64 columns, 2^19 rows of 16 231 / 225, Zipf 130 / 123; float64, 32 columns,
+// Zipf rows of 12 135 / 121).  Rows of one length lose what the sorting takes (2^20 of 16: 521 / 524), eight groups in a warp gain
+// nothing (16 columns: 40.1 / 40.3), one none (float64, 64 columns: 156 / 159), several accesses a lane spill (33 columns, Zipf 91 / 109).
 // n_dense is covered by LR * NC accesses of VW elements per entry; wider products take column tiles (gridDim.y).
 // ACCUM: add to what C holds instead of overwriting it (rows without entries are then left alone) -- the later passes
 // of a product that the host code splits into column panels of A.
@@ -182,7 +188,7 @@ spmm_tile_kernel(const S* __restrict__ data, const I* __restrict__ idx, const vo
                  const S* __restrict__ B, int64_t ldb, S* __restrict__ C, int64_t ldc,
                  const int32_t* __restrict__ tile_row, typename MmOps<S>::Acc* __restrict__ carry,
                  typename MmOps<S>::Acc* __restrict__ head, int64_t nnz, int n_dense, int LR, int piece,
-                 int use_bulk, int32_t* __restrict__ status) {
+                 int by_length, int use_bulk, int32_t* __restrict__ status) {
   typedef MmOps<S> Ops;
   typedef typename Ops::Acc A;
   constexpr int T = kMmTile;
@@ -198,6 +204,8 @@ spmm_tile_kernel(const S* __restrict__ data, const I* __restrict__ idx, const vo
   __shared__ int s_head_partial;
   __shared__ int s_failed;
   __shared__ int s_n_long, s_n_pieces;
+  __shared__ uint16_t s_order[NC == 1 ? RC : 1];          // segments by length
+  __shared__ int s_bucket[kMmBuckets];
   extern __shared__ __align__(16) unsigned char s_parts[];
 
   const int tid = threadIdx.x;
@@ -361,7 +369,32 @@ spmm_tile_kernel(const S* __restrict__ data, const I* __restrict__ idx, const vo
       return;
     }
 
-    for (int k = grp; k < m; k += ngrp) {
+    if (NC == 1 && by_length) {
+      auto bucket = [&](int k) {                 // the longest first
+        const int len = s_off[k + 1] - s_off[k];
+        return kMmBuckets - 1 - (len < 2 * kMmBuckets - 2 ? len : 2 * kMmBuckets - 2) / 2;
+      };
+      if (tid < kMmBuckets) s_bucket[tid] = 0;
+      __syncthreads();
+      for (int k = tid; k < m; k += kMmThreads) atomicAdd(&s_bucket[bucket(k)], 1);
+      __syncthreads();
+      if (tid < 32) {
+        const int c0 = s_bucket[2 * tid], c1 = s_bucket[2 * tid + 1];
+        int upto = c0 + c1;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int v = __shfl_up_sync(0xffffffffu, upto, o);
+          if (tid >= o) upto += v;
+        }
+        s_bucket[2 * tid] = upto - c0 - c1;
+        s_bucket[2 * tid + 1] = upto - c1;
+      }
+      __syncthreads();
+      for (int k = tid; k < m; k += kMmThreads) s_order[atomicAdd(&s_bucket[bucket(k)], 1)] = (uint16_t)k;
+      __syncthreads();
+    }
+    for (int q = grp; q < m; q += ngrp) {
+      const int k = NC == 1 && by_length ? s_order[q] : q;
       const int s = s_off[k], e = s_off[k + 1];
       if (LONG && e - s > 2 * piece) {
         if (lane == 0) {
@@ -480,7 +513,7 @@ struct SpmmArgs {
   void* C;
   int64_t ldc, n_rows, n_dense, nnz;
   int algo, ptype;
-  bool accumulate, long_rows;
+  bool accumulate, long_rows, uneven_rows;
   const int32_t* tile_row;
   int32_t* own_plan;      // the plan has to be made first, here (tile_row is the same address)
   void* scratch;
@@ -514,10 +547,11 @@ static int launch_spmm(const SpmmArgs& a, int LR, int piece) {
   A* head = carry + n_tiles * n_dense;
   const int bulk = a.algo != FSB_SPMM_PLAIN && aligned_to(a.data, 16) && aligned_to(a.idx, 16);
   const dim3 grid((unsigned)n_tiles, (unsigned)col_tiles);
+  const int by_length = a.uneven_rows && NC == 1 && LR >= 8 && LR < 32;
 #define FSB_SPMM_LAUNCH(LONG_, ACC_, SMEM_)                                                                          \
   spmm_tile_kernel<S, I, VW, NC, LONG_, ACC_><<<grid, kMmThreads, SMEM_, a.st>>>(                                    \
       (const S*)a.data, (const I*)a.idx, a.ptr, a.ptype == FSB_I64, (const S*)a.B, a.ldb, (S*)a.C, a.ldc, a.tile_row, \
-      carry, head, a.nnz, n_dense, LR, piece, bulk, a.status)
+      carry, head, a.nnz, n_dense, LR, piece, by_length, bulk, a.status)
   // the long segments of a tile (more than 2 * piece entries each) have at most T / piece + T / (2 * piece) pieces
   const size_t parts = a.long_rows ? (size_t)(T / piece + T / (2 * piece)) * width * sizeof(A) : 0;
   if (a.accumulate && !REAL) return FSB_EINVAL;
@@ -641,8 +675,8 @@ static int spmm_run(int vtype, int itype, int ptype, const void* data, const voi
                     size_t scratch_bytes, int32_t* status, cudaStream_t st) {
   if ((itype != FSB_I32 && itype != FSB_I64) || (ptype != FSB_I32 && ptype != FSB_I64)) return FSB_EINVAL;
   const bool accumulate = (algo & FSB_SPMM_ACCUMULATE) != 0;
-  const bool long_rows = (algo & FSB_SPMM_LONG_ROWS) != 0;
-  algo &= ~(FSB_SPMM_ACCUMULATE | FSB_SPMM_LONG_ROWS);
+  const bool long_rows = (algo & FSB_SPMM_LONG_ROWS) != 0, uneven_rows = (algo & FSB_SPMM_UNEVEN_ROWS) != 0;
+  algo &= ~(FSB_SPMM_ACCUMULATE | FSB_SPMM_LONG_ROWS | FSB_SPMM_UNEVEN_ROWS);
   if (algo != FSB_SPMM_AUTO && algo != FSB_SPMM_PLAIN && algo != FSB_SPMM_BULK) return FSB_EINVAL;
   if (n_rows < 0 || n_cols < 0 || n_dense < 0 || nnz < 0) return FSB_EINVAL;
   if (n_rows >= INT32_MAX || n_cols >= INT32_MAX || n_dense >= (1 << 24)) return FSB_ERANGE;
@@ -673,7 +707,7 @@ static int spmm_run(int vtype, int itype, int ptype, const void* data, const voi
   if (fsb_csr_num_tiles(nnz, kMmTile) >= 65535LL * 32768LL) return FSB_ERANGE;
 
   int32_t* own_plan = plan_in_scratch ? (int32_t*)((char*)scratch + parts_bytes) : nullptr;
-  SpmmArgs a{data, indices, indptr, B, ldb, C, ldc, n_rows, n_dense, nnz, algo, ptype, accumulate, long_rows,
+  SpmmArgs a{data, indices, indptr, B, ldb, C, ldc, n_rows, n_dense, nnz, algo, ptype, accumulate, long_rows, uneven_rows,
              plan_in_scratch ? own_plan : tile_row, own_plan, scratch, status, st};
   if (vtype == FSB_F32) return itype == FSB_I32 ? spmm_typed<float, int32_t>(a) : spmm_typed<float, int64_t>(a);
   if (vtype == FSB_F64) return itype == FSB_I32 ? spmm_typed<double, int32_t>(a) : spmm_typed<double, int64_t>(a);
@@ -718,7 +752,8 @@ extern "C" int fsb_spmm_csr_stored(int vtype, int ptype, const void* data, const
   if (vtype != FSB_F16 && vtype != FSB_BF16 && vtype != FSB_C64 && vtype != FSB_C128) return FSB_EINVAL;
   // staged by ordinary loads: no copy whose end would have to be waited for and reported
   return spmm_run(vtype, FSB_I32, ptype, data, indices, indptr, B, ldb, C, ldc, n_rows, n_cols, n_dense, nnz,
-                  FSB_SPMM_PLAIN | (long_rows ? FSB_SPMM_LONG_ROWS : 0), nullptr, true, scratch, scratch_bytes, nullptr,
+                  FSB_SPMM_PLAIN | (long_rows & ~FSB_SPMM_UNEVEN_ROWS ? FSB_SPMM_LONG_ROWS : 0) | (long_rows & FSB_SPMM_UNEVEN_ROWS),
+                  nullptr, true, scratch, scratch_bytes, nullptr,
                   static_cast<cudaStream_t>(stream_));
 }
 
@@ -740,7 +775,9 @@ extern "C" int fsb_spmm_csr_once(int vtype, int itype, int ptype, const void* da
   const int waited = csr_check_wait(host, st);
   if (rc != FSB_OK || waited != FSB_OK) return rc != FSB_OK ? rc : waited;
   if (!csr_check_passed(host, n_cols, nnz)) return FSB_NOT_LAUNCHED;
-  const int algo = FSB_SPMM_PLAIN | (csr_check_longest(host) > long_row ? FSB_SPMM_LONG_ROWS : 0);
+  const int64_t longest = csr_check_longest(host);
+  const int algo = FSB_SPMM_PLAIN | (longest > long_row ? FSB_SPMM_LONG_ROWS : 0) |
+                   (4 * longest * n_rows > 5 * nnz ? FSB_SPMM_UNEVEN_ROWS : 0);
   return spmm_run(vtype, itype, ptype, data, indices, indptr, B, ldb, C, ldc, n_rows, n_cols, n_dense, nnz, algo, tile_row, false,
                   scratch, parts, nullptr, st);
 }

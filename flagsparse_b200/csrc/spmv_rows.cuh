@@ -207,8 +207,8 @@ static bool rows_apply(const void* data, const void* idx, int64_t n_rows, int64_
   return n_rows >= kRowsLeast && n_rows <= (1 << 30) && nnz <= (1 << 30) && aligned_to(data, 16) && aligned_to(idx, 16);
 }
 
-// Lanes of a row: the fewest that hold four fifths of a mean row at once (complex128 half of one: 300000 rows of 24, 8 / 16 lanes
-// 46 / 50 us); more leave lanes idle (float32, 1000000 rows of 4, 2 / 4 / 8 lanes: 17 / 21 / 33 us), fewer a second turn for
+// Lanes of a row: the fewest that hold four fifths of a mean row at once (complex128 two fifths: 4 / 8 / 16 lanes, columns anywhere,
+// 1000000 rows of 12 80 / 86 / - us, 500000 rows of 36 111 / 101 / 115, 300000 rows of 60 107 / 99 / 102); more leave lanes idle (float32, 1000000 rows of 4, 2 / 4 / 8 lanes: 17 / 21 / 33 us), fewer a second turn for
 // most rows (float64, 100000 rows of 50, 16 / 8 / 4 / 2 lanes: 27 / 25 / 27 / 30 us).
 template <typename S, typename I, typename P, typename Out>
 static int rows_run(const void* data_, const void* idx_, const void* ptr_, const void* x_, Out out, int64_t n_rows, int64_t nnz,
@@ -223,7 +223,7 @@ static int rows_run(const void* data_, const void* idx_, const void* ptr_, const
   if (sms > kRowsThreads) sms = kRowsThreads;          // a thread looks at a share
   const int64_t mean = nnz / n_rows;
   int L = 2;
-  while (L < 32 && (sizeof(S) == 16 ? 2 * L * E < mean : 5 * L * E < 4 * mean)) L <<= 1;
+  while (L < 32 && 5 * L * E < (sizeof(S) == 16 ? 2 : 4) * mean) L <<= 1;
   const RowsShares shares(n_rows, nnz, sms);
   switch (L) {
     case 2: spmv_rows_kernel<S, I, P, 2, U, E><<<sms, kRowsThreads, 0, st>>>(data, idx, ptr, x, out, n_rows, nnz, shares); break;

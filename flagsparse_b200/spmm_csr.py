@@ -404,6 +404,11 @@ def _shares_long_rows(max_row_nnz, n_dense, element_size):
     return max_row_nnz > _long_row(n_dense, element_size)
 
 
+def _uneven_flag(p):
+    """FSB_SPMM_UNEVEN_ROWS where rows differ in length: segments that share a warp are then picked by length."""
+    return _lib.FSB_SPMM_UNEVEN_ROWS if 4 * p.max_row_nnz * p.n_rows > 5 * p.data.numel() else 0
+
+
 def _spmm_launch(prepared, B, C):
     """Enqueue C = A B on the current stream.  Stands in for _triton_spmm_csr_impl (spmm_csr.py:525-599)
     and _triton_spmm_csr_impl_opt_prepared (:1033-1055).  One launch of the tiled kernel per pass: the whole
@@ -424,6 +429,7 @@ def _spmm_launch(prepared, B, C):
     sv = B.element_size()
     if p.max_row_nnz > LONG_ROW_NNZ and _shares_long_rows(p.max_row_nnz, n_dense, sv):
         algo |= _lib.FSB_SPMM_LONG_ROWS
+    algo |= _uneven_flag(p)
     vt, it, pt = _VTYPE[p.data.dtype], _ITYPE[p.kernel_indices.dtype], _ITYPE[p.kernel_indptr.dtype]
     ldb, ldc = B.stride(0), C.stride(0)
     stream = _stream_ptr(dev)
@@ -468,7 +474,7 @@ def _spmm_launch_stored(prepared, B, C):
         rc = L.fsb_spmm_csr_stored(
             vt, _ITYPE[p.kernel_indptr.dtype], _ptr(p.data), _ptr(p.kernel_indices), p.kernel_indptr.data_ptr(),
             _ptr(B), B.stride(0) if B.shape[0] > 1 else n_dense, C.data_ptr(), n_dense, p.n_rows, p.n_cols, n_dense, nnz,
-            int(_shares_long_rows(p.max_row_nnz, n_dense, B.element_size())), scratch.data_ptr(), scratch.numel(), _stream_ptr(dev),
+            int(_shares_long_rows(p.max_row_nnz, n_dense, B.element_size())) | _uneven_flag(p), scratch.data_ptr(), scratch.numel(), _stream_ptr(dev),
         )
     _lib.check(rc, "fsb_spmm_csr_stored")
 

@@ -64,6 +64,7 @@ extern "C" {
 #define FSB_SPMM_BULK 2      /* tile staged by cp.async.bulk (TMA 1-D bulk copy) + mbarrier       */
 #define FSB_SPMM_ACCUMULATE 16 /* or-ed into the selector: C += A B instead of C = A B            */
 #define FSB_SPMM_LONG_ROWS 32  /* or-ed into the selector: some rows are long (see fsb_spmm_csr)  */
+#define FSB_SPMM_UNEVEN_ROWS 64 /* or-ed into the selector: the longest row is above 5/4 of the mean */
 
 int fsb_version(void);
 
@@ -371,7 +372,7 @@ int fsb_spmm_csr_wide(int vtype, int ptype, const void* data, const int32_t* ind
  * C = A B for the same four value types with B and C in the matrix's own type (half precisions: 2-byte values read as
  * they are stored, products and sums in float32, every element of C rounded once).  The tiled kernel of fsb_spmm_csr,
  * its tile plan made in scratch (fsb_spmm_stored_scratch_bytes() bytes, 16-byte aligned); long_rows != 0 is
- * FSB_SPMM_LONG_ROWS.
+ * FSB_SPMM_LONG_ROWS, but for FSB_SPMM_UNEVEN_ROWS in it, which is what it is there.
  */
 size_t fsb_spmm_stored_scratch_bytes(int vtype, int64_t nnz, int64_t n_dense);
 int fsb_spmm_csr_stored(int vtype, int ptype, const void* data, const int32_t* indices, const void* indptr,

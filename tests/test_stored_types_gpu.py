@@ -121,3 +121,21 @@ def test_spmm_rows_over_many_tiles(cuda, fsb_lib, dtype):
             B = _values((n_cols, n_dense), dtype, n_dense)
             C = fs.flagsparse_spmm_csr(vals.to(cuda), torch.from_numpy(i).to(cuda), torch.from_numpy(p).to(cuda), B.to(cuda), (len(p) - 1, n_cols))
             _check(C, vals, i, p, n_cols, B, dtype)
+
+
+@pytest.mark.parametrize("dtype", DTYPES, ids=str)
+def test_spmm_segments_by_length(cuda, fsb_lib, dtype):
+    """Tiles with more segments than threads, all of one length, none with an entry, and lengths around the last bucket; every
+    result twice, as the order inside a bucket is not fixed."""
+    n_cols = 700
+    rng = np.random.default_rng(1)
+    for lens in ([1] * 3000, [0, 2] * 1500 + [300], [int(v) for v in rng.integers(0, 4, 5000)] + [63, 64, 65, 124, 125, 126, 127, 130],
+                 [5] * 700 + [6] * 400):
+        _, i, p = handmade_csr(3, lens, n_cols)
+        vals = _values(int(p[-1]), dtype, 4)
+        d, ti, tp = vals.to(cuda), torch.from_numpy(i).to(cuda), torch.from_numpy(p).to(cuda)
+        for n_dense in (16, 32, 64, 128):
+            B = _values((n_cols, n_dense), dtype, n_dense)
+            C = fs.flagsparse_spmm_csr(d, ti, tp, B.to(cuda), (len(p) - 1, n_cols))
+            _check(C, vals, i, p, n_cols, B, dtype)
+            assert torch.equal(fs.flagsparse_spmm_csr(d, ti, tp, B.to(cuda), (len(p) - 1, n_cols)), C)
