@@ -3,6 +3,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "fsb.h"
 
 namespace fsb {
@@ -18,11 +20,16 @@ inline int cuda_rc(cudaError_t e) { return e == cudaSuccess ? FSB_OK : FSB_CUDA_
 inline bool aligned_to(const void* p, size_t a) { return (reinterpret_cast<uintptr_t>(p) & (a - 1)) == 0; }
 __device__ __forceinline__ bool aligned_to_dev(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
-// SMs of the current device
+// SMs of the current device, looked up once per device
 inline int sm_count(int* out) {
+  static std::atomic<int> known[64];
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
-  if (e == cudaSuccess) e = cudaDeviceGetAttribute(out, cudaDevAttrMultiProcessorCount, dev);
+  if (e != cudaSuccess) return cuda_rc(e);
+  *out = dev >= 0 && dev < 64 ? known[dev].load(std::memory_order_relaxed) : 0;
+  if (*out > 0) return FSB_OK;
+  e = cudaDeviceGetAttribute(out, cudaDevAttrMultiProcessorCount, dev);
+  if (e == cudaSuccess && dev >= 0 && dev < 64) known[dev].store(*out, std::memory_order_relaxed);
   return cuda_rc(e);
 }
 

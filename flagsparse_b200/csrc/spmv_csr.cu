@@ -437,7 +437,7 @@ static int run_vector(const void* data, const void* idx, const void* ptr, const 
                       int64_t n_rows, int64_t nnz, int tuning, cudaStream_t st) {
   int L = tuning & 0xff;
   if (L == 0) {
-    if (rows_apply(data, idx, n_rows, nnz)) return rows_run<V, I, P, Out>(data, idx, ptr, x, out, n_rows, nnz, st);
+    if (!(tuning & FSB_SPMV_UNEVEN_ROWS) && rows_apply(data, idx, n_rows, nnz)) return rows_run<V, I, P, Out>(data, idx, ptr, x, out, n_rows, nnz, st);
     // eight to sixteen entries (two to four 4-element groups) per lane: measured best on 32-entry rows
     const int64_t mean = n_rows > 0 ? nnz / n_rows : 0;
     L = 2;
@@ -511,7 +511,7 @@ static int spmv_typed(const SpmvArgs& a) {
   if (a.algo == FSB_SPMV_VECTOR) {
     if (a.y_peers) {
       PeerOut<V> out{(V* const*)a.y_peers, a.n_peers, a.row_offset, a.first_peer};
-      return run_vector<V, I, P, PeerOut<V>>(a.data, a.idx, a.ptr, a.x, out, a.n_rows, a.nnz, a.tuning & 0xff, a.st);
+      return run_vector<V, I, P, PeerOut<V>>(a.data, a.idx, a.ptr, a.x, out, a.n_rows, a.nnz, a.tuning, a.st);
     }
     LocalOut<V> out{(V*)a.y};
     return run_vector<V, I, P, LocalOut<V>>(a.data, a.idx, a.ptr, a.x, out, a.n_rows, a.nnz, a.tuning, a.st);

@@ -233,7 +233,7 @@ class PreparedCsrSpmmOpt:
         "data", "kernel_indices", "kernel_indptr", "shape", "n_rows", "n_cols", "max_row_nnz",
         "row_buckets", "supports_opt", "long_part_rows", "long_part_starts", "long_part_ends",
         "long_row_ids", "long_row_part_ptr", "long_row_fallback_only", "stats", "tile_nnz", "tile_row",
-        "_scratch", "_status", "_row_lengths", "wide", "_whole", "_panels", "_span", "_once",
+        "_scratch", "_status", "_row_lengths", "wide", "_whole", "_panels", "_span", "_once", "_uneven",
     )
 
     def __init__(self, data, kernel_indices, kernel_indptr, shape, n_rows, n_cols, stats, tile_nnz, tile_row,
@@ -256,6 +256,8 @@ class PreparedCsrSpmmOpt:
         self._status = None
         self._row_lengths = None
         self._once = False
+        # where rows differ in length, segments that share a warp are picked by length
+        self._uneven = _lib.FSB_SPMM_UNEVEN_ROWS if 4 * self.max_row_nnz * self.n_rows > 5 * data.numel() else 0
         self._whole = None       # the matrix as one _CsrPart (shares the tile plan)
         self._panels = {}        # number of column panels -> list of _CsrPart
         self._span = None        # columns spanned by a window of consecutive entries (median over samples)
@@ -404,11 +406,6 @@ def _shares_long_rows(max_row_nnz, n_dense, element_size):
     return max_row_nnz > _long_row(n_dense, element_size)
 
 
-def _uneven_flag(p):
-    """FSB_SPMM_UNEVEN_ROWS where rows differ in length: segments that share a warp are then picked by length."""
-    return _lib.FSB_SPMM_UNEVEN_ROWS if 4 * p.max_row_nnz * p.n_rows > 5 * p.data.numel() else 0
-
-
 def _spmm_launch(prepared, B, C):
     """Enqueue C = A B on the current stream.  Stands in for _triton_spmm_csr_impl (spmm_csr.py:525-599)
     and _triton_spmm_csr_impl_opt_prepared (:1033-1055).  One launch of the tiled kernel per pass: the whole
@@ -429,7 +426,7 @@ def _spmm_launch(prepared, B, C):
     sv = B.element_size()
     if p.max_row_nnz > LONG_ROW_NNZ and _shares_long_rows(p.max_row_nnz, n_dense, sv):
         algo |= _lib.FSB_SPMM_LONG_ROWS
-    algo |= _uneven_flag(p)
+    algo |= p._uneven
     vt, it, pt = _VTYPE[p.data.dtype], _ITYPE[p.kernel_indices.dtype], _ITYPE[p.kernel_indptr.dtype]
     ldb, ldc = B.stride(0), C.stride(0)
     stream = _stream_ptr(dev)
@@ -474,7 +471,7 @@ def _spmm_launch_stored(prepared, B, C):
         rc = L.fsb_spmm_csr_stored(
             vt, _ITYPE[p.kernel_indptr.dtype], _ptr(p.data), _ptr(p.kernel_indices), p.kernel_indptr.data_ptr(),
             _ptr(B), B.stride(0) if B.shape[0] > 1 else n_dense, C.data_ptr(), n_dense, p.n_rows, p.n_cols, n_dense, nnz,
-            int(_shares_long_rows(p.max_row_nnz, n_dense, B.element_size())) | _uneven_flag(p), scratch.data_ptr(), scratch.numel(), _stream_ptr(dev),
+            int(_shares_long_rows(p.max_row_nnz, n_dense, B.element_size())) | p._uneven, scratch.data_ptr(), scratch.numel(), _stream_ptr(dev),
         )
     _lib.check(rc, "fsb_spmm_csr_stored")
 

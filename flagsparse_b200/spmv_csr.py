@@ -115,6 +115,18 @@ def _longest_even_stored(n_rows, nnz, element_size):
     return int(max(line, _UNEVEN_PER_LANE * lanes, nnz / _UNEVEN_ENTRIES[element_size] * lanes / 4))
 
 
+# Longest row, in means (plus eight entries), up to which neighbouring rows stay on one SM (csrc/spmv_rows.cuh): its warps hold more
+# rows together than those of the kernel that spreads the rows over all SMs, and all of them wait for the longest.  600000 rows,
+# columns anywhere, Zipf lengths cut off at 4.2 / 7.1 / 11.7 / 20 means, us spread / on one SM: float16 37 / 31, 48 / 41, 62 / 51,
+# 31 / 37; float32 35 / 33, 49 / 44, 64 / 53, 29 / 37; float64 41 / 39, 61 / 66, 84 / 92, 33 / 38; complex64 41 / 37, 49 / 58, 62 / 82,
+# 29 / 33; complex128 59 / 72, 81 / 100, 104 / 153, 52 / 76.
+_NEIGHBOUR_MEANS = {2: 10, 4: 10, 8: 5, 16: 3}
+
+
+def _longest_neighbour(n_rows, nnz, element_size):
+    return _NEIGHBOUR_MEANS[element_size] * nnz // max(n_rows, 1) + 8
+
+
 def _uneven_rows(n_rows, nnz, max_row_nnz, element_size):
     """Whether the longest row leaves the lanes-per-row kernel for float16 / bfloat16 / complex values waiting for it."""
     return max_row_nnz > _longest_even_stored(n_rows, nnz, element_size)
@@ -135,7 +147,7 @@ class PreparedCsrSpmv:
     __slots__ = (
         "data", "kernel_indices", "kernel_indptr", "shape", "n_rows", "n_cols", "block_nnz",
         "max_segments", "max_row_nnz", "opt_buckets", "supports_opt", "stats", "algo", "tuning",
-        "tile_nnz", "tile_row", "scratch", "panel", "long_rows", "wide", "bins",
+        "tile_nnz", "tile_row", "scratch", "panel", "long_rows", "wide", "bins", "uneven",
     )
 
     def __init__(self, data, kernel_indices, kernel_indptr, shape, n_rows, n_cols, block_nnz,
@@ -150,6 +162,8 @@ class PreparedCsrSpmv:
         self.block_nnz = block_nnz
         self.max_segments = max_segments
         self.max_row_nnz = max_row_nnz
+        even = _longest_neighbour(n_rows, data.numel(), data.element_size())
+        self.uneven = _lib.FSB_SPMV_UNEVEN_ROWS if max_row_nnz > even else 0
         self.supports_opt = data.dtype in (torch.float32, torch.float64)
         self.stats = stats
         self.algo = algo
@@ -389,7 +403,7 @@ def _spmv_launch(prepared, x, y):
     if scratch is not None and (p.data.numel() < _STREAM_MIN_NNZ or p.bins is not None):
         scratch = torch.empty_like(scratch)
     lanes = p.tuning & 0xFF
-    tuning = p.tuning if algo == _lib.FSB_SPMV_STREAM else (lanes if lanes in (2, 4, 8, 16, 32) else 0)
+    tuning = p.tuning if algo == _lib.FSB_SPMV_STREAM else (lanes if lanes in (2, 4, 8, 16, 32) else p.uneven)
     with _on_device(dev):
         rc = L.fsb_spmv_csr(
             _VTYPE[p.data.dtype], _ITYPE[p.kernel_indices.dtype], _ITYPE[p.kernel_indptr.dtype],
@@ -416,7 +430,7 @@ def _spmv_launch_stored(prepared, x, y):
                               dtype=torch.uint8, device=dev)
     with _on_device(dev):
         rc = L.fsb_spmv_csr_stored(
-            _WIDE_VTYPE[p.data.dtype], _ITYPE[p.kernel_indptr.dtype], _ptr(p.data), _ptr(p.kernel_indices),
+            _WIDE_VTYPE[p.data.dtype], _ITYPE[p.kernel_indptr.dtype] | p.uneven, _ptr(p.data), _ptr(p.kernel_indices),
             p.kernel_indptr.data_ptr(), _ptr(x), _ptr(y), p.n_rows, p.n_cols, p.data.numel(),
             None if p.tile_row is None else p.tile_row.data_ptr(), _ptr(scratch),
             0 if scratch is None else scratch.numel(), _stream_ptr(dev),
@@ -463,7 +477,8 @@ def _spmv_once(data, indices, indptr, x, shape, out):
         y = out if out is not None else torch.empty(n_rows, dtype=dtype, device=dev)
         longest = (_longest_even_stored if stored else _longest_even)(n_rows, nnz, data.element_size())
         rc = L.fsb_spmv_csr_once(vt, it, pt, data.data_ptr(), indices.data_ptr(), indptr.data_ptr(), x.data_ptr(), y.data_ptr(),
-                                 n_rows, n_cols, nnz, longest, slot.work_ptr, slot.host_ptr, _stream_ptr(dev))
+                                 n_rows, n_cols, nnz, longest, _longest_neighbour(n_rows, nnz, data.element_size()),
+                                 slot.work_ptr, slot.host_ptr, _stream_ptr(dev))
     if rc == _lib.FSB_OK:
         return y, None
     if rc == _lib.FSB_NOT_LAUNCHED:

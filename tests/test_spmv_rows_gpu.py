@@ -57,3 +57,23 @@ def test_what_neighbours_hold_stays_out(cuda, fsb_lib):
     want = torch.full((n,), float(length), device=cuda)
     want[100], want[205] = float("inf"), float("nan")
     assert torch.equal(torch.nan_to_num(y, nan=-1.0), torch.nan_to_num(want, nan=-1.0))
+
+
+@pytest.mark.parametrize("dtype", DTYPES, ids=str)
+def test_longest_row_at_the_line(cuda, fsb_lib, dtype):
+    """Either side of the longest row from which rows are spread over all SMs; the two launches give the same sums but for their order."""
+    from flagsparse_b200 import spmv_csr
+
+    n_cols, n = 6000, 9000
+    lens = [6] * n
+    line = spmv_csr._longest_neighbour(n, 6 * n, torch.empty(0, dtype=dtype).element_size())
+    for longest in (line, line + 2):                            # the mean grows by less than what moves the line by one
+        lens[n // 2] = longest
+        _, i, p = handmade_csr(9, lens, n_cols)
+        vals, x = _values(int(p[-1]), dtype, 6), _values(n_cols, dtype, 7)
+        d, ti, tp, tx = vals.to(cuda), torch.from_numpy(i).to(cuda), torch.from_numpy(p).to(cuda), x.to(cuda)
+        prep = fs.prepare_spmv_csr(d, ti, tp, (n, n_cols))
+        assert (prep.uneven != 0) == (longest > line)
+        y = fs.flagsparse_spmv_csr(x=tx, prepared=prep)
+        _check(y, vals, i, p, n_cols, x, dtype)
+        assert torch.equal(fs.flagsparse_spmv_csr(d, ti, tp, tx, (n, n_cols)), y)
