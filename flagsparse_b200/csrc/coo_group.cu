@@ -18,8 +18,8 @@ namespace fsb {
 constexpr int kCooThreads = 256;
 constexpr int kCooWarps = kCooThreads / 32;
 constexpr int kCooMost = 16;                        // entries of a thread, at most
-// Entries of a thread: 16, but 8 up to 3 M entries, which are fewer tiles of 4096 than the SMs hold at a time (1.3 M triples, four
-// passes: moves 93 us, with 16 and the scans of half as many tiles 76; 64000: 24 and 36; 5.2 M, two passes: 165 and 162).
+// Entries of a thread: 16, but 8 up to 3 M triples, which are fewer tiles of 4096 than the SMs hold at a time (us of all kernels with 8
+// against 16: 1.3 M triples, four passes, 20 less; 64000, 10 less; 5.2 M, two passes, 3 % more).
 static int coo_items(int64_t nnz) { return nnz <= 3 << 20 ? 8 : kCooMost; }
 constexpr int kCooMaxBits = 9;                      // of a digit: 8 warps x 512 counters in shared memory
 enum { C_PTR_FIRST = 0, C_PTR_LAST, C_DECREASING, C_MIN_COL, C_MAX_COL, C_MAX_ROW_NNZ, C_EMPTY, C_LONG, C_MIN_ROW, C_MAX_ROW, C_STATS };

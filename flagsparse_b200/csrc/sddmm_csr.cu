@@ -2,7 +2,7 @@
 // CSR pattern (X is n_rows x K, Y is n_cols x K, both row-major with a row stride).
 //
 // A group of LG lanes (LG = K / VW rounded up to a power of two, at most 32; VW = elements per 128-bit access)
-// owns batches of 8 consecutive entries.  A CTA first copies the column and row ids of its tile (up to 2048
+// owns batches of 8 consecutive entries.  A CTA first copies the column and row ids of its tile (about 1024
 // entries; the row of an entry comes from the row-id array built at prepare time, 4 bytes per entry) into shared
 // memory, so that the only trip to global memory inside the loop over batches is the gather; every lane then
 // requests its slice of all eight rows of Y through the read-only path before it uses any of them, so a group has
