@@ -47,9 +47,9 @@ FALLBACK_HBM_GBS = 6650.0
 # and of the entries), scaled by 16.
 _PANEL_SOURCES = ("flagsparse_b200/csrc/spmv_panel.cu", "flagsparse_b200/panel.py")
 NCU_TRAFFIC_BYTES = {
-    "c2": (1_098_036_480 + 2_980_864, _PANEL_SOURCES, "7b7e10f9eda5"),        # profiles/spmv_panel_c2_f32.md
-    "c2f64": (1_674_077_952 + 3_125_248, _PANEL_SOURCES, "7b7e10f9eda5"),     # profiles/spmv_panel_c2_f64.md
-    "c5": (16 * (1_127_085_568 + 3_224_064), _PANEL_SOURCES, "7b7e10f9eda5"),  # profiles/spmv_panel_c5like_f32.md
+    "c2": (1_097_986_560 + 2_890_752, _PANEL_SOURCES, "3d2e646b8047"),        # profiles/spmv_panel_c2_f32.md
+    "c2f64": (1_673_763_072 + 3_127_296, _PANEL_SOURCES, "3d2e646b8047"),     # profiles/spmv_panel_c2_f64.md
+    "c5": (16 * (1_127_049_984 + 3_202_048), _PANEL_SOURCES, "3d2e646b8047"),  # profiles/spmv_panel_c5like_f32.md
 }
 
 SPMV_WORKLOADS = {
