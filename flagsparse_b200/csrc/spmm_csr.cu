@@ -174,21 +174,22 @@ __host__ __device__ constexpr int mm_ctas(int nc, size_t size, bool with_long) {
 // balances as well but pays a row-end test per entry, and an even matrix then loses what a skewed one gains (2^20 rows
 // of 16 entries, 64 columns, float32: 615 us against 531 us).  `piece` depends on the number of columns and the value
 // type only (not on the alignment, which picks VW and LR), so the order of additions does too.
-// by_length: the segments of a tile are taken in the order of their lengths, the longest first: two to four groups share a warp, and
+// BY_LENGTH: the segments of a tile are taken in the order of their lengths, the longest first: two to four groups share a warp, and
 // those whose segment is shorter wait for the longest among them (us, in the order of the rows / by length: float32, 32 columns,
 // 300000 rows of 5 37 / 33, 262144 Zipf rows of 16 87 / 81; 64 columns, 2^19 rows of 16 231 / 225, Zipf 130 / 123; float64, 32 columns,
 // Zipf rows of 12 135 / 121).  Rows of one length lose what the sorting takes (2^20 of 16: 521 / 524), eight groups in a warp gain
 // nothing (16 columns: 40.1 / 40.3), one none (float64, 64 columns: 156 / 159), several accesses a lane spill (33 columns, Zipf 91 / 109).
+// (As an argument of the launch it costs those that do without: 1390783 rows of 9, 16 columns, 108.1 us, 106.7 us as it is.)
 // n_dense is covered by LR * NC accesses of VW elements per entry; wider products take column tiles (gridDim.y).
 // ACCUM: add to what C holds instead of overwriting it (rows without entries are then left alone) -- the later passes
 // of a product that the host code splits into column panels of A.
-template <typename S, typename I, int VW, int NC, bool LONG, bool ACCUM>
+template <typename S, typename I, int VW, int NC, bool LONG, bool ACCUM, bool BY_LENGTH>
 __global__ void __launch_bounds__(kMmThreads, mm_ctas(NC, sizeof(S), LONG))
 spmm_tile_kernel(const S* __restrict__ data, const I* __restrict__ idx, const void* __restrict__ ptr, int ptr64,
                  const S* __restrict__ B, int64_t ldb, S* __restrict__ C, int64_t ldc,
                  const int32_t* __restrict__ tile_row, typename MmOps<S>::Acc* __restrict__ carry,
                  typename MmOps<S>::Acc* __restrict__ head, int64_t nnz, int n_dense, int LR, int piece,
-                 int by_length, int use_bulk, int32_t* __restrict__ status) {
+                 int use_bulk, int32_t* __restrict__ status) {
   typedef MmOps<S> Ops;
   typedef typename Ops::Acc A;
   constexpr int T = kMmTile;
@@ -204,8 +205,8 @@ spmm_tile_kernel(const S* __restrict__ data, const I* __restrict__ idx, const vo
   __shared__ int s_head_partial;
   __shared__ int s_failed;
   __shared__ int s_n_long, s_n_pieces;
-  __shared__ uint16_t s_order[NC == 1 ? RC : 1];          // segments by length
-  __shared__ int s_bucket[kMmBuckets];
+  __shared__ uint16_t s_order[BY_LENGTH ? RC : 1];        // segments by length
+  __shared__ int s_bucket[BY_LENGTH ? kMmBuckets : 1];
   extern __shared__ __align__(16) unsigned char s_parts[];
 
   const int tid = threadIdx.x;
@@ -369,7 +370,7 @@ spmm_tile_kernel(const S* __restrict__ data, const I* __restrict__ idx, const vo
       return;
     }
 
-    if (NC == 1 && by_length) {
+    if constexpr (BY_LENGTH) {
       auto bucket = [&](int k) {                 // the longest first
         const int len = s_off[k + 1] - s_off[k];
         return kMmBuckets - 1 - (len < 2 * kMmBuckets - 2 ? len : 2 * kMmBuckets - 2) / 2;
@@ -394,7 +395,7 @@ spmm_tile_kernel(const S* __restrict__ data, const I* __restrict__ idx, const vo
       __syncthreads();
     }
     for (int q = grp; q < m; q += ngrp) {
-      const int k = NC == 1 && by_length ? s_order[q] : q;
+      const int k = BY_LENGTH ? s_order[q] : q;
       const int s = s_off[k], e = s_off[k + 1];
       if (LONG && e - s > 2 * piece) {
         if (lane == 0) {
@@ -547,28 +548,34 @@ static int launch_spmm(const SpmmArgs& a, int LR, int piece) {
   A* head = carry + n_tiles * n_dense;
   const int bulk = a.algo != FSB_SPMM_PLAIN && aligned_to(a.data, 16) && aligned_to(a.idx, 16);
   const dim3 grid((unsigned)n_tiles, (unsigned)col_tiles);
-  const int by_length = a.uneven_rows && NC == 1 && LR >= 8 && LR < 32;
-#define FSB_SPMM_LAUNCH(LONG_, ACC_, SMEM_)                                                                          \
-  spmm_tile_kernel<S, I, VW, NC, LONG_, ACC_><<<grid, kMmThreads, SMEM_, a.st>>>(                                    \
+  const bool by_length = a.uneven_rows && !a.accumulate && NC == 1 && LR >= 8 && LR < 32;
+#define FSB_SPMM_LAUNCH(LONG_, ACC_, LEN_, SMEM_)                                                                    \
+  spmm_tile_kernel<S, I, VW, NC, LONG_, ACC_, LEN_><<<grid, kMmThreads, SMEM_, a.st>>>(                              \
       (const S*)a.data, (const I*)a.idx, a.ptr, a.ptype == FSB_I64, (const S*)a.B, a.ldb, (S*)a.C, a.ldc, a.tile_row, \
-      carry, head, a.nnz, n_dense, LR, piece, by_length, bulk, a.status)
+      carry, head, a.nnz, n_dense, LR, piece, bulk, a.status)
   // the long segments of a tile (more than 2 * piece entries each) have at most T / piece + T / (2 * piece) pieces
   const size_t parts = a.long_rows ? (size_t)(T / piece + T / (2 * piece)) * width * sizeof(A) : 0;
   if (a.accumulate && !REAL) return FSB_EINVAL;
   if (a.long_rows) {
     if constexpr (NC == 1 || VW * (int)sizeof(S) < 16) {       // spmm_shape gives long rows no other
       if constexpr (REAL) {
-        if (a.accumulate) FSB_SPMM_LAUNCH(true, true, parts);
+        if (a.accumulate) FSB_SPMM_LAUNCH(true, true, false, parts);
       }
-      if (!a.accumulate) FSB_SPMM_LAUNCH(true, false, parts);
+      if constexpr (NC == 1) {
+        if (by_length) FSB_SPMM_LAUNCH(true, false, true, parts);
+      }
+      if (!a.accumulate && !by_length) FSB_SPMM_LAUNCH(true, false, false, parts);
     } else {
       return FSB_EINVAL;
     }
   } else {
     if constexpr (REAL) {
-      if (a.accumulate) FSB_SPMM_LAUNCH(false, true, 0);
+      if (a.accumulate) FSB_SPMM_LAUNCH(false, true, false, 0);
     }
-    if (!a.accumulate) FSB_SPMM_LAUNCH(false, false, 0);
+    if constexpr (NC == 1) {
+      if (by_length) FSB_SPMM_LAUNCH(false, false, true, 0);
+    }
+    if (!a.accumulate && !by_length) FSB_SPMM_LAUNCH(false, false, false, 0);
   }
 #undef FSB_SPMM_LAUNCH
   FSB_RETURN_IF_LAUNCH_FAILED();
