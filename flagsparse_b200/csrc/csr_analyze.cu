@@ -234,11 +234,12 @@ int csr_check_launch(int itype, int ptype, const void* indices, const void* indp
   if (rc != FSB_OK) return rc;
   if (work == nullptr || host == nullptr) return FSB_EINVAL;
   if (!aligned_to(work, 8) || !aligned_to(host, 8)) return FSB_EALIGN;
+  // counted here, not from what the GPU wrote last: no two calls wait for the same number, however the earlier one ended
+  const int64_t ticket = ++host[kCheckTicket + 1];
   cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-  const cudaError_t e = cudaStreamIsCapturing(stream, &capturing);
+  cudaError_t e = cudaStreamIsCapturing(stream, &capturing);
   if (e != cudaSuccess) return cuda_rc(e);
   if (capturing != cudaStreamCaptureStatusNone) return FSB_CAPTURING;        // nothing would run before the wait
-  const int64_t ticket = host[kCheckTicket] + 1;
   const int wide_loads = nnz > 0 && aligned_to(indices, 16);
 #define FSB_CHECK_CSR(I_, P_)                                                                                        \
   csr_check_kernel<I_, P_><<<stats_grid(itype, n_rows, nnz), 256, 0, stream>>>(                                      \
@@ -250,9 +251,13 @@ int csr_check_launch(int itype, int ptype, const void* indices, const void* indp
     if (ptype == FSB_I32) FSB_CHECK_CSR(int64_t, int32_t); else FSB_CHECK_CSR(int64_t, int64_t);
   }
 #undef FSB_CHECK_CSR
-  FSB_RETURN_IF_LAUNCH_FAILED();
-  host[kCheckTicket + 1] = ticket;     // what the wait looks for
-  return FSB_OK;
+  e = cudaGetLastError();
+  if (e == cudaSuccess) return FSB_OK;
+  // an older error of this thread may be what is reported, with the kernel on its way: `work` and `host` are the caller's again
+  // only when it has ended
+  const int rc_launch = cuda_rc(e);
+  (void)cuda_rc(cudaStreamSynchronize(stream));
+  return rc_launch;
 }
 
 int csr_check_wait(const int64_t* host, cudaStream_t stream) {

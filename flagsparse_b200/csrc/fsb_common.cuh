@@ -9,7 +9,12 @@
 
 namespace fsb {
 
-inline int cuda_rc(cudaError_t e) { return e == cudaSuccess ? FSB_OK : FSB_CUDA_ERROR_BASE + (int)e; }
+// An error that is returned here is taken from the runtime, too: the next launch of the thread is not blamed for it.
+inline int cuda_rc(cudaError_t e) {
+  if (e == cudaSuccess) return FSB_OK;
+  (void)cudaGetLastError();
+  return FSB_CUDA_ERROR_BASE + (int)e;
+}
 
 #define FSB_RETURN_IF_LAUNCH_FAILED()                      \
   do {                                                     \

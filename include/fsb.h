@@ -91,8 +91,8 @@ int fsb_csr_analyze(int itype, int ptype, const void* indices, const void* indpt
 /*
  * The same eight numbers for a host that waits for them.  work: 7 uint64 on the device, zero before the first call and left so by
  * every call; host: 10 int64 of page-locked memory, zero before the first call: [0..7] the statistics, [8] and [9] tickets of the
- * last run and the last call.  Both belong to one call at a time (one pair per thread).  Returns when the numbers are there;
- * FSB_CAPTURING, with nothing enqueued, while the stream is being captured.
+ * last run and the last call.  Both belong to one call at a time (one pair per thread).  Returns when the numbers are there, or with
+ * an error when nothing is on its way any more; FSB_CAPTURING, with nothing enqueued, while the stream is being captured.
  */
 int fsb_csr_check(int itype, int ptype, const void* indices, const void* indptr, int64_t n_rows, int64_t nnz, void* work,
                   int64_t* host, void* stream);

@@ -115,3 +115,16 @@ def test_not_while_a_stream_is_captured(cuda, fsb_lib):
             fs.flagsparse_spmv_csr(d, i, p, x, shape)
     torch.cuda.synchronize()
     assert torch.equal(fs.flagsparse_spmv_csr(d, i, p, x, shape), want)
+
+
+def test_a_check_after_one_that_was_not_waited_for(cuda, fsb_lib):
+    """Words as a call leaves them that returned before its kernel had ended: the next one counts on from that call's ticket."""
+    d, i, p, shape = _matrix(300, 90)
+    _common._analyze_csr(i, p, 300)
+    slot = _common._check_slot(i.device)
+    words = slot.host
+    words[9] += 3
+    last = int(words[9])
+    assert int(words[8]) == last - 3
+    s = _common._analyze_csr(i, p, 300)
+    assert int(words[8]) == int(words[9]) == last + 1 and s.ptr_last == d.numel()

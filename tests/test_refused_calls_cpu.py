@@ -42,3 +42,18 @@ def test_plan_and_analysis(fsb_lib):
     assert look(0, 0, BASE + 2, BASE, BASE) == EALIGN and look(1, 0, BASE + 4, BASE, BASE) == EALIGN
     assert look(0, 0, BASE, BASE + 2, BASE) == EALIGN and look(0, 1, BASE, BASE + 4, BASE) == EALIGN
     assert look(0, 0, BASE, BASE, BASE + 4) == EALIGN
+
+
+def test_no_two_checks_wait_for_the_same_ticket(fsb_lib):
+    """Words as a call leaves them that returned before its kernel had ended (ticket 9 on its way, 7 the last that was written):
+    the next call, here one that finds no device, moves on to a number of its own."""
+    import ctypes
+
+    import torch
+
+    if torch.cuda.is_available():
+        pytest.skip("for a machine on which nothing can be launched")
+    host = (ctypes.c_int64 * 10)(*[0] * 8, 7, 9)
+    for ticket in (10, 11):
+        rc = fsb_lib.fsb_csr_check(0, 0, BASE, BASE, 100, 5000, BASE, ctypes.addressof(host), None)
+        assert rc > _lib.FSB_CUDA_ERROR_BASE and list(host) == [0] * 8 + [7, ticket]
