@@ -130,15 +130,6 @@ __device__ __forceinline__ void comp_add(double& sum, double& comp, double v) {
 }
 __device__ __forceinline__ double comp_term(double sum, double comp) { return isfinite(sum) ? comp : 0.0; }
 
-// The same for the partial sums of a row that crosses tiles, of type R.  Doubles hold so many more digits than float partial sums do
-// that nothing is gained by compensating: 64 of them add less than 2^-47 of their magnitudes.  A compensated step takes about
-// 0.23 us where one thread takes them one after the other, a plain one with its load 0.1 us.
-template <typename R>
-__device__ __forceinline__ void carry_add(double& sum, double& comp, double v) {
-  if constexpr (sizeof(R) == 4) sum += v;
-  else comp_add(sum, comp, v);
-}
-
 __device__ __forceinline__ int pow2_floor(int v) { return v <= 1 ? 1 : (1 << (31 - __clz(v))); }
 
 }  // namespace fsb

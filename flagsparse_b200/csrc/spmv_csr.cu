@@ -375,7 +375,7 @@ spmv_fixup_kernel(const P* __restrict__ ptr, const int32_t* __restrict__ tile_ro
   const bool wide = need && ((long long)t - t0) > kFixupSerial;
   if (need && !wide) {
     double sum = (double)head[t], comp = 0.0;
-    for (int64_t u = t0; u < t; ++u) carry_add<V>(sum, comp, (double)carry[u]);
+    for (int64_t u = t0; u < t; ++u) comp_add(sum, comp, (double)carry[u]);
     out.store((int64_t)ra, (V)(sum + comp_term(sum, comp)));
   }
   unsigned todo = __ballot_sync(0xffffffffu, wide);
@@ -385,18 +385,18 @@ spmv_fixup_kernel(const P* __restrict__ ptr, const int32_t* __restrict__ tile_ro
     const long long a = __shfl_sync(0xffffffffu, t0, src);
     const long long b = __shfl_sync(0xffffffffu, (long long)t, src);
     double sum = 0.0, comp = 0.0;
-    for (long long u = a + lane; u < b; u += 32) carry_add<V>(sum, comp, (double)carry[u]);
+    for (long long u = a + lane; u < b; u += 32) comp_add(sum, comp, (double)carry[u]);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       const double os = __shfl_down_sync(0xffffffffu, sum, o);
       const double oc = __shfl_down_sync(0xffffffffu, comp, o);
-      carry_add<V>(sum, comp, os);
+      comp_add(sum, comp, os);
       comp += oc;
     }
     sum = __shfl_sync(0xffffffffu, sum, 0);
     comp = __shfl_sync(0xffffffffu, comp, 0);
     if (lane == src) {
-      carry_add<V>(sum, comp, (double)head[t]);
+      comp_add(sum, comp, (double)head[t]);
       out.store((int64_t)ra, (V)(sum + comp_term(sum, comp)));
     }
   }
