@@ -87,6 +87,9 @@ SIGNATURES = {
     "fsb_spmm_csr_stored": (
         _i32, [_i32, _i32, _vp, _vp, _vp, _vp, _i64, _vp, _i64, _i64, _i64, _i64, _i64, _i32, _vp, _sz, _vp],
     ),
+    "fsb_spmm_csr_stored_rows": (
+        _i32, [_i32, _i32, _vp, _vp, _vp, _vp, _i64, _vp, _i64, _i64, _i64, _i64, _i64, _i32, _vp, _sz, _vp],
+    ),
     "fsb_spmv_stored_tile_nnz": (_i32, [_i32]),
     "fsb_spmv_stored_scratch_bytes": (_sz, [_i32, _i64]),
     "fsb_spmv_csr_stored": (_i32, [_i32, _i32, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _vp, _vp, _sz, _vp]),

@@ -785,12 +785,19 @@ extern "C" int fsb_spmm_csr_stored(int vtype, int ptype, const void* data, const
                                    const void* B, int64_t ldb, void* C, int64_t ldc, int64_t n_rows, int64_t n_cols,
                                    int64_t n_dense, int64_t nnz, int long_rows, void* scratch, size_t scratch_bytes,
                                    void* stream_) {
+  return fsb_spmm_csr_stored_rows(vtype, ptype, data, indices, indptr, B, ldb, C, ldc, n_rows, n_cols, n_dense, nnz,
+                                  long_rows ? FSB_SPMM_LONG_ROWS : 0, scratch, scratch_bytes, stream_);
+}
+
+extern "C" int fsb_spmm_csr_stored_rows(int vtype, int ptype, const void* data, const int32_t* indices, const void* indptr,
+                                        const void* B, int64_t ldb, void* C, int64_t ldc, int64_t n_rows, int64_t n_cols,
+                                        int64_t n_dense, int64_t nnz, int hints, void* scratch, size_t scratch_bytes,
+                                        void* stream_) {
   if (vtype != FSB_F16 && vtype != FSB_BF16 && vtype != FSB_C64 && vtype != FSB_C128) return FSB_EINVAL;
+  if (hints & ~(FSB_SPMM_LONG_ROWS | FSB_SPMM_UNEVEN_ROWS)) return FSB_EINVAL;
   // staged by ordinary loads: no copy whose end would have to be waited for and reported
   return spmm_run(vtype, FSB_I32, ptype, data, indices, indptr, B, ldb, C, ldc, n_rows, n_cols, n_dense, nnz,
-                  FSB_SPMM_PLAIN | (long_rows & ~FSB_SPMM_UNEVEN_ROWS ? FSB_SPMM_LONG_ROWS : 0) | (long_rows & FSB_SPMM_UNEVEN_ROWS),
-                  nullptr, true, scratch, scratch_bytes, nullptr,
-                  static_cast<cudaStream_t>(stream_));
+                  FSB_SPMM_PLAIN | hints, nullptr, true, scratch, scratch_bytes, nullptr, static_cast<cudaStream_t>(stream_));
 }
 
 extern "C" int fsb_spmm_csr_once(int vtype, int itype, int ptype, const void* data, const void* indices, const void* indptr,

@@ -261,7 +261,7 @@ class PreparedCsrSpmmOpt:
         self._whole = None       # the matrix as one _CsrPart (shares the tile plan)
         self._panels = {}        # number of column panels -> list of _CsrPart
         self._span = None        # columns spanned by a window of consecutive entries (median over samples)
-        # float16 / bfloat16 / complex values: ("native", []) -- the product goes through fsb_spmm_csr_stored
+        # float16 / bfloat16 / complex values: ("native", []) -- the product goes through fsb_spmm_csr_stored_rows
         self.wide = wide
 
     def __getattr__(self, name):
@@ -382,7 +382,7 @@ def _prepare_spmm(data, indices, indptr, shape, once, known=None):
         kernel_indices, kernel_indptr, (n_rows, n_cols), stats = indices, indptr, shape, known
     nnz = data.numel()
     if data.dtype in widetypes.WIDE_DTYPES:
-        # read as stored by fsb_spmm_csr_stored, which plans its tiles itself: no second copy of the matrix
+        # read as stored by fsb_spmm_csr_stored_rows, which plans its tiles itself: no second copy of the matrix
         return PreparedCsrSpmmOpt(data, kernel_indices, kernel_indptr, shape, n_rows, n_cols, stats, 0, None,
                                   wide=("native", []))
     tile_nnz, tile_row = 0, None
@@ -468,12 +468,13 @@ def _spmm_launch_stored(prepared, B, C):
     vt = _STORED_VTYPE[p.data.dtype]
     scratch = torch.empty(int(L.fsb_spmm_stored_scratch_bytes(vt, nnz, n_dense)), dtype=torch.uint8, device=dev)
     with _on_device(dev):
-        rc = L.fsb_spmm_csr_stored(
+        rc = L.fsb_spmm_csr_stored_rows(
             vt, _ITYPE[p.kernel_indptr.dtype], _ptr(p.data), _ptr(p.kernel_indices), p.kernel_indptr.data_ptr(),
             _ptr(B), B.stride(0) if B.shape[0] > 1 else n_dense, C.data_ptr(), n_dense, p.n_rows, p.n_cols, n_dense, nnz,
-            int(_shares_long_rows(p.max_row_nnz, n_dense, B.element_size())) | p._uneven, scratch.data_ptr(), scratch.numel(), _stream_ptr(dev),
+            (_lib.FSB_SPMM_LONG_ROWS if _shares_long_rows(p.max_row_nnz, n_dense, B.element_size()) else 0) | p._uneven,
+            scratch.data_ptr(), scratch.numel(), _stream_ptr(dev),
         )
-    _lib.check(rc, "fsb_spmm_csr_stored")
+    _lib.check(rc, "fsb_spmm_csr_stored_rows")
 
 
 def _run_spmm(prepared, B, out, return_time):

@@ -377,12 +377,16 @@ int fsb_spmm_csr_wide(int vtype, int ptype, const void* data, const int32_t* ind
  * C = A B for the same four value types with B and C in the matrix's own type (half precisions: 2-byte values read as
  * they are stored, products and sums in float32, every element of C rounded once).  The tiled kernel of fsb_spmm_csr,
  * its tile plan made in scratch (fsb_spmm_stored_scratch_bytes() bytes, 16-byte aligned); long_rows != 0 is
- * FSB_SPMM_LONG_ROWS, but for FSB_SPMM_UNEVEN_ROWS in it, which is what it is there.
+ * FSB_SPMM_LONG_ROWS.  fsb_spmm_csr_stored_rows: the same with both hints on the rows, FSB_SPMM_LONG_ROWS and
+ * FSB_SPMM_UNEVEN_ROWS or-ed together.
  */
 size_t fsb_spmm_stored_scratch_bytes(int vtype, int64_t nnz, int64_t n_dense);
 int fsb_spmm_csr_stored(int vtype, int ptype, const void* data, const int32_t* indices, const void* indptr,
                         const void* B, int64_t ldb, void* C, int64_t ldc, int64_t n_rows, int64_t n_cols,
                         int64_t n_dense, int64_t nnz, int long_rows, void* scratch, size_t scratch_bytes, void* stream);
+int fsb_spmm_csr_stored_rows(int vtype, int ptype, const void* data, const int32_t* indices, const void* indptr,
+                             const void* B, int64_t ldb, void* C, int64_t ldc, int64_t n_rows, int64_t n_cols,
+                             int64_t n_dense, int64_t nnz, int hints, void* scratch, size_t scratch_bytes, void* stream);
 
 /*
  * COO triples grouped by row (nnz > 0): values and columns in row order -- entries of a row in the order in which they are

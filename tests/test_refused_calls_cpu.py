@@ -57,3 +57,11 @@ def test_no_two_checks_wait_for_the_same_ticket(fsb_lib):
     for ticket in (10, 11):
         rc = fsb_lib.fsb_csr_check(0, 0, BASE, BASE, 100, 5000, BASE, ctypes.addressof(host), None)
         assert rc > _lib.FSB_CUDA_ERROR_BASE and list(host) == [0] * 8 + [7, ticket]
+
+
+@pytest.mark.parametrize("vtype", [_lib.FSB_F16, _lib.FSB_BF16, _lib.FSB_C64, _lib.FSB_C128])
+def test_hints_are_arguments_of_their_own(fsb_lib, vtype):
+    """Only hints that there are."""
+    for hints in (1, 16, 32 + 128):
+        assert fsb_lib.fsb_spmm_csr_stored_rows(vtype, 0, BASE, BASE, BASE, BASE, 8, BASE, 8, 100, 100, 8, 5000, hints, BASE, 1 << 30,
+                                                None) == EINVAL

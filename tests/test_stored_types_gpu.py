@@ -139,3 +139,27 @@ def test_spmm_segments_by_length(cuda, fsb_lib, dtype):
             C = fs.flagsparse_spmm_csr(d, ti, tp, B.to(cuda), (len(p) - 1, n_cols))
             _check(C, vals, i, p, n_cols, B, dtype)
             assert torch.equal(fs.flagsparse_spmm_csr(d, ti, tp, B.to(cuda), (len(p) - 1, n_cols)), C)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.complex64, torch.complex128], ids=str)
+def test_any_nonzero_long_rows_shares_them(cuda, fsb_lib, dtype):
+    """fsb_spmm_csr_stored takes long_rows as yes or no: every value but 0 gives the sums of rows that a block shares."""
+    from flagsparse_b200.spmm_csr import _STORED_VTYPE
+
+    n_cols, n_dense = 2000, 24
+    _, i, p = handmade_csr(13, [900, 3, 500, 700, 0, 8] * 20, n_cols)
+    n = len(p) - 1
+    vals, B = _values(int(p[-1]), dtype, 4), _values((n_cols, n_dense), dtype, 5)
+    d, ti, tp, tb = vals.to(cuda), torch.from_numpy(i).to(cuda), torch.from_numpy(p).to(cuda), B.to(cuda)
+    vt = _STORED_VTYPE[dtype]
+    scratch = torch.empty(fsb_lib.fsb_spmm_stored_scratch_bytes(vt, d.numel(), n_dense), dtype=torch.uint8, device=cuda)
+    got = {}
+    for yes in (0, 1, 64, 3):
+        got[yes] = torch.empty((n, n_dense), dtype=dtype, device=cuda)
+        assert fsb_lib.fsb_spmm_csr_stored(vt, 0, d.data_ptr(), ti.data_ptr(), tp.data_ptr(), tb.data_ptr(), n_dense,
+                                           got[yes].data_ptr(), n_dense, n, n_cols, n_dense, d.numel(), yes, scratch.data_ptr(),
+                                           scratch.numel(), torch.cuda.current_stream().cuda_stream) == 0
+    assert torch.equal(got[64], got[1]) and torch.equal(got[3], got[1])
+    if dtype != torch.float16 and dtype != torch.bfloat16:      # (the rounding of the result hides the order of the sums)
+        assert not torch.equal(got[0], got[1])
+    _check(got[64], vals, i, p, n_cols, B, dtype)
