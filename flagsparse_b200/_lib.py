@@ -22,7 +22,7 @@ FSB_SPMV_PANEL = 3  # host-side tag only: the panel kernel has its own entry poi
 FSB_SPMM_AUTO, FSB_SPMM_PLAIN, FSB_SPMM_BULK = 0, 1, 2
 FSB_SPMM_ACCUMULATE = 16  # or-ed into the selector: C += A B
 FSB_SPMM_LONG_ROWS = 32   # or-ed into the selector: long rows are shared by a block
-FSB_SPMV_UNEVEN_ROWS = 1024 # or-ed into the tuning of FSB_SPMV_VECTOR and the ptype of fsb_spmv_csr_stored
+FSB_SPMV_EVEN_ROWS = 1024 # or-ed into the tuning of FSB_SPMV_VECTOR: rows of about equal length
 FSB_SPMM_UNEVEN_ROWS = 64 # or-ed into the selector: the longest row is above 5/4 of the mean
 FSB_OK, FSB_NOT_LAUNCHED, FSB_CAPTURING = 0, 1, 2
 FSB_CUDA_ERROR_BASE = 1000
@@ -93,6 +93,7 @@ SIGNATURES = {
     "fsb_spmv_stored_tile_nnz": (_i32, [_i32]),
     "fsb_spmv_stored_scratch_bytes": (_sz, [_i32, _i64]),
     "fsb_spmv_csr_stored": (_i32, [_i32, _i32, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _vp, _vp, _sz, _vp]),
+    "fsb_spmv_csr_stored_even": (_i32, [_i32, _i32, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _vp]),
     "fsb_spmv_csr_wide": (_i32, [_i32, _i32, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _vp]),
     "fsb_spmm_csr_wide": (_i32, [_i32, _i32, _vp, _vp, _vp, _vp, _i64, _vp, _i64, _i64, _i64, _i64, _i64, _vp]),
     "fsb_coo_scratch_bytes": (_sz, [_i64]),

@@ -483,7 +483,7 @@ spmv_stored_fixup_kernel(const P* __restrict__ ptr, const int32_t* __restrict__ 
 
 template <typename S, typename P>
 static int stored_launch(const void* data_, const int32_t* idx, const void* ptr_, const void* x_, void* y_, int64_t n_rows,
-                         int64_t nnz, bool uneven, const int32_t* tile_row, void* scratch, cudaStream_t st) {
+                         int64_t nnz, bool even, const int32_t* tile_row, void* scratch, cudaStream_t st) {
   typedef typename StoredOps<S>::A A;
   const S* data = (const S*)data_;
   const P* ptr = (const P*)ptr_;
@@ -511,7 +511,7 @@ static int stored_launch(const void* data_, const int32_t* idx, const void* ptr_
     }
     return FSB_OK;
   }
-  if (!uneven && rows_apply(data, idx, n_rows, nnz))
+  if (even && rows_apply(data, idx, n_rows, nnz))
     return rows_run<S, int32_t, P>(data, idx, ptr, x, RowsOut<S>{y}, n_rows, nnz, st);
   // two to four groups of four entries per lane, as in the float32 / float64 kernel; entry by entry, three to six
   // (columns anywhere, 4 / 8 / 16 lanes a row: complex64, 500009 rows of 24: 70 / 64 / - us, 300000 rows of 30: 55 / 47 / 51 us,
@@ -558,13 +558,10 @@ extern "C" size_t fsb_spmv_stored_scratch_bytes(int vtype, int64_t nnz) {
   return ((size_t)fsb_csr_num_tiles(nnz, fsb_spmv_stored_tile_nnz(vtype)) * 2 * sa + 255) & ~(size_t)255;
 }
 
-extern "C" int fsb_spmv_csr_stored(int vtype, int ptype, const void* data, const int32_t* indices, const void* indptr,
-                                   const void* x, void* y, int64_t n_rows, int64_t n_cols, int64_t nnz,
-                                   const int32_t* tile_row, void* scratch, size_t scratch_bytes, void* stream_) {
-  cudaStream_t st = static_cast<cudaStream_t>(stream_);
+static int spmv_stored(int vtype, int ptype, const void* data, const int32_t* indices, const void* indptr, const void* x, void* y,
+                       int64_t n_rows, int64_t n_cols, int64_t nnz, bool even, const int32_t* tile_row, void* scratch,
+                       size_t scratch_bytes, cudaStream_t st) {
   if (vtype != FSB_F16 && vtype != FSB_BF16 && vtype != FSB_C64 && vtype != FSB_C128) return FSB_EINVAL;
-  const bool uneven = (ptype & FSB_SPMV_UNEVEN_ROWS) != 0;
-  ptype &= ~FSB_SPMV_UNEVEN_ROWS;
   if (ptype != FSB_I32 && ptype != FSB_I64) return FSB_EINVAL;
   if (n_rows < 0 || n_cols < 0 || nnz < 0) return FSB_EINVAL;
   if (n_rows >= INT32_MAX || n_cols >= INT32_MAX) return FSB_ERANGE;
@@ -584,8 +581,8 @@ extern "C" int fsb_spmv_csr_stored(int vtype, int ptype, const void* data, const
   FSB_WALK_FIRST(check_csr(FSB_I32, ptype, indices, indptr, n_rows, n_cols, nnz, st));
 #define FSB_STORED_TYPE(S_)                                                                                           \
   return ptype == FSB_I32                                                                                             \
-             ? stored_launch<S_, int32_t>(data, indices, indptr, x, y, n_rows, nnz, uneven, tile_row, scratch, st)    \
-             : stored_launch<S_, int64_t>(data, indices, indptr, x, y, n_rows, nnz, uneven, tile_row, scratch, st)
+             ? stored_launch<S_, int32_t>(data, indices, indptr, x, y, n_rows, nnz, even, tile_row, scratch, st)      \
+             : stored_launch<S_, int64_t>(data, indices, indptr, x, y, n_rows, nnz, even, tile_row, scratch, st)
   switch (vtype) {
     case FSB_F16: FSB_STORED_TYPE(__half);
     case FSB_BF16: FSB_STORED_TYPE(__nv_bfloat16);
@@ -593,6 +590,19 @@ extern "C" int fsb_spmv_csr_stored(int vtype, int ptype, const void* data, const
     default: FSB_STORED_TYPE(double2);
   }
 #undef FSB_STORED_TYPE
+}
+
+extern "C" int fsb_spmv_csr_stored(int vtype, int ptype, const void* data, const int32_t* indices, const void* indptr,
+                                   const void* x, void* y, int64_t n_rows, int64_t n_cols, int64_t nnz,
+                                   const int32_t* tile_row, void* scratch, size_t scratch_bytes, void* stream_) {
+  return spmv_stored(vtype, ptype, data, indices, indptr, x, y, n_rows, n_cols, nnz, false, tile_row, scratch, scratch_bytes,
+                     static_cast<cudaStream_t>(stream_));
+}
+
+extern "C" int fsb_spmv_csr_stored_even(int vtype, int ptype, const void* data, const int32_t* indices, const void* indptr,
+                                        const void* x, void* y, int64_t n_rows, int64_t n_cols, int64_t nnz, void* stream_) {
+  return spmv_stored(vtype, ptype, data, indices, indptr, x, y, n_rows, n_cols, nnz, true, nullptr, nullptr, 0,
+                     static_cast<cudaStream_t>(stream_));
 }
 
 // Check and product of arrays that are used once, whatever the value type.
@@ -606,10 +616,10 @@ extern "C" int fsb_spmv_csr_once(int vtype, int itype, int ptype, const void* da
   if (rc == FSB_OK) rc = csr_check_wait(host, st);
   if (rc != FSB_OK) return rc;
   if (!csr_check_passed(host, n_cols, nnz) || csr_check_longest(host) > longest) return FSB_NOT_LAUNCHED;
-  const int uneven = csr_check_longest(host) > even ? FSB_SPMV_UNEVEN_ROWS : 0;
+  const bool is_even = csr_check_longest(host) <= even;
   if (stored)
-    return fsb_spmv_csr_stored(vtype, ptype | uneven, data, (const int32_t*)indices, indptr, x, y, n_rows, n_cols, nnz, nullptr,
-                               nullptr, 0, stream_);
-  return fsb_spmv_csr(vtype, itype, ptype, data, indices, indptr, x, y, n_rows, n_cols, nnz, FSB_SPMV_VECTOR, uneven, nullptr,
-                      nullptr, 0, stream_);
+    return spmv_stored(vtype, ptype, data, (const int32_t*)indices, indptr, x, y, n_rows, n_cols, nnz, is_even, nullptr, nullptr, 0,
+                       st);
+  return fsb_spmv_csr(vtype, itype, ptype, data, indices, indptr, x, y, n_rows, n_cols, nnz, FSB_SPMV_VECTOR,
+                      is_even ? FSB_SPMV_EVEN_ROWS : 0, nullptr, nullptr, 0, stream_);
 }

@@ -162,8 +162,8 @@ class PreparedCsrSpmv:
         self.block_nnz = block_nnz
         self.max_segments = max_segments
         self.max_row_nnz = max_row_nnz
-        even = _longest_neighbour(n_rows, data.numel(), data.element_size())
-        self.uneven = _lib.FSB_SPMV_UNEVEN_ROWS if max_row_nnz > even else 0
+        # whether a row is too long for neighbouring rows to stay on one SM
+        self.uneven = max_row_nnz > _longest_neighbour(n_rows, data.numel(), data.element_size())
         self.supports_opt = data.dtype in (torch.float32, torch.float64)
         self.stats = stats
         self.algo = algo
@@ -190,6 +190,10 @@ class PreparedCsrSpmv:
         if self.long_rows is not None:
             yield self.long_rows[1].status
             yield from self.long_rows[0]._status_words()
+
+    def vector_tuning(self):
+        """What fsb_spmv_csr is told of the rows when FSB_SPMV_VECTOR picks its lanes itself."""
+        return 0 if self.uneven else _lib.FSB_SPMV_EVEN_ROWS
 
     def check_status(self):
         """Wait for the last product on this matrix and raise RuntimeError if one of its kernels gave up on a
@@ -403,7 +407,7 @@ def _spmv_launch(prepared, x, y):
     if scratch is not None and (p.data.numel() < _STREAM_MIN_NNZ or p.bins is not None):
         scratch = torch.empty_like(scratch)
     lanes = p.tuning & 0xFF
-    tuning = p.tuning if algo == _lib.FSB_SPMV_STREAM else (lanes if lanes in (2, 4, 8, 16, 32) else p.uneven)
+    tuning = p.tuning if algo == _lib.FSB_SPMV_STREAM else (lanes if lanes in (2, 4, 8, 16, 32) else p.vector_tuning())
     with _on_device(dev):
         rc = L.fsb_spmv_csr(
             _VTYPE[p.data.dtype], _ITYPE[p.kernel_indices.dtype], _ITYPE[p.kernel_indptr.dtype],
@@ -429,12 +433,13 @@ def _spmv_launch_stored(prepared, x, y):
         scratch = torch.empty(int(L.fsb_spmv_stored_scratch_bytes(_WIDE_VTYPE[p.data.dtype], p.data.numel())),
                               dtype=torch.uint8, device=dev)
     with _on_device(dev):
-        rc = L.fsb_spmv_csr_stored(
-            _WIDE_VTYPE[p.data.dtype], _ITYPE[p.kernel_indptr.dtype] | p.uneven, _ptr(p.data), _ptr(p.kernel_indices),
-            p.kernel_indptr.data_ptr(), _ptr(x), _ptr(y), p.n_rows, p.n_cols, p.data.numel(),
-            None if p.tile_row is None else p.tile_row.data_ptr(), _ptr(scratch),
-            0 if scratch is None else scratch.numel(), _stream_ptr(dev),
-        )
+        args = (_WIDE_VTYPE[p.data.dtype], _ITYPE[p.kernel_indptr.dtype], _ptr(p.data), _ptr(p.kernel_indices),
+                p.kernel_indptr.data_ptr(), _ptr(x), _ptr(y), p.n_rows, p.n_cols, p.data.numel())
+        if p.tile_row is None and not p.uneven:
+            rc = L.fsb_spmv_csr_stored_even(*args, _stream_ptr(dev))
+        else:
+            rc = L.fsb_spmv_csr_stored(*args, None if p.tile_row is None else p.tile_row.data_ptr(), _ptr(scratch),
+                                       0 if scratch is None else scratch.numel(), _stream_ptr(dev))
     _lib.check(rc, "fsb_spmv_csr_stored")
 
 

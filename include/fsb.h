@@ -64,7 +64,7 @@ extern "C" {
 #define FSB_SPMM_BULK 2      /* tile staged by cp.async.bulk (TMA 1-D bulk copy) + mbarrier       */
 #define FSB_SPMM_ACCUMULATE 16 /* or-ed into the selector: C += A B instead of C = A B            */
 #define FSB_SPMM_LONG_ROWS 32  /* or-ed into the selector: some rows are long (see fsb_spmm_csr)  */
-#define FSB_SPMV_UNEVEN_ROWS 1024 /* or-ed into the tuning of FSB_SPMV_VECTOR and the ptype of fsb_spmv_csr_stored */
+#define FSB_SPMV_EVEN_ROWS 1024 /* or-ed into the tuning of FSB_SPMV_VECTOR: rows of about equal length */
 #define FSB_SPMM_UNEVEN_ROWS 64 /* or-ed into the selector: the longest row is above 5/4 of the mean */
 
 int fsb_version(void);
@@ -101,7 +101,7 @@ int fsb_csr_check(int itype, int ptype, const void* indices, const void* indptr,
  * Check and product of CSR arrays that are used once (fsb_csr_check, then the product of checked arrays): y = A x by the kernels for
  * rows of about equal length, C = A B.  Returns FSB_OK with the product enqueued, FSB_CAPTURING, or FSB_NOT_LAUNCHED without the
  * product: the arrays are not a CSR matrix of this shape (host tells why), or, y = A x, a row has more than `longest` entries.
- * even: entries of the longest row above which the rows count as FSB_SPMV_UNEVEN_ROWS.  All value types; other than float32 /
+ * even: entries of the longest row up to which the rows count as FSB_SPMV_EVEN_ROWS.  All value types; other than float32 /
  * float64 with 32-bit indices.  long_row: longest row up to
  * which rows are not shared by a block (FSB_SPMM_LONG_ROWS); scratch as for fsb_spmm_csr_stored.
  */
@@ -133,7 +133,8 @@ int fsb_csr_tile_plan(int ptype, const void* indptr, int64_t n_rows, int64_t nnz
  *             and `scratch` of at least fsb_spmv_csr_scratch_bytes() bytes, 16-byte aligned.
  *             FSB_SPMV_AUTO picks STREAM when tile_row and scratch are given and nnz is large, else VECTOR.
  *   tuning    0 = default; otherwise kernel-specific knob (VECTOR: lanes per row, a power of two 2..32,
- *             or FSB_SPMV_UNEVEN_ROWS: rows spread over all SMs, although there are enough to keep neighbours on one;
+ *             or FSB_SPMV_EVEN_ROWS: no row is much longer than the others (float32 10 means, float64 5), so neighbours
+ *             may stay on one SM, where there are enough of them; without it rows are spread over all SMs;
  *             STREAM: bits 0-7 = 1 + the right-shift applied to a tile's mean row length to get the
  *             lanes per row; bits 8-9 = tile size, see fsb_spmv_tile_nnz).  Results stay within tolerance for any value; only speed changes.
  * The result is deterministic: the same inputs give the same bits on every call (no floating atomics).
@@ -353,16 +354,18 @@ int fsb_spmv_csr_wide(int vtype, int ptype, const void* data, const int32_t* ind
 /*
  * y = A x for the same four value types with x and y in the matrix's own type (half precisions: products and sums in
  * float32, every element of y rounded once).  Without a plan (tile_row NULL) a group of 2 to 32 lanes walks each row:
- * for rows of about equal length; FSB_SPMV_UNEVEN_ROWS in ptype keeps these rows spread over all SMs instead of neighbours
- * on one.  With tile_row (fsb_csr_tile_plan, tile_nnz = fsb_spmv_stored_tile_nnz(vtype)) the work
+ * for rows of about equal length.  With tile_row (fsb_csr_tile_plan, tile_nnz = fsb_spmv_stored_tile_nnz(vtype)) the work
  * of a block does not depend on the row lengths; scratch then holds fsb_spmv_stored_scratch_bytes() bytes, 16-byte
- * aligned.  Bit-reproducible either way.
+ * aligned.  Bit-reproducible either way.  fsb_spmv_csr_stored_even: without a plan, where no row is much longer than the
+ * others (half precisions 10 means, complex64 5, complex128 3): FSB_SPMV_EVEN_ROWS of fsb_spmv_csr.
  */
 int fsb_spmv_stored_tile_nnz(int vtype);
 size_t fsb_spmv_stored_scratch_bytes(int vtype, int64_t nnz);
 int fsb_spmv_csr_stored(int vtype, int ptype, const void* data, const int32_t* indices, const void* indptr,
                         const void* x, void* y, int64_t n_rows, int64_t n_cols, int64_t nnz,
                         const int32_t* tile_row, void* scratch, size_t scratch_bytes, void* stream);
+int fsb_spmv_csr_stored_even(int vtype, int ptype, const void* data, const int32_t* indices, const void* indptr,
+                             const void* x, void* y, int64_t n_rows, int64_t n_cols, int64_t nnz, void* stream);
 
 /*
  * C = A B for the same four value types, with the same conventions (B and C float32 for the half precisions, of the

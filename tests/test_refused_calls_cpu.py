@@ -61,7 +61,10 @@ def test_no_two_checks_wait_for_the_same_ticket(fsb_lib):
 
 @pytest.mark.parametrize("vtype", [_lib.FSB_F16, _lib.FSB_BF16, _lib.FSB_C64, _lib.FSB_C128])
 def test_hints_are_arguments_of_their_own(fsb_lib, vtype):
-    """Only hints that there are."""
+    """An index type is an index type: nothing else rides in it; and only hints that there are."""
+    for ptype in (1024, 1025):
+        assert fsb_lib.fsb_spmv_csr_stored(vtype, ptype, BASE, BASE, BASE, BASE, BASE, 100, 100, 5000, None, None, 0, None) == EINVAL
+        assert fsb_lib.fsb_spmv_csr_stored_even(vtype, ptype, BASE, BASE, BASE, BASE, BASE, 100, 100, 5000, None) == EINVAL
     for hints in (1, 16, 32 + 128):
         assert fsb_lib.fsb_spmm_csr_stored_rows(vtype, 0, BASE, BASE, BASE, BASE, 8, BASE, 8, 100, 100, 8, 5000, hints, BASE, 1 << 30,
                                                 None) == EINVAL

@@ -77,3 +77,58 @@ def test_longest_row_at_the_line(cuda, fsb_lib, dtype):
         y = fs.flagsparse_spmv_csr(x=tx, prepared=prep)
         _check(y, vals, i, p, n_cols, x, dtype)
         assert torch.equal(fs.flagsparse_spmv_csr(d, ti, tp, tx, (n, n_cols)), y)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64], ids=str)
+def test_neighbours_stay_on_one_sm_only_where_the_caller_says_even(cuda, fsb_lib, dtype):
+    """FSB_SPMV_VECTOR with tuning 0 takes lanes per row, whatever the rows; FSB_SPMV_AUTO without a plan, too."""
+    from flagsparse_b200 import _lib
+    from flagsparse_b200._common import _VTYPE
+
+    n, n_cols, lanes = 9000, 3000, 4                            # 16 * 2 < 50 + 3, 16 * 4 is not
+    _, i, p = handmade_csr(11, [50] * n, n_cols)
+    vals, x = _values(int(p[-1]), dtype, 6), _values(n_cols, dtype, 7)
+    d, ti, tp, tx = vals.to(cuda), torch.from_numpy(i).to(cuda), torch.from_numpy(p).to(cuda), x.to(cuda)
+
+    def run(algo, tuning):
+        y = torch.full((n,), float("nan"), dtype=dtype, device=cuda)
+        assert fsb_lib.fsb_spmv_csr(_VTYPE[dtype], 0, 0, d.data_ptr(), ti.data_ptr(), tp.data_ptr(), tx.data_ptr(), y.data_ptr(), n,
+                                    n_cols, d.numel(), algo, tuning, None, None, 0, torch.cuda.current_stream().cuda_stream) == 0
+        return y
+
+    spread = run(_lib.FSB_SPMV_VECTOR, lanes)
+    assert torch.equal(run(_lib.FSB_SPMV_VECTOR, 0), spread) and torch.equal(run(_lib.FSB_SPMV_AUTO, 0), spread)
+    even = run(_lib.FSB_SPMV_VECTOR, 1024)
+    assert not torch.equal(even, spread)                        # another order of the sums
+    _check(even, vals, i, p, n_cols, x, dtype)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64], ids=str)
+def test_into_several_vectors(cuda, fsb_lib, dtype):
+    """The rows kernel with the epilogue that stores every value into the vectors of all GPUs, here two vectors of this one: even
+    rows, shares of uneven weight, a row offset; the values are those of the product into one vector."""
+    from flagsparse_b200 import _lib
+    from flagsparse_b200._common import _VTYPE
+
+    n_cols = 4000
+    for lens in ([k % 9 for k in range(8192)], np.where(np.arange(30000) < 24000, 0, 9), [40] * 9001):
+        _, i, p = handmade_csr(12, [int(v) for v in lens], n_cols)
+        vals, x = _values(int(p[-1]), dtype, 6), _values(n_cols, dtype, 7)
+        n = len(p) - 1
+        d, ti, tp, tx = vals.to(cuda), torch.from_numpy(i).to(cuda), torch.from_numpy(p).to(cuda), x.to(cuda)
+        y = torch.empty(n, dtype=dtype, device=cuda)
+        st = torch.cuda.current_stream().cuda_stream
+        args = (_VTYPE[dtype], 0, 0, d.data_ptr(), ti.data_ptr(), tp.data_ptr(), tx.data_ptr())
+        assert fsb_lib.fsb_spmv_csr(*args, y.data_ptr(), n, n_cols, d.numel(), _lib.FSB_SPMV_VECTOR, 1024, None, None, 0, st) == 0
+        _check(y, vals, i, p, n_cols, x, dtype)
+        for tuning in (1024, 0):
+            out = [torch.full((n + 20,), 7.0, dtype=dtype, device=cuda) for _ in range(2)]
+            peers = torch.tensor([t.data_ptr() for t in out], dtype=torch.int64, device=cuda)
+            assert fsb_lib.fsb_spmv_csr_scatter(*args, peers.data_ptr(), 2, 1, 9, n, n_cols, d.numel(), _lib.FSB_SPMV_VECTOR, tuning,
+                                                None, None, 0, st) == 0
+            for t in out:
+                assert bool((t[:9] == 7).all()) and bool((t[9 + n:] == 7).all())
+                if tuning:
+                    assert torch.equal(t[9:9 + n], y)
+                else:
+                    _check(t[9:9 + n], vals, i, p, n_cols, x, dtype)
