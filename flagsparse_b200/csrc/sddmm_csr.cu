@@ -20,8 +20,17 @@ constexpr int kSdThreads = 256;
 constexpr int kSdBatch = 8;   // consecutive entries one group handles
 
 // Resident CTAs the register budget is set for: 64 registers, but 80 for 16-byte accesses of float64, whose eight sums take twice
-// the room (131072 rows of 16, K 200: 476 us, with 64 registers 603 us).
-__host__ __device__ constexpr int sddmm_ctas(int vw, size_t size) { return size == 8 && vw == 2 ? 3 : 4; }
+// the room (131072 rows of 16, K 200: 476 us, with 64 registers 603 us), and for rows that take several steps: with 64 the gathers of
+// a step wait for one another (float32, 2048 rows of 16, K 160: 15.4 us, 8.9 us; 209715 rows of 5, K 129: 161 us, 140 us).
+__host__ __device__ constexpr int sddmm_ctas(int vw, size_t size, bool multi) { return (size == 8 && vw == 2) || multi ? 3 : 4; }
+// Rows of several steps that take the instance for them: not those of float32 in accesses of 8 bytes (65536 rows of 16, K 130: 65 us
+// with 80 registers, 59 with 64), nor in accesses of 4 bytes where there are many tiles and most batches lie in one row or two (65536
+// rows of 16, K 129: 71 us, 66; but 209715 rows of 5: 140, 161).
+template <typename V, int VW>
+static bool sddmm_multi(int k_dim, int64_t n_rows, int64_t nnz) {
+  if (k_dim <= 32 * VW || (sizeof(V) == 4 && VW == 2)) return false;
+  return !(sizeof(V) == 4 && VW == 1 && nnz >= (1 << 19) && nnz >= 12 * n_rows);
+}
 
 // entries one CTA handles: J passes of (threads / LG) groups x 8 entries, about 1024 (262144 rows of 6, K 8: 17.3 us, with 2048
 // 20.3 us, a last wave that is a quarter full; 2^19 rows of 16, K 64: 251 us, with 512 265 us)
@@ -82,8 +91,13 @@ constexpr uint32_t kSdOne = 1u << 8, kSdTwo = 1u << 9;
 template <typename V>
 __host__ __device__ constexpr bool sddmm_vote(int VW, int LG) { return VW * (int)sizeof(V) == 16 && (LG == 8 || LG == 16); }
 
-template <typename V, int VW, int LG>
-__global__ void __launch_bounds__(kSdThreads, sddmm_ctas(VW, sizeof(V)))
+// MULTI: rows of X longer than one access per lane of a warp, walked in several steps.  With 16-byte accesses (WIDE) products are then
+// added to the sums one by one, as the pairs of lane_dot want registers of their own; and float32 has no form for batches of two
+// rows, whose second slice of X finds no room beside eight gathers: the row ids themselves tell the two forms that are left apart.
+// us, as for one step / here: float32, 65536 rows of 16, K 160 98 / 72; 2048 rows of 16, K 200 15.5 / 9.0; float64, 65536 rows of
+// 16, K 72 97 / 74, Poisson rows 90 / 74.
+template <typename V, int VW, int LG, bool MULTI>
+__global__ void __launch_bounds__(kSdThreads, sddmm_ctas(VW, sizeof(V), MULTI))
 sddmm_kernel(const int32_t* __restrict__ indices, const int32_t* __restrict__ row_ids, const V* __restrict__ X,
              int64_t ldx, const V* __restrict__ Y, int64_t ldy, const V* data, V* out,
              int64_t nnz, int k_dim, V alpha, V beta, int ids_aligned) {
@@ -96,10 +110,12 @@ sddmm_kernel(const int32_t* __restrict__ indices, const int32_t* __restrict__ ro
   constexpr int kDup = (LG > E) ? LG / E : 1;     // lanes that end up with the same result
   constexpr bool VOTE = sddmm_vote<V>(VW, LG);
   constexpr bool ONE = VOTE || LG == 32;          // batches of one row have a form of their own
+  constexpr bool WIDE = MULTI && VW * (int)sizeof(V) == 16;
+  constexpr bool TWO = !WIDE || sizeof(V) == 8;   // ... and batches of two
   __shared__ __align__(16) int32_t s_cols[T];
   __shared__ __align__(16) int32_t s_rows[T];
   __shared__ __align__(16) V s_out[T];
-  __shared__ uint32_t s_form[T / E];
+  __shared__ uint32_t s_form[!TWO ? 1 : T / E];
 
   // the tile's column and row ids go to shared memory once (entries past the end repeat the last one; they are
   // never stored), so that the loop below has one trip to global memory per batch: the gathers
@@ -118,19 +134,21 @@ sddmm_kernel(const int32_t* __restrict__ indices, const int32_t* __restrict__ ro
     }
   }
   __syncthreads();
-  for (int b = threadIdx.x; b < T / E; b += kSdThreads) {
-    const int32_t* r = s_rows + b * E;
-    const int32_t row_a = r[0], row_b = r[E - 1];
-    uint32_t form = row_a == row_b ? kSdOne : 0;
-    bool two = true;
+  if constexpr (TWO) {
+    for (int b = threadIdx.x; b < T / E; b += kSdThreads) {
+      const int32_t* r = s_rows + b * E;
+      const int32_t row_a = r[0], row_b = r[E - 1];
+      uint32_t form = row_a == row_b ? kSdOne : 0;
+      bool two = true;
 #pragma unroll
-    for (int e = 0; e < E; ++e) {
-      two = two && (r[e] == row_a || r[e] == row_b);
-      form |= (r[e] == row_a ? 1u : 0u) << e;
+      for (int e = 0; e < E; ++e) {
+        two = two && (r[e] == row_a || r[e] == row_b);
+        form |= (r[e] == row_a ? 1u : 0u) << e;
+      }
+      s_form[b] = form | (two ? kSdTwo : 0);
     }
-    s_form[b] = form | (two ? kSdTwo : 0);
+    __syncthreads();
   }
-  __syncthreads();
 
   const int lane = threadIdx.x & (LG - 1);
   const int group = threadIdx.x / LG;
@@ -148,7 +166,9 @@ sddmm_kernel(const int32_t* __restrict__ indices, const int32_t* __restrict__ ro
     V acc[E];
 #pragma unroll
     for (int e = 0; e < E; ++e) acc[e] = (V)0;
-    const uint32_t form = s_form[local / E];
+    uint32_t form;
+    if constexpr (!TWO) form = s_rows[local] == s_rows[local + E - 1] ? kSdOne : 0;
+    else form = s_form[local / E];
     bool one = (form & kSdOne) != 0, two = (form & kSdTwo) != 0;
     if constexpr (VOTE) {
       one = __all_sync(active, one);
@@ -156,7 +176,19 @@ sddmm_kernel(const int32_t* __restrict__ indices, const int32_t* __restrict__ ro
     }
     const int32_t* cols = s_cols + local;
     const int32_t* rows = s_rows + local;
-    if (ONE && one) {
+    if (WIDE && one) {
+      const V *xp = X + k0 + (int64_t)rows[0] * ldx, *yp = Y + k0;
+      for (int k = k0; k < k_dim; k += step, xp += step, yp += step) {
+        V xa[VW], yv[E][VW];
+        ld_dense<V, VW>(xp, xa);
+#pragma unroll
+        for (int e = 0; e < E; ++e) ld_dense<V, VW>(yp + (int64_t)cols[e] * ldy, yv[e]);
+#pragma unroll
+        for (int e = 0; e < E; ++e)
+#pragma unroll
+          for (int i = 0; i < VW; ++i) acc[e] += xa[i] * yv[e][i];
+      }
+    } else if (ONE && one) {
       const char *xp = reinterpret_cast<const char*>(row_at<V>(Xk, rows[0], xs)), *yp = Yk;
       for (int k = k0; k < k_dim; k += step, xp += step * sizeof(V), yp += step * sizeof(V)) {
         V xa[VW], yv[E][VW];
@@ -166,7 +198,7 @@ sddmm_kernel(const int32_t* __restrict__ indices, const int32_t* __restrict__ ro
 #pragma unroll
         for (int e = 0; e < E; ++e) acc[e] += lane_dot(xa, yv[e]);
       }
-    } else if (two) {
+    } else if (TWO && two) {
       const char *xp = reinterpret_cast<const char*>(row_at<V>(Xk, rows[0], xs)), *yp = Yk;
       const char *xq = reinterpret_cast<const char*>(row_at<V>(Xk, rows[E - 1], xs));
       for (int k = k0; k < k_dim; k += step, xp += step * sizeof(V), xq += step * sizeof(V), yp += step * sizeof(V)) {
@@ -177,10 +209,20 @@ sddmm_kernel(const int32_t* __restrict__ indices, const int32_t* __restrict__ ro
         for (int e = 0; e < E; ++e) ld_dense<V, VW>(row_at<V>(yp, cols[e], ys), yv[e]);
 #pragma unroll
         for (int e = 0; e < E; ++e) {
-          V t;                       // (a branch of the group; choosing the slice first takes an instruction per element)
-          if (form >> e & 1) t = lane_dot(xa, yv[e]);
-          else t = lane_dot(xb, yv[e]);
-          acc[e] += t;
+          if constexpr (WIDE) {
+            if (form >> e & 1) {
+#pragma unroll
+              for (int i = 0; i < VW; ++i) acc[e] += xa[i] * yv[e][i];
+            } else {
+#pragma unroll
+              for (int i = 0; i < VW; ++i) acc[e] += xb[i] * yv[e][i];
+            }
+          } else {
+            V t;                     // (a branch of the group; choosing the slice first takes an instruction per element)
+            if (form >> e & 1) t = lane_dot(xa, yv[e]);
+            else t = lane_dot(xb, yv[e]);
+            acc[e] += t;
+          }
         }
       }
     } else {
@@ -236,13 +278,15 @@ sddmm_kernel(const int32_t* __restrict__ indices, const int32_t* __restrict__ ro
 }
 
 template <typename V, int VW>
-static int sddmm_launch(int LG, unsigned blocks, cudaStream_t st, const int32_t* indices, const int32_t* row_ids,
+static int sddmm_launch(int LG, int64_t n_rows, unsigned blocks, cudaStream_t st, const int32_t* indices, const int32_t* row_ids,
                         const V* X, int64_t ldx, const V* Y, int64_t ldy, const V* data, V* out, int64_t nnz,
                         int k_dim, V alpha, V beta, int ids_aligned) {
+#define FSB_SDDMM_LAUNCH(LG_, MULTI_)                                                                            \
+  sddmm_kernel<V, VW, LG_, MULTI_><<<blocks, kSdThreads, 0, st>>>(indices, row_ids, X, ldx, Y, ldy, data, out,   \
+                                                                  nnz, k_dim, alpha, beta, ids_aligned)
 #define FSB_SDDMM_CASE(LG_)                                                                                      \
   case LG_:                                                                                                      \
-    sddmm_kernel<V, VW, LG_><<<blocks, kSdThreads, 0, st>>>(indices, row_ids, X, ldx, Y, ldy, data, out, nnz,    \
-                                                            k_dim, alpha, beta, ids_aligned);                   \
+    FSB_SDDMM_LAUNCH(LG_, false);                                                                                \
     break
   switch (LG) {
     FSB_SDDMM_CASE(1);
@@ -250,17 +294,21 @@ static int sddmm_launch(int LG, unsigned blocks, cudaStream_t st, const int32_t*
     FSB_SDDMM_CASE(4);
     FSB_SDDMM_CASE(8);
     FSB_SDDMM_CASE(16);
-    FSB_SDDMM_CASE(32);
+    case 32:
+      if (sddmm_multi<V, VW>(k_dim, n_rows, nnz)) FSB_SDDMM_LAUNCH(32, true);
+      else FSB_SDDMM_LAUNCH(32, false);
+      break;
     default: return FSB_EINVAL;
   }
 #undef FSB_SDDMM_CASE
+#undef FSB_SDDMM_LAUNCH
   FSB_RETURN_IF_LAUNCH_FAILED();
   return FSB_OK;
 }
 
 template <typename V>
 static int sddmm_typed(const int32_t* indices, const int32_t* row_ids, const void* X, int64_t ldx, const void* Y,
-                       int64_t ldy, const void* data, void* out, int64_t nnz, int k_dim, double alpha, double beta,
+                       int64_t ldy, const void* data, void* out, int64_t n_rows, int64_t nnz, int k_dim, double alpha, double beta,
                        cudaStream_t st) {
   constexpr int VMAX = 16 / sizeof(V);
   int vw = VMAX;
@@ -281,13 +329,13 @@ static int sddmm_typed(const int32_t* indices, const int32_t* row_ids, const voi
   V* ov = (V*)out;
   if constexpr (VMAX == 4) {
     if (vw == 4)
-      return sddmm_launch<V, 4>(LG, (unsigned)blocks, st, indices, row_ids, Xv, ldx, Yv, ldy, dv, ov, nnz, k_dim,
+      return sddmm_launch<V, 4>(LG, n_rows, (unsigned)blocks, st, indices, row_ids, Xv, ldx, Yv, ldy, dv, ov, nnz, k_dim,
                                 (V)alpha, (V)beta, ids_aligned);
   }
   if (vw == 2)
-    return sddmm_launch<V, 2>(LG, (unsigned)blocks, st, indices, row_ids, Xv, ldx, Yv, ldy, dv, ov, nnz, k_dim,
+    return sddmm_launch<V, 2>(LG, n_rows, (unsigned)blocks, st, indices, row_ids, Xv, ldx, Yv, ldy, dv, ov, nnz, k_dim,
                               (V)alpha, (V)beta, ids_aligned);
-  return sddmm_launch<V, 1>(LG, (unsigned)blocks, st, indices, row_ids, Xv, ldx, Yv, ldy, dv, ov, nnz, k_dim,
+  return sddmm_launch<V, 1>(LG, n_rows, (unsigned)blocks, st, indices, row_ids, Xv, ldx, Yv, ldy, dv, ov, nnz, k_dim,
                             (V)alpha, (V)beta, ids_aligned);
 }
 
@@ -311,6 +359,6 @@ extern "C" int fsb_sddmm_csr(int vtype, const int32_t* indices, const int32_t* r
     return FSB_EALIGN;
   FSB_WALK_FIRST(check_entry_ids(indices, row_ids, n_rows, n_cols, nnz, st));
   if (vtype == FSB_F32)
-    return sddmm_typed<float>(indices, row_ids, X, ldx, Y, ldy, data, out, nnz, (int)k_dim, alpha, beta, st);
-  return sddmm_typed<double>(indices, row_ids, X, ldx, Y, ldy, data, out, nnz, (int)k_dim, alpha, beta, st);
+    return sddmm_typed<float>(indices, row_ids, X, ldx, Y, ldy, data, out, n_rows, nnz, (int)k_dim, alpha, beta, st);
+  return sddmm_typed<double>(indices, row_ids, X, ldx, Y, ldy, data, out, n_rows, nnz, (int)k_dim, alpha, beta, st);
 }

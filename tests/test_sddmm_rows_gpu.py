@@ -48,3 +48,35 @@ def test_ends_of_tiles(cuda, fsb_lib, dtype, u, k):
         # the dot product's (k + 1) u, and a rounding for beta * data and one for the sum
         bound = (k + 1) * u * 0.5 * np.abs(xd * yd).sum(1) + 2 * u * (0.5 * np.abs((xd * yd).sum(1)) + 2 * np.abs(d.double().numpy()))
         assert np.all(np.abs(out.cpu().double().numpy() - (0.5 * (xd * yd).sum(1) - 2 * d.double().numpy())) <= 1.0001 * bound), nnz
+
+
+@pytest.mark.parametrize("dtype,u", [(torch.float32, 2.0 ** -24), (torch.float64, 2.0 ** -53)], ids=str)
+@pytest.mark.parametrize("name", sorted(LENS))
+def test_rows_of_several_steps(cuda, fsb_lib, dtype, u, name):
+    """More than one access per lane of a warp: 16-byte accesses (float32 from 132, float64 from 66 on), single elements and pairs, whole
+    last steps and short ones, tiles that end in the middle."""
+    n_cols = 200
+    _, i, p = handmade_csr(2, LENS[name], n_cols)
+    n_rows = len(p) - 1
+    row = np.repeat(np.arange(n_rows), np.diff(p))
+    prep = fs.prepare_sddmm_csr(torch.from_numpy(i).to(cuda), torch.from_numpy(p).to(cuda), (n_rows, n_cols))
+    for k in (35, 65, 68, 129, 132, 134, 192, 256, 257, 260, 388):
+        rng = np.random.default_rng(k)
+        x, y = (torch.from_numpy(rng.uniform(-1, 1, (n, k))).to(dtype) for n in (n_rows, n_cols))
+        d = torch.from_numpy(rng.uniform(-1, 1, len(i))).to(dtype)
+        out = fs.flagsparse_sddmm_csr(d.to(cuda), x=x.to(cuda), y=y.to(cuda), beta=1.0, prepared=prep).cpu().double().numpy()
+        xy, dd = x.double().numpy()[row] * y.double().numpy()[i], d.double().numpy()
+        bound = (k + 1) * u * np.abs(xy).sum(1) + 2 * u * (np.abs(xy.sum(1)) + np.abs(dd))
+        assert np.all(np.abs(out - xy.sum(1) - dd) <= 1.0001 * bound), k
+
+
+def test_single_elements_in_many_tiles(cuda, fsb_lib):
+    """Either side of the sizes from which float32 rows of an odd number of elements take the instance for one step."""
+    for n_rows, length, k in ((1 << 15, 16, 33), ((1 << 15) - 1, 16, 33), (1 << 16, 11, 35), (1 << 14, 40, 129)):
+        gen = torch.Generator(device="cuda").manual_seed(k)
+        i = torch.randint(0, 500, (n_rows * length,), generator=gen, device=cuda, dtype=torch.int32)
+        p = torch.arange(n_rows + 1, device=cuda) * length
+        x, y = (torch.empty(n, k, device=cuda).uniform_(-1, 1, generator=gen) for n in (n_rows, 500))
+        out = fs.flagsparse_sddmm_csr(x=x, y=y, prepared=fs.prepare_sddmm_csr(i, p, (n_rows, 500)))
+        xy = x.double().repeat_interleave(length, 0) * y.double()[i.long()]
+        assert bool(((out.double() - xy.sum(1)).abs() <= (k + 1) * 2.0 ** -24 * 1.0001 * xy.abs().sum(1)).all())
