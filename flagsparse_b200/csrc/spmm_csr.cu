@@ -248,9 +248,13 @@ spmm_tile_kernel(const S* __restrict__ data, const I* __restrict__ idx, const vo
 
   // Row c of B: one wide multiply-add from a stride in bytes, and one for the high word, where several accesses per lane, small ones
   // or conversions leave the arithmetic in the way of the gathers (float32, 262144 rows of 16, 33 columns: 102 us, from the stride in
-  // elements 112 us; float16, 200003 rows of 20, 70 columns: 132 / 146, 200 columns: 229 / 241; complex64, 32 columns: 81 / 86).  float64 and 16-byte gathers of
-  // one access lose registers to it (float64, 75 columns: 179 / 161; float32, 64 columns: 256 / 233).
+  // elements 112 us; float16, 200003 rows of 20, 70 columns: 132 / 146, 200 columns: 229 / 241; complex64, 32 columns: 81 / 86).  float64
+  // and 16-byte gathers of one access lose registers to it (float64, 75 columns: 179 / 161; float32, 64 columns: 256 / 233).
+  // ROWS_FIRST: the four rows before the first of their gathers; single floats, one access, left each gather waiting for its own row
+  // where few tiles run (5461 rows of 24, 13 / 21 columns: stride in elements 8.6 / 12.3 us, in bytes 9.5 / 13.9, here 8.3 / 11.7; 174762
+  // rows of 24, 21 columns: 81.5, 71.7, 66.7).  Others lose to it (float32, 70 columns 2 %, float64, 33 columns 12 %) or do not care.
   constexpr bool FROM_BYTES = RealOf<S>::parts == 2 || sizeof(S) == 2 || (sizeof(S) == 4 && VW * (int)sizeof(S) < 16);
+  constexpr bool ROWS_FIRST = sizeof(S) == 4 && VW == 1 && NC == 1;
   const char* B0 = reinterpret_cast<const char*>(B + col0);
   const uint64_t row_bytes = (uint64_t)ldb * sizeof(S);
   auto row_of = [&](I c) {
@@ -284,9 +288,14 @@ spmm_tile_kernel(const S* __restrict__ data, const I* __restrict__ idx, const vo
     if (CHAINS == 2) clear(odd);
     for (; p + U <= e; p += U) {
       Pack<S, VW> b[U][NC];
+      const S* rows[ROWS_FIRST ? U : 1];
+      if constexpr (ROWS_FIRST) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) rows[u] = row_of(s_idx[p + u]);
+      }
 #pragma unroll
       for (int u = 0; u < U; ++u) {
-        const S* row = row_of(s_idx[p + u]);
+        const S* row = ROWS_FIRST ? rows[ROWS_FIRST ? u : 0] : row_of(s_idx[p + u]);
 #pragma unroll
         for (int i = 0; i < NC; ++i)
           if (i == 0 || col0 + i * LR * VW < n_dense) b[u][i].gather(row + i * LR * VW);
