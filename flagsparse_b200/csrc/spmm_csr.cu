@@ -382,7 +382,9 @@ spmm_tile_kernel(const S* __restrict__ data, const I* __restrict__ idx, const vo
       return;
     }
 
-    if constexpr (BY_LENGTH) {
+    // (a group has one segment at most: nothing to choose from.  float64, 682 rows of 48, 16 columns: sorted 8.7 us, 8.4 us)
+    const bool sorted = BY_LENGTH && m > ngrp;
+    if (sorted) {
       auto bucket = [&](int k) {                 // the longest first
         const int len = s_off[k + 1] - s_off[k];
         return kMmBuckets - 1 - (len < 2 * kMmBuckets - 2 ? len : 2 * kMmBuckets - 2) / 2;
@@ -407,7 +409,7 @@ spmm_tile_kernel(const S* __restrict__ data, const I* __restrict__ idx, const vo
       __syncthreads();
     }
     for (int q = grp; q < m; q += ngrp) {
-      const int k = BY_LENGTH ? s_order[q] : q;
+      const int k = sorted ? s_order[BY_LENGTH ? q : 0] : q;
       const int s = s_off[k], e = s_off[k + 1];
       if (LONG && e - s > 2 * piece) {
         if (lane == 0) {

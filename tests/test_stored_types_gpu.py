@@ -163,3 +163,21 @@ def test_any_nonzero_long_rows_shares_them(cuda, fsb_lib, dtype):
     if dtype != torch.float16 and dtype != torch.bfloat16:      # (the rounding of the result hides the order of the sums)
         assert not torch.equal(got[0], got[1])
     _check(got[64], vals, i, p, n_cols, B, dtype)
+
+
+@pytest.mark.parametrize("dtype", DTYPES, ids=str)
+def test_spmm_few_segments_in_a_tile(cuda, fsb_lib, dtype):
+    """As many segments as a block has groups (16 or 32), one less, one more: from there on they are taken by length.  Every tile ends
+    with a row, and the last one holds a few rows only."""
+    n_cols = 700
+    for count in (15, 16, 17, 31, 32, 33):
+        short = 1024 // count - 3
+        tile = [short] * (count - 2) + [1024 - short * (count - 2) - 1, 1]
+        lens = tile * 4 + [7, 0, 3, 90]
+        _, i, p = handmade_csr(3, lens, n_cols)
+        vals = _values(int(p[-1]), dtype, 4)
+        d, ti, tp = vals.to(cuda), torch.from_numpy(i).to(cuda), torch.from_numpy(p).to(cuda)
+        for n_dense in (16, 32, 64, 128):
+            B = _values((n_cols, n_dense), dtype, n_dense)
+            C = fs.flagsparse_spmm_csr(d, ti, tp, B.to(cuda), (len(p) - 1, n_cols))
+            _check(C, vals, i, p, n_cols, B, dtype)
