@@ -437,7 +437,7 @@ static int run_vector(const void* data, const void* idx, const void* ptr, const 
                       int64_t n_rows, int64_t nnz, int tuning, cudaStream_t st) {
   int L = tuning & 0xff;
   if (L == 0) {
-    if ((tuning & FSB_SPMV_EVEN_ROWS) && rows_apply(data, idx, n_rows, nnz))
+    if ((tuning & FSB_SPMV_EVEN_ROWS) && rows_apply<V>(data, idx, n_rows, nnz))
       return rows_run<V, I, P, Out>(data, idx, ptr, x, out, n_rows, nnz, st);
     // eight to sixteen entries (two to four 4-element groups) per lane: measured best on 32-entry rows
     const int64_t mean = n_rows > 0 ? nnz / n_rows : 0;

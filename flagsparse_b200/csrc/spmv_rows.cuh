@@ -199,17 +199,38 @@ struct RowsOut {
 template <typename S> __host__ __device__ constexpr int rows_each() { return sizeof(S) == 16 ? 2 : 4; }
 template <typename S> __host__ __device__ constexpr int rows_together() { return sizeof(S) <= 4 ? 2 : 1; }
 
-// Matrices that take the kernel: up to 2^30 rows and entries (row + 2 * hop fits 32 bits), from 8192 rows on (float32 by lanes per
-// row and here: 4096 rows of 16 and of 48 5.5 and 5.6 us, 10000 rows of 24 5.5 and 5.6, with one of 120 among them 8.3 and 5.6,
-// 65536 rows of 16 8.2 and 6.2).
-constexpr int kRowsLeast = 8192;
-static bool rows_apply(const void* data, const void* idx, int64_t n_rows, int64_t nnz) {
-  return n_rows >= kRowsLeast && n_rows <= (1 << 30) && nnz <= (1 << 30) && aligned_to(data, 16) && aligned_to(idx, 16);
+// Lanes of a row: the fewest that hold four fifths of a mean row at once (complex128 two fifths: 4 / 8 / 16 lanes, columns anywhere,
+// 1000000 rows of 12 80 / 86 / - us, 500000 rows of 36 111 / 101 / 115, 300000 rows of 60 107 / 99 / 102); more leave lanes idle
+// (float32, 1000000 rows of 4, 2 / 4 / 8 lanes: 17 / 21 / 33 us), fewer a second turn for most rows (float64, 100000 rows of 50,
+// 16 / 8 / 4 / 2 lanes: 27 / 25 / 27 / 30 us).
+template <typename S>
+static int rows_lanes(int64_t mean) {
+  int L = 2;
+  while (L < 32 && 5 * L * rows_each<S>() < (sizeof(S) == 16 ? 2 : 4) * mean) L <<= 1;
+  return L;
 }
 
-// Lanes of a row: the fewest that hold four fifths of a mean row at once (complex128 two fifths: 4 / 8 / 16 lanes, columns anywhere,
-// 1000000 rows of 12 80 / 86 / - us, 500000 rows of 36 111 / 101 / 115, 300000 rows of 60 107 / 99 / 102); more leave lanes idle (float32, 1000000 rows of 4, 2 / 4 / 8 lanes: 17 / 21 / 33 us), fewer a second turn for
-// most rows (float64, 100000 rows of 50, 16 / 8 / 4 / 2 lanes: 27 / 25 / 27 / 30 us).
+// Mean row from which fewer rows than warps are no hindrance: the lanes-per-row kernel then has its own trouble with them.
+template <typename S> constexpr int64_t rows_long() { return sizeof(S) == 4 ? 24 : 10; }
+template <> constexpr int64_t rows_long<float2>() { return 0; }
+template <> constexpr int64_t rows_long<double2>() { return INT32_MAX; }
+
+// Matrices that take the kernel: 8192 to 2^30 rows, up to 2^30 entries (row + 2 * hop fits 32 bits), and rows for four fifths of the
+// warps (32 to 1024 rows an SM) or rows that are long: short rows leave most warps without any.  us through lanes per row / here:
+// float32, 8192 rows of 4 2.2 / 2.6, 32768 Poisson rows of 8 3.6 / 4.5, 80000 rows of 4 3.3 / 3.6, 131072 such rows 4.6 / 4.3; 12000
+// Poisson rows of 30 4.4 / 4.2; float64, 32768 rows of 4 2.6 / 2.8, 20000 Poisson rows of 20 5.7 / 4.5; bfloat16, 32768 rows of 4 2.6 /
+// 3.0; complex128, 12000 rows of 8 2.6 / 3.1, Poisson rows of 30 4.3 / 4.7; complex64, 20000 rows of 8 2.9 / 3.0, Poisson 4.6 / 3.5.
+constexpr int kRowsLeast = 8192;
+template <typename S>
+static bool rows_apply(const void* data, const void* idx, int64_t n_rows, int64_t nnz) {
+  if (n_rows < kRowsLeast || n_rows > (1 << 30) || nnz > (1 << 30) || !aligned_to(data, 16) || !aligned_to(idx, 16)) return false;
+  const int64_t mean = nnz / n_rows;
+  int sms = 0;
+  if (mean >= rows_long<S>()) return true;
+  if (sm_count(&sms) != FSB_OK) return false;
+  return 5 * n_rows >= 4 * (int64_t)sms * (kRowsThreads / 32) * rows_together<S>() * (32 / rows_lanes<S>(mean));
+}
+
 template <typename S, typename I, typename P, typename Out>
 static int rows_run(const void* data_, const void* idx_, const void* ptr_, const void* x_, Out out, int64_t n_rows, int64_t nnz,
                     cudaStream_t st) {
@@ -221,11 +242,8 @@ static int rows_run(const void* data_, const void* idx_, const void* ptr_, const
   const int rc = sm_count(&sms);
   if (rc != FSB_OK) return rc;
   if (sms > kRowsThreads) sms = kRowsThreads;          // a thread looks at a share
-  const int64_t mean = nnz / n_rows;
-  int L = 2;
-  while (L < 32 && 5 * L * E < (sizeof(S) == 16 ? 2 : 4) * mean) L <<= 1;
   const RowsShares shares(n_rows, nnz, sms);
-  switch (L) {
+  switch (rows_lanes<S>(nnz / n_rows)) {
     case 2: spmv_rows_kernel<S, I, P, 2, U, E><<<sms, kRowsThreads, 0, st>>>(data, idx, ptr, x, out, n_rows, nnz, shares); break;
     case 4: spmv_rows_kernel<S, I, P, 4, U, E><<<sms, kRowsThreads, 0, st>>>(data, idx, ptr, x, out, n_rows, nnz, shares); break;
     case 8: spmv_rows_kernel<S, I, P, 8, U, E><<<sms, kRowsThreads, 0, st>>>(data, idx, ptr, x, out, n_rows, nnz, shares); break;

@@ -511,7 +511,7 @@ static int stored_launch(const void* data_, const int32_t* idx, const void* ptr_
     }
     return FSB_OK;
   }
-  if (even && rows_apply(data, idx, n_rows, nnz))
+  if (even && rows_apply<S>(data, idx, n_rows, nnz))
     return rows_run<S, int32_t, P>(data, idx, ptr, x, RowsOut<S>{y}, n_rows, nnz, st);
   // two to four groups of four entries per lane, as in the float32 / float64 kernel; entry by entry, three to six
   // (columns anywhere, 4 / 8 / 16 lanes a row: complex64, 500009 rows of 24: 70 / 64 / - us, 300000 rows of 30: 55 / 47 / 51 us,

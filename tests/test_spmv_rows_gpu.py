@@ -111,7 +111,7 @@ def test_into_several_vectors(cuda, fsb_lib, dtype):
     from flagsparse_b200._common import _VTYPE
 
     n_cols = 4000
-    for lens in ([k % 9 for k in range(8192)], np.where(np.arange(30000) < 24000, 0, 9), [40] * 9001):
+    for lens in ([20 + k % 9 for k in range(8192)], np.where(np.arange(30000) < 6000, 0, 40), [k % 9 for k in range(125000)]):
         _, i, p = handmade_csr(12, [int(v) for v in lens], n_cols)
         vals, x = _values(int(p[-1]), dtype, 6), _values(n_cols, dtype, 7)
         n = len(p) - 1
@@ -132,3 +132,40 @@ def test_into_several_vectors(cuda, fsb_lib, dtype):
                     assert torch.equal(t[9:9 + n], y)
                 else:
                     _check(t[9:9 + n], vals, i, p, n_cols, x, dtype)
+
+
+@pytest.mark.parametrize("dtype", DTYPES, ids=str)
+def test_enough_rows_for_the_warps(cuda, fsb_lib, dtype):
+    """Short rows, 2 and 4 lanes each, either side of the number of rows from which neighbours stay on one SM: 32 rows a warp (values
+    of 8 and 16 bytes: 16) with two lanes a row, half as many with four."""
+    from flagsparse_b200 import _lib
+    from flagsparse_b200._common import _VTYPE
+
+    size = torch.empty(0, dtype=dtype).element_size()
+    together, n_cols = (2 if size <= 4 else 1), 500
+    sms = torch.cuda.get_device_properties(cuda).multi_processor_count
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    for lanes in (2, 4):
+        mean = 9 if lanes == 2 else 12               # (float64 and half precisions: rows of 12 are long, whatever their number)
+        line = -(-4 * sms * 32 * together * (32 // lanes) // 5)
+        for n in (line - 1, line):
+            p = torch.arange(n + 1, device=cuda, dtype=torch.int32) * mean
+            i = torch.randint(0, n_cols, (n * mean,), device=cuda, generator=gen, dtype=torch.int32)
+            d, x = _values(n * mean, dtype, 1).to(cuda), _values(n_cols, dtype, 2).to(cuda)
+            y = fs.flagsparse_spmv_csr(d, i, p, x, (n, n_cols))
+            wide = torch.complex128 if dtype.is_complex else torch.float64
+            prod = (d.to(wide) * x.to(wide)[i.long()]).view(n, mean)
+            ref, mag = prod.sum(1), prod.abs().sum(1)
+            u = {4: 2.0 ** -24, 8: 2.0 ** -53}[4 if dtype in (torch.float16, torch.bfloat16, torch.float32, torch.complex64) else 8]
+            bound = (4 if dtype.is_complex else 1) * (mean + 1) * u * mag
+            if size == 2:
+                v = {torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8}[dtype]
+                bound = bound * (1 + v) + v * ref.abs() + (2.0 ** -25 if dtype == torch.float16 else 0)
+            assert bool(((y.to(wide) - ref).abs() <= 1.0001 * bound).all()), n
+            assert torch.equal(fs.flagsparse_spmv_csr(x=x, prepared=fs.prepare_spmv_csr(d, i, p, (n, n_cols))), y)
+            if dtype in (torch.float32, torch.float64) and lanes == 2:
+                spread = torch.empty_like(y)         # two lanes a row, and no neighbours
+                assert fsb_lib.fsb_spmv_csr(_VTYPE[dtype], 0, 0, d.data_ptr(), i.data_ptr(), p.data_ptr(), x.data_ptr(), spread.data_ptr(),
+                                            n, n_cols, d.numel(), _lib.FSB_SPMV_VECTOR, 2, None, None, 0,
+                                            torch.cuda.current_stream().cuda_stream) == 0
+                assert torch.equal(y, spread) == (n < line)
