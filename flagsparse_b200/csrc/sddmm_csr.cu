@@ -23,15 +23,6 @@ constexpr int kSdBatch = 8;   // consecutive entries one group handles
 // the room (131072 rows of 16, K 200: 476 us, with 64 registers 603 us), and for rows that take several steps: with 64 the gathers of
 // a step wait for one another (float32, 2048 rows of 16, K 160: 15.4 us, 8.9 us; 209715 rows of 5, K 129: 161 us, 140 us).
 __host__ __device__ constexpr int sddmm_ctas(int vw, size_t size, bool multi) { return (size == 8 && vw == 2) || multi ? 3 : 4; }
-// Rows of several steps that take the instance for them: not those of float32 in accesses of 8 bytes (65536 rows of 16, K 130: 65 us
-// with 80 registers, 59 with 64), nor in accesses of 4 bytes where there are many tiles and most batches lie in one row or two (65536
-// rows of 16, K 129: 71 us, 66; but 209715 rows of 5: 140, 161).
-template <typename V, int VW>
-static bool sddmm_multi(int k_dim, int64_t n_rows, int64_t nnz) {
-  if (k_dim <= 32 * VW || (sizeof(V) == 4 && VW == 2)) return false;
-  return !(sizeof(V) == 4 && VW == 1 && nnz >= (1 << 19) && nnz >= 12 * n_rows);
-}
-
 // entries one CTA handles: J passes of (threads / LG) groups x 8 entries, about 1024 (262144 rows of 6, K 8: 17.3 us, with 2048
 // 20.3 us, a last wave that is a quarter full; 2^19 rows of 16, K 64: 251 us, with 512 265 us)
 __host__ __device__ constexpr int sddmm_passes(int LG) {
@@ -275,6 +266,23 @@ sddmm_kernel(const int32_t* __restrict__ indices, const int32_t* __restrict__ ro
     if (data != nullptr) v += __ldcs(data + tile0 + i) * beta;
     __stcs(out + tile0 + i, v);
   }
+}
+
+// Which rows of several steps take the instance for them: not those of float32 in accesses of 8 bytes (65536 rows of 16, K 130: 65 us
+// with 80 registers, 59 with 64); not where four CTAs an SM hold all tiles and three do not (float32, 262144 entries, rows of 5 and
+// Poisson rows of 16, K 200: 37.6 / 26.4 us and 27.3 / 22.9); nor in single elements where there are more tiles than that and most batches
+// lie in one row or two (float32, 65536 rows of 16, K 129: 71 us, 66; but 209715 rows of 5 140, 161; float64 from more tiles on:
+// 262144 rows of 16, K 33 275, 248, and 25000 such rows 24.6, 26.0).
+template <typename V, int VW>
+static bool sddmm_multi(int k_dim, int64_t n_rows, int64_t nnz) {
+  constexpr bool SINGLE = sizeof(V) == 4;
+  if (k_dim <= 32 * VW || (SINGLE && VW == 2)) return false;
+  if (sddmm_ctas(VW, sizeof(V), false) == sddmm_ctas(VW, sizeof(V), true)) return true;
+  int sms = 0;
+  if (sm_count(&sms) != FSB_OK) return true;
+  const int64_t tiles = (nnz + sddmm_tile(32) - 1) / sddmm_tile(32);
+  if (tiles > 3 * sms && tiles <= 4 * sms) return false;
+  return !(VW == 1 && tiles > (SINGLE ? 4 : 14) * sms && nnz >= 12 * n_rows);
 }
 
 template <typename V, int VW>

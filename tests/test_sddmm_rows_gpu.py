@@ -70,13 +70,19 @@ def test_rows_of_several_steps(cuda, fsb_lib, dtype, u, name):
         assert np.all(np.abs(out - xy.sum(1) - dd) <= 1.0001 * bound), k
 
 
-def test_single_elements_in_many_tiles(cuda, fsb_lib):
-    """Either side of the sizes from which float32 rows of an odd number of elements take the instance for one step."""
-    for n_rows, length, k in ((1 << 15, 16, 33), ((1 << 15) - 1, 16, 33), (1 << 16, 11, 35), (1 << 14, 40, 129)):
+@pytest.mark.parametrize("dtype,u", [(torch.float32, 2.0 ** -24), (torch.float64, 2.0 ** -53)], ids=str)
+def test_several_steps_in_the_instance_for_one(cuda, fsb_lib, dtype, u):
+    """Numbers of tiles for which rows of several steps take the instance for one: more than three an SM and up to four; single elements
+    in more tiles than that (float64: from 14 an SM on), with rows of 12 entries and more."""
+    for n_rows, length, k in ((1 << 15, 16, 33), (1 << 16, 11, 35), (1 << 14, 40, 129), (1 << 14, 16, 132), (1 << 14, 16, 260),
+                              (1 << 14, 16, 65), (80000, 14, 35), (1 << 13, 16, 260)):
         gen = torch.Generator(device="cuda").manual_seed(k)
         i = torch.randint(0, 500, (n_rows * length,), generator=gen, device=cuda, dtype=torch.int32)
         p = torch.arange(n_rows + 1, device=cuda) * length
-        x, y = (torch.empty(n, k, device=cuda).uniform_(-1, 1, generator=gen) for n in (n_rows, 500))
+        x, y = (torch.empty(n, k, device=cuda, dtype=dtype).uniform_(-1, 1, generator=gen) for n in (n_rows, 500))
         out = fs.flagsparse_sddmm_csr(x=x, y=y, prepared=fs.prepare_sddmm_csr(i, p, (n_rows, 500)))
-        xy = x.double().repeat_interleave(length, 0) * y.double()[i.long()]
-        assert bool(((out.double() - xy.sum(1)).abs() <= (k + 1) * 2.0 ** -24 * 1.0001 * xy.abs().sum(1)).all())
+        for a in range(0, n_rows, 4096):                        # (in parts: the products of all entries would be large)
+            some = slice(a * length, min(n_rows, a + 4096) * length)
+            xy = x[a:a + 4096].double().repeat_interleave(length, 0) * y.double()[i[some].long()]
+            # (the sum that is compared with has roundings of its own)
+            assert bool(((out[some].double() - xy.sum(1)).abs() <= ((k + 1) * u + k * 2.0 ** -53) * 1.0001 * xy.abs().sum(1)).all())
