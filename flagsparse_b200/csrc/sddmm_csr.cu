@@ -270,9 +270,9 @@ sddmm_kernel(const int32_t* __restrict__ indices, const int32_t* __restrict__ ro
 
 // Which rows of several steps take the instance for them: not those of float32 in accesses of 8 bytes (65536 rows of 16, K 130: 65 us
 // with 80 registers, 59 with 64); not where four CTAs an SM hold all tiles and three do not (float32, 262144 entries, rows of 5 and
-// Poisson rows of 16, K 200: 37.6 / 26.4 us and 27.3 / 22.9); nor in single elements where there are more tiles than that and most batches
+// Poisson rows of 16, K 200: 37.6 / 26.6 us and 27.5 / 22.6); nor in single elements where there are more tiles than that and most batches
 // lie in one row or two (float32, 65536 rows of 16, K 129: 71 us, 66; but 209715 rows of 5 140, 161; float64 from more tiles on:
-// 262144 rows of 16, K 33 275, 248, and 25000 such rows 24.6, 26.0).
+// 262144 rows of 16, K 33 275, 241, and 25000 such rows 26.5, 27.2).
 template <typename V, int VW>
 static bool sddmm_multi(int k_dim, int64_t n_rows, int64_t nnz) {
   constexpr bool SINGLE = sizeof(V) == 4;
