@@ -179,7 +179,7 @@ __host__ __device__ constexpr int mm_ctas(int nc, size_t size, bool with_long) {
 // 300000 rows of 5 37 / 33, 262144 Zipf rows of 16 87 / 81; 64 columns, 2^19 rows of 16 231 / 225, Zipf 130 / 123; float64, 32 columns,
 // Zipf rows of 12 135 / 121).  Rows of one length lose what the sorting takes (2^20 of 16: 521 / 524), eight groups in a warp gain
 // nothing (16 columns: 40.1 / 40.3), one none (float64, 64 columns: 156 / 159), several accesses a lane spill (33 columns, Zipf 91 / 109),
-// and complex64 has no registers left for it (32 columns, Zipf rows: 87381 of 24 67 / 81, 419430 of 5 145 / 185).
+// and complex64 with long rows has no registers left for it (32 columns, Zipf rows: 87381 of 24 67 / 81, 419430 of 5 145 / 185).
 // (As an argument of the launch it costs those that do without: 1390783 rows of 9, 16 columns, 108.1 us, 106.7 us as it is.)
 // n_dense is covered by LR * NC accesses of VW elements per entry; wider products take column tiles (gridDim.y).
 // ACCUM: add to what C holds instead of overwriting it (rows without entries are then left alone) -- the later passes
@@ -254,8 +254,8 @@ spmm_tile_kernel(const S* __restrict__ data, const I* __restrict__ idx, const vo
   // ROWS_FIRST: the four rows before the first of their gathers; single floats, one access, left each gather waiting for its own row
   // where few tiles run (5461 rows of 24, 13 / 21 columns: stride in elements 8.6 / 12.3 us, in bytes 9.5 / 13.9, here 8.3 / 11.7; 174762
   // rows of 24, 21 columns: 81.5, 71.7, 66.7).  Others lose to it (float32, 70 columns 2 %, float64, 33 columns 12 %) or do not care.
-  // Eight half-precision values at a time taken by length: the same (bfloat16, 128 columns, 419430 Zipf rows of 5: 164 / 147).
-  constexpr bool FROM_BYTES = RealOf<S>::parts == 2 || (sizeof(S) == 2 && !(BY_LENGTH && VW == 8)) ||
+  // Eight half-precision values at a time, long rows, by length: the same (bfloat16, 128 columns, 419430 Zipf rows of 5: 164 / 147).
+  constexpr bool FROM_BYTES = RealOf<S>::parts == 2 || (sizeof(S) == 2 && !(BY_LENGTH && LONG && VW == 8)) ||
                               (sizeof(S) == 4 && VW * (int)sizeof(S) < 16);
   constexpr bool ROWS_FIRST = sizeof(S) == 4 && VW == 1 && NC == 1;
   const char* B0 = reinterpret_cast<const char*>(B + col0);
@@ -591,8 +591,8 @@ static int launch_spmm(const SpmmArgs& a, int LR, int piece) {
   A* head = carry + n_tiles * n_dense;
   const int bulk = a.algo != FSB_SPMM_PLAIN && aligned_to(a.data, 16) && aligned_to(a.idx, 16);
   const dim3 grid((unsigned)n_tiles, (unsigned)col_tiles);
-  constexpr bool SORTS = NC == 1 && !(RealOf<S>::parts == 2 && sizeof(S) == 8);
-  const bool by_length = SORTS && a.uneven_rows && !a.accumulate && LR >= 8 && LR < 32;
+  constexpr bool SORTS_LONG = NC == 1 && !(RealOf<S>::parts == 2 && sizeof(S) == 8);
+  const bool by_length = a.uneven_rows && !a.accumulate && (a.long_rows ? SORTS_LONG : NC == 1) && LR >= 8 && LR < 32;
 #define FSB_SPMM_LAUNCH(LONG_, ACC_, LEN_, SMEM_)                                                                    \
   spmm_tile_kernel<S, I, VW, NC, LONG_, ACC_, LEN_><<<grid, kMmThreads, SMEM_, a.st>>>(                              \
       (const S*)a.data, (const I*)a.idx, a.ptr, a.ptype == FSB_I64, (const S*)a.B, a.ldb, (S*)a.C, a.ldc, a.tile_row, \
@@ -605,7 +605,7 @@ static int launch_spmm(const SpmmArgs& a, int LR, int piece) {
       if constexpr (REAL) {
         if (a.accumulate) FSB_SPMM_LAUNCH(true, true, false, parts);
       }
-      if constexpr (SORTS) {
+      if constexpr (SORTS_LONG) {
         if (by_length) FSB_SPMM_LAUNCH(true, false, true, parts);
       }
       if (!a.accumulate && !by_length) FSB_SPMM_LAUNCH(true, false, false, parts);
@@ -616,7 +616,7 @@ static int launch_spmm(const SpmmArgs& a, int LR, int piece) {
     if constexpr (REAL) {
       if (a.accumulate) FSB_SPMM_LAUNCH(false, true, false, 0);
     }
-    if constexpr (SORTS) {
+    if constexpr (NC == 1) {
       if (by_length) FSB_SPMM_LAUNCH(false, false, true, 0);
     }
     if (!a.accumulate && !by_length) FSB_SPMM_LAUNCH(false, false, false, 0);
