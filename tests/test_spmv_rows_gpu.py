@@ -1,6 +1,6 @@
-"""The SpMV kernel that walks neighbouring rows on one SM (from 8192 rows on): every number of lanes, rows that take one turn and
-several, shares of even and uneven weight, ends of the arrays, every value type and index width.  Reference and bound as for
-the tiled kernels: the product of the stored values in complex128."""
+"""The SpMV kernel that walks neighbouring rows on one SM (from 8192 rows on, of short rows as many as its warps take): every number of
+lanes, rows that take one turn and several, shares of even and uneven weight, ends of the arrays, every value type and index
+width.  Reference and bound as for the tiled kernels: the product of the stored values in complex128."""
 
 import numpy as np
 import pytest
@@ -13,23 +13,32 @@ from test_stored_types_gpu import DTYPES, _check, _values
 pytestmark = pytest.mark.gpu
 
 
-def _lengths():
+def _lengths(size):
+    """Row lengths that take the kernel, whatever the values of `size` bytes."""
     rng = np.random.default_rng(5)
-    yield "least", [k % 6 for k in range(8192)]
-    yield "one more", [k % 6 for k in range(8193)]
-    for mean in (1, 5, 13, 27, 60, 130):                       # 2, 2, 4, 8, 16, 32 lanes for four entries at a time
-        yield f"mean {mean}", rng.poisson(mean, 8200 + mean)
-    yield "several turns", np.where(np.arange(9001) % 97 == 5, 90, 4)
-    yield "empty, then rows", np.where(np.arange(30000) < 24000, 0, 9)     # uneven shares: dealt in turn
-    yield "long rows first", np.where(np.arange(20003) < 2500, 70, 8)
-    yield "last entry", [0] * 20000 + [1]
+    most = 125000 if size <= 4 else 63000                      # rows for the warps with two lanes a row
+    yield "least", [24 + k % 6 for k in range(8192)] if size != 16 else [60 + k % 6 for k in range(8192)]
+    yield "one more", [24 + k % 6 for k in range(8193)] if size != 16 else [60 + k % 6 for k in range(8193)]
+    # 2, 2, 4, 8, 16, 32 lanes for four entries at a time, 2, 2, 4, 8, 16, 32 for two (complex128)
+    for mean, n in ((1, most), (5, most), (13, most // 2), (27, 16000), (60, 8260), (130, 8330)):
+        yield f"mean {mean}", rng.poisson(mean, n)
+    yield "several turns", np.where(np.arange(16001) % 97 == 5, 75, 30)
+    yield "empty, then rows", np.where(np.arange(30000) < 6000, 0, 30)     # uneven shares: dealt in turn
+    yield "long rows first", np.where(np.arange(70003) < 9000, 26, 9)
+    yield "last entry", [0] * (most + 20000) + [1]
+
+
+def _csr(lens, n_cols):
+    p = np.zeros(len(lens) + 1, dtype=np.int32)
+    np.cumsum(lens, out=p[1:])
+    return np.random.default_rng(7).integers(0, n_cols, int(p[-1])).astype(np.int32), p
 
 
 @pytest.mark.parametrize("dtype", DTYPES, ids=str)
 def test_against_the_stored_values(cuda, fsb_lib, dtype):
     n_cols = 12000
-    for name, lens in _lengths():
-        _, i, p = handmade_csr(7, [int(v) for v in lens], n_cols)
+    for name, lens in _lengths(torch.empty(0, dtype=dtype).element_size()):
+        i, p = _csr(lens, n_cols)
         vals, x = _values(int(p[-1]), dtype, 4), _values(n_cols, dtype, 5)
         shape = (len(p) - 1, n_cols)
         d, ti, tp, tx = vals.to(cuda), torch.from_numpy(i).to(cuda), torch.from_numpy(p).to(cuda), x.to(cuda)
@@ -38,6 +47,7 @@ def test_against_the_stored_values(cuda, fsb_lib, dtype):
         for wi, wp in ((ti.long(), tp), (ti, tp.long()), (ti.long(), tp.long())):
             assert torch.equal(fs.flagsparse_spmv_csr(d, wi, wp, tx, shape), y), name
         prep = fs.prepare_spmv_csr(d, ti, tp, shape)
+        assert not prep.uneven, name
         assert torch.equal(fs.flagsparse_spmv_csr(x=tx, prepared=prep), y), name
         if vals.numel() > 1:                                    # arrays that start off a 16-byte boundary: lanes per row
             off = torch.cat([d[:1], d])[1:], torch.cat([ti[:1], ti])[1:]

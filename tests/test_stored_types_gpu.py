@@ -125,15 +125,17 @@ def test_spmm_rows_over_many_tiles(cuda, fsb_lib, dtype):
 
 @pytest.mark.parametrize("dtype", DTYPES, ids=str)
 def test_spmm_segments_by_length(cuda, fsb_lib, dtype):
-    """Tiles with more segments than threads, all of one length, none with an entry, and lengths around the last bucket; every
-    result twice, as the order inside a bucket is not fixed."""
+    """Tiles with more segments than threads, all of one length but for one row of the matrix, chunks of segments none of which has an
+    entry, and lengths around the last bucket; every result twice, as the order inside a bucket is not fixed."""
     n_cols = 700
     rng = np.random.default_rng(1)
-    for lens in ([1] * 3000, [0, 2] * 1500 + [300], [int(v) for v in rng.integers(0, 4, 5000)] + [63, 64, 65, 124, 125, 126, 127, 130],
-                 [5] * 700 + [6] * 400):
+    for lens in ([1] * 3000 + [2], [0, 2] * 1500 + [300], [3] * 300 + [0] * 2500 + [3] * 300 + [9], [5] * 700 + [6] * 400 + [8],
+                 [int(v) for v in rng.integers(0, 4, 5000)] + [63, 64, 65, 124, 125, 126, 127, 130]):
         _, i, p = handmade_csr(3, lens, n_cols)
         vals = _values(int(p[-1]), dtype, 4)
         d, ti, tp = vals.to(cuda), torch.from_numpy(i).to(cuda), torch.from_numpy(p).to(cuda)
+        if dtype in (torch.float32, torch.float64):
+            assert fs.prepare_spmm_csr_opt(d, ti, tp, (len(p) - 1, n_cols))._uneven     # all of these are taken by length
         for n_dense in (16, 32, 64, 128):
             B = _values((n_cols, n_dense), dtype, n_dense)
             C = fs.flagsparse_spmm_csr(d, ti, tp, B.to(cuda), (len(p) - 1, n_cols))
