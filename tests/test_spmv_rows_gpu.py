@@ -31,7 +31,9 @@ def _lengths(size):
 def _csr(lens, n_cols):
     p = np.zeros(len(lens) + 1, dtype=np.int32)
     np.cumsum(lens, out=p[1:])
-    return np.random.default_rng(7).integers(0, n_cols, int(p[-1])).astype(np.int32), p
+    row = np.repeat(np.arange(len(lens)), lens)
+    start = np.random.default_rng(7).integers(0, n_cols - 7 * int(max(lens)), len(lens))
+    return (start[row] + 7 * (np.arange(int(p[-1])) - p[row])).astype(np.int32), p       # ascending inside a row
 
 
 @pytest.mark.parametrize("dtype", DTYPES, ids=str)
