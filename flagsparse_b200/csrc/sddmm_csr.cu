@@ -19,10 +19,14 @@ namespace fsb {
 constexpr int kSdThreads = 256;
 constexpr int kSdBatch = 8;   // consecutive entries one group handles
 
-// Resident CTAs the register budget is set for: 64 registers, but 80 for 16-byte accesses of float64, whose eight sums take twice
-// the room (131072 rows of 16, K 200: 476 us, with 64 registers 603 us), and for rows that take several steps: with 64 the gathers of
-// a step wait for one another (float32, 2048 rows of 16, K 160: 15.4 us, 8.9 us; 209715 rows of 5, K 129: 161 us, 140 us).
-__host__ __device__ constexpr int sddmm_ctas(int vw, size_t size, bool multi) { return (size == 8 && vw == 2) || multi ? 3 : 4; }
+// Resident CTAs the register budget is set for: 64 registers, but 80 for 16-byte accesses (float64, 131072 rows of 16, K 200: 476 us,
+// with 64 registers 603 us; float32, 69905 rows of 30, K 60: 46 and 67 us, 87381 rows of 48, K 16 37 and 46 us), except for groups of
+// one lane or two, whose CTAs handle one batch a group (262144 rows of 16, K 8: 47 and 40 us), and for rows that take several steps:
+// with 64 the gathers of a step wait for one another (float32, 2048 rows of 16, K 160: 15.4 us, 8.9 us; 209715 rows of 5, K 129: 161 us, 140 us).
+__host__ __device__ constexpr int sddmm_ctas(int vw, size_t size, int LG, bool multi) {
+  return (vw * (int)size == 16 && !(size == 4 && LG <= 2)) || multi ? 3 : 4;
+}
+
 // entries one CTA handles: J passes of (threads / LG) groups x 8 entries, about 1024 (262144 rows of 6, K 8: 17.3 us, with 2048
 // 20.3 us, a last wave that is a quarter full; 2^19 rows of 16, K 64: 251 us, with 512 265 us)
 __host__ __device__ constexpr int sddmm_passes(int LG) {
@@ -37,7 +41,8 @@ __device__ __forceinline__ const V* row_at(const char* base, int32_t id, uint64_
   return reinterpret_cast<const V*>(base + (uint64_t)(uint32_t)id * stride);
 }
 
-// dot product of what one lane holds of two rows; pairs of floats go through the packed multiply-add
+// dot product of what one lane holds of two rows (one product after the other: pairs of floats in packed multiply-adds end with one more
+// addition of two sums, 2 % more rms error at K 8, 16, 100 and 128)
 template <typename V, int VW>
 __device__ __forceinline__ V lane_dot(const V (&a)[VW], const V (&b)[VW]) {
   V s = a[0] * b[0];
@@ -45,20 +50,6 @@ __device__ __forceinline__ V lane_dot(const V (&a)[VW], const V (&b)[VW]) {
   for (int i = 1; i < VW; ++i) s = fma(a[i], b[i], s);
   return s;
 }
-__device__ __forceinline__ uint64_t pack2(float x, float y) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
-  return r;
-}
-__device__ __forceinline__ float lane_dot(const float (&a)[4], const float (&b)[4]) {
-  uint64_t t;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(t) : "l"(pack2(a[0], a[1])), "l"(pack2(b[0], b[1])));
-  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(t) : "l"(pack2(a[2], a[3])), "l"(pack2(b[2], b[3])));
-  float x, y;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(t));
-  return x + y;
-}
-
 // The form of a batch of eight entries: bit e is set where entry e lies in the row of the first one; kSdOne: all of them do;
 // kSdTwo: the others lie in the row of the last one.
 //
@@ -73,10 +64,10 @@ __device__ __forceinline__ float lane_dot(const float (&a)[4], const float (&b)[
 // What bounded the kernel before its present shape was its own arithmetic: 340 warp instructions for 16 entries (2^19 rows of
 // 16, K 64, float32), of which the gathers, the products and their sums need about a third; 4.8 of the 10.2 cycles that a
 // warp took per instruction were spent waiting for memory.  So the forms are worked out once per batch while the ids are staged
-// (not by every lane of the group), rows are found by one wide multiply-add from a stride in bytes, pairs of floats are
-// multiplied by one instruction, and the results leave through shared memory with alpha, beta and `data` at the end.
-// That case 290 us before, 251 us now (gathers at 8.6 TB/s, DRAM traffic 1.2 GB); 131072 rows of 32: 117 us, 95 us; K 33:
-// 268 us, 173 us; float64, 2^18 rows of 16, K 32: 228 us, 146 us.  A group that walks whole rows instead, as the SpMM kernel
+// (not by every lane of the group), rows are found by one wide multiply-add from a stride in bytes, and the results leave
+// through shared memory with alpha, beta and `data` at the end.
+// That case 254 us before, 234 us now, Poisson rows 290 and 249; 131072 rows of 32: 108 us, 95 us; K 33: 554 us, 362 us; float64,
+// 2^18 rows of 16, K 32: 131 us, 120 us.  A group that walks whole rows instead, as the SpMM kernel
 // does, with the next row's slice of X on its way: 309 us (groups of a warp wait for the longest row among theirs).
 constexpr uint32_t kSdOne = 1u << 8, kSdTwo = 1u << 9;
 template <typename V>
@@ -88,7 +79,7 @@ __host__ __device__ constexpr bool sddmm_vote(int VW, int LG) { return VW * (int
 // us, as for one step / here: float32, 65536 rows of 16, K 160 98 / 72; 2048 rows of 16, K 200 15.5 / 9.0; float64, 65536 rows of
 // 16, K 72 97 / 74, Poisson rows 90 / 74.
 template <typename V, int VW, int LG, bool MULTI>
-__global__ void __launch_bounds__(kSdThreads, sddmm_ctas(VW, sizeof(V), MULTI))
+__global__ void __launch_bounds__(kSdThreads, sddmm_ctas(VW, sizeof(V), LG, MULTI))
 sddmm_kernel(const int32_t* __restrict__ indices, const int32_t* __restrict__ row_ids, const V* __restrict__ X,
              int64_t ldx, const V* __restrict__ Y, int64_t ldy, const V* data, V* out,
              int64_t nnz, int k_dim, V alpha, V beta, int ids_aligned) {
@@ -186,8 +177,16 @@ sddmm_kernel(const int32_t* __restrict__ indices, const int32_t* __restrict__ ro
         ld_dense<V, VW>(reinterpret_cast<const V*>(xp), xa);
 #pragma unroll
         for (int e = 0; e < E; ++e) ld_dense<V, VW>(row_at<V>(yp, cols[e], ys), yv[e]);
+        // (four floats onto the sum itself: 2^19 rows of 16, K 64 234 us, as a product of its own 235; 32768 rows of 16, K 64 1 % less)
 #pragma unroll
-        for (int e = 0; e < E; ++e) acc[e] += lane_dot(xa, yv[e]);
+        for (int e = 0; e < E; ++e) {
+          if constexpr (sizeof(V) == 4 && VW == 4) {
+#pragma unroll
+            for (int i = 0; i < VW; ++i) acc[e] = fma(xa[i], yv[e][i], acc[e]);
+          } else {
+            acc[e] += lane_dot(xa, yv[e]);
+          }
+        }
       }
     } else if (TWO && two) {
       const char *xp = reinterpret_cast<const char*>(row_at<V>(Xk, rows[0], xs)), *yp = Yk;
@@ -269,15 +268,15 @@ sddmm_kernel(const int32_t* __restrict__ indices, const int32_t* __restrict__ ro
 }
 
 // Which rows of several steps take the instance for them: not those of float32 in accesses of 8 bytes (65536 rows of 16, K 130: 65 us
-// with 80 registers, 59 with 64); not where four CTAs an SM hold all tiles and three do not (float32, 262144 entries, rows of 5 and
-// Poisson rows of 16, K 200: 37.6 / 26.6 us and 27.5 / 22.6); nor in single elements where there are more tiles than that and most batches
+// with 80 registers, 59 with 64); of single elements not where four CTAs an SM hold all tiles and three do not (float32, 16384 rows of
+// 16, K 65: 15 % less with 64), nor where there are more tiles than that and most batches
 // lie in one row or two (float32, 65536 rows of 16, K 129: 71 us, 66; but 209715 rows of 5 140, 161; float64 from more tiles on:
 // 262144 rows of 16, K 33 275, 241, and 25000 such rows 26.5, 27.2).
 template <typename V, int VW>
 static bool sddmm_multi(int k_dim, int64_t n_rows, int64_t nnz) {
   constexpr bool SINGLE = sizeof(V) == 4;
   if (k_dim <= 32 * VW || (SINGLE && VW == 2)) return false;
-  if (sddmm_ctas(VW, sizeof(V), false) == sddmm_ctas(VW, sizeof(V), true)) return true;
+  if (sddmm_ctas(VW, sizeof(V), 32, false) == sddmm_ctas(VW, sizeof(V), 32, true)) return true;
   int sms = 0;
   if (sm_count(&sms) != FSB_OK) return true;
   const int64_t tiles = (nnz + sddmm_tile(32) - 1) / sddmm_tile(32);

@@ -60,3 +60,32 @@ def test_no_less_accurate_than_two_sums_over_a_row(cuda, fsb_lib, dtype, length)
         assert rc == 0
         a, b = _rms(new, exact), _rms(old.to(dtype), exact)
         assert a <= 1.03 * b, (n_dense, a, b)
+
+
+@pytest.mark.parametrize("k", [8, 16, 64, 100, 128])
+def test_sddmm_no_less_accurate_than_products_one_by_one(cuda, fsb_lib, k):
+    """float32, four elements a lane: the rms error against that of the same sum with the four products added one after the other by fused
+    multiply-adds and the lanes added in a tree.  The bound leaves half a percent for the last place in which the model's
+    double rounding may differ."""
+    n_rows, length, n_cols = 4000, 12, 500
+    rng = np.random.default_rng(k)
+    i = rng.integers(0, n_cols, n_rows * length).astype(np.int32)
+    x, y = rng.uniform(-1, 1, (n_rows, k)).astype(np.float32), rng.uniform(-1, 1, (n_cols, k)).astype(np.float32)
+    p = torch.arange(n_rows + 1, device=cuda) * length
+    prep = fs.prepare_sddmm_csr(torch.from_numpy(i).to(cuda), p, (n_rows, n_cols))
+    out = fs.flagsparse_sddmm_csr(x=torch.from_numpy(x).to(cuda), y=torch.from_numpy(y).to(cuda), prepared=prep).cpu().numpy()
+    prod = np.repeat(x.astype(np.float64), length, 0) * y.astype(np.float64)[i]          # exact
+    lanes = 1
+    while 4 * lanes < k:
+        lanes *= 2
+    part = np.zeros((len(i), lanes, 4))
+    part.reshape(len(i), -1)[:, :k] = prod
+    s = np.zeros((len(i), lanes), dtype=np.float32)
+    for j in range(4):
+        s = (s + part[:, :, j]).astype(np.float32)
+    while lanes > 1:
+        lanes //= 2
+        s = s[:, :lanes] + s[:, lanes:]
+    exact = prod.astype(np.longdouble).sum(1)
+    rms = lambda v: float(np.sqrt(np.mean((v - exact) ** 2)))  # noqa: E731
+    assert rms(out.astype(np.longdouble)) <= 1.005 * rms(s[:, 0].astype(np.longdouble))
