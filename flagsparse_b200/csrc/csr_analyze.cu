@@ -48,8 +48,8 @@ __device__ __forceinline__ long long warp_min(long long v) {
 // 250007 rows, 64-bit: two launches, 33 us; 10 us in this one; 2.1 M entries, 150001 rows: 30 us and 7 us).
 // Thread k < 6 of a block returns what the block found: longest row, decreasing and empty rows, long rows, smallest and largest index.
 template <typename I, typename P>
-__device__ __forceinline__ long long csr_stats_block(const P* __restrict__ ptr, int64_t n_rows, int64_t long_len, const I* __restrict__ idx, int64_t nnz,
-                 int wide_loads) {
+__device__ __forceinline__ long long csr_stats_block(const P* __restrict__ ptr, int64_t n_rows, int64_t long_len,
+                                                     const I* __restrict__ idx, int64_t nnz, int wide_loads) {
   constexpr int E = 16 / (int)sizeof(I);
   constexpr int U = 4;                       // requests in flight
   __shared__ long long s_part[8][6];

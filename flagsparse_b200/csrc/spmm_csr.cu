@@ -152,13 +152,14 @@ struct Pack {
 
 // Resident CTAs the register budget is set for.  One access per lane: 40 registers hold four gathers of 4-byte values; left
 // to itself the compiler fits 32 at times and issues them one after the other (54 columns, 28386 rows of 45 entries, float32:
-// 39 us, 37 us).  Four gathers and the sums of 8-byte values take 48, and so do four gathers of eight half-precision values with
-// their eight sums (float16, 2^20 rows of 10, 128 columns: 558 us with 40, 454 us; bfloat16, 200003 Zipf rows of 20, 128 columns:
-// 157 us, 148 us; both with rows found by their stride in bytes); 8-byte values (float64, 60000 rows of 31, 40 / 64 / 128 columns with 40
-// registers: 70.6 / 77.8 / 145 us, with 48: 59.6 / 67.7 / 130 us; with 64: 66 / 74 / 146 us).  Several accesses: 64 (60000
-// rows of 31, 65 columns with 80 registers: float32 80.0 us, float64 114 us; with 64: 78.0 us, 98.8 us), four of them 80, which
-// 64 would spill.  With long rows the pieces' arithmetic comes on top (float64, 33 columns, one row of 300 among 60000 of 31:
-// 102 us with 128 registers, 82 us with 80, 88 us with 64).
+// 39 us, 37 us).  Four gathers and the sums of 8-byte values take 48 (float64, 60000 rows of 31, 40 / 64 / 128 columns with 40
+// registers: 70.6 / 77.8 / 145 us, with 48: 59.6 / 67.7 / 130 us, with 64: 66 / 74 / 146 us), and so do four gathers of eight
+// half-precision values with their eight sums (float16, 2^20 rows of 10, 128 columns: 558 us with 40, 454 us; bfloat16, 200003 Zipf
+// rows of 20, 128 columns: 157 us, 148 us; both with rows found by their stride in bytes).  Several accesses: 64 (60000 rows of 31, 65
+// columns with 80 registers: float32 80.0 us, float64 114 us; with 64: 78.0 us, 98.8 us), four of them 80, which leaves 12 bytes to
+// spill where rows are found by their stride in bytes (198 columns: rows of one length 4 % slower than without, others 2 to 10 %
+// faster).  With long rows the pieces' arithmetic comes on top (float64, 33 columns, one row of 300 among 60000 of 31: 102 us with
+// 128 registers, 82 us with 80, 88 us with 64).
 __host__ __device__ constexpr int mm_ctas(int nc, size_t size, bool with_long) {
   if (nc == 1) return size == 16 ? 4 : size == 8 || size == 2 ? 5 : 6;
   if (with_long) return nc == 4 || (nc == 3 && size == 4) ? 2 : 3;

@@ -10,7 +10,8 @@
  * Conventions
  *   - Every pointer is a DEVICE pointer unless the comment says "host".
  *   - vtype: value dtype of data / x / B / y / C.  itype: dtype of `indices`.  ptype: dtype of `indptr`.
- *   - All work is enqueued on `stream` (a cudaStream_t passed as void*); no call synchronises the host
+ *   - All work is enqueued on `stream` (a cudaStream_t passed as void*); no call waits for the GPU but
+ *     fsb_csr_check and the fsb_*_csr_once entry points, which need an answer of it,
  *     and no call allocates or frees device memory -- the caller owns every buffer, scratch included (the one
  *     exception is fsb_spmv_csr_noalloc, whose scratch is an array built into the library).
  *   - Return value: 0 on success, a negative FSB_E* code for an argument error detected on the host, or
