@@ -488,12 +488,7 @@ spmm_fixup_kernel(const P* __restrict__ ptr, const int32_t* __restrict__ tile_ro
   const R first = head[t * n_dense + j];
   const int n = (int)(t - (p >> log2_tile));          // partial sums in the tiles before
   const R* from = carry + (t - n) * n_dense + j;
-  auto batch = [&](int u, R (&v)[8]) {
-#pragma unroll
-    for (int k = 0; k < 8; ++k) v[k] = __ldg(from + (int64_t)(u + k) * n_dense);
-  };
   double sum = (double)first, comp = 0.0;
-  bool exact = false;
   if constexpr (sizeof(R) == 4) {
     // the largest magnitude, and the smallest that is not zero, less one
     uint32_t most = __float_as_uint(first) & 0x7FFFFFFFu, least = most - 1u;
@@ -505,23 +500,28 @@ spmm_fixup_kernel(const P* __restrict__ ptr, const int32_t* __restrict__ tile_ro
     };
     int u = 0;
     for (; u + 8 <= n; u += 8) {
-      R v[8];
-      batch(u, v);
+      float v[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] = __ldg(from + (int64_t)(u + k) * n_dense);
 #pragma unroll
       for (int k = 0; k < 8; ++k) add(v[k]);
     }
     for (; u < n; ++u) add(__ldg(from + (int64_t)u * n_dense));
     // n + 1 numbers of 24 bits, exponents `range` apart: every sum of them has at most this many bits
     const int low = (int)((least + 1u) >> 23), range = (int)(most >> 23) - (low > 0 ? low : 1);
-    exact = 24 + range + (32 - __clz(n)) <= 53;
-  }
-  if (!exact) {
+    if (24 + range + (32 - __clz(n)) > 53) {
+      sum = (double)first;
+#pragma unroll 1
+      for (int u = 0; u < n; ++u) comp_add(sum, comp, (double)__ldg(from + (int64_t)u * n_dense));
+    }
+  } else {
     // (eight and more: four sums in turn, or each would wait for the one before it)
     double sums[4] = {(double)first, 0.0, 0.0, 0.0}, comps[4] = {0.0, 0.0, 0.0, 0.0};
     int u = 0;
     for (; u + 8 <= n; u += 8) {
       R v[8];
-      batch(u, v);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] = __ldg(from + (int64_t)(u + k) * n_dense);
 #pragma unroll
       for (int k = 0; k < 8; ++k) comp_add(sums[k & 3], comps[k & 3], (double)v[k]);
     }
