@@ -363,7 +363,7 @@ class ShardedCsrSpmv(_ShardedBase):
                     _VTYPE[p.data.dtype], _ITYPE[p.kernel_indices.dtype], _ITYPE[p.kernel_indptr.dtype],
                     _ptr(p.data), _ptr(p.kernel_indices), p.kernel_indptr.data_ptr(), _ptr(x),
                     self._peer_ptrs.data_ptr(), self.world, self.rank, base + self.row_start, p.n_rows, p.n_cols,
-                    p.data.numel(), algo, p.tuning if algo == _lib.FSB_SPMV_STREAM else p.vector_tuning(),
+                    p.data.numel(), algo, p.tuning if algo == _lib.FSB_SPMV_STREAM else p.vector_tuning,
                     None if p.tile_row is None else p.tile_row.data_ptr(),
                     None if p.scratch is None else p.scratch.data_ptr(),
                     0 if p.scratch is None else p.scratch.numel(), _stream_ptr(self.device),

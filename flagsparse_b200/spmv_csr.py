@@ -147,7 +147,7 @@ class PreparedCsrSpmv:
     __slots__ = (
         "data", "kernel_indices", "kernel_indptr", "shape", "n_rows", "n_cols", "block_nnz",
         "max_segments", "max_row_nnz", "opt_buckets", "supports_opt", "stats", "algo", "tuning",
-        "tile_nnz", "tile_row", "scratch", "panel", "long_rows", "wide", "bins", "uneven",
+        "tile_nnz", "tile_row", "scratch", "panel", "long_rows", "wide", "bins", "uneven", "vector_tuning",
     )
 
     def __init__(self, data, kernel_indices, kernel_indptr, shape, n_rows, n_cols, block_nnz,
@@ -164,6 +164,8 @@ class PreparedCsrSpmv:
         self.max_row_nnz = max_row_nnz
         # whether a row is too long for neighbouring rows to stay on one SM
         self.uneven = max_row_nnz > _longest_neighbour(n_rows, data.numel(), data.element_size())
+        # what fsb_spmv_csr is told of the rows where FSB_SPMV_VECTOR picks its lanes itself
+        self.vector_tuning = 0 if self.uneven else _lib.FSB_SPMV_EVEN_ROWS
         self.supports_opt = data.dtype in (torch.float32, torch.float64)
         self.stats = stats
         self.algo = algo
@@ -190,10 +192,6 @@ class PreparedCsrSpmv:
         if self.long_rows is not None:
             yield self.long_rows[1].status
             yield from self.long_rows[0]._status_words()
-
-    def vector_tuning(self):
-        """What fsb_spmv_csr is told of the rows when FSB_SPMV_VECTOR picks its lanes itself."""
-        return 0 if self.uneven else _lib.FSB_SPMV_EVEN_ROWS
 
     def check_status(self):
         """Wait for the last product on this matrix and raise RuntimeError if one of its kernels gave up on a
@@ -407,7 +405,7 @@ def _spmv_launch(prepared, x, y):
     if scratch is not None and (p.data.numel() < _STREAM_MIN_NNZ or p.bins is not None):
         scratch = torch.empty_like(scratch)
     lanes = p.tuning & 0xFF
-    tuning = p.tuning if algo == _lib.FSB_SPMV_STREAM else (lanes if lanes in (2, 4, 8, 16, 32) else p.vector_tuning())
+    tuning = p.tuning if algo == _lib.FSB_SPMV_STREAM else (lanes if lanes in (2, 4, 8, 16, 32) else p.vector_tuning)
     with _on_device(dev):
         rc = L.fsb_spmv_csr(
             _VTYPE[p.data.dtype], _ITYPE[p.kernel_indices.dtype], _ITYPE[p.kernel_indptr.dtype],
